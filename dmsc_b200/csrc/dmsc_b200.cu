@@ -1122,8 +1122,10 @@ int extract_batch_impl(dmsc_b200_context* ctx, int B, const float* img, const in
     int per = 0;
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, label_exit_kernel<true>, 256, 0));
     const unsigned eg = (unsigned)std::max(1, per) * ctx->num_sms;
-    if (F.groups) LK(label_exit_kernel<true><<<eg, 256, 0, st>>>(I, exf, nex + 0, LF.perim, OF, (int)nltile + 2, ctx->status));
-    if (V.groups) LK(label_exit_kernel<false><<<eg, 256, 0, st>>>(I, exv, nex + 1, LV.perim, OV, (int)nltile + 2, ctx->status));
+    // a path enters a tile through each of its border cells at most once
+    const int hops = (int)std::min<long long>(nltile * kPerim + 2, 2147483647LL);
+    if (F.groups) LK(label_exit_kernel<true><<<eg, 256, 0, st>>>(I, exf, nex + 0, LF.perim, OF, hops, ctx->status));
+    if (V.groups) LK(label_exit_kernel<false><<<eg, 256, 0, st>>>(I, exv, nex + 1, LV.perim, OV, hops, ctx->status));
     LAUNCH_CHECK("label_exit_kernel");
   }
   mark(ctx, 10, st);
