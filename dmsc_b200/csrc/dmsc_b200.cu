@@ -48,7 +48,7 @@ enum SideSlot {
   X_ROUT, X_SVT, X_SVL, X_SVR, X_DYING, X_GRP, X_LINK, X_MINE, X_ACT0, X_ACT1, X_CNT, X_PAIR, X_ALIVE,
   X_ALIVEI, X_TOOUTX, X_TOOUT, X_UF, X_CROOT, X_CKEY, X_CVAL, X_NODE,
   X_ALEN, X_ACL, X_AROOT, X_PLEN, X_SEND, X_APOS, X_EROWC, X_EROWO, X_Q0, X_Q1, X_QB, X_G12,
-  X_GBASE, X_WX, X_WA, X_CENDS, kSideSlots
+  X_GBASE, X_WX, X_WA, X_CENDS, X_SOLO, kSideSlots
 };
 
 struct Buf {
@@ -182,6 +182,7 @@ struct dmsc_b200_context {
   int emit_shape = 0;    // expansion chain tasks per thread batch: 0 -> 1, 1 -> 2
   int seg_cursors = 1;  // raw-arc cursors per lane of the segment writer
   bool label_smem_set = false;  // dynamic shared memory limit raised for the label kernels
+  bool pair_smem_set = false;   // and for the pairing's tile kernel
   int cap_pair_rounds = 0, cap_replay_rounds = 0, cap_emit_levels = 0;
 };
 
@@ -329,10 +330,10 @@ void mark(dmsc_b200_context* ctx, int k, cudaStream_t st) {
 }
 
 // Cooperative launch of a persistent kernel: as many blocks as can be
-// co-resident, so grid-wide barriers are safe.
+// co-resident (at most `most`, when given), so grid-wide barriers are safe.
 template <class T>
 void coop_launch(dmsc_b200_context* ctx, void (*kernel)(T), T args, cudaStream_t st, const char* name,
-                 int per_cap = 0) {
+                 int per_cap = 0, int most = 0) {
   int per = 0;
   CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, 256, 0));
   if (per < 1) {
@@ -341,7 +342,8 @@ void coop_launch(dmsc_b200_context* ctx, void (*kernel)(T), T args, cudaStream_t
   }
   if (per_cap > 0 && per_cap < per) per = per_cap;
   void* a[] = {&args};
-  CK(cudaLaunchCooperativeKernel((void*)kernel, dim3(per * ctx->num_sms), dim3(256), a, 0, st));
+  const int grid = most > 0 ? std::min(per * ctx->num_sms, most) : per * ctx->num_sms;
+  CK(cudaLaunchCooperativeKernel((void*)kernel, dim3(grid), dim3(256), a, 0, st));
   ++ctx->launches;
 }
 
@@ -493,17 +495,42 @@ PairArgs pairing_args(dmsc_b200_context* ctx, int si, Side& S) {
   A.status = ctx->status;
   A.max_rounds = capped(M + 2, ctx->cap_pair_rounds);
   A.rounds = get<int>(ctx, S_STATS, 8) + 0 + si;
+  A.handover = get<int>(ctx, S_STATS, 8) + 6;
+  A.node = sget<int>(ctx, si, X_CROOT, M + 1);  // free until the thresholded union-find
+  A.solo_key = sget<unsigned long long>(ctx, si, X_SOLO, kPairSoloEdges + kPairSoloEdges / 2 + kPairSoloNodes);
+  A.solo_ext = (int2*)(A.solo_key + kPairSoloEdges);
+  A.solo_ends = (uint32_t*)(A.solo_ext + kPairSoloNodes);
   A.timeline = get<unsigned long long>(ctx, S_TIMELINE, kTimelineSlots) + si * kTimeline;
   return A;
 }
 
-// Both sides' pairing rounds in one cooperative launch.
-void run_pairing(dmsc_b200_context* ctx, cudaStream_t st) {
+// Both sides' pairing: the tile pass over `nltile` tiles, then the global
+// rounds on what it leaves undecided: in one cooperative launch while they
+// are many, in one block per side at the end.
+void run_pairing(dmsc_b200_context* ctx, PairTileArgs T, int nltile, cudaStream_t st) {
   PairArgs2 P;
-  for (int si = 0; si < 2; ++si) P.s[si] = pairing_args(ctx, si, ctx->side[si]);
-  if (ctx->nsad > 0)
-    coop_launch(ctx, ctx->pair_shape ? pairing_persistent_kernel<4, 4> : pairing_persistent_kernel<2, 5>, P, st,
-                "pairing_persistent_kernel", ctx->pair_per_sm);
+  for (int si = 0; si < 2; ++si) {
+    P.s[si] = pairing_args(ctx, si, ctx->side[si]);
+    T.act[si] = P.s[si].act0;
+    T.roots[si] = P.s[si].roots0;
+    T.key[si] = P.s[si].key;
+  }
+  if (ctx->nsad <= 0) return;
+  constexpr int kSm = (int)sizeof(PairTileSmem), kSolo = (int)sizeof(PairSoloSmem);
+  if (!ctx->pair_smem_set) {  // more than the 48 KB of static shared memory
+    CK(cudaFuncSetAttribute(pair_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSm));
+    CK(cudaFuncSetAttribute(pair_solo_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSolo));
+    ctx->pair_smem_set = true;
+  }
+  LK(pair_tile_kernel<<<2u * (unsigned)nltile, kTilePairNT, kSm, st>>>(ctx->I, T));
+  LAUNCH_CHECK("pair_tile_kernel");
+  // one block per 1024 saddles, up to all that are resident: a grid barrier
+  // costs 3 us more on 740 blocks than on 148, and the tile pass leaves about
+  // 200 saddles of 1024
+  coop_launch(ctx, ctx->pair_shape ? pairing_persistent_kernel<4, 4> : pairing_persistent_kernel<2, 4>, P, st,
+              "pairing_persistent_kernel", ctx->pair_per_sm, (ctx->nsad + 1023) / 1024);
+  LK(pair_solo_kernel<<<2, kSoloNT, kSolo, st>>>(P));
+  LAUNCH_CHECK("pair_solo_kernel");
 }
 
 // Persistence, cancellation, thresholded union-find and output ranks of one side.
@@ -895,12 +922,12 @@ int extract_batch_impl(dmsc_b200_context* ctx, int B, const float* img, const in
   // the pairing's starting state (side 0: faces / maxima, side 1: vertices /
   // minima), set up by the compaction and the saddle walks
   PairStart ps;
-  ps.nsad = nsad;
   ps.sval = sval;
   for (int si = 0; si < 2; ++si) {
     const int M = si ? nmin : nmax;
     ps.M[si] = M;
     ps.minedge[si] = sget<unsigned long long>(ctx, si, X_MINE, M + 1);
+    ps.leave[si] = sget<unsigned>(ctx, si, X_CROOT, M + 1);  // free until the thresholded union-find
     ps.link[si] = sget<int>(ctx, si, X_LINK, M + 1);
     ps.cnt[si] = sget<int>(ctx, si, X_CNT, 8);
     ps.g12[si] = sget<int2>(ctx, si, X_G12, nsad);
@@ -968,7 +995,17 @@ int extract_batch_impl(dmsc_b200_context* ctx, int B, const float* img, const in
   uint8_t* canc = get<uint8_t>(ctx, S_CANC, nsad + 4);
   mark(ctx, 4, st);
   CK(cudaMemsetAsync(canc, 0, nsad + 4, st));
-  run_pairing(ctx, st);
+  {
+    PairTileArgs T{};
+    T.ps = ps;
+    T.off[0] = off[2];
+    T.off[1] = off[0];
+    T.bits[0] = bmax;
+    T.bits[1] = bmin;
+    T.off_sad = off[1];
+    T.seg_sad = seg[1];
+    run_pairing(ctx, T, (int)nltile, st);
+  }
   mark(ctx, 5, st);
   // the two sides' persistence, thresholded union-find and ranks are
   // independent (disjoint buffers; their cancellation bits are ORed into the
@@ -1767,7 +1804,7 @@ int dmsc_b200_tuning_limits(dmsc_b200_context* ctx, int* out, int n) {
   int v[9] = {kGradShapes, kLabelShapes, 0, 0, 0, kSegCursorShapes, kPairShapes, kReplayShapes, kEmitShapes};
   if (cudaSetDevice(ctx->device) != cudaSuccess ||
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-          &v[2], ctx->pair_shape ? pairing_persistent_kernel<4, 4> : pairing_persistent_kernel<2, 5>, 256, 0) !=
+          &v[2], ctx->pair_shape ? pairing_persistent_kernel<4, 4> : pairing_persistent_kernel<2, 4>, 256, 0) !=
           cudaSuccess ||
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(
           &v[3], ctx->replay_shape ? replay_persistent_kernel<2, 3> : replay_persistent_kernel<1, 4>, 256, 0) !=

@@ -753,15 +753,9 @@ static __global__ void __launch_bounds__(256) compact_kernel(
   if (seg0 == 0 && lane == 0) {  // the pairing's void groups and round counters
 #pragma unroll
     for (int sd = 0; sd < 2; ++sd) {
-      ps.minedge[sd][ps.M[sd]] = ~0ull;
       ps.link[sd][ps.M[sd]] = ps.M[sd];
-      int* c = ps.cnt[sd];
-      c[0] = ps.nsad;  // round 0 takes every saddle
-      c[1] = 0;        // the saddles still active after it (counted by the walks)
-      c[2] = 0;
-      c[3] = ps.M[sd] + 1;
-      c[4] = 0;
-      c[5] = 0;
+#pragma unroll
+      for (int k = 0; k < 6; ++k) ps.cnt[sd][k] = 0;
     }
   }
   const unsigned lt = (1u << lane) - 1u;
@@ -814,6 +808,7 @@ static __global__ void __launch_bounds__(256) compact_kernel(
       min_img[q] = bk;
       min_key[q] = make_int2(__float_as_int(cv.v), (int)(4 * gidx));
       ps.minedge[1][q] = ~0ull;  // a single-extremum group without outgoing saddles yet
+      ps.leave[1][q] = ~0u;
       ps.link[1][q] = q;
     }
     if (m & 8u) {
@@ -821,6 +816,7 @@ static __global__ void __launch_bounds__(256) compact_kernel(
       max_img[q] = bk;
       max_key[q] = make_int2(__float_as_int(cv.f), (int)(4 * gidx + 3));
       ps.minedge[0][q] = ~0ull;
+      ps.leave[0][q] = ~0u;
       ps.link[0][q] = q;
     }
 #pragma unroll

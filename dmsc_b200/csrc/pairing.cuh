@@ -26,6 +26,7 @@
 #include <cuda/atomic>
 
 #include "common.cuh"
+#include "gradient.cuh"
 #include "replay.cuh"
 
 namespace dmsc {
@@ -47,7 +48,6 @@ __device__ __forceinline__ int sweep_key_saddle(unsigned long long k, bool desc)
   const int lo = (int)(uint32_t)k;
   return desc ? 0x7FFFFFFF - lo : lo;
 }
-constexpr int kUndecided = -2;
 
 // older(a, b) for extremum dense indices of one image; `void_id` is older
 // than all. Older = smaller (value, cell) under value_less on the vertex side
@@ -61,13 +61,22 @@ __device__ __forceinline__ bool older(int a, int b, int void_id, const int2* __r
   return older_less ? tie_lt(va, ka.y, vb, kb.y) : tie_lt(vb, kb.y, va, ka.y);
 }
 
+// Ends of a saddle as the walks record them for the tile pass below. A local
+// saddle has its two ends inside its own 64 x 64 index tile or in the void:
+// each end is ~(r * 64 + c) of the extremum's cell in the tile (negative), or
+// ~kLocalVoid. Any other saddle holds the ends' groups (>= 0, the void M), a
+// cycle kCycleEnd twice.
+constexpr int kLocalVoid = 0x7FFF;
+constexpr int kCycleEnd = (int)0x80000000;
+
 // K4: per saddle, both face walks and the vertex walks. Writes per saddle and
 // side one record {target 0, target 1, cells 0, cells 1}: each arc's dense
-// target index (or -1) and its raw arc's cell count; then runs the pairing's round-0 saddle phase for both sides (all
-// groups are still single extrema, so the ends are the groups): a saddle
-// whose two ends coincide is a cycle, the others record their ends' groups
-// and reduce their sweep key into both groups' minimum, and each block adds
-// the saddles that stay active to the side's round-1 counter.
+// target index (or -1) and its raw arc's cell count; and the pairing's
+// starting state: a saddle whose two ends coincide is a cycle, the others
+// record their ends and reduce their sweep key into both ends' minima
+// (nothing waits for these reductions: 0.03 ms of the 0.33 ms at 4096^2), and
+// a saddle that is not local to its tile reduces the value part of its key
+// into its ends' `leave` too.
 __global__ void __launch_bounds__(256) saddle_walk_kernel(Imgs I, const uint8_t* __restrict__ flow, int nsad,
                                                           const int* __restrict__ crit_sad,
                                                           const int* __restrict__ sad_img,
@@ -78,59 +87,468 @@ __global__ void __launch_bounds__(256) saddle_walk_kernel(Imgs I, const uint8_t*
                                                           int4* __restrict__ arc_f, int4* __restrict__ arc_v,
                                                           long long cap, PairStart ps, unsigned* status) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  int keep[2] = {0, 0};
-  if (s < nsad) {
-    const int b = sad_img[s];
-    const int H = I.H[b], W = I.W[b], Nx = W + 1;
-    const int sc = crit_sad[s];
-    int te[2][2], len[2][2];
+  if (s >= nsad) return;
+  const int b = sad_img[s];
+  const int H = I.H[b], W = I.W[b], Nx = W + 1;
+  const int sc = crit_sad[s];
+  const int sl = (sc >> 2) - I.idx_base[b], sy = sl / Nx, sx = sl - sy * Nx;
+  int te[2][2], len[2][2], loc[2][2];  // loc: the end's cell in the saddle's tile, -1 when it lies in another
 #pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      long long steps;
-      const int end = flow_walk<4>(flow, face_start(sc, j, Nx) >> 2, Nx, cap, &steps, status);
-      const int target = seg_rank(I, b, end, Nx, off_max, max_bits);
-      te[0][j] = target;
-      len[0][j] = target >= 0 ? (int)steps + 1 : 0;  // cells of the raw arc, start and end included
+  for (int j = 0; j < 2; ++j) {
+    long long steps;
+    const int end = flow_walk<4>(flow, face_start(sc, j, Nx) >> 2, Nx, cap, &steps, status);
+    int y, x;
+    const int target = seg_rank(I, b, end, Nx, off_max, max_bits, y, x);
+    te[0][j] = target;
+    len[0][j] = target >= 0 ? (int)steps + 1 : 0;  // cells of the raw arc, start and end included
+    loc[0][j] = ((y ^ sy) | (x ^ sx)) >> 6 ? -1 : (y & 63) << 6 | (x & 63);
+  }
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    const int start = vertex_start(sc, j, H, W, Nx, I.idx_base[b]);
+    long long steps = 0;
+    int target = -1, at = kLocalVoid;
+    if (start >= 0) {
+      const int end = flow_walk<0>(flow, start >> 2, Nx, cap, &steps, status);
+      int y, x;
+      target = seg_rank(I, b, end, Nx, off_min, min_bits, y, x);
+      at = ((y ^ sy) | (x ^ sx)) >> 6 ? -1 : (y & 63) << 6 | (x & 63);
     }
+    te[1][j] = target;
+    len[1][j] = target >= 0 ? (int)steps + 1 : 0;  // an arc that leaves the image is empty
+    loc[1][j] = at;
+  }
+  // a raw arc has fewer cells than the batch (cell ids are int32)
+  arc_f[s] = make_int4(te[0][0], te[0][1], len[0][0], len[0][1]);
+  arc_v[s] = make_int4(te[1][0], te[1][1], len[1][0], len[1][1]);
+  // descending sweep on the face side in the primal and the vertex side in
+  // the dual
+  const bool d = I.dual[b];
 #pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      const int start = vertex_start(sc, j, H, W, Nx, I.idx_base[b]);
-      long long steps = 0;
-      int target = -1;
-      if (start >= 0) {
-        const int end = flow_walk<0>(flow, start >> 2, Nx, cap, &steps, status);
-        target = seg_rank(I, b, end, Nx, off_min, min_bits);
-      }
-      te[1][j] = target;
-      len[1][j] = target >= 0 ? (int)steps + 1 : 0;  // an arc that leaves the image is empty
+  for (int sd = 0; sd < 2; ++sd) {
+    const int M = ps.M[sd];
+    const int ga = te[sd][0] < 0 ? M : te[sd][0], gb = te[sd][1] < 0 ? M : te[sd][1];
+    if (ga == gb) {
+      ps.g12[sd][s] = make_int2(kCycleEnd, kCycleEnd);
+      continue;
     }
-    // a raw arc has fewer cells than the batch (cell ids are int32)
-    arc_f[s] = make_int4(te[0][0], te[0][1], len[0][0], len[0][1]);
-    arc_v[s] = make_int4(te[1][0], te[1][1], len[1][0], len[1][1]);
-    // round 0 of the pairing: descending sweep on the face side in the
-    // primal and the vertex side in the dual
-    const bool d = I.dual[b];
-    const float v = ps.sval[s];
-#pragma unroll
-    for (int sd = 0; sd < 2; ++sd) {
-      const int M = ps.M[sd];
-      const int ga = te[sd][0] < 0 ? M : te[sd][0], gb = te[sd][1] < 0 ? M : te[sd][1];
-      if (ga == gb) {
-        ps.dying[sd][s] = -1;
-        continue;
-      }
-      ps.dying[sd][s] = kUndecided;
-      ps.g12[sd][s] = make_int2(ga, gb);
-      const unsigned long long k = sweep_key(v, s, sd == 0 ? !d : d);
-      atomicMin(ps.minedge[sd] + ga, k);  // result unused: a reduction
+    const bool local = (loc[sd][0] | loc[sd][1]) >= 0;
+    ps.g12[sd][s] = local ? make_int2(~loc[sd][0], ~loc[sd][1]) : make_int2(ga, gb);
+    const unsigned long long k = sweep_key(ps.sval[s], s, sd == 0 ? !d : d);
+    if (ga != M) {
+      atomicMin(ps.minedge[sd] + ga, k);  // results unused: reductions
+      if (!local) atomicMin(ps.leave[sd] + ga, (unsigned)(k >> 32));
+    }
+    if (gb != M) {
       atomicMin(ps.minedge[sd] + gb, k);
-      keep[sd] = 1;
+      if (!local) atomicMin(ps.leave[sd] + gb, (unsigned)(k >> 32));
     }
   }
-  const int c0 = __syncthreads_count(keep[0]), c1 = __syncthreads_count(keep[1]);
-  if (threadIdx.x == 0) {
-    if (c0) atomicAdd(ps.cnt[0] + 1, c0);
-    if (c1) atomicAdd(ps.cnt[1] + 1, c1);
+}
+
+// K5a: the pairing's rounds inside one 64 x 64 index tile and side per block,
+// on groups and saddles held in shared memory. A round's decision needs a
+// group's first outgoing saddle and the oldest member of the group behind it,
+// nothing else, so a block may decide any group whose first outgoing saddle
+// is local to the tile, at any time: the saddles that leave the tile enter
+// only through the smallest value key among them at each extremum (`leave`,
+// from the walks), and a group that reaches it waits for the global rounds.
+// Round 0 decides from the walks' minima. The saddles that stay undecided are
+// listed again each round, so a round costs what is left of them. After the
+// rounds only the first of the saddles between the same two groups is kept
+// (when a later one is swept the two are joined already: a cycle); the block
+// then writes the decisions (-1 for a cycle, and for now for what stays
+// undecided), links every dead group to its root and appends the saddles and
+// roots that remain to the lists of the global rounds. A tile with more
+// extrema or saddles than fit (kTileNodes, kTileEdges: above those of i.i.d.
+// noise, 820 and 1460 of 4096 cells) hands everything on.
+//
+// Bound: instruction issue (short dependent shared-memory chains and block
+// barriers, 48 warps per SM). On the bump fields 12% of the saddles and 8% of
+// the groups are left to the global rounds, on i.i.d. noise 15% and 10% (with
+// tiles of 128: 5 to 8%, but one block per SM). Measured, the whole pairing
+// stage without and with this pass and the last block's rounds: 4096^2 bumps
+// 1.13 -> 0.76 ms (this pass 0.37), 8192^2 noise 7.80 -> 4.75, 509 x 1531
+// 0.287 -> 0.166.
+constexpr int kTileNodes = 896, kTileEdges = 1664;
+constexpr int kTilePairNT = 256, kTilePairWarps = kTilePairNT / 32;
+constexpr int kTileRounds = 6;    // later rounds decide less than 1% of what is left
+constexpr int kTilePairs = 512;   // slots of the table of group pairs
+constexpr int kTileList = (kTileEdges / 32 + kTilePairWarps - 1) / kTilePairWarps * 32;  // a warp's edges
+constexpr unsigned kTileVoid = 0xFFFEu;
+// `ends` of an edge that is no longer undecided: dead node | kTileDead, or a
+// cycle (or not the first between its groups); of one that leaves the tile
+constexpr uint32_t kTileDead = 0xFFFF0000u, kTileCycle = 0xFFFFFFFFu, kTileOut = 0xFFFEFFFEu;
+
+struct PairTileSmem {
+  unsigned long long minedge[kTileNodes];  // (value key, edge or its complement) of a root's first local saddle
+  float val[kTileNodes];
+  uint32_t leave[kTileNodes];   // value key of the group's first saddle out of the tile
+  uint32_t ends[kTileEdges];    // nodes of both ends (roots as of the last phase A)
+  uint32_t hi[kTileEdges];      // value key
+  uint16_t list[kTilePairWarps][kTileList];  // each warp's undecided edges
+  uint16_t link[kTileNodes];
+  uint8_t seg[kTileNodes];      // segment of each node
+  uint8_t row[kTileEdges];      // row of each edge
+  uint32_t bits[2 * kLT];       // extrema of each (row, 32-column segment)
+  uint16_t npre[2 * kLT + 1];   // nodes before each segment
+  int noff[2 * kLT];            // first rank of each segment
+  uint16_t spre[kLT + 1];       // edges before each row
+  int sbase[kLT];               // first saddle of each row
+  int n_live;
+};
+
+struct PairTileArgs {
+  PairStart ps;
+  const int* off[2];        // segment offsets of each side's extrema
+  const uint32_t* bits[2];  // segment bit masks of each side's extrema
+  const int2* key[2];       // (value bits, cell) of each extremum
+  const int* off_sad;       // segment offsets and counts of the saddles
+  const int* seg_sad;
+  int* act[2];    // active saddles for the global rounds
+  int* roots[2];  // live roots
+};
+
+// Root of node x in the tile's forest (path halving; at most kTileNodes steps).
+__device__ __forceinline__ unsigned tile_root(volatile uint16_t* link, unsigned x) {
+  if (x == kTileVoid) return x;
+  unsigned p = link[x];
+  for (int k = 0; k <= kTileNodes; ++k) {
+    if (p == x || p == kTileVoid) return p;
+    const unsigned pp = link[p];
+    if (pp == p) return p;
+    link[x] = (uint16_t)pp;
+    if (pp == kTileVoid) return pp;
+    x = pp;
+    p = link[x];
+  }
+  return x;
+}
+
+__global__ void __launch_bounds__(kTilePairNT, 6) pair_tile_kernel(Imgs I, PairTileArgs A) {
+  extern __shared__ __align__(16) unsigned char pair_tile_smem[];
+  PairTileSmem& S = *reinterpret_cast<PairTileSmem*>(pair_tile_smem);
+  constexpr int NT = kTilePairNT, NW = kTilePairWarps, kNodesPer = (kTileNodes + NT - 1) / NT;
+  const bool s1 = blockIdx.x & 1;  // consecutive blocks: the two sides of one tile
+  const LabelTile g = label_tile_of(I, blockIdx.x >> 1);
+  const bool dual = I.dual[g.b];
+  const bool desc = s1 ? dual : !dual, older_less = s1 ? !dual : dual;
+  unsigned long long* minedge = s1 ? A.ps.minedge[1] : A.ps.minedge[0];
+  int* glink = s1 ? A.ps.link[1] : A.ps.link[0];
+  int2* g12 = s1 ? A.ps.g12[1] : A.ps.g12[0];
+  int* dying = s1 ? A.ps.dying[1] : A.ps.dying[0];
+  int* cnt = s1 ? A.ps.cnt[1] : A.ps.cnt[0];
+  int* act = s1 ? A.act[1] : A.act[0];
+  int* roots = s1 ? A.roots[1] : A.roots[0];
+  const int M = s1 ? A.ps.M[1] : A.ps.M[0];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const unsigned lt = (1u << lane) - 1u;
+  // ---- segment tables: extrema by (row, segment), saddles by row ----
+  const int nsegx = (g.W + kTileX) / kTileX;
+  if (tid < 2 * kLT) {
+    const int r = tid >> 1, y = g.y0 + r, sx = (g.x0 >> 5) + (tid & 1);
+    const bool in = y <= g.H && sx < nsegx;
+    const long long q = (long long)I.seg_base[g.b] + (long long)y * nsegx + sx;
+    S.bits[tid] = in ? __ldg((s1 ? A.bits[1] : A.bits[0]) + q) : 0u;
+    S.noff[tid] = in ? __ldg((s1 ? A.off[1] : A.off[0]) + q) : 0;
+    const int so = in ? __ldg(A.off_sad + q) : 0x7FFFFFFF, sn = in ? __ldg(A.seg_sad + q) : 0;
+    const int both = sn + __shfl_xor_sync(0xffffffffu, sn, 1);
+    if ((tid & 1) == 0) {
+      S.sbase[r] = so;
+      S.spre[r + 1] = (uint16_t)both;
+    }
+  } else if (tid == NT - 1) {
+    S.n_live = 0;
+  }
+  __syncthreads();
+  if (tid < 32) {  // exclusive sums: 128 segments (4 per lane), 64 rows (2 per lane)
+    int c[4], n = 0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) n += c[k] = __popc(S.bits[4 * lane + k]);
+    const int e0 = S.spre[2 * lane + 1], e1 = S.spre[2 * lane + 2];
+    int xn = n, xe = e0 + e1;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int yn = __shfl_up_sync(0xffffffffu, xn, o), ye = __shfl_up_sync(0xffffffffu, xe, o);
+      if (lane >= o) {
+        xn += yn;
+        xe += ye;
+      }
+    }
+    int at = xn - n;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      S.npre[4 * lane + k] = (uint16_t)at;
+      at += c[k];
+    }
+    if (lane == 31) S.npre[2 * kLT] = (uint16_t)at;
+    __syncwarp();
+    S.spre[2 * lane + 1] = (uint16_t)(xe - e1);
+    S.spre[2 * lane + 2] = (uint16_t)xe;
+    if (lane == 0) S.spre[0] = 0;
+  }
+  __syncthreads();
+  const int nn = S.npre[2 * kLT], ne = S.spre[kLT];
+  auto saddle_in_row = [&](int k, int r) { return S.sbase[r] + k - S.spre[r]; };
+  auto edge_of = [&](int s) {  // edge of a saddle of the tile
+    int lo = 0;
+#pragma unroll
+    for (int w = kLT / 2; w > 0; w >>= 1)
+      if (S.sbase[lo + w] <= s) lo += w;
+    return S.spre[lo] + s - S.sbase[lo];
+  };
+  auto local_rank = [&](int enc, bool node) -> int {  // node or list rank of a local end
+    const int p = ~enc;
+    if (p == kLocalVoid) return node ? (int)kTileVoid : M;
+    const int q = p >> 5;
+    return (node ? S.npre[q] : S.noff[q]) + __popc(S.bits[q] & ((1u << (p & 31)) - 1u));
+  };
+  if (nn > kTileNodes || ne > kTileEdges) {  // does not fit: all to the global rounds
+    for (int k0 = 0; k0 < max(ne, kLTN); k0 += NT) {
+      const int k = k0 + tid;
+      int s = -1, x = -1;
+      if (k < ne) {
+        int r = 0;
+        for (int w = kLT / 2; w > 0; w >>= 1)
+          if (S.spre[r + w] <= k) r += w;
+        s = saddle_in_row(k, r);
+        dying[s] = -1;
+        const int2 e = g12[s];
+        if (e.x == kCycleEnd)
+          s = -1;
+        else if (e.x < 0)
+          g12[s] = make_int2(local_rank(e.x, false), local_rank(e.y, false));
+      }
+      if (k < kLTN) {  // the cell at position k of the tile
+        const unsigned m = S.bits[k >> 5];
+        if ((m >> (k & 31)) & 1u) {
+          x = S.noff[k >> 5] + __popc(m & ((1u << (k & 31)) - 1u));
+          minedge[x] = kNoEdge;
+        }
+      }
+      int ps, px;
+      block_reserve2(cnt, s >= 0, cnt + 3, x >= 0, ps, px);
+      if (s >= 0) act[ps] = s;
+      if (x >= 0) roots[px] = x;
+    }
+    return;
+  }
+  {  // row of every edge, segment of every node
+    const int r = tid >> 2, q = tid >> 1;
+    for (int k = S.spre[r] + (tid & 3); k < S.spre[r + 1]; k += 4) S.row[k] = (uint8_t)r;
+    for (int i = S.npre[q] + (tid & 1); i < S.npre[q + 1]; i += 2) S.seg[i] = (uint8_t)q;
+  }
+  __syncthreads();
+  auto saddle_of = [&](int k) { return saddle_in_row(k, S.row[k]); };
+  auto rank_of = [&](unsigned i) {
+    const int q = S.seg[i];
+    return S.noff[q] + (int)i - S.npre[q];
+  };
+  // ---- nodes i = tid + NT j; edges in chunks of 32, chunk c to warp c % NW ----
+  unsigned long long me[kNodesPer];
+#pragma unroll
+  for (int j = 0; j < kNodesPer; ++j) {
+    const int i = tid + NT * j;
+    me[j] = kNoEdge;
+    if (i >= nn) continue;
+    const int x = rank_of(i);
+    me[j] = minedge[x];
+    S.val[i] = __int_as_float(__ldg(&(s1 ? A.key[1] : A.key[0])[x].x));
+    S.leave[i] = (s1 ? A.ps.leave[1] : A.ps.leave[0])[x];
+    S.minedge[i] = kNoEdge;
+    S.link[i] = (uint16_t)i;
+  }
+  uint16_t* const list = S.list[warp];
+  int n = 0;  // edges in the warp's list
+  constexpr int kBatch = 4;  // chunks whose loads are issued together
+  for (int c0 = warp; c0 * 32 < ne; c0 += NW * kBatch) {
+    int2 en[kBatch];
+    float sv[kBatch];
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u) {
+      const int k = (c0 + NW * u) * 32 + lane;
+      en[u] = make_int2(kCycleEnd, kCycleEnd);
+      sv[u] = 0.f;
+      if (k < ne) {
+        const int sd = saddle_of(k);
+        en[u] = g12[sd];
+        sv[u] = __ldg(A.ps.sval + sd);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u) {
+      const int k = (c0 + NW * u) * 32 + lane;
+      if ((c0 + NW * u) * 32 >= ne) break;  // warp-uniform
+      uint32_t e = en[u].x == kCycleEnd ? kTileCycle : kTileOut;
+      const bool take = en[u].x < 0 && en[u].x != kCycleEnd;
+      if (take) e = (uint32_t)local_rank(en[u].x, true) | (uint32_t)local_rank(en[u].y, true) << 16;
+      if (k < ne) {
+        const uint32_t o = orderable_key(sv[u]);
+        S.hi[k] = desc ? ~o : o;
+        S.ends[k] = e;
+      }
+      const unsigned m = __ballot_sync(0xffffffffu, take);
+      if (take) list[n + __popc(m & lt)] = (uint16_t)k;
+      n += __popc(m);
+    }
+  }
+  __syncthreads();
+  // A root's decision on its first outgoing edge k (value key h1): it dies
+  // there when the group behind it is older and no saddle out of the tile
+  // comes first. (The other end's root may read `ends` after it was marked:
+  // it finds the dead node, its own partner, there.)
+  auto decide = [&](int i, uint32_t h1, int k) -> bool {
+    const uint32_t e = S.ends[k];
+    const unsigned h = (e & 0xFFFFu) == (unsigned)i ? e >> 16 : e & 0xFFFFu;
+    if (h != kTileVoid) {  // nodes are numbered in cell order
+      const float vh = S.val[h], vi = S.val[i];
+      if (!(older_less ? tie_lt(vh, (int)h, vi, i) : tie_lt(vi, i, vh, (int)h))) return false;
+    }
+    S.ends[k] = kTileDead | (uint32_t)i;
+    S.link[i] = (uint16_t)h;
+    return true;
+  };
+  unsigned died = 0;  // bit j: node tid + NT j died in the previous round
+#pragma unroll
+  for (int j = 0; j < kNodesPer; ++j) {
+    const int i = tid + NT * j;
+    if (i >= nn || me[j] == kNoEdge) continue;
+    const uint32_t h1 = (uint32_t)(me[j] >> 32);
+    if (S.leave[i] <= h1) continue;  // its first saddle leaves the tile, or may
+    if (decide(i, h1, edge_of(sweep_key_saddle(me[j], desc)))) died |= 1u << j;
+  }
+  int any = __syncthreads_or(died);
+  for (int round = 1; any && round < kTileRounds; ++round) {
+    // a dead group's first saddle out of the tile now belongs to its root
+    if (died) {
+#pragma unroll
+      for (int j = 0; j < kNodesPer; ++j) {
+        if (!((died >> j) & 1u)) continue;
+        const int i = tid + NT * j;
+        const unsigned r = tile_root(S.link, i);
+        if (r != kTileVoid) atomicMin(&S.leave[r], S.leave[i]);
+      }
+    }
+    // phase A: both ends' roots; cycles and the edges decided in the previous
+    // round leave the warp's list, the others reduce their key into both
+    // roots' minimum
+    int kept = 0;
+    for (int q0 = 0; q0 < n; q0 += 32) {
+      bool keep = false;
+      int k = 0;
+      if (q0 + lane < n) {
+        k = list[q0 + lane];
+        const uint32_t e = S.ends[k];
+        if (e < kTileDead) {
+          const unsigned a = tile_root(S.link, e & 0xFFFFu), b = tile_root(S.link, e >> 16);
+          keep = a != b;
+          S.ends[k] = keep ? a | b << 16 : kTileCycle;
+          if (keep) {
+            const unsigned long long m = ((unsigned long long)S.hi[k] << 32) | (uint32_t)(desc ? 0xFFFF - k : k);
+            if (a != kTileVoid && m < *(volatile unsigned long long*)&S.minedge[a]) atomicMin(&S.minedge[a], m);
+            if (b != kTileVoid && m < *(volatile unsigned long long*)&S.minedge[b]) atomicMin(&S.minedge[b], m);
+          }
+        }
+      }
+      const unsigned m = __ballot_sync(0xffffffffu, keep);
+      __syncwarp();  // the chunk is read before its slots are written again
+      if (keep) list[kept + __popc(m & lt)] = (uint16_t)k;
+      kept += __popc(m);
+    }
+    n = kept;
+    __syncthreads();
+    // phase B
+    died = 0;
+#pragma unroll
+    for (int j = 0; j < kNodesPer; ++j) {
+      const int i = tid + NT * j;
+      if (i >= nn || S.link[i] != i) continue;
+      const unsigned long long m = S.minedge[i];
+      if (m == kNoEdge) continue;
+      S.minedge[i] = kNoEdge;
+      const uint32_t h1 = (uint32_t)(m >> 32);
+      if (S.leave[i] <= h1) continue;
+      if (decide(i, h1, desc ? 0xFFFF - (int)(uint32_t)m : (int)(uint32_t)m)) died |= 1u << j;
+    }
+    any = __syncthreads_or(died);
+  }
+  // ---- the first edge between each pair of groups, by a hash table (it
+  // takes the arrays of the minima and of the keys out of the tile, which
+  // are not read any more) ----
+  static_assert(kTilePairs <= kTileNodes, "the table reuses the nodes' arrays");
+  uint32_t* tab = S.leave;                // group pair of each slot
+  unsigned long long* first = S.minedge;  // its first edge's key
+  for (int q = tid; q < kTilePairs; q += NT) {
+    tab[q] = kTileCycle;
+    first[q] = kNoEdge;
+  }
+  if (lane == 0) atomicAdd(&S.n_live, n);
+  __syncthreads();
+  const bool dedupe = S.n_live <= kTilePairs;
+  for (int q = lane; q < n; q += 32) {
+    const int k = list[q];
+    const uint32_t e = S.ends[k];
+    if (e >= kTileDead) continue;
+    const unsigned a = tile_root(S.link, e & 0xFFFFu), b = tile_root(S.link, e >> 16);
+    const uint32_t pr = a == b ? kTileCycle : min(a, b) | max(a, b) << 16;  // the void is the larger node
+    S.ends[k] = pr;
+    if (!dedupe || a == b) continue;
+    unsigned h = (pr * 0x9E3779B1u) >> 23;  // 9 bits; there are no more pairs than slots
+    for (int t = 0; t < kTilePairs; ++t) {
+      const uint32_t old = atomicCAS(&tab[h], kTileCycle, pr);
+      if (old == kTileCycle || old == pr) break;
+      h = (h + 1) & (kTilePairs - 1);
+    }
+    atomicMin(&first[h], ((unsigned long long)S.hi[k] << 32) | (uint32_t)(desc ? 0xFFFF - k : k));
+    S.hi[k] = h;
+  }
+  __syncthreads();
+  // ---- decisions, links and what remains for the global rounds ----
+  int n_act = 0, n_root = 0;
+  if (dedupe) {
+    for (int q = lane; q < n; q += 32) {
+      const int k = list[q];
+      if (S.ends[k] >= kTileDead) continue;
+      const int lo = (int)(uint32_t)first[S.hi[k]];
+      if ((desc ? 0xFFFF - lo : lo) != k) S.ends[k] = kTileCycle;
+    }
+  }
+  __syncwarp();  // a warp's edges are those of its chunks
+  for (int c = warp; c * 32 < ne; c += NW) {
+    const int k = c * 32 + lane;
+    if (k >= ne) continue;
+    const uint32_t e = S.ends[k];
+    dying[saddle_of(k)] = e >= kTileDead && e != kTileCycle ? rank_of(e & 0xFFFFu) : -1;
+    n_act += e < kTileDead;
+  }
+#pragma unroll
+  for (int j = 0; j < kNodesPer; ++j) {
+    const int i = tid + NT * j;
+    if (i >= nn) continue;
+    const unsigned r = tile_root(S.link, i);
+    if (r == (unsigned)i)
+      ++n_root;
+    else
+      glink[rank_of(i)] = r == kTileVoid ? M : rank_of(r);
+  }
+  int pa, pr;
+  block_reserve2(cnt, n_act, cnt + 3, n_root, pa, pr);
+  for (int c = warp; c * 32 < ne; c += NW) {
+    const int k = c * 32 + lane;
+    if (k >= ne) continue;
+    const uint32_t e = S.ends[k];
+    if (e >= kTileDead) continue;
+    const int s = saddle_of(k);
+    if (e != kTileOut) g12[s] = make_int2(rank_of(e & 0xFFFFu), (e >> 16) == kTileVoid ? M : rank_of(e >> 16));
+    act[pa++] = s;
+  }
+#pragma unroll
+  for (int j = 0; j < kNodesPer; ++j) {
+    const int i = tid + NT * j;
+    if (i >= nn || S.link[i] != i) continue;
+    const int x = rank_of(i);
+    minedge[x] = kNoEdge;  // the global rounds start empty
+    roots[pr++] = x;
   }
 }
 

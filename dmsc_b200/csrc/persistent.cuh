@@ -74,16 +74,17 @@ __device__ __forceinline__ long long chunk_size(long long n, int blocks) {
   return 256LL * max(1LL, min((long long)kChunkPer, (n + lanes - 1) / lanes));
 }
 
-// Round loops whose active set has shrunk below a threshold finish in block 0
-// alone: the other blocks leave (all decide alike, from the same counters
-// read after the grid barrier that ended the previous round), and block 0
-// separates the remaining phases with block barriers instead of grid
-// barriers, which cost several microseconds each. The pairing's items are
-// short (a few dependent loads each), so block 0 takes over while each of
-// its threads still has several; a replay item walks whole parent chains, so
-// the replay goes solo only at one item per thread.
-constexpr long long kPairSoloItems = 2048;
+// Round loops whose active set has shrunk below a threshold leave the grid,
+// whose barriers cost several microseconds each. The replay and the geometry
+// expansion finish in block 0 alone (the other blocks leave: all decide
+// alike, from the same counters read after the grid barrier that ended the
+// previous round), with block barriers between the phases; a replay item
+// walks whole parent chains, so the replay does so only at one item per
+// thread. The pairing hands over to a kernel that holds what is left of a
+// side in one block's shared memory (pair_solo_kernel).
 constexpr long long kReplaySoloItems = 256;
+constexpr int kPairSoloEdges = 8192, kPairSoloNodes = 4096;  // per side
+constexpr unsigned kSoloVoid = 0x7FFFu;                      // the void's node
 
 __device__ __forceinline__ void chunk_start(ChunkLists& L) {
   if (threadIdx.x < 2) L.n[threadIdx.x] = 0;
@@ -91,14 +92,6 @@ __device__ __forceinline__ void chunk_start(ChunkLists& L) {
 }
 
 __device__ __forceinline__ void chunk_keep(ChunkLists& L, int side, int v) { L.buf[side][atomicAdd(&L.n[side], 1)] = v; }
-// the same, counting only (no list is written)
-__device__ __forceinline__ void chunk_count(ChunkLists& L, int side) { atomicAdd(&L.n[side], 1); }
-__device__ __forceinline__ void chunk_flush_count(ChunkLists& L, int* cnt0, int* cnt1) {
-  __syncthreads();
-  if (threadIdx.x < 2 && L.n[threadIdx.x] > 0) atomicAdd(threadIdx.x == 0 ? cnt0 : cnt1, L.n[threadIdx.x]);
-  __syncthreads();
-}
-
 __device__ __forceinline__ void chunk_flush(ChunkLists& L, int* cnt0, int* out0, int* cnt1, int* out1) {
   const int t = threadIdx.x;
   __syncthreads();
@@ -136,23 +129,32 @@ struct PairArgs {
   unsigned* status;
   int max_rounds;
   int* rounds;                   // receives the number of rounds (statistics)
+  // what the grid hands over to the solo kernel: the round (-1: it reached its
+  // cap), and the side's edges (sweep key; node | node << 16 | descending << 31)
+  // and nodes, the live roots in list order
+  int* handover;
+  unsigned long long* solo_key;  // [kPairSoloEdges]
+  uint32_t* solo_ends;           // [kPairSoloEdges]
+  int2* solo_ext;                // [kPairSoloNodes] (value bits, cell)
+  int* node;                     // [M] node of each live root
   unsigned long long* timeline;  // [kTimeline] round start times (ns), optional
 };
 
 // Both sides' persistence pairing in one cooperative launch; each round
 // processes both sides' active saddles and live roots, so the two sides share
 // their grid barriers. Per round and side: (A) every active saddle finds its
-// ends' groups, cycles are decided, the rest reduce their sweep key into
-// both groups' minimum (no returned value needed) and stay active; (B) every
+// ends' groups; those whose ends are in one group leave (cycles, whose
+// decision is -1 from the start, and the saddles decided in the round before,
+// whose ends are joined now), the rest reduce their sweep key into both
+// groups' minimum (no returned value needed) and stay active; (B) every
 // live root with an outgoing saddle decides whether it dies there, and a
 // root that dies links itself under the other group's root at once (phase B
 // reads no link, and the next reader is the next round's phase A, behind the
 // round's barrier); the others stay live; roots without outgoing saddles
-// leave for good. Round 0's phase A runs in the saddle walks (all groups are
-// single extrema then, so it needs no lookups), which also leave the round
-// counters; the groups' union-find and minima are set up by the compaction
-// (PairStart). Rounds 0 and 1 scan every saddle and group instead of reading
-// lists (see the round loop). A side with no active saddle just idles.
+// leave for good. The rounds start from the saddles and roots that the tile
+// pass (pair_tile_kernel) left undecided. The void is no list's member: it
+// never dies, so nothing is reduced into it. A side with no active saddle
+// just idles.
 struct PairArgs2 {
   PairArgs s[2];
 };
@@ -161,21 +163,20 @@ struct PairArgs2 {
 // is issued for all of them before any is used, so a thread waits on U
 // independent chains of dependent loads at once instead of one after the
 // other (the stores and atomics between items would otherwise keep the
-// compiler from overlapping them). Two shapes (tuned): U = 2 with 5 resident
-// blocks per SM (48 registers) and U = 4 with 4 (64 registers).
+// compiler from overlapping them). Two shapes (tuned): U = 2 and U = 4, both
+// with at most 4 resident blocks per SM (64 registers).
 constexpr int kPairShapes = 2;
 
 // Per-side fields picked by a flag (the parameter struct is only indexed
 // with constants, so it stays in the constant bank).
 #define PSIDE(f) (s1 ? P.s[1].f : P.s[0].f)
 
-// Phase A for the thread's items i0 + 256 u (u < U) below cend: side 0's
-// items come first (i < n0). In a scan the items are the saddles themselves
-// (the decided ones are skipped), else the active list; the saddles that stay
-// active are appended to the next list (`lists`) or only counted.
+// Phase A for the thread's items i0 + 256 u (u < U) below cend of the active
+// lists: side 0's items come first (i < n0); the saddles that stay active are
+// appended to the next list.
 template <int U>
 __device__ __forceinline__ void pair_batch_a(const PairArgs2& P, int r, long long i0, long long cend, int n0,
-                                             bool scan, bool lists, ChunkLists& L) {
+                                             ChunkLists& L) {
   int e[U], ga[U], gb[U];
   float sv[U];
   unsigned act = 0, s1m = 0, du = 0;
@@ -188,25 +189,20 @@ __device__ __forceinline__ void pair_batch_a(const PairArgs2& P, int r, long lon
       const long long j = s1 ? i - n0 : i;
       act |= 1u << u;
       s1m |= (unsigned)s1 << u;
-      e[u] = scan ? (int)j : ((r & 1) ? PSIDE(act1) : PSIDE(act0))[j];
+      e[u] = ((r & 1) ? PSIDE(act1) : PSIDE(act0))[j];
     }
   }
-  // the saddle's state, ends and key value, all issued together
-  int dy[U];
+  int2 g[U];  // the ends' groups of the previous round
 #pragma unroll
   for (int u = 0; u < U; ++u) {
-    dy[u] = kUndecided;
     ga[u] = gb[u] = 0;
+    g[u] = make_int2(0, 0);
     if (!((act >> u) & 1u)) continue;
     const bool s1 = (s1m >> u) & 1u;
-    dy[u] = PSIDE(dying)[e[u]];
-    const int2 g = PSIDE(g12)[e[u]];  // the ends' groups of the previous round
-    ga[u] = g.x;
-    gb[u] = g.y;
+    g[u] = PSIDE(g12)[e[u]];
+    ga[u] = g[u].x;
+    gb[u] = g[u].y;
   }
-#pragma unroll
-  for (int u = 0; u < U; ++u)
-    if (dy[u] != kUndecided) act &= ~(1u << u);
   {
     // the groups' current roots: path-halving finds of all 2U ends in lockstep
     unsigned live = 0;
@@ -260,30 +256,22 @@ __device__ __forceinline__ void pair_batch_a(const PairArgs2& P, int r, long lon
   for (int u = 0; u < U; ++u) {
     if (!((act >> u) & 1u)) continue;
     const bool s1 = (s1m >> u) & 1u;
-    if (ga[u] == gb[u]) {
-      PSIDE(dying)[e[u]] = -1;
-      continue;
-    }
-    PSIDE(g12)[e[u]] = make_int2(ga[u], gb[u]);
+    if (ga[u] == gb[u]) continue;  // a cycle, or decided in the previous round
+    if (ga[u] != g[u].x || gb[u] != g[u].y) PSIDE(g12)[e[u]] = make_int2(ga[u], gb[u]);
     const unsigned long long k = sweep_key(sv[u], e[u], (du >> u) & 1u);
-    atomicMin(PSIDE(minedge) + ga[u], k);  // result unused: a reduction
-    atomicMin(PSIDE(minedge) + gb[u], k);
-    if (lists)
-      chunk_keep(L, s1, e[u]);
-    else
-      chunk_count(L, s1);
+    if (ga[u] != PSIDE(M)) atomicMin(PSIDE(minedge) + ga[u], k);  // result unused: a reduction
+    if (gb[u] != PSIDE(M)) atomicMin(PSIDE(minedge) + gb[u], k);
+    chunk_keep(L, s1, e[u]);
   }
 }
 
 // Phase B for the thread's live roots k0 + 256 u (u < U) below cend (side 0's
-// first, k < nr0; in a scan every group, in index order, and the groups
-// without an outgoing saddle are skipped): each root with an outgoing saddle
-// decides there and a dying root links itself under the other group's root;
-// the void never dies; roots without outgoing saddles leave for good. The
-// roots that stay live are listed when `lists` is set.
+// first, k < nr0): each root with an outgoing saddle decides there and a
+// dying root links itself under the other group's root; roots without
+// outgoing saddles leave for good. The roots that stay live are listed.
 template <int U>
 __device__ __forceinline__ void pair_batch_b(const PairArgs2& P, int r, long long k0, long long cend, int nr0,
-                                             bool scan, bool lists, ChunkLists& L) {
+                                             ChunkLists& L) {
   int g[U];
   unsigned act = 0, s1m = 0;
 #pragma unroll
@@ -295,7 +283,7 @@ __device__ __forceinline__ void pair_batch_b(const PairArgs2& P, int r, long lon
       const long long j = s1 ? k - nr0 : k;
       act |= 1u << u;
       s1m |= (unsigned)s1 << u;
-      g[u] = scan ? (int)j : ((r & 1) ? PSIDE(roots1) : PSIDE(roots0))[j];
+      g[u] = ((r & 1) ? PSIDE(roots1) : PSIDE(roots0))[j];
     }
   }
   unsigned long long me[U];
@@ -307,7 +295,7 @@ __device__ __forceinline__ void pair_batch_b(const PairArgs2& P, int r, long lon
     if (!((act >> u) & 1u)) continue;
     const bool s1 = (s1m >> u) & 1u;
     me[u] = PSIDE(minedge)[g[u]];
-    if (g[u] < PSIDE(M)) kg[u] = PSIDE(key)[g[u]];
+    kg[u] = PSIDE(key)[g[u]];
   }
   int e[U];
   unsigned older_less = 0;
@@ -321,11 +309,6 @@ __device__ __forceinline__ void pair_batch_b(const PairArgs2& P, int r, long lon
       continue;
     }
     PSIDE(minedge)[g[u]] = kNoEdge;
-    if (g[u] == PSIDE(M)) {  // the void is older than every group: it never dies
-      if (lists) chunk_keep(L, s1, g[u]);
-      act &= ~(1u << u);
-      continue;
-    }
     // g is an extremum of one image; its image (from its cell) gives the
     // sweep direction of the key and the age order: value_less on the vertex
     // side in the primal and the face side in the dual
@@ -363,7 +346,7 @@ __device__ __forceinline__ void pair_batch_b(const PairArgs2& P, int r, long lon
     if (dies) {
       PSIDE(dying)[e[u]] = g[u];
       PSIDE(link)[g[u]] = h[u];
-    } else if (lists) {
+    } else {
       chunk_keep(L, s1, g[u]);
     }
   }
@@ -374,22 +357,14 @@ template <int U, int MINB>
 __global__ void __launch_bounds__(256, MINB) pairing_persistent_kernel(PairArgs2 P) {
   __shared__ ChunkLists L;
   cg::grid_group grid = cg::this_grid();
-  const long long tid = grid.thread_rank(), nth = grid.size();
-  bool done0 = false, done1 = false, solo = false;
-  // Round 0 takes every group and keeps no list (nearly all stay live; its
-  // saddle phase ran in the saddle walks, which also counted the saddles
-  // that stay active); round 1 scans every saddle (skipping the decided ones) and every
-  // group (skipping those without an outgoing saddle) and writes the lists
-  // that the later rounds read. Scanning all items in later rounds too, while
-  // many are active, measured slower (1.58 against 1.28 ms at 4096^2: the
-  // decided items still cost their loads).
-  bool scan = true;
+  const long long tid = grid.thread_rank();
+  const int bid = (int)blockIdx.x, nblk = (int)gridDim.x;
+  bool done0 = false, done1 = false;
   for (int r = 0;; ++r) {
     const int n0 = *(volatile int*)(P.s[0].cnt + r % 3), n1 = *(volatile int*)(P.s[1].cnt + r % 3);
     // a side whose active list is empty is finished: its roots are not visited
-    const int nr0 = n0 && !scan ? *(volatile int*)(P.s[0].cnt + 3 + r % 3) : 0;
-    const int nr1 = n1 && !scan ? *(volatile int*)(P.s[1].cnt + 3 + r % 3) : 0;
-    const bool lists = !scan || r >= 1;
+    const int nr0 = n0 ? *(volatile int*)(P.s[0].cnt + 3 + r % 3) : 0;
+    const int nr1 = n1 ? *(volatile int*)(P.s[1].cnt + 3 + r % 3) : 0;
     if (tid == 0) {
       for (int sd = 0; sd < 2; ++sd) {
         const PairArgs& A = P.s[sd];
@@ -403,74 +378,197 @@ __global__ void __launch_bounds__(256, MINB) pairing_persistent_kernel(PairArgs2
         done = done || n == 0;
       }
     }
-    if (n0 == 0 && n1 == 0) break;
-    if (!solo && !scan && (long long)n0 + n1 + nr0 + nr1 <= kPairSoloItems) {
-      solo = true;
-      if (blockIdx.x != 0) break;
+    // both sides fit the solo kernel (or are finished): the whole grid digests
+    // the edges and nodes for it (one block gathering them alone took 35 us)
+    // and every thread leaves
+    if (n0 <= kPairSoloEdges && n1 <= kPairSoloEdges && nr0 <= kPairSoloNodes && nr1 <= kPairSoloNodes) {
+      if (tid == 0) *P.s[0].handover = r;
+      if (n0 == 0 && n1 == 0) break;
+      for (long long j = tid; j < nr0 + nr1; j += grid.size()) {
+        const PairArgs& A = j < nr0 ? P.s[0] : P.s[1];
+        const int i = (int)(j < nr0 ? j : j - nr0);
+        const int g = ((r & 1) ? A.roots1 : A.roots0)[i];
+        A.node[g] = i;
+        A.solo_ext[i] = A.key[g];
+      }
+      grid.sync();
+      for (long long j = tid; j < n0 + n1; j += grid.size()) {
+        const bool s1 = j >= n0;
+        const PairArgs& A = s1 ? P.s[1] : P.s[0];
+        const int k = (int)(s1 ? j - n0 : j), s = ((r & 1) ? A.act1 : A.act0)[k];
+        const int2 e = A.g12[s];
+        const float v = A.sval[s];
+        const bool d = A.dual[A.B > 1 ? A.sad_img[s] : 0], desc = s1 ? d : !d;
+        const int a = find_halving(A.link, e.x, A.M + 2, A.status), b = find_halving(A.link, e.y, A.M + 2, A.status);
+        A.solo_key[k] = sweep_key(v, s, desc);
+        A.solo_ends[k] = (a == A.M ? kSoloVoid : (unsigned)A.node[a]) | (b == A.M ? kSoloVoid : (unsigned)A.node[b]) << 16 |
+                         (unsigned)desc << 31;
+      }
+      break;
     }
     if (r >= max(P.s[0].max_rounds, P.s[1].max_rounds)) {
       // every thread leaves here in the same round (the counters it read are
-      // the same); saddles still undecided become cycles, so the kernels
+      // the same); saddles still undecided stay cycles (-1), so the kernels
       // that run before the host sees the status read valid extremum indices
-      if (tid == 0) set_status(P.s[0].status, kStatusRoundCap);
-      const long long t0 = solo ? threadIdx.x : tid, nt = solo ? blockDim.x : nth;
-      for (int sd = 0; sd < 2; ++sd)
-        for (long long i = t0; i < P.s[sd].nsad; i += nt)
-          if (P.s[sd].dying[i] == kUndecided) P.s[sd].dying[i] = -1;
+      if (tid == 0) {
+        set_status(P.s[0].status, kStatusRoundCap);
+        *P.s[0].handover = -1;
+      }
       break;
     }
-    const int bid = solo ? 0 : (int)blockIdx.x, nblk = solo ? 1 : (int)gridDim.x;
     if (tid == 0) {
       for (int sd = 0; sd < 2; ++sd) {
         P.s[sd].cnt[(r + 2) % 3] = 0;
         P.s[sd].cnt[3 + (r + 2) % 3] = 0;
       }
     }
-    // phase A over both sides' active saddles (or every saddle in a scan);
-    // round 0's ran in the saddle walks
-    if (r > 0) {
-      const int na0 = scan ? P.s[0].nsad : n0, na1 = scan ? P.s[1].nsad : n1;
-      const long long n = (long long)na0 + na1, chunk = chunk_size(n, nblk);
+    {  // phase A: both sides' active saddles
+      const long long n = (long long)n0 + n1, chunk = chunk_size(n, nblk);
       for (long long c0 = (long long)bid * chunk; c0 < n; c0 += (long long)nblk * chunk) {
         chunk_start(L);
         const long long cend = min(n, c0 + chunk);
-        for (long long i0 = c0 + threadIdx.x; i0 < cend; i0 += 256LL * U)
-          pair_batch_a<U>(P, r, i0, cend, na0, scan, lists, L);
-        if (lists)
-          chunk_flush(L, P.s[0].cnt + (r + 1) % 3, (r & 1) ? P.s[0].act0 : P.s[0].act1, P.s[1].cnt + (r + 1) % 3,
-                      (r & 1) ? P.s[1].act0 : P.s[1].act1);
-        else
-          chunk_flush_count(L, P.s[0].cnt + (r + 1) % 3, P.s[1].cnt + (r + 1) % 3);
+        for (long long i0 = c0 + threadIdx.x; i0 < cend; i0 += 256LL * U) pair_batch_a<U>(P, r, i0, cend, n0, L);
+        chunk_flush(L, P.s[0].cnt + (r + 1) % 3, (r & 1) ? P.s[0].act0 : P.s[0].act1, P.s[1].cnt + (r + 1) % 3,
+                    (r & 1) ? P.s[1].act0 : P.s[1].act1);
       }
-      if (solo)
-        __syncthreads();
-      else
-        grid.sync();
     }
+    grid.sync();
     if (tid == 0 && r < kTimeline)  // side sd's phase-B starts: block 12 + sd
       for (int sd = 0; sd < 2; ++sd)
         if (P.s[sd].timeline) P.s[sd].timeline[kTimelinePhaseB + r] = global_ns();
-    // phase B: live roots (or every group in a scan) decide on their first
-    // outgoing saddle
-    {
-      const int nb0 = scan ? P.s[0].M + 1 : nr0, nb1 = scan ? P.s[1].M + 1 : nr1;
-      const long long n = (long long)nb0 + nb1, chunk = chunk_size(n, nblk);
+    {  // phase B: live roots decide on their first outgoing saddle
+      const long long n = (long long)nr0 + nr1, chunk = chunk_size(n, nblk);
       for (long long c0 = (long long)bid * chunk; c0 < n; c0 += (long long)nblk * chunk) {
-        if (lists) chunk_start(L);
+        chunk_start(L);
         const long long cend = min(n, c0 + chunk);
-        for (long long k0 = c0 + threadIdx.x; k0 < cend; k0 += 256LL * U)
-          pair_batch_b<U>(P, r, k0, cend, nb0, scan, lists, L);
-        if (lists)
-          chunk_flush(L, P.s[0].cnt + 3 + (r + 1) % 3, (r & 1) ? P.s[0].roots0 : P.s[0].roots1,
-                      P.s[1].cnt + 3 + (r + 1) % 3, (r & 1) ? P.s[1].roots0 : P.s[1].roots1);
+        for (long long k0 = c0 + threadIdx.x; k0 < cend; k0 += 256LL * U) pair_batch_b<U>(P, r, k0, cend, nr0, L);
+        chunk_flush(L, P.s[0].cnt + 3 + (r + 1) % 3, (r & 1) ? P.s[0].roots0 : P.s[0].roots1,
+                    P.s[1].cnt + 3 + (r + 1) % 3, (r & 1) ? P.s[1].roots0 : P.s[1].roots1);
       }
     }
-    scan = scan && !lists;
-    if (solo)
-      __syncthreads();
-    else
-      grid.sync();
+    grid.sync();
   }
+}
+
+// The pairing's last rounds, one block per side: the saddles and live roots
+// that the grid (or the tile pass) left, held in shared memory. A round costs
+// a few block barriers and shared-memory reads here, 12 to 16 us with grid
+// barriers and dependent global loads, however few its saddles are. Phase B
+// runs over the edges: the one whose (unique) key is its root's minimum
+// decides for that root and clears the minimum.
+constexpr int kSoloNT = 1024, kSoloList = kPairSoloEdges / (kSoloNT / 32);
+
+struct PairSoloSmem {
+  unsigned long long minedge[kPairSoloNodes];
+  unsigned long long key[kPairSoloEdges];  // sweep key of each edge
+  uint32_t ends[kPairSoloEdges];           // node | node << 16 | descending sweep << 31
+  int2 ext[kPairSoloNodes];                // (value bits, cell) of each node
+  int rank[kPairSoloNodes];
+  uint16_t link[kPairSoloNodes];
+  uint16_t list[kSoloNT / 32][kSoloList];  // each warp's undecided edges
+};
+
+__device__ __forceinline__ unsigned solo_root(volatile uint16_t* link, unsigned x) {
+  if (x == kSoloVoid) return x;
+  unsigned p = link[x];
+  for (int k = 0; k <= kPairSoloNodes; ++k) {  // links never form a cycle
+    if (p == x || p == kSoloVoid) return p;
+    const unsigned pp = link[p];
+    if (pp == p) return p;
+    link[x] = (uint16_t)pp;
+    if (pp == kSoloVoid) return pp;
+    x = pp;
+    p = link[x];
+  }
+  return x;
+}
+
+__global__ void __launch_bounds__(kSoloNT) pair_solo_kernel(PairArgs2 P) {
+  extern __shared__ __align__(16) unsigned char pair_solo_smem[];
+  PairSoloSmem& S = *reinterpret_cast<PairSoloSmem*>(pair_solo_smem);
+  const bool s1 = blockIdx.x != 0;
+  const PairArgs& A = s1 ? P.s[1] : P.s[0];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const unsigned lt = (1u << lane) - 1u;
+  const int r0 = *P.s[0].handover;
+  if (r0 < 0) return;  // the grid reached its cap
+  const int ne = A.cnt[r0 % 3], nr = A.cnt[3 + r0 % 3];
+  if (ne == 0) return;
+  const int* roots = (r0 & 1) ? A.roots1 : A.roots0;
+  for (int i = tid; i < nr; i += kSoloNT) {
+    S.rank[i] = roots[i];
+    S.ext[i] = A.solo_ext[i];
+    S.minedge[i] = kNoEdge;
+    S.link[i] = (uint16_t)i;
+  }
+  // edges in chunks of 32, chunk c to warp c % 32
+  uint16_t* const list = S.list[warp];
+  int n = 0;
+  for (int c = warp; c * 32 < ne; c += kSoloNT / 32) {
+    const int k = c * 32 + lane;
+    if (k < ne) {
+      S.key[k] = A.solo_key[k];
+      S.ends[k] = A.solo_ends[k];
+      list[n + lane] = (uint16_t)k;
+    }
+    n += min(32, ne - c * 32);
+  }
+  const int max_rounds = max(P.s[0].max_rounds, P.s[1].max_rounds);
+  int r = r0;
+  while (__syncthreads_or(n > 0)) {
+    if (r >= max_rounds) {  // what is undecided stays a cycle (-1)
+      if (tid == 0) set_status(A.status, kStatusRoundCap);
+      break;
+    }
+    if (tid == 0 && A.timeline && r < kTimeline && r > r0) A.timeline[r] = global_ns();
+    // phase A
+    int kept = 0;
+    for (int q0 = 0; q0 < n; q0 += 32) {
+      bool keep = false;
+      int k = 0;
+      if (q0 + lane < n) {
+        k = list[q0 + lane];
+        const uint32_t e = S.ends[k];
+        const unsigned a = solo_root(S.link, e & 0x7FFFu), b = solo_root(S.link, (e >> 16) & 0x7FFFu);
+        keep = a != b;  // else a cycle, or decided in the previous round
+        if (keep) {
+          S.ends[k] = a | b << 16 | (e & 0x80000000u);
+          const unsigned long long m = S.key[k];
+          if (a != kSoloVoid && m < *(volatile unsigned long long*)&S.minedge[a]) atomicMin(&S.minedge[a], m);
+          if (b != kSoloVoid && m < *(volatile unsigned long long*)&S.minedge[b]) atomicMin(&S.minedge[b], m);
+        }
+      }
+      const unsigned m = __ballot_sync(0xffffffffu, keep);
+      __syncwarp();  // the chunk is read before its slots are written again
+      if (keep) list[kept + __popc(m & lt)] = (uint16_t)k;
+      kept += __popc(m);
+    }
+    n = kept;
+    __syncthreads();
+    // phase B (the list is the warp's own: no barrier is needed before it)
+    for (int q = lane; q < n; q += 32) {
+      const int k = list[q];
+      const uint32_t e = S.ends[k];
+      const unsigned long long m = S.key[k];
+      const bool older_less = !(e >> 31);
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const unsigned g = (j ? e >> 16 : e) & 0x7FFFu, h = (j ? e : e >> 16) & 0x7FFFu;
+        if (g == kSoloVoid || *(volatile unsigned long long*)&S.minedge[g] != m) continue;
+        S.minedge[g] = kNoEdge;
+        if (h != kSoloVoid) {
+          const int2 kh = S.ext[h], kg = S.ext[g];
+          const float vh = __int_as_float(kh.x), vg = __int_as_float(kg.x);
+          if (!(older_less ? tie_lt(vh, kh.y, vg, kg.y) : tie_lt(vg, kg.y, vh, kh.y))) continue;
+        }
+        A.dying[sweep_key_saddle(m, e >> 31)] = S.rank[g];
+        S.link[g] = (uint16_t)h;
+      }
+    }
+    ++r;
+  }
+  if (tid == 0 && A.rounds) *A.rounds = r;
+  if (tid == 0 && A.timeline && r < kTimeline && r > r0) A.timeline[r] = global_ns();
 }
 
 // ---------------------------------------------------------------------------

@@ -57,12 +57,14 @@ __device__ __forceinline__ int flow_walk(const uint8_t* __restrict__ flow, int i
 }
 
 // Dense rank in its critical list of the extremum at global index g of image
-// b: its 32-index row segment's first rank (the compaction's exclusive scan)
-// plus the extrema before it in the segment's bit mask.
+// b, whose coordinates (y, x) are returned: its 32-index row segment's first
+// rank (the compaction's exclusive scan) plus the extrema before it in the
+// segment's bit mask.
 __device__ __forceinline__ int seg_rank(const Imgs& I, int b, int g, int Nx, const int* __restrict__ off,
-                                        const uint32_t* __restrict__ bits) {
+                                        const uint32_t* __restrict__ bits, int& y, int& x) {
   const int l = g - I.idx_base[b];
-  const int y = l / Nx, x = l - y * Nx;
+  y = l / Nx;
+  x = l - y * Nx;
   const int seg = I.seg_base[b] + y * ((Nx + 31) >> 5) + (x >> 5);
   return __ldg(off + seg) + __popc(__ldg(bits + seg) & ((1u << (x & 31)) - 1u));
 }

@@ -12,7 +12,7 @@ changes an output bit:
 * ``label_shape``: 64 x 64 label tiles on 1024 or 512 threads (4 or 8 cells
   per thread in the barrier-free pointer jumping);
 * ``pair_shape``: pairing items each thread advances together (2 or 4,
-  with 5 or 4 resident blocks per SM);
+  with at most 4 resident blocks per SM);
 * ``replay_shape``: replay cancellations each thread advances together (1 or
   2, with 4 or 3 resident blocks per SM);
 * ``emit_shape``: geometry-expansion chain tasks each thread advances
