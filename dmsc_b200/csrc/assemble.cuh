@@ -35,18 +35,6 @@ struct RouteF {
   }
 };
 
-__global__ void u8_to_int_kernel(const uint8_t* __restrict__ a, int n, int* __restrict__ b) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) b[i] = a[i];
-}
-
-// to_out[x] = batch-wide output rank of alive extremum x (-1 otherwise).
-__global__ void to_out_kernel(int n, const uint8_t* __restrict__ alive, const int* __restrict__ to_out_excl,
-                              int* __restrict__ to_out) {
-  int x = blockIdx.x * blockDim.x + threadIdx.x;
-  if (x < n) to_out[x] = alive[x] ? to_out_excl[x] : -1;
-}
-
 // Surviving extrema, image-local cell ids, into the routed point lists.
 __global__ void points_kernel(int n, const uint8_t* __restrict__ alive, const int* __restrict__ to_out_excl,
                               const int* __restrict__ alive_base, const int2* __restrict__ key,
@@ -58,18 +46,31 @@ __global__ void points_kernel(int n, const uint8_t* __restrict__ alive, const in
   if (dst) dst[to_out_excl[x] - alive_base[b]] = key[x].y - 4 * I.idx_base[b];
 }
 
-// flag[s] = 1 when saddle s (list order) survives both sides.
-__global__ void survivor_flag_kernel(int nsad, const uint8_t* __restrict__ cancelled, int* __restrict__ flag) {
-  int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= nsad) return;
-  flag[s] = cancelled[s] == 0;
+// Survivor count and first survivor of every image, from the exclusive scan
+// `pos` of the survivors' flags; the count, the two cancellation counts and
+// the status word go straight to the mapped readback area.
+__global__ void survivor_base_kernel(int B, const int* __restrict__ sad_base, int nsad,
+                                     const uint8_t* __restrict__ survive, const int* __restrict__ pos,
+                                     const int* __restrict__ n_cancel, const unsigned* __restrict__ status,
+                                     int* __restrict__ surv_base, long long* __restrict__ rb) {
+  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+  if (b > B) return;
+  const int total = nsad > 0 ? pos[nsad - 1] + survive[nsad - 1] : 0;
+  const int f = b < B ? sad_base[b] : nsad;
+  surv_base[b] = f < nsad ? pos[f] : total;
+  if (b == 0) {
+    rb[0] = total;
+    rb[1] = n_cancel[0];
+    rb[2] = n_cancel[1];
+    rb[3] = *status;
+  }
 }
 
 // The survivors in list order with their sort keys ((image, s_val) order:
 // the image id above the orderable value, so one sort orders every image;
 // a 32-bit key of the value alone for one image).
 template <class K>
-__global__ void survivor_gather_kernel(int nsad, const int* __restrict__ flag, const int* __restrict__ pos,
+__global__ void survivor_gather_kernel(int nsad, const uint8_t* __restrict__ flag, const int* __restrict__ pos,
                                        const float* __restrict__ sval, const int* __restrict__ sad_img,
                                        K* __restrict__ key_out, int* __restrict__ idx_out) {
   int s = blockIdx.x * blockDim.x + threadIdx.x;

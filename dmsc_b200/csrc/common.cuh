@@ -120,8 +120,8 @@ struct Imgs {
 // The persistence pairing's starting state, written by the kernels that
 // produce its inputs instead of a pass of its own: the ordered compaction
 // sets every group's union-find link (itself) and smallest outgoing keys
-// (none) as it lists the extrema, plus the void's link and the round
-// counters; the saddle walks record each saddle's ends as they find them and
+// (none) and its alive flag as it lists the extrema, plus the void's link
+// and the counters; the saddle walks record each saddle's ends as they find them and
 // reduce the saddles' keys into the minima (see pairing.cuh). Side 0
 // is the face side (maxima), side 1 the vertex side (minima).
 struct PairStart {
@@ -130,6 +130,8 @@ struct PairStart {
   unsigned* leave[2];              // [M] smallest value key of the saddles out of the extremum's tile
   int* link[2];                    // [M + 1] group union-find
   int* cnt[2];                     // [6] rotating active-saddle and live-root counters
+  int* n_cancel;                   // [2] cancellation counters
+  uint8_t* alive[2];               // [M] extrema that no cancelled saddle kills
   int2* g12[2];                    // [nsad] groups of each saddle's two ends
   int* dying[2];                   // [nsad] decision of each saddle
   const float* sval;               // [nsad] saddle values

@@ -15,6 +15,7 @@
 #include <chrono>
 #include <cub/cub.cuh>
 #include <cudaTypedefs.h>
+#include <thrust/iterator/transform_iterator.h>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -40,13 +41,13 @@ namespace {
 enum Slot {
   S_MASK, S_FLOW, S_SEG0, S_SEG1, S_SEG2, S_OFF0, S_OFF1, S_OFF2, S_TOT, S_TAB, S_BASES,
   S_CSAD, S_IMIN, S_ISAD, S_IMAX, S_MINBITS, S_MAXBITS, S_KMIN, S_KMAX, S_SVAL, S_SKEY2, S_IOTA,
-  S_ASC, S_ARCF, S_ARCV, S_CANC, S_FLAG, S_FPOS, S_SURV, S_STATUS, S_NCANC, S_STATS, S_TIMELINE, S_ROUTE,
+  S_ASC, S_ARCF, S_ARCV, S_ALIVE, S_RANK, S_FLAG, S_FPOS, S_SURV, S_STATUS, S_NCANC, S_STATS, S_TIMELINE, S_ROUTE,
   S_BKEY, S_BIDX, S_BKEY2, S_BIDX2, S_PERF, S_PERV, S_EXF, S_EXV, S_NEX, S_SKEY32B, S_SKEYS, S_SURVIC,
   S_SIDE0,  // per-side slots start here, kSideSlots each
 };
 enum SideSlot {
-  X_ROUT, X_SVT, X_SVL, X_SVR, X_DYING, X_GRP, X_LINK, X_MINE, X_ACT0, X_ACT1, X_CNT, X_PAIR, X_ALIVE,
-  X_ALIVEI, X_TOOUTX, X_TOOUT, X_UF, X_CROOT, X_CKEY, X_CVAL, X_NODE,
+  X_ROUT, X_SVT, X_SVL, X_SVR, X_DYING, X_GRP, X_LINK, X_MINE, X_ACT0, X_ACT1, X_CNT, X_PAIR,
+  X_UF, X_CROOT, X_CKEY, X_CVAL, X_NODE,
   X_ALEN, X_ACL, X_AROOT, X_PLEN, X_SEND, X_APOS, X_EROWC, X_EROWO, X_Q0, X_Q1, X_QB, X_G12,
   X_GBASE, X_WX, X_WA, X_CENDS, X_SOLO, kSideSlots
 };
@@ -83,8 +84,7 @@ struct Side {
   int* dying = nullptr;
   int2* pp = nullptr;               // [nsad] paired extremum (-1: none) and persistence bits
   uint8_t* alive = nullptr;
-  int* to_out_excl = nullptr;
-  int* to_out = nullptr;
+  int* to_out_excl = nullptr;   // [M] alive extrema before each (over both sides' lists)
   ReplayState R{};
   int C = 0;
   long long* arc_len = nullptr;
@@ -293,8 +293,8 @@ void* cub_tmp(dmsc_b200_context* ctx, size_t bytes, cudaStream_t st) {
   return b.p;
 }
 
-template <class In, class Out>
-void excl_sum(dmsc_b200_context* ctx, const In* in, Out* out, int n, cudaStream_t st) {
+template <class It, class Out>
+void excl_sum(dmsc_b200_context* ctx, It in, Out* out, int n, cudaStream_t st) {
   if (n <= 0) return;
   size_t bytes = 0;
   CK(cub::DeviceScan::ExclusiveSum(nullptr, bytes, in, out, n, st));
@@ -533,52 +533,65 @@ void run_pairing(dmsc_b200_context* ctx, PairTileArgs T, int nltile, cudaStream_
   LAUNCH_CHECK("pair_solo_kernel");
 }
 
-// Persistence, cancellation, thresholded union-find and output ranks of one side.
-void finish_pairing(dmsc_b200_context* ctx, int si, Side& S, cudaStream_t st) {
-  const int nsad = ctx->nsad, M = S.M;
-  // persistence, cancellation, alive flags
-  S.pp = sget<int2>(ctx, si, X_PAIR, nsad);
-  S.alive = sget<uint8_t>(ctx, si, X_ALIVE, M + 4);
-  CK(cudaMemsetAsync(S.alive, 1, M + 4, st));
-  uint8_t* canc = get<uint8_t>(ctx, S_CANC, nsad + 4);
-  int* ncanc = get<int>(ctx, S_NCANC, 4) + si;
-  CK(cudaMemsetAsync(ncanc, 0, sizeof(int), st));
-  int2* cends = sget<int2>(ctx, si, X_CENDS, nsad);
-  // the replay's cancellation list (keys and saddles) comes out of the same
-  // pass when this side's arcs are simplified
-  unsigned long long* ckey = S.arcs ? sget<unsigned long long>(ctx, si, X_CKEY, nsad) : nullptr;
-  int* cval = S.arcs ? sget<int>(ctx, si, X_CVAL, nsad) : nullptr;
-  ReplayNode* node = S.arcs ? sget<ReplayNode>(ctx, si, X_NODE, M + 1) : nullptr;
-  if (nsad > 0) {
-    LK(persistence_kernel<<<grid_for(nsad, TB), TB, 0, st>>>(
-        nsad, !S.faces, ctx->I.dual, ctx->I.thr, ctx->sad_img, S.dying, get<float>(ctx, S_SVAL, nsad), S.key,
-        S.pp, canc, (uint8_t)(S.faces ? 1 : 2), S.alive, ncanc, S.arc, cends, ctx->crit_sad, ckey,
-        cval, node));
-    LAUNCH_CHECK("persistence_kernel");
+struct ByteToInt {
+  __host__ __device__ int operator()(uint8_t v) const { return v; }
+};
+
+// Persistence, cancellation, thresholded union-find and output ranks of both
+// sides; `survive` / `pos`: the surviving saddles and their exclusive scan.
+void finish_pairing(dmsc_b200_context* ctx, uint8_t* survive, int* pos, cudaStream_t st) {
+  const int nsad = ctx->nsad;
+  PersistArgs P{};
+  UtArgs U{};
+  P.nsad = nsad;
+  P.dual = ctx->I.dual;
+  P.thr = ctx->I.thr;
+  P.sad_img = ctx->sad_img;
+  P.crit_sad = ctx->crit_sad;
+  P.sval = get<float>(ctx, S_SVAL, nsad);
+  P.survive = survive;
+  P.n_cancel = get<int>(ctx, S_NCANC, 4);
+  U.count = P.n_cancel;
+  U.status = ctx->status;
+  const int Mf = ctx->side[0].M, Mv = ctx->side[1].M, most = std::max(Mf, Mv) + 1;
+  // both sides' flags and ranks back to back, so one scan ranks them all (a
+  // side's ranks are only used relative to its images' first ones)
+  uint8_t* alive = get<uint8_t>(ctx, S_ALIVE, (size_t)Mf + Mv);
+  int* rank = get<int>(ctx, S_RANK, (size_t)Mf + Mv);
+  for (int si = 0; si < 2; ++si) {
+    Side& S = ctx->side[si];
+    S.pp = sget<int2>(ctx, si, X_PAIR, nsad);
+    S.alive = alive + (si ? Mf : 0);
+    S.to_out_excl = rank + (si ? Mf : 0);
+    S.rout = sget<int>(ctx, si, X_ROUT, S.M + 1);
+    P.M[si] = U.M[si] = S.M;
+    P.dying[si] = S.dying;
+    P.key[si] = S.key;
+    P.pp[si] = S.pp;
+    P.alive[si] = S.alive;
+    P.arc[si] = S.arc;
+    P.ends[si] = sget<int2>(ctx, si, X_CENDS, nsad);
+    // the replay's cancellation list (keys and saddles) comes out of the same
+    // pass when this side's arcs are simplified
+    P.ckey[si] = S.arcs ? sget<unsigned long long>(ctx, si, X_CKEY, nsad) : nullptr;
+    P.cval[si] = S.arcs ? sget<int>(ctx, si, X_CVAL, nsad) : nullptr;
+    P.node[si] = S.arcs ? sget<ReplayNode>(ctx, si, X_NODE, S.M + 1) : nullptr;
+    P.uf[si] = sget<int>(ctx, si, X_UF, S.M + 1);
+    U.ends[si] = P.ends[si];
+    U.p[si] = P.uf[si];
+    U.alive[si] = S.alive;
+    U.comp_root[si] = sget<int>(ctx, si, X_CROOT, S.M + 1);
+    U.rank[si] = S.to_out_excl;
+    U.rout[si] = S.rout;
   }
-  // thresholded union-find roots
-  int* uf = sget<int>(ctx, si, X_UF, M + 1);
-  int* croot = sget<int>(ctx, si, X_CROOT, M + 1);
-  LK(iota_kernel<<<grid_for(M + 1, TB), TB, 0, st>>>(uf, M + 1));
-  if (nsad > 0)
-    LK(ut_union_kernel<<<grid_for(nsad, TB), TB, 0, st>>>(cends, ncanc, M, uf, M + 2, ctx->status));
-  LK(ut_flatten_kernel<<<grid_for((M + 1 + kUtBatch - 1) / kUtBatch, TB), TB, 0, st>>>(M + 1, uf, M + 2,
-                                                                                       ctx->status));
-  LK(ut_mark_kernel<<<grid_for(M + 1, TB), TB, 0, st>>>(M, uf, S.alive, croot));
-  LAUNCH_CHECK("thresholded union-find");
-  // batch-wide output rank of alive extrema
-  int* alive_i = sget<int>(ctx, si, X_ALIVEI, M + 1);
-  S.to_out_excl = sget<int>(ctx, si, X_TOOUTX, M + 1);
-  S.to_out = sget<int>(ctx, si, X_TOOUT, M + 1);
-  if (M > 0) {
-    LK(u8_to_int_kernel<<<grid_for(M, TB), TB, 0, st>>>(S.alive, M, alive_i));
-    excl_sum(ctx, alive_i, S.to_out_excl, M, st);
-    LK(to_out_kernel<<<grid_for(M, TB), TB, 0, st>>>(M, S.alive, S.to_out_excl, S.to_out));
-    LAUNCH_CHECK("to_out_kernel");
-  }
-  S.rout = sget<int>(ctx, si, X_ROUT, M + 1);
-  if (M > 0) LK(root_out_kernel<<<grid_for(M, TB), TB, 0, st>>>(M, uf, croot, S.to_out, S.rout));
-  LAUNCH_CHECK("root_out_kernel");
+  LK(persistence_kernel<<<grid_for(std::max(nsad, most), TB), TB, 0, st>>>(P));
+  if (nsad > 0) LK(ut_union_kernel<<<dim3(grid_for(nsad, TB), 2), TB, 0, st>>>(U));
+  LK(ut_flatten_kernel<<<dim3(grid_for((most + kUtBatch - 1) / kUtBatch, TB), 2), TB, 0, st>>>(U));
+  auto as_int = [](const uint8_t* p) { return thrust::make_transform_iterator(p, ByteToInt{}); };
+  excl_sum(ctx, as_int(alive), rank, Mf + Mv, st);
+  LK(root_out_kernel<<<dim3(grid_for(most, TB), 2), TB, 0, st>>>(U));
+  excl_sum(ctx, as_int(survive), pos, nsad, st);
+  LAUNCH_CHECK("persistence and ranks");
 }
 
 // Replay inputs of one side (batch); returns the replay kernel's arguments,
@@ -923,7 +936,9 @@ int extract_batch_impl(dmsc_b200_context* ctx, int B, const float* img, const in
   // minima), set up by the compaction and the saddle walks
   PairStart ps;
   ps.sval = sval;
+  ps.n_cancel = get<int>(ctx, S_NCANC, 4);
   for (int si = 0; si < 2; ++si) {
+    ps.alive[si] = get<uint8_t>(ctx, S_ALIVE, (size_t)nmax + nmin) + (si ? nmax : 0);
     const int M = si ? nmin : nmax;
     ps.M[si] = M;
     ps.minedge[si] = sget<unsigned long long>(ctx, si, X_MINE, M + 1);
@@ -992,9 +1007,7 @@ int extract_batch_impl(dmsc_b200_context* ctx, int B, const float* img, const in
     S->groups = (S->groups_primal && any_primal) || (S->groups_dual && any_dual);
   }
 
-  uint8_t* canc = get<uint8_t>(ctx, S_CANC, nsad + 4);
   mark(ctx, 4, st);
-  CK(cudaMemsetAsync(canc, 0, nsad + 4, st));
   {
     PairTileArgs T{};
     T.ps = ps;
@@ -1007,42 +1020,25 @@ int extract_batch_impl(dmsc_b200_context* ctx, int B, const float* img, const in
     run_pairing(ctx, T, (int)nltile, st);
   }
   mark(ctx, 5, st);
-  // the two sides' persistence, thresholded union-find and ranks are
-  // independent (disjoint buffers; their cancellation bits are ORed into the
-  // shared byte map with atomics): the vertex side runs on side_st
-  CK(cudaEventRecord(ctx->fork_ev, st));
-  CK(cudaStreamWaitEvent(ctx->side_st, ctx->fork_ev, 0));
-  finish_pairing(ctx, 0, F, st);
-  finish_pairing(ctx, 1, V, ctx->side_st);
-  CK(cudaEventRecord(ctx->join_ev, ctx->side_st));
-  CK(cudaStreamWaitEvent(st, ctx->join_ev, 0));
+  uint8_t* flag = get<uint8_t>(ctx, S_FLAG, nsad);  // surviving saddles
+  int* fpos = get<int>(ctx, S_FPOS, nsad);
+  finish_pairing(ctx, flag, fpos, st);
   mark(ctx, 6, st);
 
   // ---- surviving saddles in minima-sweep (vertex side) order ----
-  int* flag = get<int>(ctx, S_FLAG, nsad);
-  int* fpos = get<int>(ctx, S_FPOS, nsad);
   ctx->surv = get<int>(ctx, S_SURV, nsad);
-  ctx->nsurv = 0;
-  if (nsad > 0) {
-    LK(survivor_flag_kernel<<<grid_for(nsad, TB), TB, 0, st>>>(nsad, canc, flag));
-    excl_sum(ctx, flag, fpos, nsad, st);
-    LK(last_plus_kernel<int><<<1, 1, 0, st>>>(fpos, flag, nsad, tot));
-    LK(copy2_kernel<<<1, 1, 0, st>>>(get<int>(ctx, S_NCANC, 4), tot + 1));
-    LAUNCH_CHECK("survivors");
-    // the status word rides along: a capped pairing or union-find loop ends
-    // the call here, before the replay
-    rb_reserve(ctx, 4 * sizeof(long long));
-    rb_copy(ctx, st, 0, tot, 3 * sizeof(long long));
-    rb_copy(ctx, st, 3 * sizeof(long long), ctx->status, sizeof(unsigned));
-    wait_stream(ctx, st);
-    raise_status(ctx, *(const unsigned*)(ctx->rb_h + 3 * sizeof(long long)));
-    ctx->nsurv = (int)rb_ll(ctx)[0];
-    F.C = (int)rb_ll(ctx)[1];
-    V.C = (int)rb_ll(ctx)[2];
-  }
+  // the status word rides along: a capped pairing or union-find loop ends the
+  // call here, before the replay
+  rb_reserve(ctx, 4 * sizeof(long long));
+  LK(survivor_base_kernel<<<grid_for(B + 1LL, TB), TB, 0, st>>>(B, BS.sad, nsad, flag, fpos, get<int>(ctx, S_NCANC, 4),
+                                                               ctx->status, BS.surv, (long long*)ctx->rb_d));
+  LAUNCH_CHECK("survivor_base_kernel");
+  wait_stream(ctx, st);
+  raise_status(ctx, (unsigned)rb_ll(ctx)[3]);
+  ctx->nsurv = (int)rb_ll(ctx)[0];
+  F.C = (int)rb_ll(ctx)[1];
+  V.C = (int)rb_ll(ctx)[2];
   const int nsurv = ctx->nsurv;
-  LK(image_base_kernel<<<grid_for(B + 1LL, TB), TB, 0, st>>>(B, BS.sad, nsad, fpos, nsurv, BS.surv));
-  LAUNCH_CHECK("survivor bases");
   // the survivor order and records run on side_st, overlapping the replay
   // and the labels (neither reads them); the final arcs wait for them
   cudaStream_t ss = ctx->side_st;

@@ -756,6 +756,7 @@ static __global__ void __launch_bounds__(256) compact_kernel(
       ps.link[sd][ps.M[sd]] = ps.M[sd];
 #pragma unroll
       for (int k = 0; k < 6; ++k) ps.cnt[sd][k] = 0;
+      ps.n_cancel[sd] = 0;
     }
   }
   const unsigned lt = (1u << lane) - 1u;
@@ -810,6 +811,7 @@ static __global__ void __launch_bounds__(256) compact_kernel(
       ps.minedge[1][q] = ~0ull;  // a single-extremum group without outgoing saddles yet
       ps.leave[1][q] = ~0u;
       ps.link[1][q] = q;
+      ps.alive[1][q] = 1;
     }
     if (m & 8u) {
       const int q = o_max[k] + __popc(bmax & lt);
@@ -818,6 +820,7 @@ static __global__ void __launch_bounds__(256) compact_kernel(
       ps.minedge[0][q] = ~0ull;
       ps.leave[0][q] = ~0u;
       ps.link[0][q] = q;
+      ps.alive[0][q] = 1;
     }
 #pragma unroll
     for (int t = 1; t <= 2; ++t) {

@@ -552,75 +552,87 @@ __global__ void __launch_bounds__(kTilePairNT, 6) pair_tile_kernel(Imgs I, PairT
   }
 }
 
-__global__ void iota_kernel(int* __restrict__ a, int n) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) a[i] = i;
-}
-
 // Persistence of each decided saddle and cancellation (persistence.hxx:82-104,
-// 139-161), with the saddle's image's orientation and threshold: pp[s] =
-// (paired extremum or -1, persistence bits; -1 for a cycle); `sbit` marks the
-// side in `cancelled`.
-__global__ void __launch_bounds__(256) persistence_kernel(int nsad, bool min_side, const uint8_t* __restrict__ dual,
-                                                          const float* __restrict__ thr,
-                                                          const int* __restrict__ sad_img,
-                                                          const int* __restrict__ dying,
-                                                          const float* __restrict__ sad_val,
-                                                          const int2* __restrict__ ext_key,
-                                                          int2* __restrict__ pp,
-                                                          uint8_t* __restrict__ cancelled, uint8_t sbit,
-                                                          uint8_t* __restrict__ alive, int* __restrict__ n_cancel,
-                                                          const int4* __restrict__ arc,
-                                                          int2* __restrict__ canc_ends,
-                                                          const int* __restrict__ crit_sad,
-                                                          unsigned long long* __restrict__ ckey,
-                                                          int* __restrict__ cval, ReplayNode* __restrict__ node) {
+// 139-161), both sides of a saddle in one thread, with the saddle's image's
+// orientation and threshold: pp[s] = (paired extremum or -1, persistence
+// bits; -1 for a cycle), alive[d] = 0 for an extremum that a cancelled saddle
+// kills, survive[s] = 1 when neither side cancels the saddle; and the starting
+// links of the thresholded union-find.
+struct PersistArgs {
+  int nsad;
+  int M[2];
+  const uint8_t* dual;
+  const float* thr;
+  const int* sad_img;
+  const int* crit_sad;
+  const float* sval;
+  uint8_t* survive;
+  int* n_cancel;               // [2]
+  const int* dying[2];
+  const int2* key[2];          // (value bits, cell) of each extremum
+  int2* pp[2];
+  uint8_t* alive[2];
+  const int4* arc[2];
+  int2* ends[2];               // cancelled saddles' arc ends, compacted
+  unsigned long long* ckey[2];  // and their replay keys and saddles (nullptr: arcs not simplified)
+  int* cval[2];
+  ReplayNode* node[2];
+  int* uf[2];                  // [M + 1]
+};
+
+__global__ void __launch_bounds__(256) persistence_kernel(PersistArgs A) {
   // saddles in list order: every per-saddle access is sequential
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  bool canc = false;
-  int d = -1;
-  float p = -1.0f;
-  if (s < nsad) {
-    d = dying[s];
-    if (d < 0) {
-      d = -1;
-    } else {
-      const int b = sad_img[s];
-      const bool du = dual[b];
-      float sv = sad_val[s], ev = __int_as_float(ext_key[d].x);
-      if (min_side)
-        p = du ? sub_like_host(ev, sv) : sub_like_host(sv, ev);
-      else
-        p = du ? sub_like_host(sv, ev) : sub_like_host(ev, sv);
-      if (p <= thr[b]) {
-        canc = true;
-        atomicOr((unsigned*)(cancelled + (s & ~3)), (unsigned)sbit << (8 * (s & 3)));
-        alive[d] = 0;
+  bool canc[2] = {false, false};
+  int d[2] = {-1, -1};
+  float p[2] = {-1.0f, -1.0f};
+#pragma unroll
+  for (int sd = 0; sd < 2; ++sd)
+    if (s <= A.M[sd]) A.uf[sd][s] = s;
+  if (s < A.nsad) {
+    const int b = A.sad_img[s];
+    const bool du = A.dual[b];
+    const float sv = A.sval[s], thr = A.thr[b];
+#pragma unroll
+    for (int sd = 0; sd < 2; ++sd) d[sd] = A.dying[sd][s];
+    float ev[2];
+#pragma unroll
+    for (int sd = 0; sd < 2; ++sd) ev[sd] = d[sd] >= 0 ? __int_as_float(A.key[sd][d[sd]].x) : 0.f;
+#pragma unroll
+    for (int sd = 0; sd < 2; ++sd) {
+      if (d[sd] >= 0) {
+        // saddle - extremum on the vertex side in the primal and on the face
+        // side in the dual, extremum - saddle otherwise
+        p[sd] = (sd == 1) != du ? sub_like_host(sv, ev[sd]) : sub_like_host(ev[sd], sv);
+        canc[sd] = p[sd] <= thr;
+        if (canc[sd]) A.alive[sd][d[sd]] = 0;
       }
+      A.pp[sd][s] = make_int2(d[sd], __float_as_int(p[sd]));
     }
-    pp[s] = make_int2(d, __float_as_int(p));
+    A.survive[s] = !(canc[0] || canc[1]);
   }
   // cancelled edges' ends, compacted for the thresholded union-find, and (when
   // the side's arcs are simplified) the same cancellations with their replay
   // keys (CancelEvent::operator<, cpu/persistence_struct.hxx:16-21):
   // (persistence, saddle cell); a saddle is cancelled at most once per side,
   // so the pair is unique and the target cell never breaks a tie
-  const int slot = block_append(n_cancel, canc);
-  if (canc) {
-    const int4 a = arc[s];
-    canc_ends[slot] = make_int2(a.x, a.y);
-    if (ckey) {
-      const unsigned long long key = ((unsigned long long)orderable_key(p) << 32) | (unsigned)crit_sad[s];
-      ckey[slot] = key;
-      cval[slot] = s;
-      // the killed extremum's replay record: its cancellation key, undecided
-      // (the other records are never read, see replay.cuh)
-      node[d].ctime = key;
-      node[d].status = kPending;
-    }
+  int slot[2];
+  block_reserve2(A.n_cancel, canc[0], A.n_cancel + 1, canc[1], slot[0], slot[1]);
+#pragma unroll
+  for (int sd = 0; sd < 2; ++sd) {
+    if (!canc[sd]) continue;
+    const int4 a = A.arc[sd][s];
+    A.ends[sd][slot[sd]] = make_int2(a.x, a.y);
+    if (!A.ckey[sd]) continue;
+    const unsigned long long key = ((unsigned long long)orderable_key(p[sd]) << 32) | (unsigned)A.crit_sad[s];
+    A.ckey[sd][slot[sd]] = key;
+    A.cval[sd][slot[sd]] = s;
+    // the killed extremum's replay record: its cancellation key, undecided
+    // (the other records are never read, see replay.cuh)
+    A.node[sd][d[sd]].ctime = key;
+    A.node[sd][d[sd]].status = kPending;
   }
 }
-
 
 // Thresholded union-find (the reference's uf_min / uf_max, persistence.hxx:
 // 90-104, 147-161): lock-free union of the ends of every cancelled saddle
@@ -628,10 +640,23 @@ __global__ void __launch_bounds__(256) persistence_kernel(int nsad, bool min_sid
 // cancelled edges written by persistence_kernel. Every link points to a
 // smaller index, so a root search takes at most n steps and every failed CAS
 // means another thread linked one of the two roots (at most n - 1 links
-// exist); both loops are capped at `cap` anyway, and a cap sets
+// exist); both loops are capped at the node count anyway, and a cap sets
 // kStatusFindCap and returns the node reached (a valid index). One edge per
 // thread: advancing 4 edges' searches in lockstep measured slower here (the
 // forest is deep while the unions run, and a thread waits for its longest).
+// Both sides in one launch (blockIdx.y).
+struct UtArgs {
+  int M[2];                  // the void is node M
+  const int2* ends[2];
+  const int* count;          // [2] cancelled edges
+  int* p[2];                 // [M + 1] links
+  const uint8_t* alive[2];
+  int* comp_root[2];         // [M + 1] alive member of each root's component, -1 for the void's
+  const int* rank[2];        // [M] alive extrema before each extremum
+  int* rout[2];              // [M] rank of each extremum's thresholded root, -1 for the void
+  unsigned* status;
+};
+
 __device__ __forceinline__ int uf_root(int* p, int x, int cap, unsigned* status) {
   for (int k = 0;; ++k) {
     int px = p[x];
@@ -646,21 +671,22 @@ __device__ __forceinline__ int uf_root(int* p, int x, int cap, unsigned* status)
   }
 }
 
-__global__ void __launch_bounds__(256) ut_union_kernel(const int2* __restrict__ ends, const int* __restrict__ count,
-                                                       int void_id, int* __restrict__ p, int cap,
-                                                       unsigned* status) {
-  const int n = *count;
+__global__ void __launch_bounds__(256) ut_union_kernel(UtArgs A) {
+  const bool s1 = blockIdx.y != 0;
+  const int2* __restrict__ ends = s1 ? A.ends[1] : A.ends[0];
+  int* p = s1 ? A.p[1] : A.p[0];
+  const int void_id = s1 ? A.M[1] : A.M[0], cap = void_id + 2, n = A.count[s1];
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
     const int2 e = ends[q];
     int a = e.x < 0 ? void_id : e.x;
     int b = e.y < 0 ? void_id : e.y;
     for (int tries = 0;; ++tries) {
       if (tries >= cap) {
-        set_status(status, kStatusFindCap);
+        set_status(A.status, kStatusFindCap);
         break;
       }
-      a = uf_root(p, a, cap, status);
-      b = uf_root(p, b, cap, status);
+      a = uf_root(p, a, cap, A.status);
+      b = uf_root(p, b, cap, A.status);
       if (a == b) break;
       if (a > b) {
         int t = a;
@@ -675,8 +701,14 @@ __global__ void __launch_bounds__(256) ut_union_kernel(const int2* __restrict__ 
 constexpr int kUtBatch = 4;
 
 // Every node's root, kUtBatch nodes per thread with their pointer chains
-// followed in lockstep (a written root is an ancestor for every reader).
-__global__ void ut_flatten_kernel(int n, int* __restrict__ p, int cap, unsigned* status) {
+// followed in lockstep (a written root is an ancestor for every reader), and
+// each component's alive member.
+__global__ void ut_flatten_kernel(UtArgs A) {
+  const bool s1 = blockIdx.y != 0;
+  int* p = s1 ? A.p[1] : A.p[0];
+  const uint8_t* alive = s1 ? A.alive[1] : A.alive[0];
+  int* comp_root = s1 ? A.comp_root[1] : A.comp_root[0];
+  const int M = s1 ? A.M[1] : A.M[0], n = M + 1, cap = M + 2;
   const long long nt = (long long)gridDim.x * blockDim.x;
   const long long x0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   int r[kUtBatch];
@@ -690,7 +722,7 @@ __global__ void ut_flatten_kernel(int n, int* __restrict__ p, int cap, unsigned*
   const unsigned own = live;
   for (int k = 0; live; ++k) {
     if (k >= cap) {
-      set_status(status, kStatusFindCap);
+      set_status(A.status, kStatusFindCap);
       break;
     }
     int pr[kUtBatch];
@@ -703,30 +735,26 @@ __global__ void ut_flatten_kernel(int n, int* __restrict__ p, int cap, unsigned*
     }
   }
 #pragma unroll
-  for (int u = 0; u < kUtBatch; ++u)
-    if ((own >> u) & 1u) p[x0 + nt * u] = r[u];
+  for (int u = 0; u < kUtBatch; ++u) {
+    if (!((own >> u) & 1u)) continue;
+    const int x = (int)(x0 + nt * u);
+    p[x] = r[u];
+    if (x == M)
+      comp_root[r[u]] = -1;
+    else if (alive[x])
+      comp_root[r[u]] = x;
+  }
 }
 
-// Component root = its alive member, or -1 for the void's component.
-__global__ void ut_mark_kernel(int n_ext, const int* __restrict__ p, const uint8_t* __restrict__ alive,
-                               int* __restrict__ comp_root) {
-  int x = blockIdx.x * blockDim.x + threadIdx.x;
-  if (x > n_ext) return;
-  if (x == n_ext)
-    comp_root[p[x]] = -1;
-  else if (alive[x])
-    comp_root[p[x]] = x;
-}
-
-// Out rank of each extremum's thresholded root: the component's alive
-// member (comp_root of its flattened union-find root; -1 for the void's
-// component), which always has an out rank.
-__global__ void root_out_kernel(int n_ext, const int* __restrict__ p, const int* __restrict__ comp_root,
-                                const int* __restrict__ to_out, int* __restrict__ rout) {
-  int x = blockIdx.x * blockDim.x + threadIdx.x;
-  if (x >= n_ext) return;
-  const int u = comp_root[p[x]];
-  rout[x] = u >= 0 ? to_out[u] : -1;
+// Rank of each extremum's thresholded root among the alive extrema: the
+// component's alive member (comp_root of its flattened union-find root; -1
+// for the void's component).
+__global__ void root_out_kernel(UtArgs A) {
+  const bool s1 = blockIdx.y != 0;
+  const int x = blockIdx.x * blockDim.x + threadIdx.x;
+  if (x >= (s1 ? A.M[1] : A.M[0])) return;
+  const int u = (s1 ? A.comp_root[1] : A.comp_root[0])[(s1 ? A.p[1] : A.p[0])[x]];
+  (s1 ? A.rout[1] : A.rout[0])[x] = u >= 0 ? (s1 ? A.rank[1] : A.rank[0])[u] : -1;
 }
 
 }  // namespace dmsc
