@@ -66,6 +66,11 @@ __global__ void survivor_base_kernel(int B, const int* __restrict__ sad_base, in
   }
 }
 
+// Image, global cell and list index of a survivor, in output order.
+struct SurvHead {
+  int img, cell, sad, pad;
+};
+
 // The survivors in list order with their sort keys ((image, s_val) order:
 // the image id above the orderable value, so one sort orders every image;
 // a 32-bit key of the value alone for one image).
@@ -80,45 +85,6 @@ __global__ void survivor_gather_kernel(int nsad, const uint8_t* __restrict__ fla
   idx_out[pos[s]] = s;
 }
 
-// Surviving saddles in the vertex side's sweep order (arcs_topology.hxx:99-102):
-// `sorted` lists them by ascending (image, s_val, cell id); an image whose
-// vertex side sweeps descending (dual) takes its range reversed. Also
-// gathers each survivor's image and cell in output order (`ic`), so the
-// later per-survivor kernels read them in order.
-__global__ void survivor_order_kernel(int n, const int* __restrict__ sorted, const int* __restrict__ sad_img,
-                                      const int* __restrict__ crit_sad, const uint8_t* __restrict__ dual,
-                                      const int* __restrict__ surv_base, int* __restrict__ surv,
-                                      int2* __restrict__ ic) {
-  int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= n) return;
-  const int s = sorted[p], b = sad_img[s];
-  int q = p;
-  if (dual[b]) {
-    const int base = surv_base[b], cnt = surv_base[b + 1] - base;
-    q = base + cnt - 1 - (p - base);
-  }
-  surv[q] = s;
-  ic[q] = make_int2(b, crit_sad[s]);
-}
-
-// Per-survivor records of one side gathered once in output (sweep) order, so
-// the later per-survivor kernels read them in order instead of gathering
-// from the list-ordered saddle arrays again: its arc ends, raw-arc lengths
-// and the record of its outputs (out ranks of its ends' thresholded roots,
-// persistence, out rank of its pair's root; -1 for the void).
-__global__ void surv_side_kernel(int nsurv, const int* __restrict__ surv, const int4* __restrict__ arc,
-                                 const int2* __restrict__ pp, const int* __restrict__ rout, int2* __restrict__ sv_t,
-                                 longlong2* __restrict__ sv_len, int4* __restrict__ sv_rec) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nsurv) return;
-  const int s = surv[i];
-  const int4 a = arc[s];
-  const int2 pr = pp[s];
-  sv_t[i] = make_int2(a.x, a.y);
-  sv_len[i] = make_longlong2(a.z, a.w);
-  sv_rec[i] = make_int4(a.x >= 0 ? rout[a.x] : -1, a.y >= 0 ? rout[a.y] : -1, pr.y, pr.x >= 0 ? rout[pr.x] : -1);
-}
-
 // Per-image first positions (B + 1 entries, the last one the total):
 // base[b] = excl[first[b]] where first[] are the image's first items.
 __global__ void image_base_kernel(int B, const int* __restrict__ first, int n_items, const int* __restrict__ excl,
@@ -129,23 +95,49 @@ __global__ void image_base_kernel(int B, const int* __restrict__ first, int n_it
   base[b] = f < n_items ? excl[f] : total;
 }
 
-// The same with the total read from the device.
-__global__ void image_base_dev_kernel(int B, const int* __restrict__ first, int n_items, const int* __restrict__ excl,
-                                      const long long* __restrict__ total, int* __restrict__ base) {
-  int b = blockIdx.x * blockDim.x + threadIdx.x;
+// First rank of each image's alive extrema on both sides (B + 1 entries, the
+// last one the side's total), from the scan over both sides' flags.
+__global__ void alive_base_kernel(int B, int M0, int M1, const int* __restrict__ first0, const int* __restrict__ first1,
+                                  const int* __restrict__ rank, const uint8_t* __restrict__ alive,
+                                  int* __restrict__ base0, int* __restrict__ base1) {
+  const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b > B) return;
-  int f = b < B ? first[b] : n_items;
-  base[b] = f < n_items ? excl[f] : (int)*total;
+  const int n = M0 + M1;
+  const int total = n > 0 ? rank[n - 1] + alive[n - 1] : 0;
+  const int f0 = b < B ? first0[b] : M0, f1 = M0 + (b < B ? first1[b] : M1);
+  base0[b] = f0 < n ? rank[f0] : total;
+  base1[b] = f1 < n ? rank[f1] : total;
 }
 
-// The survivor of output position q when an image's survivors are visited in
-// reverse (maxima sweep) or forward (minima sweep) order.
-__device__ __forceinline__ int visit(int q, bool reversed, const int* __restrict__ surv_base, int B, int* b_out) {
-  int b = find_image(surv_base, B, q);
-  *b_out = b;
-  if (!reversed) return q;
-  int base = surv_base[b], n = surv_base[b + 1] - base;
-  return base + n - 1 - (q - base);
+// Two 32-bit counts scanned at once in one 64-bit sum: side 0 in the low half,
+// side 1 in the high half (a total of 2^31 or more fails the call, so no count
+// that is used ever carries).
+__device__ __forceinline__ unsigned long long pack2(unsigned f, unsigned v) { return f | (unsigned long long)v << 32; }
+__device__ __forceinline__ int half_of(unsigned long long p, int sd) { return (int)(unsigned)(sd ? p >> 32 : p); }
+
+// Everything the host reads back for the sizes, straight to the mapped area:
+// the integer bases (first min, saddle, max, survivor, alive ranks and e rows
+// of both sides; B + 1 entries each), the geometry starts of both sides and
+// the status word. Also leaves the e row and geometry starts on the device.
+__global__ void sizes_kernel(int B, const int* __restrict__ surv_base, const unsigned long long* __restrict__ lens,
+                             const unsigned long long* __restrict__ rows, const unsigned long long* __restrict__ total,
+                             int* __restrict__ bases, long long* __restrict__ gbase0, long long* __restrict__ gbase1,
+                             const unsigned* __restrict__ status, int* __restrict__ rb_int,
+                             long long* __restrict__ rb_long, unsigned* __restrict__ rb_status) {
+  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+  if (b > B) return;
+  const int n = B + 1, f = surv_base[b];
+#pragma unroll
+  for (int k = 0; k < 6; ++k) rb_int[k * n + b] = bases[k * n + b];
+#pragma unroll
+  for (int sd = 0; sd < 2; ++sd) {
+    bases[(6 + sd) * n + b] = half_of(rows[f], sd);
+    rb_int[(6 + sd) * n + b] = half_of(rows[f], sd);
+    const long long g = b < B ? (long long)half_of(lens[f], sd) : (long long)total[sd];  // the exact total
+    (sd ? gbase1 : gbase0)[b] = g;
+    rb_long[sd * n + b] = g;
+  }
+  if (b == 0) *rb_status = *status;
 }
 
 // e rows of one survivor (cpu/workspace.hxx:175-195, 197-219) from the out
@@ -167,102 +159,66 @@ __device__ __forceinline__ int erow_ends(int r1, int r2, int* o1, int* o2) {
   return n;
 }
 
-__global__ void erow_count_kernel(int nsurv, bool reversed, const int* __restrict__ surv_base, int B,
-                                  const int4* __restrict__ sv_rec, int* __restrict__ cnt) {
-  int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= nsurv) return;
-  int b;
-  const int i = visit(q, reversed, surv_base, B, &b);
-  const int4 r = sv_rec[i];
-  int a, c;
-  cnt[q] = erow_ends(r.x, r.y, &a, &c);
-}
+// Per-survivor outputs of both sides: the saddle points, persistence, pairs,
+// e rows and the CSR offsets of the arcs (cpu/workspace.hxx:247-287: offsets[0]
+// = 0, offsets[k+1] = end of survivor k, arc_offsets[k] = end of its first
+// arc), all image-local, in the arrays that the image's orientation selects.
+struct SurvSideOut {
+  RouteF p;
+  Route pp, e, off, aoff;
+  const int* alive_base;   // [B + 1]
+  const long long* gbase;  // [B + 1]
+  const int4* out;         // [nsurv] ranks of the ends' roots, persistence bits, rank of the pair's root
+  const int4* arc;         // [nsurv] arc ends and raw-arc lengths
+  const int4* fin;         // [nsurv] chain lengths and roots of the final arcs (nullptr: no arcs)
+};
 
-// Per-survivor scalars and e rows of one side. `row_off` is the batch-wide
-// exclusive scan of the row counts in visiting order; `row_base[b]` its value
-// at image b's first survivor.
-__global__ void side_outputs_kernel(int nsurv, bool reversed, const int* __restrict__ surv_base, Imgs I,
-                                    const int4* __restrict__ sv_rec, const int* __restrict__ alive_base,
-                                    const int* __restrict__ row_off, const int* __restrict__ row_base, RouteF P,
-                                    Route PP, Route E) {
-  int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= nsurv) return;
-  int b;
-  int i = visit(q, reversed, surv_base, I.B, &b);
-  const bool d = I.dual[b];
-  const int li = i - surv_base[b];
-  const int4 r = sv_rec[i];
-  if (float* p = P.at(d, b)) p[li] = __int_as_float(r.z);
-  if (int* pp = PP.at(d, b)) pp[li] = r.w >= 0 ? r.w - alive_base[b] : -1;
-  if (int* e = E.at(d, b)) {
-    int a = 0, c = 0;
-    int n = erow_ends(r.x, r.y, &a, &c);
-    int o = row_off[q] - row_base[b];
-    if (n >= 1) {
-      e[2 * o] = li;
-      e[2 * o + 1] = a - alive_base[b];
-    }
-    if (n == 2) {
-      e[2 * o + 2] = li;
-      e[2 * o + 3] = c - alive_base[b];
-    }
-  }
-}
-
-__global__ void sad_pts_kernel(int nsurv, const int2* __restrict__ surv_ic, const int* __restrict__ surv_base, Imgs I,
-                               int* __restrict__ out, const int* __restrict__ out_off) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nsurv) return;
-  const int2 ic = surv_ic[i];
-  const int b = ic.x;
-  out[out_off[b] + (i - surv_base[b])] = ic.y - 4 * I.idx_base[b];
-}
-
-// Geometry start of every image on one side (B + 1 entries).
-__global__ void geom_base_kernel(int B, const int* __restrict__ surv_base, int nsurv,
-                                 const long long* __restrict__ saddle_end_incl, const long long* __restrict__ plen,
-                                 const long long* __restrict__ total, long long* __restrict__ gbase) {
-  int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b > B) return;
-  int f = b < B ? surv_base[b] : nsurv;
-  gbase[b] = f < nsurv ? saddle_end_incl[f] - plen[f] : *total;
-}
-
-// Image-local output position of every arc (its start inside its image's
-// geometry of this side), for the geometry expansion and writer.
-__global__ void arc_pos_kernel(int nsurv, const long long* __restrict__ arc_len,
-                               const long long* __restrict__ saddle_end_incl, const int2* __restrict__ surv_ic,
-                               const long long* __restrict__ gbase, long long* __restrict__ arc_pos) {
+__global__ void __launch_bounds__(256) survivor_outputs_kernel(int nsurv, Imgs I, const int* __restrict__ surv_base,
+                                                               const SurvHead* __restrict__ head,
+                                                               const unsigned long long* __restrict__ lens,
+                                                               const unsigned long long* __restrict__ rows,
+                                                               int* __restrict__ sad_pts, SurvSideOut F,
+                                                               SurvSideOut V) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nsurv) return;
-  const longlong2 al = *reinterpret_cast<const longlong2*>(arc_len + 2 * i);
-  const long long start = saddle_end_incl[i] - gbase[surv_ic[i].x] - al.x - al.y;
-  *reinterpret_cast<longlong2*>(arc_pos + 2 * i) = make_longlong2(start, start + al.x);
-}
-
-// CSR offsets of one side's arcs, per image (cpu/workspace.hxx:247-287):
-// offsets[0] = 0, offsets[k+1] = end of survivor k, arc_offsets[k] = end of
-// its first arc, image-local. `off_off[b]` / `arc_off[b]` place image b's
-// block (n_b + 1 and n_b entries) in the routed arrays.
-__global__ void arc_offsets_kernel(int nsurv, int B, const int* __restrict__ surv_base, const uint8_t* __restrict__ dual,
-                                   const long long* __restrict__ arc_len,
-                                   const long long* __restrict__ saddle_end_incl, const long long* __restrict__ gbase,
-                                   Route OFF, Route AOFF) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nsurv + B) return;
-  if (i >= nsurv) {  // one leading zero per image
-    int b = i - nsurv;
-    if (int* o = OFF.at(dual[b], b)) o[0] = 0;
-    return;
+  if (i < I.B) {  // one leading zero per image
+#pragma unroll
+    for (int sd = 0; sd < 2; ++sd)
+      if (int* o = (sd ? V : F).off.at(I.dual[i], i)) o[0] = 0;
   }
-  int b = find_image(surv_base, B, i);
-  const bool d = dual[b];
-  const longlong2 al = *reinterpret_cast<const longlong2*>(arc_len + 2 * i);
-  long long end = saddle_end_incl[i] - gbase[b];
-  long long start = end - al.x - al.y;
-  int li = i - surv_base[b];
-  if (int* o = OFF.at(d, b)) o[li + 1] = (int)end;
-  if (int* a = AOFF.at(d, b)) a[li] = (int)(start + al.x);
+  if (i >= nsurv) return;
+  const int2 ic = *reinterpret_cast<const int2*>(head + i);
+  const int b = ic.x;
+  const bool d = I.dual[b];
+  const int first = surv_base[b], last = surv_base[b + 1], li = i - first;
+  if (sad_pts) sad_pts[i] = ic.y - 4 * I.idx_base[b];
+  const unsigned long long r0 = rows[i], r1 = rows[i + 1];
+#pragma unroll
+  for (int sd = 0; sd < 2; ++sd) {
+    const SurvSideOut& S = sd ? V : F;
+    const int4 r = S.out[i];
+    const int ab = S.alive_base[b];
+    if (float* p = S.p.at(d, b)) p[li] = __int_as_float(r.z);
+    if (int* pp = S.pp.at(d, b)) pp[li] = r.w >= 0 ? r.w - ab : -1;
+    if (int* e = S.e.at(d, b)) {
+      int x = 0, y = 0;
+      const int n = erow_ends(r.x, r.y, &x, &y);
+      // the vertex side's rows follow the minima sweep (this order), the face
+      // side's the maxima sweep, its reverse
+      const int o = sd ? half_of(r0, 1) - half_of(rows[first], 1) : half_of(rows[last], 0) - half_of(r1, 0);
+      if (n >= 1) {
+        e[2 * o] = li;
+        e[2 * o + 1] = x - ab;
+      }
+      if (n == 2) {
+        e[2 * o + 2] = li;
+        e[2 * o + 3] = y - ab;
+      }
+    }
+    if (!S.fin) continue;
+    const int g = (int)S.gbase[b];
+    if (int* o = S.off.at(d, b)) o[li + 1] = half_of(lens[i + 1], sd) - g;
+    if (int* a = S.aoff.at(d, b)) a[li] = half_of(lens[i], sd) - g + S.arc[i].z + S.fin[i].x;
+  }
 }
 
 }  // namespace dmsc

@@ -41,14 +41,15 @@ namespace {
 enum Slot {
   S_MASK, S_FLOW, S_SEG0, S_SEG1, S_SEG2, S_OFF0, S_OFF1, S_OFF2, S_TOT, S_TAB, S_BASES,
   S_CSAD, S_IMIN, S_ISAD, S_IMAX, S_MINBITS, S_MAXBITS, S_KMIN, S_KMAX, S_SVAL, S_SKEY2, S_IOTA,
-  S_ASC, S_ARCF, S_ARCV, S_ALIVE, S_RANK, S_FLAG, S_FPOS, S_SURV, S_STATUS, S_NCANC, S_STATS, S_TIMELINE, S_ROUTE,
-  S_BKEY, S_BIDX, S_BKEY2, S_BIDX2, S_PERF, S_PERV, S_EXF, S_EXV, S_NEX, S_SKEY32B, S_SKEYS, S_SURVIC,
+  S_ASC, S_ARC, S_ALIVE, S_RANK, S_FLAG, S_FPOS, S_STATUS, S_NCANC, S_STATS, S_TIMELINE, S_ROUTE,
+  S_BKEY, S_BIDX, S_BKEY2, S_BIDX2, S_PERF, S_PERV, S_EXF, S_EXV, S_NEX, S_SKEY32B, S_SKEYS,
+  S_SHEAD, S_LENS, S_ROWS, S_PP,
   S_SIDE0,  // per-side slots start here, kSideSlots each
 };
 enum SideSlot {
-  X_ROUT, X_SVT, X_SVL, X_SVR, X_DYING, X_GRP, X_LINK, X_MINE, X_ACT0, X_ACT1, X_CNT, X_PAIR,
+  X_ROUT, X_DYING, X_GRP, X_LINK, X_MINE, X_ACT0, X_ACT1, X_CNT,
   X_UF, X_CROOT, X_CKEY, X_CVAL, X_NODE,
-  X_ALEN, X_ACL, X_AROOT, X_PLEN, X_SEND, X_APOS, X_EROWC, X_EROWO, X_Q0, X_Q1, X_QB, X_G12,
+  X_SARC, X_SOUT, X_SFIN, X_Q0, X_Q1, X_QB, X_G12,
   X_GBASE, X_WX, X_WA, X_CENDS, X_SOLO, kSideSlots
 };
 
@@ -76,27 +77,19 @@ struct Side {
   bool groups_primal = false, groups_dual = false;
   int* ext_img = nullptr;
   const int2* key = nullptr;  // (value bits, global cell id) per extremum, list order
-  int4* arc = nullptr;              // [nsad] per saddle (list order): arc ends and raw-arc cells
+  const int4* arc = nullptr;        // per saddle (list order, every second record): arc ends and raw-arc cells
   int* rout = nullptr;              // [M] out rank of each extremum's thresholded root (-1: the void)
-  int2* sv_t = nullptr;             // [nsurv] per survivor (output order): arc ends
-  longlong2* sv_len = nullptr;      // raw-arc lengths
-  int4* sv_rec = nullptr;           // out ranks of the ends' roots, persistence, out rank of the pair's root
   int* dying = nullptr;
-  int2* pp = nullptr;               // [nsad] paired extremum (-1: none) and persistence bits
+  const int2* pp = nullptr;         // paired extremum (-1: none) and persistence bits of each saddle (every second)
   uint8_t* alive = nullptr;
   int* to_out_excl = nullptr;   // [M] alive extrema before each (over both sides' lists)
   ReplayState R{};
   int C = 0;
-  long long* arc_len = nullptr;
-  long long* arc_cl = nullptr;
-  int* arc_root = nullptr;
-  long long* send = nullptr;
-  long long* plen = nullptr;
+  int4* s_arc = nullptr;       // [nsurv] per survivor (output order): arc ends and raw-arc lengths
+  int4* s_out = nullptr;       // [nsurv] ranks of the ends' roots, persistence bits, rank of the pair's root
+  int4* s_fin = nullptr;       // [nsurv] chain lengths and roots of the final arcs
   long long* gbase = nullptr;  // [B+1] geometry start of each image
   long long total = 0;
-  int n_alive = 0;
-  int n_erows = 0;
-  int* erow_off = nullptr;
 };
 
 }  // namespace
@@ -126,8 +119,9 @@ struct dmsc_b200_context {
   const float* img = nullptr;  // input of the last extract (read again by fetch_pair_pixels)
   int* crit_sad = nullptr;
   int* sad_img = nullptr;
-  int* surv = nullptr;
-  int2* surv_ic = nullptr;  // [nsurv] image and cell of each survivor (output order)
+  SurvHead* head = nullptr;  // [nsurv] image, cell and list index of each survivor (output order)
+  unsigned long long* lens = nullptr;  // [nsurv + 1] where its geometry starts (both sides packed)
+  unsigned long long* rows = nullptr;  // [nsurv + 1] and its e rows
   unsigned* status = nullptr;
   Side side[2];
   std::vector<dmsc_b200_sizes> sizes;
@@ -195,25 +189,6 @@ __global__ void totals3_kernel(const int* o0, const int* s0, const int* o1, cons
   out[0] = (long long)o0[n - 1] + s0[n - 1];
   out[1] = (long long)o1[n - 1] + s1[n - 1];
   out[2] = (long long)o2[n - 1] + s2[n - 1];
-}
-
-template <class T>
-__global__ void last_plus_kernel(const T* excl, const T* val, int n, long long* out) {
-  *out = n > 0 ? (long long)excl[n - 1] + (long long)val[n - 1] : 0;
-}
-
-__global__ void copy2_kernel(const int* a, long long* out) {
-  out[0] = a[0];
-  out[1] = a[1];
-}
-
-template <class T>
-__global__ void last_kernel(const T* a, int n, long long* out) {
-  *out = n > 0 ? (long long)a[n - 1] : 0;
-}
-
-__global__ void u8_last_plus_kernel(const int* excl, const uint8_t* v, int n, long long* out) {
-  *out = n > 0 ? (long long)excl[n - 1] + v[n - 1] : 0;
 }
 
 // 32-bit words from device memory into the mapped readback area.
@@ -551,6 +526,8 @@ void finish_pairing(dmsc_b200_context* ctx, uint8_t* survive, int* pos, cudaStre
   P.sval = get<float>(ctx, S_SVAL, nsad);
   P.survive = survive;
   P.n_cancel = get<int>(ctx, S_NCANC, 4);
+  P.pp = get<int4>(ctx, S_PP, nsad);
+  P.arc = ctx->side[0].arc;
   U.count = P.n_cancel;
   U.status = ctx->status;
   const int Mf = ctx->side[0].M, Mv = ctx->side[1].M, most = std::max(Mf, Mv) + 1;
@@ -560,16 +537,14 @@ void finish_pairing(dmsc_b200_context* ctx, uint8_t* survive, int* pos, cudaStre
   int* rank = get<int>(ctx, S_RANK, (size_t)Mf + Mv);
   for (int si = 0; si < 2; ++si) {
     Side& S = ctx->side[si];
-    S.pp = sget<int2>(ctx, si, X_PAIR, nsad);
+    S.pp = (const int2*)P.pp + si;
     S.alive = alive + (si ? Mf : 0);
     S.to_out_excl = rank + (si ? Mf : 0);
     S.rout = sget<int>(ctx, si, X_ROUT, S.M + 1);
     P.M[si] = U.M[si] = S.M;
     P.dying[si] = S.dying;
     P.key[si] = S.key;
-    P.pp[si] = S.pp;
     P.alive[si] = S.alive;
-    P.arc[si] = S.arc;
     P.ends[si] = sget<int2>(ctx, si, X_CENDS, nsad);
     // the replay's cancellation list (keys and saddles) comes out of the same
     // pass when this side's arcs are simplified
@@ -627,20 +602,38 @@ ReplayArgs replay_prepare(dmsc_b200_context* ctx, int si, Side& S, cudaStream_t 
   return A;
 }
 
-// Final arcs of one side's survivors after the replay: lengths, chain roots
-// and the side's geometry total (device, into *total).
-void replay_final(dmsc_b200_context* ctx, int si, Side& S, long long* total, cudaStream_t st) {
+// The survivors in output order with their final arcs (after the replay and
+// the sort, `sorted`), and the scans of their geometry cells and e rows; the
+// exact geometry totals stay on the device (read back with the sizes).
+void replay_final(dmsc_b200_context* ctx, const int* sorted, unsigned long long* total, cudaStream_t st) {
   const int nsurv = ctx->nsurv;
-  S.arc_len = sget<long long>(ctx, si, X_ALEN, 2 * (size_t)nsurv);
-  S.arc_cl = sget<long long>(ctx, si, X_ACL, 2 * (size_t)nsurv);
-  S.arc_root = sget<int>(ctx, si, X_AROOT, 2 * (size_t)nsurv);
-  S.plen = sget<long long>(ctx, si, X_PLEN, nsurv);
-  S.send = sget<long long>(ctx, si, X_SEND, nsurv);
-  LK(final_arcs_kernel<<<grid_for(nsurv, TB), TB, 0, st>>>(nsurv, ctx->surv_ic, ctx->I.dual, S.arcs_primal,
-                                                           S.arcs_dual, S.sv_t, S.sv_len, S.alive, S.R, ctx->nsad + 1,
-                                                           S.arc_len, S.arc_cl, S.arc_root, S.plen, ctx->status));
-  incl_sum(ctx, S.plen, S.send, nsurv, st);
-  LK(last_kernel<long long><<<1, 1, 0, st>>>(S.send, nsurv, total));
+  ctx->head = get<SurvHead>(ctx, S_SHEAD, nsurv);
+  ctx->lens = get<unsigned long long>(ctx, S_LENS, (size_t)nsurv + 1);
+  ctx->rows = get<unsigned long long>(ctx, S_ROWS, (size_t)nsurv + 1);
+  FinalSide A[2] = {};
+  for (int si = 0; si < 2; ++si) {
+    Side& S = ctx->side[si];
+    S.s_out = sget<int4>(ctx, si, X_SOUT, nsurv);
+    S.s_arc = S.arcs ? sget<int4>(ctx, si, X_SARC, nsurv) : nullptr;
+    S.s_fin = S.arcs ? sget<int4>(ctx, si, X_SFIN, nsurv) : nullptr;
+    FinalSide& P = A[si];
+    P.arc = ctx->side[0].arc;
+    P.pp = ctx->side[0].pp;
+    P.rout = S.rout;
+    P.s_arc = S.s_arc;
+    P.s_out = S.s_out;
+    P.s_fin = S.s_fin;
+    P.alive = S.alive;
+    P.S = S.R;
+    P.primal = S.arcs_primal;
+    P.dual = S.arcs_dual;
+  }
+  CK(cudaMemsetAsync(total, 0, 2 * sizeof(unsigned long long), st));
+  LK(survivor_final_kernel<<<grid_for(2 * (nsurv + 1LL), TB), TB, 0, st>>>(
+      nsurv, sorted, ctx->B, ctx->sad_img, ctx->crit_sad, ctx->I.dual, ctx->bases.surv, A[0], A[1], ctx->nsad + 1,
+      ctx->head, ctx->lens, ctx->rows, total, ctx->status));
+  excl_sum(ctx, ctx->lens, ctx->lens, nsurv + 1, st);
+  excl_sum(ctx, ctx->rows, ctx->rows, nsurv + 1, st);
   LAUNCH_CHECK("final arcs");
 }
 
@@ -952,7 +945,7 @@ int extract_batch_impl(dmsc_b200_context* ctx, int B, const float* img, const in
       I, img, nseg, flow, off[0], off[1], off[2], csad, imin, isad, imax, bmin, bmax, kmin, kmax, sval, ps));
   LAUNCH_CHECK("compact_kernel");
   // per-image bases of the critical lists (B + 1 entries each)
-  int* bases = get<int>(ctx, S_BASES, 9 * (size_t)(B + 1));
+  int* bases = get<int>(ctx, S_BASES, 8 * (size_t)(B + 1));
   Bases& BS = ctx->bases;
   BS.min = bases;
   BS.sad = bases + (B + 1);
@@ -970,11 +963,10 @@ int extract_batch_impl(dmsc_b200_context* ctx, int B, const float* img, const in
 
   // ---- K4 saddle walks ----
   // per saddle and side: arc ends and raw-arc lengths (cells)
-  int4* arc_f = get<int4>(ctx, S_ARCF, nsad);
-  int4* arc_v = get<int4>(ctx, S_ARCV, nsad);
+  int4* arc = get<int4>(ctx, S_ARC, 2 * (size_t)nsad);
   if (nsad > 0) {
     LK(saddle_walk_kernel<<<grid_for(nsad, TB), TB, 0, st>>>(I, flow, nsad, csad, isad, off[2], bmax, off[0], bmin,
-                                                             arc_f, arc_v, ncells, ps, ctx->status));
+                                                             arc, ncells, ps, ctx->status));
     LAUNCH_CHECK("saddle_walk_kernel");
   }
 
@@ -991,8 +983,8 @@ int extract_batch_impl(dmsc_b200_context* ctx, int B, const float* img, const in
   V.ext_img = imin;
   F.key = kmax;
   V.key = kmin;
-  F.arc = arc_f;
-  V.arc = arc_v;
+  F.arc = arc;
+  V.arc = arc + 1;
   // faces: ridges/peaks in the primal, valleys/basins in the dual (workspace.hxx:322-362)
   F.arcs_primal = f_ridges;
   F.arcs_dual = f_valleys;
@@ -1026,7 +1018,6 @@ int extract_batch_impl(dmsc_b200_context* ctx, int B, const float* img, const in
   mark(ctx, 6, st);
 
   // ---- surviving saddles in minima-sweep (vertex side) order ----
-  ctx->surv = get<int>(ctx, S_SURV, nsad);
   // the status word rides along: a capped pairing or union-find loop ends the
   // call here, before the replay
   rb_reserve(ctx, 4 * sizeof(long long));
@@ -1039,8 +1030,8 @@ int extract_batch_impl(dmsc_b200_context* ctx, int B, const float* img, const in
   F.C = (int)rb_ll(ctx)[1];
   V.C = (int)rb_ll(ctx)[2];
   const int nsurv = ctx->nsurv;
-  // the survivor order and records run on side_st, overlapping the replay
-  // and the labels (neither reads them); the final arcs wait for them
+  // the survivors' sort runs on side_st, overlapping the replay and the
+  // labels (neither reads it); the final arcs wait for it
   cudaStream_t ss = ctx->side_st;
   CK(cudaEventRecord(ctx->fork_ev, st));
   mark(ctx, 7, st);
@@ -1066,54 +1057,35 @@ int extract_batch_impl(dmsc_b200_context* ctx, int B, const float* img, const in
   // the survivors' side-stream work is enqueued after the replay's launch,
   // so the device starts the replay while the host sets up the sort
   CK(cudaStreamWaitEvent(ss, ctx->fork_ev, 0));
+  int* sorted = get<int>(ctx, S_ASC, nsurv);
   if (nsurv > 0) {
     // the survivors (list order) sorted by (image, s_val) with the list index
     // as the stable tie-break, then each image's range in its vertex-side
     // sweep direction (reversed for a dual image)
     int* sidx = get<int>(ctx, S_IOTA, nsurv);
-    int* sorted = get<int>(ctx, S_ASC, nsurv);
     if (B > 1) {
       unsigned long long* k = get<unsigned long long>(ctx, S_SKEY2, nsurv);
-      LK(survivor_gather_kernel<unsigned long long><<<grid_for(nsad, TB), TB, 0, ss>>>(
-          nsad, flag, fpos, get<float>(ctx, S_SVAL, nsad), ctx->sad_img, k, sidx));
+      LK(survivor_gather_kernel<unsigned long long><<<grid_for(nsad, TB), TB, 0, ss>>>(nsad, flag, fpos, sval, isad, k,
+                                                                                       sidx));
       sort_pairs(ctx, k, get<unsigned long long>(ctx, S_SKEYS, nsurv), sidx, sorted, nsurv, ss, 32 + bits_for(B));
     } else {
       uint32_t* k = get<uint32_t>(ctx, S_SKEY32B, nsurv);
-      LK(survivor_gather_kernel<uint32_t><<<grid_for(nsad, TB), TB, 0, ss>>>(
-          nsad, flag, fpos, get<float>(ctx, S_SVAL, nsad), ctx->sad_img, k, sidx));
+      LK(survivor_gather_kernel<uint32_t><<<grid_for(nsad, TB), TB, 0, ss>>>(nsad, flag, fpos, sval, isad, k, sidx));
       sort_pairs(ctx, k, get<uint32_t>(ctx, S_SKEYS, nsurv), sidx, sorted, nsurv, ss, 32);
     }
-    // the survivors in output order, with their records gathered once
-    ctx->surv_ic = get<int2>(ctx, S_SURVIC, nsurv);
-    LK(survivor_order_kernel<<<grid_for(nsurv, TB), TB, 0, ss>>>(nsurv, sorted, ctx->sad_img, ctx->crit_sad, I.dual,
-                                                               BS.surv, ctx->surv, ctx->surv_ic));
     LAUNCH_CHECK("survivor order");
-    for (int si = 0; si < 2; ++si) {
-      Side& S = ctx->side[si];
-      S.sv_t = sget<int2>(ctx, si, X_SVT, nsurv);
-      S.sv_len = sget<longlong2>(ctx, si, X_SVL, nsurv);
-      S.sv_rec = sget<int4>(ctx, si, X_SVR, nsurv);
-      LK(surv_side_kernel<<<grid_for(nsurv, TB), TB, 0, ss>>>(nsurv, ctx->surv, S.arc, S.pp,
-                                                            S.rout, S.sv_t, S.sv_len, S.sv_rec));
-    }
-    LAUNCH_CHECK("survivor records");
   }
   CK(cudaEventRecord(ctx->join_ev, ss));
 
   // ---- labels (region id = rank among the image's alive extrema) ----
+  // alive bases first (needed by the labels and the outputs)
+  LK(alive_base_kernel<<<grid_for(B + 1LL, TB), TB, 0, st>>>(B, nmax, nmin, BS.max, BS.min, F.to_out_excl, F.alive,
+                                                            BS.alive[0], BS.alive[1]));
+  LAUNCH_CHECK("alive bases");
   LabelOut OF{}, OV{};
   LabelSide LF{}, LV{};
   for (int si = 0; si < 2; ++si) {
     Side& S = ctx->side[si];
-    // alive bases first (needed by the labels and the outputs)
-    long long* at = get<long long>(ctx, S_TOT, 8) + 4 + si;
-    if (S.M > 0)
-      LK(u8_last_plus_kernel<<<1, 1, 0, st>>>(S.to_out_excl, S.alive, S.M, at));
-    else
-      CK(cudaMemsetAsync(at, 0, sizeof(long long), st));
-    LK(image_base_dev_kernel<<<grid_for(B + 1LL, TB), TB, 0, st>>>(B, S.faces ? BS.max : BS.min, S.M, S.to_out_excl,
-                                                                   at, BS.alive[si]));
-    LAUNCH_CHECK("alive bases");
     if (!S.groups) continue;
     LabelOut& O = S.faces ? OF : OV;
     if (S.faces) {
@@ -1168,52 +1140,23 @@ int extract_batch_impl(dmsc_b200_context* ctx, int B, const float* img, const in
 
   // ---- final arc lengths (after the survivor records on side_st) ----
   CK(cudaStreamWaitEvent(st, ctx->join_ev, 0));
-  {
-    // geometry totals stay on the device (read back with the sizes)
-    long long* tot = get<long long>(ctx, S_TOT, 8);
-    CK(cudaMemsetAsync(tot, 0, 2 * sizeof(long long), st));
-    for (int si = 0; si < 2; ++si) {
-      Side& S = ctx->side[si];
-      S.gbase = sget<long long>(ctx, si, X_GBASE, B + 1);
-      S.total = 0;
-      if (S.arcs && nsad > 0) {
-        if (nsurv > 0) replay_final(ctx, si, S, tot + si, st);
-        LK(geom_base_kernel<<<grid_for(B + 1LL, TB), TB, 0, st>>>(B, BS.surv, nsurv, S.send, S.plen, tot + si,
-                                                                  S.gbase));
-        LAUNCH_CHECK("geom_base_kernel");
-      } else {
-        CK(cudaMemsetAsync(S.gbase, 0, (B + 1) * sizeof(long long), st));
-      }
-    }
-    mark(ctx, 9, st);
-  }
-
-  // ---- e rows ----
   for (int si = 0; si < 2; ++si) {
-    Side& S = ctx->side[si];
-    int* ec = sget<int>(ctx, si, X_EROWC, nsurv);
-    S.erow_off = sget<int>(ctx, si, X_EROWO, nsurv);
-    long long* et = get<long long>(ctx, S_TOT, 8) + 6 + si;
-    if (nsurv > 0) {
-      LK(erow_count_kernel<<<grid_for(nsurv, TB), TB, 0, st>>>(nsurv, S.faces, BS.surv, B, S.sv_rec, ec));
-      excl_sum(ctx, ec, S.erow_off, nsurv, st);
-      LK(last_plus_kernel<int><<<1, 1, 0, st>>>(S.erow_off, ec, nsurv, et));
-    } else {
-      CK(cudaMemsetAsync(et, 0, sizeof(long long), st));
-    }
-    LK(image_base_dev_kernel<<<grid_for(B + 1LL, TB), TB, 0, st>>>(B, BS.surv, nsurv, S.erow_off, et, BS.erow[si]));
-    LAUNCH_CHECK("e rows");
+    ctx->side[si].gbase = sget<long long>(ctx, si, X_GBASE, B + 1);
+    ctx->side[si].total = 0;
   }
+  unsigned long long* total = get<unsigned long long>(ctx, S_TOT, 8) + 4;
+  replay_final(ctx, sorted, total, st);
+  mark(ctx, 9, st);
 
   // ---- per-image sizes: one read of the bases ----
   {
     // int bases, then (8-byte aligned) the two geometry bases, then the status word
-    size_t ib = (9 * (size_t)(B + 1) * sizeof(int) + 7) & ~(size_t)7, lb = 2 * (size_t)(B + 1) * sizeof(long long);
+    size_t ib = (8 * (size_t)(B + 1) * sizeof(int) + 7) & ~(size_t)7, lb = 2 * (size_t)(B + 1) * sizeof(long long);
     rb_reserve(ctx, ib + lb + 64);
-    rb_copy(ctx, st, 0, bases, 9 * (size_t)(B + 1) * sizeof(int));
-    rb_copy(ctx, st, ib, F.gbase, (B + 1) * sizeof(long long));
-    rb_copy(ctx, st, ib + (B + 1) * sizeof(long long), V.gbase, (B + 1) * sizeof(long long));
-    rb_copy(ctx, st, ib + lb, ctx->status, sizeof(unsigned));
+    LK(sizes_kernel<<<grid_for(B + 1LL, TB), TB, 0, st>>>(
+        B, BS.surv, ctx->lens, ctx->rows, total, bases, F.gbase, V.gbase, ctx->status, (int*)ctx->rb_d, (long long*)(ctx->rb_d + ib),
+        (unsigned*)(ctx->rb_d + ib + lb)));
+    LAUNCH_CHECK("sizes_kernel");
     wait_stream(ctx, st);
     mark(ctx, 11, st);
     const char* h = ctx->rb_h;
@@ -1278,9 +1221,6 @@ void emit_expand(dmsc_b200_context* ctx, int si, Side& S, cudaStream_t st) {
   const int nsurv = ctx->nsurv;
   ctx->expanded[si] = false;
   if (!S.arcs || S.total <= 0 || nsurv <= 0) return;
-  long long* arc_pos = sget<long long>(ctx, si, X_APOS, 2 * (size_t)nsurv);
-  LK(arc_pos_kernel<<<grid_for(nsurv, TB), TB, 0, st>>>(nsurv, S.arc_len, S.send, ctx->surv_ic, S.gbase, arc_pos));
-  LAUNCH_CHECK("arc_pos_kernel");
   const long long cap = S.total;
   EmitArgs& A = ctx->emit[si];
   A = EmitArgs{};
@@ -1294,12 +1234,11 @@ void emit_expand(dmsc_b200_context* ctx, int si, Side& S, cudaStream_t st) {
   E.status = ctx->status;
   A.nsurv = nsurv;
   E.nvirt = 2 * nsurv;
-  E.surv_ic = ctx->surv_ic;
-  E.sv_t = S.sv_t;
-  E.sv_len = S.sv_len;
-  E.arc_pos = arc_pos;
-  A.arc_cl = S.arc_cl;
-  A.arc_root = S.arc_root;
+  E.head = ctx->head;
+  E.arc = S.s_arc;
+  E.fin = S.s_fin;
+  E.lens = ctx->lens;
+  E.gbase = S.gbase;
   A.q0 = sget<int4>(ctx, si, X_Q0, cap);
   A.q1 = sget<int4>(ctx, si, X_Q1, cap);
   A.cnt = sget<int>(ctx, si, X_CNT, 8);
@@ -1313,15 +1252,11 @@ void emit_expand(dmsc_b200_context* ctx, int si, Side& S, cudaStream_t st) {
   ctx->expanded[si] = true;
 }
 
-// Geometry of one side, second half (fetch): the CSR offsets and the writer
-// of every raw-arc segment into the caller's arrays (`dst_off[b]`: image b's
-// start in its destination).
+// Geometry of one side, second half (fetch): the writer of every raw-arc
+// segment into the caller's arrays (`dst_off[b]`: image b's start in its
+// destination).
 void emit_write(dmsc_b200_context* ctx, int si, Side& S, int32_t* flat_primal, int32_t* flat_dual, const int* dst_off,
-                Route OFF, Route AOFF, cudaStream_t st) {
-  const int nsurv = ctx->nsurv, B = ctx->B;
-  LK(arc_offsets_kernel<<<grid_for(nsurv + (long long)B, TB), TB, 0, st>>>(nsurv, B, ctx->bases.surv, ctx->I.dual,
-                                                                           S.arc_len, S.send, S.gbase, OFF, AOFF));
-  LAUNCH_CHECK("arc_offsets_kernel");
+                cudaStream_t st) {
   if (!ctx->expanded[si] || (!flat_primal && !flat_dual)) return;
   EmitArgs& A = ctx->emit[si];
   EmitCtx E = A.E;
@@ -1394,23 +1329,34 @@ int fetch_batch_impl(dmsc_b200_context* ctx, const dmsc_b200_outputs* o, cudaStr
       LK(points_kernel<<<grid_for(S.M, TB), TB, 0, st>>>(S.M, S.alive, S.to_out_excl, ctx->bases.alive[si], S.key,
                                                          S.ext_img, I, R));
   }
-  if (nsurv > 0 && o->sad_pts)
-    LK(sad_pts_kernel<<<grid_for(nsurv, TB), TB, 0, st>>>(nsurv, ctx->surv_ic, ctx->bases.surv, I, o->sad_pts,
-                                                          ctx->bases.surv));
-  LAUNCH_CHECK("point lists");
-  // per-saddle scalars and e rows
-  if (nsurv > 0) {
-    for (int si = 0; si < 2; ++si) {
-      Side& S = ctx->side[si];
-      RouteF P{S.faces ? o->p_max : o->p_min, S.faces ? o->p_min : o->p_max, ctx->bases.surv};
-      Route PP{S.faces ? o->ppairs_max : o->ppairs_min, S.faces ? o->ppairs_min : o->ppairs_max, ctx->bases.surv};
-      Route E{S.faces ? o->e_max : o->e_min, S.faces ? o->e_min : o->e_max, rt_of(si == 0 ? R_E0 : R_E1)};
-      LK(side_outputs_kernel<<<grid_for(nsurv, TB), TB, 0, st>>>(nsurv, S.faces, ctx->bases.surv, I, S.sv_rec,
-                                                                 ctx->bases.alive[si], S.erow_off,
-                                                                 ctx->bases.erow[si], P, PP, E));
-    }
-    LAUNCH_CHECK("side_outputs_kernel");
+  // per-survivor outputs; a side's arcs go to the arrays that some image takes
+  // (faces: ridges in the primal, valleys in the dual)
+  SurvSideOut SO[2];
+  int32_t* geom_out[2][2] = {};
+  for (int si = 0; si < 2; ++si) {
+    Side& S = ctx->side[si];
+    const bool f = S.faces;
+    SurvSideOut& A = SO[si];
+    A.p = RouteF{f ? o->p_max : o->p_min, f ? o->p_min : o->p_max, ctx->bases.surv};
+    A.pp = Route{f ? o->ppairs_max : o->ppairs_min, f ? o->ppairs_min : o->ppairs_max, ctx->bases.surv};
+    A.e = Route{f ? o->e_max : o->e_min, f ? o->e_min : o->e_max, rt_of(si == 0 ? R_E0 : R_E1)};
+    A.off = Route{f ? o->ridge_offsets : o->valley_offsets, f ? o->valley_offsets : o->ridge_offsets,
+                  rt_of(si == 0 ? R_OFF0 : R_OFF1)};
+    A.aoff = Route{f ? o->ridge_arc_offsets : o->valley_arc_offsets, f ? o->valley_arc_offsets : o->ridge_arc_offsets,
+                   rt_of(si == 0 ? R_AOFF0 : R_AOFF1)};
+    if (!S.arcs_primal) A.off.primal = A.aoff.primal = nullptr;
+    if (!S.arcs_dual) A.off.dual = A.aoff.dual = nullptr;
+    geom_out[si][0] = S.arcs_primal ? (f ? o->ridges : o->valleys) : nullptr;
+    geom_out[si][1] = S.arcs_dual ? (f ? o->valleys : o->ridges) : nullptr;
+    A.alive_base = ctx->bases.alive[si];
+    A.gbase = S.gbase;
+    A.out = S.s_out;
+    A.arc = S.s_arc;
+    A.fin = S.s_fin;
   }
+  LK(survivor_outputs_kernel<<<grid_for(std::max(nsurv, B), TB), TB, 0, st>>>(
+      nsurv, I, ctx->bases.surv, ctx->head, ctx->lens, ctx->rows, o->sad_pts, SO[0], SO[1]));
+  LAUNCH_CHECK("survivor_outputs_kernel");
   mark(ctx, 13, st);
   // per-field totals over the batch (elements)
   long long tot_n[15] = {0};
@@ -1431,28 +1377,9 @@ int fetch_batch_impl(dmsc_b200_context* ctx, const dmsc_b200_outputs* o, cudaStr
   if (ctx->host_fetch_set)  // lists and per-saddle outputs are final: copy them while the geometry is built
     for (int k = 0; k < 9; ++k) copy_out_async(ctx, host_f[k], dev_f[k], 4 * (size_t)tot_n[k], st);
   // arc geometry
-  for (int si = 0; si < 2; ++si) {
-    Side& S = ctx->side[si];
-    if (!S.arcs) continue;
-    // faces: ridges in the primal, valleys in the dual
-    int32_t* gp = S.faces ? o->ridges : o->valleys;
-    int32_t* gd = S.faces ? o->valleys : o->ridges;
-    Route OFF{S.faces ? o->ridge_offsets : o->valley_offsets, S.faces ? o->valley_offsets : o->ridge_offsets,
-              rt_of(si == 0 ? R_OFF0 : R_OFF1)};
-    Route AOFF{S.faces ? o->ridge_arc_offsets : o->valley_arc_offsets,
-               S.faces ? o->valley_arc_offsets : o->ridge_arc_offsets, rt_of(si == 0 ? R_AOFF0 : R_AOFF1)};
-    if (!S.arcs_primal) {
-      gp = nullptr;
-      OFF.primal = nullptr;
-      AOFF.primal = nullptr;
-    }
-    if (!S.arcs_dual) {
-      gd = nullptr;
-      OFF.dual = nullptr;
-      AOFF.dual = nullptr;
-    }
-    emit_write(ctx, si, S, gp, gd, rt_of(si == 0 ? R_G0 : R_G1), OFF, AOFF, st);
-  }
+  for (int si = 0; si < 2; ++si)
+    if (ctx->side[si].arcs)
+      emit_write(ctx, si, ctx->side[si], geom_out[si][0], geom_out[si][1], rt_of(si == 0 ? R_G0 : R_G1), st);
   mark(ctx, 14, st);
   if (ctx->host_fetch_set)
     for (int k = 9; k < 15; ++k) copy_out_async(ctx, host_f[k], dev_f[k], 4 * (size_t)tot_n[k], st);
@@ -1478,8 +1405,7 @@ int fetch_pair_pixels_impl(dmsc_b200_context* ctx, int32_t* plus_max, int32_t* m
     Route PLUS{S.faces ? plus_max : plus_min, S.faces ? plus_min : plus_max, ctx->bases.surv};
     Route MINUS{S.faces ? minus_max : minus_min, S.faces ? minus_min : minus_max, ctx->bases.surv};
     LK(pair_pixels_kernel<<<grid_for(nsurv, TB), TB, 0, st>>>(nsurv, S.faces, ctx->bases.surv, ctx->I, ctx->img,
-                                                              ctx->surv, ctx->crit_sad, S.pp, S.key, PLUS,
-                                                              MINUS));
+                                                              ctx->head, S.pp, S.key, PLUS, MINUS));
   }
   LAUNCH_CHECK("pair_pixels_kernel");
   return kOk;

@@ -71,8 +71,9 @@ constexpr int kCycleEnd = (int)0x80000000;
 
 // K4: per saddle, both face walks and the vertex walks. Writes per saddle and
 // side one record {target 0, target 1, cells 0, cells 1}: each arc's dense
-// target index (or -1) and its raw arc's cell count; and the pairing's
-// starting state: a saddle whose two ends coincide is a cycle, the others
+// target index (or -1) and its raw arc's cell count (a saddle's two records
+// in one 32-byte sector, for the random reads); and the pairing's starting
+// state: a saddle whose two ends coincide is a cycle, the others
 // record their ends and reduce their sweep key into both ends' minima
 // (nothing waits for these reductions: 0.03 ms of the 0.33 ms at 4096^2), and
 // a saddle that is not local to its tile reduces the value part of its key
@@ -84,8 +85,7 @@ __global__ void __launch_bounds__(256) saddle_walk_kernel(Imgs I, const uint8_t*
                                                           const uint32_t* __restrict__ max_bits,
                                                           const int* __restrict__ off_min,
                                                           const uint32_t* __restrict__ min_bits,
-                                                          int4* __restrict__ arc_f, int4* __restrict__ arc_v,
-                                                          long long cap, PairStart ps, unsigned* status) {
+                                                          int4* __restrict__ arc, long long cap, PairStart ps, unsigned* status) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= nsad) return;
   const int b = sad_img[s];
@@ -119,8 +119,8 @@ __global__ void __launch_bounds__(256) saddle_walk_kernel(Imgs I, const uint8_t*
     loc[1][j] = at;
   }
   // a raw arc has fewer cells than the batch (cell ids are int32)
-  arc_f[s] = make_int4(te[0][0], te[0][1], len[0][0], len[0][1]);
-  arc_v[s] = make_int4(te[1][0], te[1][1], len[1][0], len[1][1]);
+  arc[2 * (long long)s] = make_int4(te[0][0], te[0][1], len[0][0], len[0][1]);
+  arc[2 * (long long)s + 1] = make_int4(te[1][0], te[1][1], len[1][0], len[1][1]);
   // descending sweep on the face side in the primal and the vertex side in
   // the dual
   const bool d = I.dual[b];
@@ -554,8 +554,8 @@ __global__ void __launch_bounds__(kTilePairNT, 6) pair_tile_kernel(Imgs I, PairT
 
 // Persistence of each decided saddle and cancellation (persistence.hxx:82-104,
 // 139-161), both sides of a saddle in one thread, with the saddle's image's
-// orientation and threshold: pp[s] = (paired extremum or -1, persistence
-// bits; -1 for a cycle), alive[d] = 0 for an extremum that a cancelled saddle
+// orientation and threshold: pp[s] = (paired extremum or -1, persistence bits;
+// -1 for a cycle) of the face and the vertex side, alive[d] = 0 for an extremum that a cancelled saddle
 // kills, survive[s] = 1 when neither side cancels the saddle; and the starting
 // links of the thresholded union-find.
 struct PersistArgs {
@@ -570,9 +570,9 @@ struct PersistArgs {
   int* n_cancel;               // [2]
   const int* dying[2];
   const int2* key[2];          // (value bits, cell) of each extremum
-  int2* pp[2];
+  int4* pp;                    // [nsad] both sides
   uint8_t* alive[2];
-  const int4* arc[2];
+  const int4* arc;             // [2 nsad]
   int2* ends[2];               // cancelled saddles' arc ends, compacted
   unsigned long long* ckey[2];  // and their replay keys and saddles (nullptr: arcs not simplified)
   int* cval[2];
@@ -607,8 +607,8 @@ __global__ void __launch_bounds__(256) persistence_kernel(PersistArgs A) {
         canc[sd] = p[sd] <= thr;
         if (canc[sd]) A.alive[sd][d[sd]] = 0;
       }
-      A.pp[sd][s] = make_int2(d[sd], __float_as_int(p[sd]));
     }
+    A.pp[s] = make_int4(d[0], __float_as_int(p[0]), d[1], __float_as_int(p[1]));
     A.survive[s] = !(canc[0] || canc[1]);
   }
   // cancelled edges' ends, compacted for the thresholded union-find, and (when
@@ -621,7 +621,7 @@ __global__ void __launch_bounds__(256) persistence_kernel(PersistArgs A) {
 #pragma unroll
   for (int sd = 0; sd < 2; ++sd) {
     if (!canc[sd]) continue;
-    const int4 a = A.arc[sd][s];
+    const int4 a = A.arc[2 * (long long)s + sd];
     A.ends[sd][slot[sd]] = make_int2(a.x, a.y);
     if (!A.ckey[sd]) continue;
     const unsigned long long key = ((unsigned long long)orderable_key(p[sd]) << 32) | (unsigned)A.crit_sad[s];

@@ -79,27 +79,25 @@ __device__ __forceinline__ int value_pixel(const float* __restrict__ img_all, co
   return I.dual[b] ? cell_pixel_g<true>(img, cell & 3, y, x, H, W) : cell_pixel_g<false>(img, cell & 3, y, x, H, W);
 }
 
-// Per surviving saddle of one side, in the order of that side's p output
-// (survivor order; the face side visits each image's survivors reversed),
-// the image-local pixels entering its persistence with sign + and -
+// Per surviving saddle of one side, in survivor order (the order of its p
+// output), the image-local pixels entering its persistence with sign + and -
 // (-1, -1 for a cycle, whose persistence is the constant -1). The sign
 // follows persistence_kernel: p = saddle - extremum on the vertex side in the
 // primal and on the face side in the dual, extremum - saddle otherwise.
 __global__ void pair_pixels_kernel(int nsurv, bool faces, const int* __restrict__ surv_base, Imgs I,
-                                   const float* __restrict__ img_all, const int* __restrict__ surv_sad,
-                                   const int* __restrict__ crit_sad, const int2* __restrict__ pp,
-                                   const int2* __restrict__ ext_key, Route PLUS, Route MINUS) {
-  int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= nsurv) return;
-  int b;
-  int i = visit(q, faces, surv_base, I.B, &b);
+                                   const float* __restrict__ img_all, const SurvHead* __restrict__ head,
+                                   const int2* __restrict__ pp, const int2* __restrict__ ext_key, Route PLUS,
+                                   Route MINUS) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= nsurv) return;
+  const int4 h = *reinterpret_cast<const int4*>(head + i);
+  const int b = h.x;
   const bool d = I.dual[b];
   const int li = i - surv_base[b];
-  const int s = surv_sad[i];
-  const int e = pp[s].x;
+  const int e = pp[2 * (long long)h.z].x;
   int plus = -1, minus = -1;
   if (e >= 0) {
-    const int sp = value_pixel(img_all, I, b, crit_sad[s]);
+    const int sp = value_pixel(img_all, I, b, h.y);
     const int ep = value_pixel(img_all, I, b, ext_key[e].y);
     const bool saddle_plus = (!faces) != d;
     plus = saddle_plus ? sp : ep;

@@ -579,7 +579,7 @@ struct ReplayArgs {
   const unsigned long long* key;     // [C] replay key of each cancellation
   const int* cj;                     // [C] saddle (list index) of each cancellation
   const int* dying;  // [nsad] in saddle list order
-  const int4* arc;   // [nsad] {end 0, end 1, raw-arc cells 0, raw-arc cells 1} of each saddle, list order
+  const int4* arc;   // {end 0, end 1, raw-arc cells 0, raw-arc cells 1} of each saddle, list order (every second record)
   const uint8_t* alive;  // [M] extrema that no cancellation kills (their records are never read)
   const int* crit_sad;   // [nsad] global cell id of each saddle
   ReplayState S;
@@ -653,7 +653,7 @@ __device__ __forceinline__ void replay_batch(const ReplayArgs2& P, int rd, long 
     for (int u = 0; u < U; ++u) {
       if (!((act >> u) & 1u)) continue;
       const bool s1 = (s1m >> u) & 1u;
-      const int4 w = RSIDE(arc)[sd[u]];
+      const int4 w = RSIDE(arc)[2 * (long long)sd[u]];
       x[2 * u] = w.x;
       x[2 * u + 1] = w.y;
     }
@@ -736,7 +736,7 @@ __device__ __forceinline__ void replay_batch(const ReplayArgs2& P, int rd, long 
       k = 1;
     ReplayNode* node = RSIDE(S.node);
     if (k >= 0) {
-      const int4 ar = RSIDE(arc)[s];
+      const int4 ar = RSIDE(arc)[2 * (long long)s];
       const int2 tt = make_int2(ar.x, ar.y);
       const longlong2 bl = make_longlong2(ar.z, ar.w);
       *reinterpret_cast<longlong2*>(&node[dd].cl_dy) = make_longlong2(k == 0 ? a0 : a1, k == 0 ? a1 : a0);
@@ -851,8 +851,6 @@ __global__ void __launch_bounds__(256, MINB) replay_persistent_kernel(ReplayArgs
 struct EmitArgs {
   EmitCtx E;
   int nsurv;
-  const long long* arc_cl;
-  const int* arc_root;
   int4* q0;
   int4* q1;
   int* cnt;  // [0..2] rotating level counts, [3] raw-arc segment count
@@ -1015,19 +1013,21 @@ __global__ void __launch_bounds__(256, MINB) emit_persistent_kernel(EmitArgs A) 
   int* const n_base = A.cnt + 3;
   // level 0: the chain of each surviving arc (its own raw arc is a segment
   // item of the writer, read from the survivor records). A block takes
-  // kLevel0Arcs arcs per thread at a time: it counts their chains, reserves
+  // kLevel0 survivors per thread at a time: it counts their chains, reserves
   // queue slots once for all of them and then writes the tasks, so the
   // blocks queue on the shared counter once per 4096 arcs instead of once
   // per 256 (each reservation waits on the atomic's return).
-  constexpr int kLevel0Arcs = 16;
-  const long long narcs = 2LL * A.nsurv, span = (long long)blockDim.x * kLevel0Arcs;
-  for (long long base = (long long)blockIdx.x * span; base < narcs; base += (long long)gridDim.x * span) {
-    // a chain exists only on arcs that the image's output takes (arc_cl = 0 otherwise)
+  constexpr int kLevel0 = 8;
+  const long long span = (long long)blockDim.x * kLevel0;
+  for (long long base = (long long)blockIdx.x * span; base < A.nsurv; base += (long long)gridDim.x * span) {
+    // a chain exists only on arcs that the image's output takes (length 0 otherwise)
     int mine = 0;
 #pragma unroll
-    for (int k = 0; k < kLevel0Arcs; ++k) {
-      const long long q = base + (long long)k * blockDim.x + threadIdx.x;
-      mine += q < narcs && A.arc_cl[q] > 0;
+    for (int k = 0; k < kLevel0; ++k) {
+      const long long i = base + (long long)k * blockDim.x + threadIdx.x;
+      if (i >= A.nsurv) continue;
+      const int2 cl = *reinterpret_cast<const int2*>(E.fin + i);
+      mine += (cl.x > 0) + (cl.y > 0);
     }
     // most arcs have no chain (at threshold 0 nearly all): a block reserves
     // queue slots only when one of its threads has a task
@@ -1035,17 +1035,22 @@ __global__ void __launch_bounds__(256, MINB) emit_persistent_kernel(EmitArgs A) 
     int p, pb;
     block_reserve2(A.cnt, mine, n_base, 0, p, pb);
     if (mine == 0) continue;
-    for (int k = 0; k < kLevel0Arcs; ++k) {
-      const long long q = base + (long long)k * blockDim.x + threadIdx.x;
-      if (q >= narcs || A.arc_cl[q] <= 0) continue;
-      const int i = (int)(q >> 1), j = (int)(q & 1);
-      const int2 tt = E.sv_t[i];
-      const longlong2 bl = E.sv_len[i];
-      if (p < E.q_cap)
-        A.q0[p] = make_task(kTaskChain, 0, j ? tt.y : tt.x, A.arc_root[q], E.arc_pos[q] + (j ? bl.y : bl.x));
-      else
-        set_status(E.status, kStatusQueueOverflow);
-      ++p;
+    for (int k = 0; k < kLevel0; ++k) {
+      const long long i = base + (long long)k * blockDim.x + threadIdx.x;
+      if (i >= A.nsurv) break;
+      const int4 fin = E.fin[i];
+      if (fin.x <= 0 && fin.y <= 0) continue;
+      const int4 a = E.arc[i];
+      const int pos = surv_start(E, (int)i, E.head[i].img);
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        if ((j ? fin.y : fin.x) <= 0) continue;
+        if (p < E.q_cap)
+          A.q0[p] = make_task(kTaskChain, 0, j ? a.y : a.x, j ? fin.w : fin.z, pos + a.z + (j ? fin.x + a.w : 0));
+        else
+          set_status(E.status, kStatusQueueOverflow);
+        ++p;
+      }
     }
   }
   grid.sync();

@@ -27,6 +27,7 @@
 // their start cells when written.
 #pragma once
 
+#include "assemble.cuh"
 #include "common.cuh"
 #include "walks.cuh"
 
@@ -119,41 +120,98 @@ __device__ __forceinline__ bool walk_root(const ReplayState& S, const uint8_t* _
   return true;
 }
 
-// Final arcs of the surviving saddles: length and the chain root of each
-// (survivor i in output order, arcs 0 and 1), and the survivor's total path
-// length, from the survivors' gathered records (image, arc ends, raw-arc
-// lengths). Images whose output does not take this side's arcs
-// (`arcs_primal` / `arcs_dual` by orientation) get empty arcs.
-__global__ void final_arcs_kernel(int nsurv, const int2* __restrict__ surv_ic, const uint8_t* __restrict__ dual,
-                                  bool arcs_primal, bool arcs_dual, const int2* __restrict__ sv_t,
-                                  const longlong2* __restrict__ sv_len, const uint8_t* __restrict__ alive,
-                                  ReplayState S, int max_steps, long long* __restrict__ arc_len,
-                                  long long* __restrict__ arc_cl, int* __restrict__ arc_root,
-                                  long long* __restrict__ plen, unsigned* status) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nsurv) return;
-  const int2 tt = sv_t[i];
-  const longlong2 bl = sv_len[i];
-  const bool take = dual[surv_ic[i].x] ? arcs_dual : arcs_primal;
-  long long len[2] = {0, 0}, cl[2] = {0, 0};
-  int root[2] = {-1, -1};
+// The survivors in output order and their final arcs, two threads (sides) a
+// survivor. `sorted` lists them by ascending (image, s_val, cell id), the
+// vertex side's sweep order (arcs_topology.hxx:99-102); an image whose vertex
+// side sweeps descending (dual) takes its range reversed. A side's thread
+// gathers its arc ends and raw-arc lengths, its persistence and the ranks of
+// the thresholded roots of its ends and pair (-1 for the void), walks its
+// ends' chains to their final roots, and writes all of it in output order, so
+// that the later per-survivor kernels read in order; the survivor's geometry
+// cells and e rows go to the scans (entry nsurv is zero: the totals). Images
+// whose output does not take a side's arcs (`primal` / `dual` by orientation)
+// get empty arcs there.
+//
+// Bound by L2 sectors (180 G/s): the sort's random permutation makes every
+// read its own sector, so both sides' records of a saddle are interleaved.
+// Measured at 4096^2 noise, threshold 0 (5.9 M survivors), gathers, final
+// arcs, row counts, scans and positions: 0.76 ms in eleven passes, 0.58 ms in
+// this one and two scans.
+struct FinalSide {
+  const int4* arc;        // [2 nsad] both sides' records, interleaved
+  const int2* pp;         // [2 nsad] paired extremum and persistence bits, interleaved
+  const int* rout;        // [M] rank of each extremum's root
+  int4* s_arc;            // [nsurv] arc ends, raw-arc lengths
+  int4* s_out;            // [nsurv] ranks of the ends' roots, persistence bits, rank of the pair's root
+  int4* s_fin;            // [nsurv] chain lengths and roots; nullptr: no image takes the arcs
+  const uint8_t* alive;
+  ReplayState S;
+  bool primal, dual;
+};
+
+__global__ void __launch_bounds__(256) survivor_final_kernel(
+    int nsurv, const int* __restrict__ sorted, int B, const int* __restrict__ sad_img,
+    const int* __restrict__ crit_sad, const uint8_t* __restrict__ dual, const int* __restrict__ surv_base, FinalSide F,
+    FinalSide V, int max_steps, SurvHead* __restrict__ head, unsigned long long* __restrict__ lens,
+    unsigned long long* __restrict__ rows, unsigned long long* __restrict__ total, unsigned* status) {
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const int p = (int)(t >> 1), sd = (int)(t & 1);
+  __shared__ unsigned long long sum[2];
+  if (threadIdx.x < 2) sum[threadIdx.x] = 0;
+  __syncthreads();
+  int q = p;
+  unsigned n_rows = 0;
+  unsigned long long len = 0;
+  if (p < nsurv) {
+    const int s = sorted[p], b = B > 1 ? sad_img[s] : 0;
+    const bool d = dual[b];
+    if (d) {
+      const int base = surv_base[b], cnt = surv_base[b + 1] - base;
+      q = base + cnt - 1 - (p - base);
+    }
+    const FinalSide& A = sd ? V : F;
+    const int4 a = A.arc[2 * (long long)s + sd];
+    const int2 pr = A.pp[2 * (long long)s + sd];
+    const int4 o = make_int4(a.x >= 0 ? A.rout[a.x] : -1, a.y >= 0 ? A.rout[a.y] : -1, pr.y,
+                             pr.x >= 0 ? A.rout[pr.x] : -1);
+    A.s_out[q] = o;
+    int x, y;
+    n_rows = erow_ends(o.x, o.y, &x, &y);
+    if (A.s_fin) {
+      int4 fin = make_int4(0, 0, -1, -1);
+      if (d ? A.dual : A.primal) {
+        long long c[2] = {0, 0};
+        int root[2];
 #pragma unroll
-  for (int j = 0; j < 2; ++j) {
-    const int T = j ? tt.y : tt.x;
-    if (T < 0 || !take) continue;
-    // an extremum that no cancellation kills (alive) is its own final root;
-    // only the others walk their parent chains
-    int R = T;
-    long long a = 0;
-    if (!alive[T]) walk_root(S, alive, T, kNever, &R, &a, max_steps, status);
-    len[j] = (j ? bl.y : bl.x) + a;
-    cl[j] = a;
-    root[j] = R;
+        for (int j = 0; j < 2; ++j) {
+          const int T = j ? a.y : a.x;
+          root[j] = T;
+          // an extremum that no cancellation kills (alive) is its own final
+          // root; only the others walk their parent chains
+          if (T >= 0 && !A.alive[T]) walk_root(A.S, A.alive, T, kNever, &root[j], &c[j], max_steps, status);
+        }
+        // a chain beyond 32 bits makes the side's geometry overflow (the
+        // exact total says so): its stored length is not used then
+        fin = make_int4((int)c[0], (int)c[1], root[0], root[1]);
+        len = (unsigned long long)((long long)a.z + a.w + c[0] + c[1]);
+      }
+      A.s_arc[q] = a;
+      A.s_fin[q] = fin;
+    }
+    if (sd == 0) *reinterpret_cast<int4*>(head + q) = make_int4(b, crit_sad[s], s, 0);
   }
-  *reinterpret_cast<longlong2*>(arc_len + 2 * i) = make_longlong2(len[0], len[1]);
-  *reinterpret_cast<longlong2*>(arc_cl + 2 * i) = make_longlong2(cl[0], cl[1]);
-  *reinterpret_cast<int2*>(arc_root + 2 * i) = make_int2(root[0], root[1]);
-  plen[i] = len[0] + len[1];
+  const unsigned other_rows = __shfl_xor_sync(0xffffffffu, n_rows, 1);
+  const unsigned other_len = __shfl_xor_sync(0xffffffffu, (unsigned)len, 1);
+  if (sd == 0 && p <= nsurv) {  // p == nsurv: q == p, all zero
+    lens[q] = pack2((unsigned)len, other_len);
+    rows[q] = pack2(n_rows, other_rows);
+  }
+  // the exact geometry totals
+#pragma unroll
+  for (int o = 2; o < 32; o <<= 1) len += __shfl_xor_sync(0xffffffffu, len, o);
+  if ((threadIdx.x & 31) < 2 && len) atomicAdd(&sum[sd], len);
+  __syncthreads();
+  if (threadIdx.x < 2 && sum[threadIdx.x]) atomicAdd(total + threadIdx.x, sum[threadIdx.x]);
 }
 
 // ---------------------------------------------------------------------------
@@ -179,13 +237,19 @@ struct EmitCtx {
   // the survivors' own raw arcs (segment items 0 .. 2 nsurv - 1 of the
   // writer, read from the survivor records instead of a task list)
   int nvirt;                 // 2 nsurv
-  const int2* surv_ic;       // [nsurv] image and cell of each survivor (output order)
-  const int2* sv_t;          // [nsurv] this side's arc ends
-  const longlong2* sv_len;   // [nsurv] this side's raw-arc lengths
-  const long long* arc_pos;  // [2 nsurv] image-local output position of each arc
+  const SurvHead* head;      // [nsurv] image and cell of each survivor (output order)
+  const int4* arc;           // [nsurv] arc ends and raw-arc lengths
+  const int4* fin;           // [nsurv] chain lengths and roots
+  const unsigned long long* lens;  // [nsurv + 1] where each survivor's geometry starts (both sides packed)
+  const long long* gbase;    // [B + 1] where each image's does
   int max_steps;
   unsigned* status;
 };
+
+// Image-local output position of a survivor's first arc.
+__device__ __forceinline__ int surv_start(const EmitCtx& E, int i, int b) {
+  return half_of(E.lens[i], E.faces ? 0 : 1) - (int)E.gbase[b];
+}
 
 // A raw-arc segment task of the chain expansion: {reversed | arc << 1,
 // saddle cell, cells, output position}: the writer finds the arc's start
@@ -220,14 +284,13 @@ __device__ __forceinline__ void seg_start(const EmitCtx& E, long long q, SegCurs
   bool rev;
   if (q < E.nvirt) {
     const int i = (int)(q >> 1), j = (int)(q & 1);
-    const int2 tt = E.sv_t[i];
-    const longlong2 bl = E.sv_len[i];
-    len = (int)(j ? bl.y : bl.x);
-    if ((j ? tt.y : tt.x) < 0 || len <= 0) return;
-    const int2 ic = E.surv_ic[i];
+    const int4 a = E.arc[i];
+    len = j ? a.w : a.z;
+    if ((j ? a.y : a.x) < 0 || len <= 0) return;
+    const int2 ic = *reinterpret_cast<const int2*>(E.head + i);
     b = ic.x;
     idx = arc_start_of_cell(E, ic.y, j, b);
-    pos = (int)E.arc_pos[q];
+    pos = surv_start(E, i, b) + (j ? a.z + E.fin[i].x : 0);
     rev = false;
   } else {
     const int4 t = E.base_q[q - E.nvirt];
