@@ -26,6 +26,7 @@ EXPORTS = (
     "dmsc_b200_set_host_input",
     "dmsc_b200_extract_batch",
     "dmsc_b200_fetch_pair_pixels",
+    "dmsc_b200_fetch_pairs",
     "dmsc_b200_scatter_pair_grads",
     "dmsc_b200_error_string",
     "dmsc_b200_last_error",
@@ -106,6 +107,8 @@ def load():
         lib.dmsc_b200_extract_batch.restype = ctypes.c_int
         lib.dmsc_b200_fetch_pair_pixels.argtypes = [ctypes.c_void_p] + [ctypes.c_void_p] * 5
         lib.dmsc_b200_fetch_pair_pixels.restype = ctypes.c_int
+        lib.dmsc_b200_fetch_pairs.argtypes = [ctypes.c_void_p] * 10
+        lib.dmsc_b200_fetch_pairs.restype = ctypes.c_int
         lib.dmsc_b200_scatter_pair_grads.argtypes = [
             ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int64, ctypes.c_void_p,
             ctypes.c_int64, ctypes.c_void_p]

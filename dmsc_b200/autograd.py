@@ -25,7 +25,7 @@ from dataclasses import dataclass
 import torch
 
 from . import _lib
-from .dmsc import _batch_raw, _ptr, _validate
+from .dmsc import _extract_raw, _ptr, _validate
 
 
 @dataclass
@@ -53,29 +53,19 @@ class PersistencePairs:
 
 def _run(x3, thresholds, duals):
     """Forward on a contiguous [B, H, W] CUDA tensor: the values, metadata and
-    the pixel pairs as flat pixel ids of ``x3`` (-1 for cycles)."""
-    B, H, W = x3.shape
-    imgs = list(x3.unbind(0))
-    out, lens, _, _, _, _ = _batch_raw(imgs, thresholds, duals, 0, flat=x3.reshape(-1), pair_pixels=True)
+    the pixel pairs, then the pairs as flat pixel ids of ``x3`` (-1 for
+    cycles)."""
     dev = x3.device
-    n_min = torch.tensor(lens["p_min"], device=dev)
-    n_max = torch.tensor(lens["p_max"], device=dev)
-    ids = torch.arange(B, device=dev)
-    img_min = torch.repeat_interleave(ids, n_min)
-    img_max = torch.repeat_interleave(ids, n_max)
-    # per image: its p_min entries, then its p_max entries
-    order_key = torch.cat([img_min * 2, img_max * 2 + 1])
-    perm = torch.sort(order_key, stable=True).indices
-    cat = lambda a, b: torch.cat([a, b])[perm]  # noqa: E731
-    p = cat(out["p_min"], out["p_max"])
-    image = cat(img_min, img_max)
-    side = cat(torch.zeros_like(img_min, dtype=torch.int8), torch.ones_like(img_max, dtype=torch.int8))
-    ppairs = cat(out["ppairs_min"], out["ppairs_max"])
-    plus = cat(out["plus_min"], out["plus_max"])
-    minus = cat(out["minus_min"], out["minus_max"])
-    base = (image * (H * W)).to(torch.int32)
-    plus_g = torch.where(plus >= 0, plus + base, plus)
-    minus_g = torch.where(minus >= 0, minus + base, minus)
+    sizes, s = _extract_raw(x3, thresholds, duals)
+    n = 2 * sum(int(z.sad_pts) for z in sizes)  # a surviving saddle has an entry on both sides
+    p = torch.empty(n, dtype=torch.float32, device=dev)
+    image = torch.empty(n, dtype=torch.int64, device=dev)
+    side = torch.empty(n, dtype=torch.int8, device=dev)
+    ppairs, plus, minus, plus_g, minus_g = (torch.empty(n, dtype=torch.int32, device=dev) for _ in range(5))
+    ctx = _lib.context(dev.index if dev.index is not None else torch.cuda.current_device())
+    ctx.check(ctx.lib.dmsc_b200_fetch_pairs(
+        ctx.h, *(_ptr(t) for t in (p, image, side, ppairs, plus, minus, plus_g, minus_g)),
+        ctypes.c_void_p(s.cuda_stream)), "dmsc_b200_fetch_pairs")
     return p, image, side, ppairs, plus, minus, plus_g, minus_g
 
 

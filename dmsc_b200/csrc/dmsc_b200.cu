@@ -1411,6 +1411,30 @@ int fetch_pair_pixels_impl(dmsc_b200_context* ctx, int32_t* plus_max, int32_t* m
   return kOk;
 }
 
+// Persistence entries of the last extract in the autograd order (pairs.cuh).
+int fetch_pairs_impl(dmsc_b200_context* ctx, PairEntries E, cudaStream_t st) {
+  if (!ctx->valid) {
+    set_err(ctx, "fetch_pairs without a successful extract");
+    return kErrInvalidArgument;
+  }
+  const int nsurv = ctx->nsurv;
+  if (nsurv > 0 && (!E.p || !E.image || !E.side || !E.ppairs || !E.plus || !E.minus || !E.plus_flat || !E.minus_flat)) {
+    set_err(ctx, "invalid argument");
+    return kErrInvalidArgument;
+  }
+  CK(cudaSetDevice(ctx->device));
+  if (nsurv == 0) return kOk;
+  PairSide P[2];
+  for (int si = 0; si < 2; ++si) {
+    const Side& S = ctx->side[si];
+    P[si] = PairSide{S.pp, S.key, S.s_out, ctx->bases.alive[si]};
+  }
+  LK(pair_entries_out_kernel<<<grid_for(2LL * nsurv, TB), TB, 0, st>>>(nsurv, ctx->I, ctx->bases.surv, ctx->img,
+                                                                       ctx->head, P[0], P[1], E));
+  LAUNCH_CHECK("pair_entries_out_kernel");
+  return kOk;
+}
+
 // grad_img[0, npx) = deterministic scatter of +-grad[i] onto (plus[i], minus[i]).
 int scatter_pair_grads_impl(dmsc_b200_context* ctx, const int32_t* plus, const int32_t* minus, const float* grad,
                             long long n, float* grad_img, long long npx, cudaStream_t st) {
@@ -1595,6 +1619,20 @@ int dmsc_b200_fetch_pair_pixels(dmsc_b200_context* ctx, int32_t* plus_max, int32
   ctx->err.clear();
   try {
     return fetch_pair_pixels_impl(ctx, plus_max, minus_max, plus_min, minus_min, (cudaStream_t)stream);
+  } catch (const Fail& f) {
+    return f.code;
+  }
+}
+
+int dmsc_b200_fetch_pairs(dmsc_b200_context* ctx, float* persistence, int64_t* image, int8_t* side, int32_t* ppairs,
+                          int32_t* plus_pixel, int32_t* minus_pixel, int32_t* plus_flat, int32_t* minus_flat,
+                          void* stream) {
+  if (!ctx) return kErrInvalidArgument;
+  ctx->err.clear();
+  try {
+    const PairEntries E{persistence, (long long*)image, (signed char*)side, ppairs,
+                        plus_pixel,  minus_pixel,       plus_flat,          minus_flat};
+    return fetch_pairs_impl(ctx, E, (cudaStream_t)stream);
   } catch (const Fail& f) {
     return f.code;
   }

@@ -283,13 +283,30 @@ _SIZE_OF = dict(max_pts="max_pts", min_pts="min_pts", sad_pts="sad_pts", e_max="
                 valley_offsets="valley_offsets", valley_arc_offsets="valley_arc_offsets")
 
 
-def _batch_raw(images, thresholds, is_dual, flags: int, stream=None, flat=None, pair_pixels=False, host_fixed=False):
+def _extract_raw(x3, thresholds, duals):
+    """The first C-ABI phase alone on a contiguous [B, H, W] CUDA tensor, with
+    no gradient, arcs or labels: the sizes of every image and the stream."""
+    B, H, W = (int(v) for v in x3.shape)
+    dev = x3.device
+    ctx = _lib.context(dev.index if dev.index is not None else torch.cuda.current_device())
+    s = torch.cuda.current_stream(dev)
+    tuning.apply(ctx, B * H * W)
+    sz = (_lib.Sizes * B)()
+    rc = ctx.lib.dmsc_b200_extract_batch(
+        ctx.h, ctypes.c_void_p(x3.data_ptr()), B, (ctypes.c_int * B)(*([H] * B)), (ctypes.c_int * B)(*([W] * B)),
+        (ctypes.c_float * B)(*[float(t) for t in thresholds]), (ctypes.c_ubyte * B)(*[int(d) for d in duals]), 0,
+        _ptr(None), _ptr(None), _ptr(None), sz, ctypes.c_void_p(s.cuda_stream))
+    if rc == _lib.ERR_TOO_LARGE and B == 1:
+        raise RuntimeError(f"Input is too large for 32-bit cell IDs: {H}x{W}")
+    ctx.check(rc, "dmsc_b200_extract_batch")
+    return sz, s
+
+
+def _batch_raw(images, thresholds, is_dual, flags: int, stream=None, host_fixed=False):
     """Both C-ABI phases of one device batch. Returns the batch-wide output
     tensors (``out``, field -> tensor, images back to back), the per-image
     lengths of each (``lens``), the image shapes and orientations and the
-    stream. ``flat`` may hold the images already back to back; with
-    ``pair_pixels`` the pixel pairs of every p_max / p_min entry are fetched
-    too (``plus_max``, ``minus_max``, ``plus_min``, ``minus_min``)."""
+    stream."""
     B = len(images)
     dev = images[0].device
     ctx = _lib.context(dev.index if dev.index is not None else torch.cuda.current_device())
@@ -298,8 +315,7 @@ def _batch_raw(images, thresholds, is_dual, flags: int, stream=None, flat=None, 
     Hs = [int(x.shape[0]) for x in images]
     Ws = [int(x.shape[1]) for x in images]
     duals = [bool(d) for d in is_dual]
-    if flat is None:
-        flat = images[0].reshape(-1) if B == 1 else torch.cat([x.reshape(-1) for x in images])
+    flat = images[0].reshape(-1) if B == 1 else torch.cat([x.reshape(-1) for x in images])
     nidx = [(h + 1) * (w + 1) for h, w in zip(Hs, Ws)]
     npx = [h * w for h, w in zip(Hs, Ws)]
     tuning.apply(ctx, sum(npx))
@@ -334,14 +350,6 @@ def _batch_raw(images, thresholds, is_dual, flags: int, stream=None, flat=None, 
     ctx.check(ctx.lib.dmsc_b200_fetch(ctx.h, ctypes.byref(o), ctypes.c_void_p(s.cuda_stream)), "dmsc_b200_fetch")
     if host_fixed:
         out = hout
-    if pair_pixels:
-        for f in ("plus_max", "minus_max", "plus_min", "minus_min"):
-            side = f.split("_")[1]
-            out[f] = torch.empty(out["p_" + side].numel(), **i32)
-            lens[f] = lens["p_" + side]
-        ctx.check(ctx.lib.dmsc_b200_fetch_pair_pixels(
-            ctx.h, _ptr(out["plus_max"]), _ptr(out["minus_max"]), _ptr(out["plus_min"]), _ptr(out["minus_min"]),
-            ctypes.c_void_p(s.cuda_stream)), "dmsc_b200_fetch_pair_pixels")
     if host_fixed:
         grad, peaks, basins = hg, hp, hb
     if grad is not None:

@@ -183,6 +183,18 @@ int dmsc_b200_extract_batch(dmsc_b200_context* ctx, const float* images, int B, 
 int dmsc_b200_fetch_pair_pixels(dmsc_b200_context* ctx, int32_t* plus_max, int32_t* minus_max, int32_t* plus_min,
                                 int32_t* minus_min, void* stream);
 
+/* Persistence values of the last extract with their metadata, 2 n entries (n:
+   the sum of the images' sad_pts): per image the entries of p_min, then those
+   of p_max. image: index of the image; side: 0 min, 1 max; ppairs: the
+   matching ppairs_min / ppairs_max entry; plus_pixel / minus_pixel: the
+   image-local pixels entering the value with sign + and - (-1 for a cycle);
+   plus_flat / minus_flat: the same counted over the whole batch. No
+   dmsc_b200_fetch() is needed before; the input image must be unchanged.
+   Every array holds 2 n entries. */
+int dmsc_b200_fetch_pairs(dmsc_b200_context* ctx, float* persistence, int64_t* image, int8_t* side, int32_t* ppairs,
+                          int32_t* plus_pixel, int32_t* minus_pixel, int32_t* plus_flat, int32_t* minus_flat,
+                          void* stream);
+
 /* Backward scatter: grad_img[0 .. npx) = 0, then for every i < n,
    grad_img[plus[i]] += grad[i] and grad_img[minus[i]] -= grad[i] (ends
    outside [0, npx), such as -1, are skipped). Deterministic: the terms of
