@@ -92,6 +92,7 @@ __device__ __forceinline__ void chunk_start(ChunkLists& L) {
 }
 
 __device__ __forceinline__ void chunk_keep(ChunkLists& L, int side, int v) { L.buf[side][atomicAdd(&L.n[side], 1)] = v; }
+
 __device__ __forceinline__ void chunk_flush(ChunkLists& L, int* cnt0, int* out0, int* cnt1, int* out1) {
   const int t = threadIdx.x;
   __syncthreads();
@@ -602,23 +603,35 @@ struct ReplayArgs2 {
   ReplayArgs s[2];
 };
 
+// A round that holds every pending cancellation in a thread of its own lets
+// the walks wait for the decisions they need instead of ending the round:
+// each wait is a re-read of under a microsecond, against 10 to 20 us for a
+// round. Measured, the replay stage with rounds only and with waits: 0.37 ->
+// 0.14 ms on a 1080 x 1920 field of 256 levels (30 rounds before), 0.34 -> 0.24
+// at 2048^2, threshold 0.25, 0.91 -> 0.80 at 4096^2, 0.085 -> 0.045 at 256^2.
+// The first round and the rounds with more items than threads do not wait: a
+// decision there is as often many strides away (4 looks: 1.16 ms at 4096^2).
+constexpr int kReplayWait = 256;
+
 // One batch of a thread's pending cancellations, the items i0 + nt u (u < U)
-// below na + nb (side 0's first): both walks of every item resume where the
+// below n (side 0's first, i < na): both walks of every item resume where the
 // previous round left them and advance in lockstep (2U independent chains of
-// node loads at once); an item whose walks meet an undecided node keeps its
-// walk positions and stays pending, the others decide (link or skip). The
-// batch's pending items are appended to the next round's lists with one block
-// reservation.
+// node loads at once), then the item decides (link or skip). An item with a
+// walk that meets an undecided node keeps its walks' positions and stays
+// pending for the next round. With WAIT such a walk looks at the node again,
+// up to kReplayWait times, and an item decides inside the loop, as soon as
+// both its walks have ended, so that lanes of its own warp may wait for it.
 #define RSIDE(f) (s1 ? P.s[1].f : P.s[0].f)
-template <int U>
-__device__ __forceinline__ void replay_batch(const ReplayArgs2& P, int rd, long long i0, long long nt, int na, int nb) {
+template <int U, bool WAIT>
+__device__ __forceinline__ void replay_batch(const ReplayArgs2& P, int rd, long long i0, long long nt,
+                                             long long n, int na, ChunkLists& L) {
   int r[U];
   unsigned act = 0, s1m = 0;
 #pragma unroll
   for (int u = 0; u < U; ++u) {
     const long long i = i0 + nt * u;
     r[u] = 0;
-    if (i < (long long)na + nb) {
+    if (i < n) {
       const bool s1 = i >= na;
       act |= 1u << u;
       s1m |= (unsigned)s1 << u;
@@ -664,69 +677,15 @@ __device__ __forceinline__ void replay_batch(const ReplayArgs2& P, int rd, long 
     const bool s1 = (s1m >> u) & 1u;
     d[u] = ((act >> u) & 1u) ? RSIDE(dying)[sd[u]] : 0;
   }
-  // the walks, resumed where the previous round left them and advanced in
-  // lockstep (the root as of the step's key, with the length summed on the
-  // way): bit c of `live` is a walk still
-  // moving, bit c of `wait` one that met an undecided node
-  unsigned live = 0, wait = 0;
+  // bit c of `live` is a walk that has not ended (the root as of the step's
+  // key is not reached), bit c of `wait` one that met an undecided node
+  unsigned live = 0;
 #pragma unroll
   for (int c = 0; c < 2 * U; ++c)
     if (((act >> (c >> 1)) & 1u) && x[c] >= 0) live |= 1u << c;
-  // a chain is at most its side's node count long (a side without arcs takes
-  // no part and has no bound of its own)
-  const int cap = max(P.s[0].max_steps, P.s[1].max_steps);
-  for (int steps = 0; live; ++steps) {
-    if (steps > cap) {
-      set_status(P.s[0].status, kStatusChainCap);
-      break;
-    }
-    longlong2 kl[2 * U];
-    int2 w[2 * U];  // status, parent
-    bool al[2 * U];
-#pragma unroll
-    for (int c = 0; c < 2 * U; ++c) {
-      const bool s1 = (s1m >> (c >> 1)) & 1u;
-      if ((live >> c) & 1u) {  // the alive flag and the record's sector, issued together
-        al[c] = RSIDE(alive)[x[c]];
-        kl[c] = node_keylen_cg(RSIDE(S.node), x[c]);
-        w[c] = __ldcg(reinterpret_cast<const int2*>(&RSIDE(S.node)[x[c]].status));
-      }
-    }
-#pragma unroll
-    for (int c = 0; c < 2 * U; ++c) {
-      if (!((live >> c) & 1u)) continue;
-      // never cancelled (its record is not written), or not linked before
-      // this step: the root
-      if (al[c] || (unsigned long long)kl[c].x >= tk[c >> 1]) {
-        live &= ~(1u << c);
-        continue;
-      }
-      const int st = w[c].x;
-      if (status_kind(st) == kPending || (st >> 2) > rd) {  // undecided, or decided in this round
-        live &= ~(1u << c);
-        wait |= 1u << c;
-        continue;
-      }
-      if (status_kind(st) == kRootForever) {
-        live &= ~(1u << c);
-        continue;
-      }
-      a[c] += kl[c].y;
-      x[c] = w[c].y;
-      if (x[c] < 0) live &= ~(1u << c);
-    }
-  }
-  unsigned keep = 0;
-#pragma unroll
-  for (int u = 0; u < U; ++u) {
-    if (!((act >> u) & 1u)) continue;
+  auto decide = [&](int u) {
+    act &= ~(1u << u);
     const bool s1 = (s1m >> u) & 1u;
-    if ((wait >> (2 * u)) & 3u) {  // still waiting on an earlier cancellation
-      keep |= 1u << u;
-      *reinterpret_cast<int2*>(RSIDE(wx) + 2 * r[u]) = make_int2(x[2 * u], x[2 * u + 1]);
-      *reinterpret_cast<longlong2*>(RSIDE(wa) + 2 * r[u]) = make_longlong2(a[2 * u], a[2 * u + 1]);
-      continue;
-    }
     const int R0 = x[2 * u], R1 = x[2 * u + 1], dd = d[u], s = sd[u];
     const long long a0 = a[2 * u], a1 = a[2 * u + 1];
     int k = -1;
@@ -737,34 +696,79 @@ __device__ __forceinline__ void replay_batch(const ReplayArgs2& P, int rd, long 
     ReplayNode* node = RSIDE(S.node);
     if (k >= 0) {
       const int4 ar = RSIDE(arc)[2 * (long long)s];
-      const int2 tt = make_int2(ar.x, ar.y);
-      const longlong2 bl = make_longlong2(ar.z, ar.w);
       *reinterpret_cast<longlong2*>(&node[dd].cl_dy) = make_longlong2(k == 0 ? a0 : a1, k == 0 ? a1 : a0);
       *reinterpret_cast<int4*>(&node[dd].t_dy) =
-          make_int4(k == 0 ? tt.x : tt.y, k == 0 ? tt.y : tt.x, (int)(k == 0 ? bl.x : bl.y),
-                    (int)(k == 0 ? bl.y : bl.x));
-      node[dd].wlen = bl.x + bl.y + a0 + a1;
-      // status, parent, the dying side with what W(d) expands to (its
-      // non-empty chains and raw-arc segments), and the saddle, in one store;
-      // a walk of this round uses no field of a record whose status carries
-      // this round's tag, so the order of these stores does not matter
-      *reinterpret_cast<int4*>(&node[dd].status) =
-          make_int4(status_word(kLinked, rd), k == 0 ? R1 : R0,
-                    side_word(k, (a0 > 0) + (a1 > 0), (bl.x > 0) + (bl.y > 0)), RSIDE(crit_sad)[s]);
+          make_int4(k == 0 ? ar.x : ar.y, k == 0 ? ar.y : ar.x, k == 0 ? ar.z : ar.w, k == 0 ? ar.w : ar.z);
+      // the dying side with what W(d) expands to (its non-empty chains and
+      // raw-arc segments), and the saddle
+      *reinterpret_cast<int2*>(&node[dd].side) =
+          make_int2(side_word(k, (a0 > 0) + (a1 > 0), (ar.z > 0) + (ar.w > 0)), RSIDE(crit_sad)[s]);
+      node_link_set(node, dd, NodeLink{kLinked, k == 0 ? R1 : R0, (long long)ar.z + ar.w + a0 + a1});
     } else {
-      node[dd].status = status_word(kRootForever, rd);
+      node_link_set(node, dd, NodeLink{kRootForever, -1, 0});
+    }
+  };
+  // a chain is at most its side's node count long (a side without arcs takes
+  // no part and has no bound of its own)
+  const int cap = max(P.s[0].max_steps, P.s[1].max_steps);
+  int steps = 0, waited = 0;
+  while (true) {
+    unsigned long long key[2 * U];
+    NodeLink w[2 * U];
+    bool al[2 * U];
+#pragma unroll
+    for (int c = 0; c < 2 * U; ++c) {
+      const bool s1 = (s1m >> (c >> 1)) & 1u;
+      if ((live >> c) & 1u) {  // the alive flag and the record's sector, issued together
+        al[c] = RSIDE(alive)[x[c]];
+        key[c] = __ldcg(&RSIDE(S.node)[x[c]].ctime);
+        w[c] = node_link_live(RSIDE(S.node), x[c]);
+      }
+    }
+    unsigned wait = 0;
+#pragma unroll
+    for (int c = 0; c < 2 * U; ++c) {
+      if (!((live >> c) & 1u)) continue;
+      // never cancelled (its record is not written), or not linked before
+      // this step: the root
+      if (al[c] || key[c] >= tk[c >> 1]) {
+        live &= ~(1u << c);
+        continue;
+      }
+      if (w[c].status == kPending) {
+        wait |= 1u << c;
+        continue;
+      }
+      if (w[c].status == kRootForever) {
+        live &= ~(1u << c);
+        continue;
+      }
+      a[c] += w[c].wlen;
+      x[c] = w[c].parent;
+      if (x[c] < 0) live &= ~(1u << c);
+    }
+    if (WAIT) {
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (((act >> u) & 1u) && !((live >> (2 * u)) & 3u)) decide(u);
+      if (!act) return;
+      if (wait == live && ++waited >= kReplayWait) break;  // only waiting walks are left
+    } else if (wait == live) {
+      break;
+    }
+    if (++steps > 2 * U * (cap + 1) + kReplayWait) {
+      set_status(P.s[0].status, kStatusChainCap);
+      break;
     }
   }
-  // every thread of the block takes part in the reservation (a side without
-  // cancellations reserves nothing and its counter is not touched)
-  const int n0 = __popc(keep & ~s1m), n1 = __popc(keep & s1m);
-  int p0, p1;
-  block_reserve2(P.s[0].cnt + (rd + 1) % 3, n0, P.s[1].cnt + (rd + 1) % 3, n1, p0, p1);
 #pragma unroll
   for (int u = 0; u < U; ++u) {
-    if (!((keep >> u) & 1u)) continue;
+    if (!WAIT && ((act >> u) & 1u) && !((live >> (2 * u)) & 3u)) decide(u);
+    if (!((act >> u) & 1u)) continue;
     const bool s1 = (s1m >> u) & 1u;
-    ((rd & 1) ? RSIDE(act0) : RSIDE(act1))[s1 ? p1++ : p0++] = r[u];
+    *reinterpret_cast<int2*>(RSIDE(wx) + 2 * r[u]) = make_int2(x[2 * u], x[2 * u + 1]);
+    *reinterpret_cast<longlong2*>(RSIDE(wa) + 2 * r[u]) = make_longlong2(a[2 * u], a[2 * u + 1]);
+    chunk_keep(L, s1, r[u]);
   }
 }
 #undef RSIDE
@@ -774,6 +778,7 @@ constexpr int kReplayShapes = 2;
 
 template <int U, int MINB>
 __global__ void __launch_bounds__(256, MINB) replay_persistent_kernel(ReplayArgs2 P) {
+  __shared__ ChunkLists L;
   cg::grid_group grid = cg::this_grid();
   const long long tid = grid.thread_rank(), nth = grid.size();
   for (int sd = 0; sd < 2; ++sd) {
@@ -790,7 +795,7 @@ __global__ void __launch_bounds__(256, MINB) replay_persistent_kernel(ReplayArgs
     }
   }
   grid.sync();
-  bool done0 = false, done1 = false, solo = false;
+  bool done0 = false, done1 = false;
   for (int rd = 0;; ++rd) {
     const int na = P.s[0].n_cancel ? *(volatile int*)(P.s[0].cnt + rd % 3) : 0;
     const int nb = P.s[1].n_cancel ? *(volatile int*)(P.s[1].cnt + rd % 3) : 0;
@@ -812,18 +817,14 @@ __global__ void __launch_bounds__(256, MINB) replay_persistent_kernel(ReplayArgs
     }
     done0 = done0 || na == 0;
     done1 = done1 || nb == 0;
-    if (na == 0 && nb == 0) break;
-    if (!solo && (long long)na + nb <= kReplaySoloItems) {  // block 0 finishes alone
-      solo = true;
-      if (blockIdx.x != 0) break;
-    }
-    const long long t0 = solo ? threadIdx.x : tid, nt = solo ? blockDim.x : nth;
+    const long long n = (long long)na + nb;
+    if (n == 0) break;
     if (rd >= max(P.s[0].max_rounds, P.s[1].max_rounds)) {
       if (tid == 0) set_status(P.s[0].n_cancel ? P.s[0].status : P.s[1].status, kStatusRoundCap);
       // the cancellations still pending are dropped (their dying nodes
       // become roots), so the chain walks of the kernels that run before the
       // host sees the status meet decided nodes only
-      for (long long i = t0; i < (long long)na + nb; i += nt) {
+      for (long long i = tid; i < n; i += nth) {
         const ReplayArgs& A = i < na ? P.s[0] : P.s[1];
         const long long k = i < na ? i : i - na;
         const int r = rd == 0 ? (int)k : ((rd & 1) ? A.act1 : A.act0)[k];
@@ -834,14 +835,23 @@ __global__ void __launch_bounds__(256, MINB) replay_persistent_kernel(ReplayArgs
     if (tid == 0)
       for (int sd = 0; sd < 2; ++sd)
         if (P.s[sd].n_cancel) P.s[sd].cnt[(rd + 2) % 3] = 0;
-    // grid-stride over both sides' pending cancellations, U per thread at a
-    // time (a cancellation decided earlier in the same round is visible to
-    // later walks)
-    for (long long base = 0; base < (long long)na + nb; base += nt * U) replay_batch<U>(P, rd, base + t0, nt, na, nb);
-    if (solo)
-      __syncthreads();
-    else
-      grid.sync();
+    // grid-stride over both sides' pending cancellations (the grid works on
+    // neighbouring ones at any time, which keeps their nodes in L2: contiguous
+    // chunks per block took 366 us instead of 252 for the first round at
+    // 4096^2), with one reservation per kChunkPer strides
+    const bool wait = rd > 0 && n <= nth;
+    for (long long base = 0; base < n; base += nth * kChunkPer) {
+      chunk_start(L);
+      const long long end = min(n, base + nth * kChunkPer);
+      for (long long i0 = base + tid; i0 < end; i0 += nth * U)
+        if (wait)
+          replay_batch<U, true>(P, rd, i0, nth, end, na, L);
+        else
+          replay_batch<U, false>(P, rd, i0, nth, end, na, L);
+      chunk_flush(L, P.s[0].cnt + (rd + 1) % 3, (rd & 1) ? P.s[0].act0 : P.s[0].act1, P.s[1].cnt + (rd + 1) % 3,
+                  (rd & 1) ? P.s[1].act0 : P.s[1].act1);
+    }
+    grid.sync();
   }
 }
 
@@ -902,21 +912,21 @@ __device__ __forceinline__ void emit_batch(const EmitCtx& E, int4* __restrict__ 
       act &= ~live;  // the capped tasks are dropped
       break;
     }
-    longlong2 kl[U];
-    int4 w[U];
+    NodeLink l[U];
+    int2 w[U];
 #pragma unroll
     for (int u = 0; u < U; ++u)
       if ((live >> u) & 1u) {
-        kl[u] = node_keylen(E.S.node, z[u]);
+        l[u] = node_link(E.S.node, z[u]);
         w[u] = node_words(E.S.node, z[u]);
       }
 #pragma unroll
     for (int u = 0; u < U; ++u)
       if ((live >> u) & 1u) {
-        tot[u] += kl[u].y;
-        nc[u] += chains_of(w[u].z);  // counts stored at link time
-        nb[u] += bases_of(w[u].z);
-        z[u] = w[u].y;
+        tot[u] += l[u].wlen;
+        nc[u] += chains_of(w[u].x);  // counts stored at link time
+        nb[u] += bases_of(w[u].x);
+        z[u] = l[u].parent;
         if (z[u] == stop[u] || z[u] < 0) live &= ~(1u << u);
       }
   }
@@ -952,15 +962,16 @@ __device__ __forceinline__ void emit_batch(const EmitCtx& E, int4* __restrict__ 
   for (int u = 0; u < U; ++u)
     if (((act >> u) & 1u) && z[u] != stop[u] && z[u] >= 0) live |= 1u << u;
   while (live) {
-    int4 w[U], te[U];  // (status, parent, side, saddle), (arc ends, raw-arc lengths)
-    long long wl[U];
+    NodeLink l[U];
+    int2 w[U];   // (side, saddle)
+    int4 te[U];  // (arc ends, raw-arc lengths)
     longlong2 cl[U];
 #pragma unroll
     for (int u = 0; u < U; ++u)
       if ((live >> u) & 1u) {  // the node's two sectors, issued together
         const ReplayNode* nd = E.S.node + z[u];
         w[u] = node_words(E.S.node, z[u]);
-        wl[u] = nd->wlen;
+        l[u] = node_link(E.S.node, z[u]);
         cl[u] = *reinterpret_cast<const longlong2*>(&nd->cl_dy);
         te[u] = *reinterpret_cast<const int4*>(&nd->t_dy);
       }
@@ -968,11 +979,11 @@ __device__ __forceinline__ void emit_batch(const EmitCtx& E, int4* __restrict__ 
     for (int u = 0; u < U; ++u) {
       if (!((live >> u) & 1u)) continue;
       // W(z) = reverse(chain(Tk -> z)) + reverse(arc k) + arc o + chain(To -> R)
-      const int d = z[u], k = side_of(w[u].z), s = w[u].w, R = w[u].y;  // s: the saddle's cell
+      const int d = z[u], k = side_of(w[u].x), s = w[u].y, R = l[u].parent;  // s: the saddle's cell
       const int Tk = te[u].x, To = te[u].y;
       const long long la = cl[u].x, lb = te[u].z, lc = te[u].w, ld = cl[u].y;
       const bool rv = (rev >> u) & 1u;
-      const long long at = rv ? pos[u] + tot[u] - off[u] - wl[u] : pos[u] + off[u];
+      const long long at = rv ? pos[u] + tot[u] - off[u] - l[u].wlen : pos[u] + off[u];
       int& q = pc[u];
       int& qb = pbc[u];
       if (!rv) {
@@ -986,8 +997,8 @@ __device__ __forceinline__ void emit_batch(const EmitCtx& E, int4* __restrict__ 
         if (lb > 0) E.base_q[qb++] = make_saddle_seg(s, k, 0, lb, at + ld + lc);
         if (la > 0) q_out[q++] = make_task(kTaskChain, 0, Tk, d, at + ld + lc + lb);
       }
-      off[u] += wl[u];
-      z[u] = w[u].y;
+      off[u] += l[u].wlen;
+      z[u] = l[u].parent;
       if (z[u] == stop[u] || z[u] < 0) live &= ~(1u << u);
     }
   }

@@ -35,27 +35,22 @@ namespace dmsc {
 
 constexpr unsigned long long kNever = ~0ull;  // replay key of a node that is never cancelled
 enum : int { kPending = 0, kLinked = 1, kRootForever = 2 };
-// A replay status word is kind | tag << 2; a decision made in replay round r
-// carries tag r + 1 (the initial kRootForever of never-cancelled nodes has
-// tag 0). Walks in round r use only decisions with tag <= r: those were
-// written before the grid barrier that opened round r, which orders them, so
-// plain (L2) loads see them complete and no acquire/release is needed.
-__device__ __forceinline__ int status_kind(int st) { return st & 3; }
-__device__ __forceinline__ int status_word(int kind, int round) { return kind | ((round + 1) << 2); }
 
-// A replay node in one 64-byte line: everything a chain walk reads, in the
-// first 32-byte sector as two 16-byte halves, (ctime, wlen) and (status,
-// parent, side, saddle cell); in the second, what the emission needs to expand
-// W(node) without touching the saddle's arrays: the two chain lengths, the
-// saddle's arc ends on the dying and the other side and their raw-arc
-// lengths (written at link time).
+// A replay node in one 64-byte line. The first 32-byte sector holds all that a
+// chain walk reads: its key with the emission's words, and the link (status,
+// parent, length of W(node)) in 16 bytes that are written and read as one, so
+// a walk that sees the status sees the whole decision, in the round in which
+// it is made, with no fence. The second sector holds what the emission needs
+// to expand W(node) without touching the saddle's arrays: the two chain
+// lengths, the saddle's arc ends on the dying and the other side and their
+// raw-arc lengths (written before the kernel ends, read by later kernels).
 struct alignas(64) ReplayNode {
   unsigned long long ctime;  // replay key of the cancellation killing the node, kNever if none
-  long long wlen;            // length of W(node)
-  int status;                // kPending / kLinked / kRootForever, with the deciding round's tag
-  int parent;                // link target (-1 = void) when kLinked
   int side;                  // side_word: dying side of the node's cancellation and what W(node) expands to
   int scell;                 // global cell id of the saddle of the node's cancellation
+  int status;                // kPending / kLinked / kRootForever
+  int parent;                // link target (-1 = void) when kLinked
+  long long wlen;            // length of W(node)
   long long cl_dy;           // chain length T_dying -> node at link time
   long long cl_ot;           // chain length T_other -> parent at link time
   int t_dy, t_ot;            // the saddle's arc ends on the dying and the other side
@@ -67,16 +62,43 @@ struct ReplayState {
   ReplayNode* node;  // [M + 1]
 };
 
-// The halves of a node's record: through L2 inside the replay (other blocks
-// write records during the launch), plain loads after it.
-__device__ __forceinline__ longlong2 node_keylen_cg(const ReplayNode* n, int x) {
-  return __ldcg(reinterpret_cast<const longlong2*>(&n[x].ctime));
+struct NodeLink {
+  int status, parent;
+  long long wlen;
+};
+// The link while other blocks may be writing it (one 16-byte access through
+// L2), and after the replay.
+__device__ __forceinline__ NodeLink node_link_live(const ReplayNode* n, int x) {
+  unsigned long long lo, hi;
+  asm volatile(
+      "{\n"
+      ".reg .b128 t;\n"
+      "ld.relaxed.gpu.global.b128 t, [%2];\n"
+      "mov.b128 {%0, %1}, t;\n"
+      "}\n"
+      : "=l"(lo), "=l"(hi)
+      : "l"(__cvta_generic_to_global(&n[x].status))
+      );
+  return NodeLink{(int)(unsigned)lo, (int)(unsigned)(lo >> 32), (long long)hi};
 }
-__device__ __forceinline__ longlong2 node_keylen(const ReplayNode* n, int x) {
-  return *reinterpret_cast<const longlong2*>(&n[x].ctime);
+__device__ __forceinline__ void node_link_set(ReplayNode* n, int x, NodeLink l) {
+  const unsigned long long lo = (unsigned)l.status | (unsigned long long)(unsigned)l.parent << 32;
+  asm volatile(
+      "{\n"
+      ".reg .b128 t;\n"
+      "mov.b128 t, {%1, %2};\n"
+      "st.relaxed.gpu.global.b128 [%0], t;\n"
+      "}\n" ::"l"(__cvta_generic_to_global(&n[x].status)),
+      "l"(lo), "l"((unsigned long long)l.wlen)
+      );
 }
-__device__ __forceinline__ int4 node_words(const ReplayNode* n, int x) {
-  return *reinterpret_cast<const int4*>(&n[x].status);
+__device__ __forceinline__ NodeLink node_link(const ReplayNode* n, int x) {
+  const int4 v = *reinterpret_cast<const int4*>(&n[x].status);
+  return NodeLink{v.x, v.y, (long long)((unsigned long long)(unsigned)v.w << 32 | (unsigned)v.z)};
+}
+// The emission's words (side, saddle cell).
+__device__ __forceinline__ int2 node_words(const ReplayNode* n, int x) {
+  return *reinterpret_cast<const int2*>(&n[x].side);
 }
 
 // Node records are written only for the nodes a cancellation kills: the
@@ -102,14 +124,13 @@ __device__ __forceinline__ bool walk_root(const ReplayState& S, const uint8_t* _
   long long a = 0;
   int steps = 0;
   while (x >= 0 && !alive[x]) {
-    const longlong2 kl = node_keylen(S.node, x);
-    const int4 w = node_words(S.node, x);
-    if ((unsigned long long)kl.x >= t) break;
-    const int st = status_kind(w.x);
-    if (st == kPending) return false;
-    if (st == kRootForever) break;
-    a += kl.y;
-    x = w.y;
+    const unsigned long long key = S.node[x].ctime;
+    const NodeLink l = node_link(S.node, x);
+    if (key >= t) break;
+    if (l.status == kPending) return false;
+    if (l.status == kRootForever) break;
+    a += l.wlen;
+    x = l.parent;
     if (++steps > max_steps) {
       set_status(status, kStatusChainCap);
       break;
