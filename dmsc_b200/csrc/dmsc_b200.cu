@@ -765,7 +765,7 @@ int bits_for(int n) {
   return b;
 }
 
-void emit_expand(dmsc_b200_context* ctx, int si, Side& S, cudaStream_t st);
+void emit_expand(dmsc_b200_context* ctx, cudaStream_t st);
 
 int extract_batch_impl(dmsc_b200_context* ctx, int B, const float* img, const int* hH, const int* hW,
                        const float* hthr, const unsigned char* hdual, unsigned flags, int32_t* grad_out,
@@ -1207,70 +1207,78 @@ int extract_batch_impl(dmsc_b200_context* ctx, int B, const float* img, const in
   // the geometry's chain expansion needs no output buffer: it runs now,
   // while the caller allocates the outputs of the fetch
   mark(ctx, 17, st);
-  for (int si = 0; si < 2; ++si) emit_expand(ctx, si, ctx->side[si], st);
+  emit_expand(ctx, st);
   mark(ctx, 18, st);
   ctx->valid = true;
   return kOk;
 }
 
-// Geometry of one side, first half (end of extract, before the caller has
-// allocated the outputs): the arcs' image-local positions and the
-// breadth-first chain expansion into the segment list. The writer runs in
-// fetch (emit_write); the device runs this while the host allocates.
-void emit_expand(dmsc_b200_context* ctx, int si, Side& S, cudaStream_t st) {
+// Geometry, first half (end of extract, before the caller has allocated the
+// outputs): the breadth-first chain expansion of both sides into their segment
+// lists. The writer runs in fetch (emit_write); the device runs this while
+// the host allocates.
+void emit_expand(dmsc_b200_context* ctx, cudaStream_t st) {
   const int nsurv = ctx->nsurv;
-  ctx->expanded[si] = false;
-  if (!S.arcs || S.total <= 0 || nsurv <= 0) return;
-  const long long cap = S.total;
-  EmitArgs& A = ctx->emit[si];
-  A = EmitArgs{};
-  EmitCtx& E = A.E;
-  E.flow = ctx->flow;
-  E.I = ctx->I;
-  E.faces = S.faces;
-  E.S = S.R;
-  E.q_cap = cap;
-  E.max_steps = ctx->nsad + 1;
-  E.status = ctx->status;
-  A.nsurv = nsurv;
-  E.nvirt = 2 * nsurv;
-  E.head = ctx->head;
-  E.arc = S.s_arc;
-  E.fin = S.s_fin;
-  E.lens = ctx->lens;
-  E.gbase = S.gbase;
-  A.q0 = sget<int4>(ctx, si, X_Q0, cap);
-  A.q1 = sget<int4>(ctx, si, X_Q1, cap);
-  A.cnt = sget<int>(ctx, si, X_CNT, 8);
-  E.base_q = sget<int4>(ctx, si, X_QB, cap);
-  E.base_cap = cap;
-  A.max_levels = capped(ctx->nsad + 4, ctx->cap_emit_levels);
-  A.levels = get<int>(ctx, S_STATS, 8) + 4 + si;
-  A.timeline = get<unsigned long long>(ctx, S_TIMELINE, kTimelineSlots) + (2 + si) * kTimeline;
-  coop_launch(ctx, ctx->emit_shape ? emit_persistent_kernel<2, 3> : emit_persistent_kernel<1, 5>, A, st,
-              "emit_persistent_kernel", ctx->emit_per_sm);
-  ctx->expanded[si] = true;
+  EmitArgs2 P{};
+  long long most = 0;
+  for (int si = 0; si < 2; ++si) {
+    Side& S = ctx->side[si];
+    ctx->expanded[si] = S.arcs && S.total > 0 && nsurv > 0;
+    if (!ctx->expanded[si]) continue;
+    const long long cap = S.total;
+    EmitArgs& A = P.s[si];
+    EmitCtx& E = A.E;
+    E.flow = ctx->flow;
+    E.I = ctx->I;
+    E.faces = S.faces;
+    E.S = S.R;
+    E.q_cap = cap;
+    E.max_steps = ctx->nsad + 1;
+    E.status = ctx->status;
+    A.nsurv = nsurv;
+    E.nvirt = 2 * nsurv;
+    E.head = ctx->head;
+    E.arc = S.s_arc;
+    E.fin = S.s_fin;
+    E.lens = ctx->lens;
+    E.gbase = S.gbase;
+    A.q0 = sget<int4>(ctx, si, X_Q0, cap);
+    A.q1 = sget<int4>(ctx, si, X_Q1, cap);
+    A.cnt = sget<int>(ctx, si, X_CNT, 8);
+    E.base_q = sget<int4>(ctx, si, X_QB, cap);
+    E.base_cap = cap;
+    A.max_levels = capped(ctx->nsad + 4, ctx->cap_emit_levels);
+    A.levels = get<int>(ctx, S_STATS, 8) + 4 + si;
+    A.timeline = get<unsigned long long>(ctx, S_TIMELINE, kTimelineSlots) + (2 + si) * kTimeline;
+    ctx->emit[si] = A;
+    most += cap;
+  }
+  // few tasks for small geometry: a grid barrier costs less on fewer blocks
+  if (most > 0)
+    coop_launch(ctx, ctx->emit_shape ? emit_persistent_kernel<2, 3> : emit_persistent_kernel<1, 5>, P, st,
+                "emit_persistent_kernel", ctx->emit_per_sm, (int)std::min<long long>(2 + most / 512, 1 << 20));
 }
 
-// Geometry of one side, second half (fetch): the writer of every raw-arc
-// segment into the caller's arrays (`dst_off[b]`: image b's start in its
-// destination).
-void emit_write(dmsc_b200_context* ctx, int si, Side& S, int32_t* flat_primal, int32_t* flat_dual, const int* dst_off,
-                cudaStream_t st) {
-  if (!ctx->expanded[si] || (!flat_primal && !flat_dual)) return;
-  EmitArgs& A = ctx->emit[si];
-  EmitCtx E = A.E;
-  E.out_primal = flat_primal;
-  E.out_dual = flat_dual;
-  E.dst_off = dst_off;
-  int per = 0;
-  if (ctx->seg_cursors == 1) {
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, emit_segments_kernel<1>, 256, 0));
-    LK(emit_segments_kernel<1><<<dim3(per * ctx->num_sms * 4), 256, 0, st>>>(E, A.cnt + 3));
-  } else {
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, emit_segments_kernel<2>, 256, 0));
-    LK(emit_segments_kernel<2><<<dim3(per * ctx->num_sms * 4), 256, 0, st>>>(E, A.cnt + 3));
+// Geometry, second half (fetch): the writer of every raw-arc segment into the
+// caller's arrays (out[side][orientation]; `dst_off[side][b]`: image b's start
+// in its destination).
+void emit_write(dmsc_b200_context* ctx, int32_t* const (*out)[2], const int* const* dst_off, cudaStream_t st) {
+  SegArgs A{};
+  bool any = false;
+  for (int si = 0; si < 2; ++si) {
+    if (!ctx->expanded[si] || (!out[si][0] && !out[si][1])) continue;
+    any = true;
+    A.E[si] = ctx->emit[si].E;
+    A.E[si].out_primal = out[si][0];
+    A.E[si].out_dual = out[si][1];
+    A.E[si].dst_off = dst_off[si];
+    A.count[si] = ctx->emit[si].cnt + 3;
   }
+  if (!any) return;
+  int per = 0;
+  auto kernel = ctx->seg_cursors == 1 ? emit_segments_kernel<1> : emit_segments_kernel<2>;
+  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, 256, 0));
+  LK(kernel<<<dim3(per * ctx->num_sms * 4, 2), 256, 0, st>>>(A));
   LAUNCH_CHECK("emit_segments_kernel");
 }
 
@@ -1377,9 +1385,8 @@ int fetch_batch_impl(dmsc_b200_context* ctx, const dmsc_b200_outputs* o, cudaStr
   if (ctx->host_fetch_set)  // lists and per-saddle outputs are final: copy them while the geometry is built
     for (int k = 0; k < 9; ++k) copy_out_async(ctx, host_f[k], dev_f[k], 4 * (size_t)tot_n[k], st);
   // arc geometry
-  for (int si = 0; si < 2; ++si)
-    if (ctx->side[si].arcs)
-      emit_write(ctx, si, ctx->side[si], geom_out[si][0], geom_out[si][1], rt_of(si == 0 ? R_G0 : R_G1), st);
+  const int* const dst_off[2] = {rt_of(R_G0), rt_of(R_G1)};
+  emit_write(ctx, geom_out, dst_off, st);
   mark(ctx, 14, st);
   if (ctx->host_fetch_set)
     for (int k = 9; k < 15; ++k) copy_out_async(ctx, host_f[k], dev_f[k], 4 * (size_t)tot_n[k], st);

@@ -868,6 +868,10 @@ struct EmitArgs {
   int* levels;                   // receives the number of levels (statistics)
   unsigned long long* timeline;  // [kTimeline] level start times (ns), optional
 };
+// Both sides; a side with no geometry has cnt == nullptr.
+struct EmitArgs2 {
+  EmitArgs s[2];
+};
 
 // One batch of a thread's chain tasks at one expansion level, in[i0 + nt u]
 // (u < U) below n: the U chains are counted in lockstep (one node-record load
@@ -1006,22 +1010,24 @@ __device__ __forceinline__ void emit_batch(const EmitCtx& E, int4* __restrict__ 
 // Expansion shapes (tuned): U = 1 with 5 resident blocks per SM, U = 2 with 3.
 constexpr int kEmitShapes = 2;
 
-// Geometry of one side: breadth-first expansion of the chain and W tasks
-// (replay.cuh), collecting the raw-arc segments with their output positions,
-// then one parallel pass that walks and writes every segment.
+// Geometry: breadth-first expansion of both sides' chain and W tasks
+// (replay.cuh), collecting the raw-arc segments with their output positions.
+// Levels are chain depths and most are bound by the latency of their longest
+// chain, so the two sides share every level (and its grid barrier): at each
+// level the blocks are split between them by their task counts, and a level's
+// tasks go to the warps of all its blocks, 32 at a time. The geometry stage
+// with a launch per side and together: 0.344 -> 0.182 ms at 2048^2, threshold
+// 0.25, 0.187 -> 0.106 at 256^2, 0.573 -> 0.420 on 1080 x 1920 pixels of 256
+// levels, 1.10 -> 0.98 at 4096^2, threshold 0.05.
 template <int U, int MINB>
-__global__ void __launch_bounds__(256, MINB) emit_persistent_kernel(EmitArgs A) {
+__global__ void __launch_bounds__(256, MINB) emit_persistent_kernel(EmitArgs2 P) {
   cg::grid_group grid = cg::this_grid();
-  const long long tid = grid.thread_rank(), nth = grid.size();
-  if (tid == 0) {
-    A.cnt[0] = 0;
-    A.cnt[1] = 0;
-    A.cnt[2] = 0;
-    A.cnt[3] = 0;
+  const long long tid = grid.thread_rank();
+  if (tid < 8) {
+    const EmitArgs& A = tid < 4 ? P.s[0] : P.s[1];
+    if (A.cnt) A.cnt[tid & 3] = 0;
   }
   grid.sync();
-  const EmitCtx& E = A.E;
-  int* const n_base = A.cnt + 3;
   // level 0: the chain of each surviving arc (its own raw arc is a segment
   // item of the writer, read from the survivor records). A block takes
   // kLevel0 survivors per thread at a time: it counts their chains, reserves
@@ -1030,68 +1036,108 @@ __global__ void __launch_bounds__(256, MINB) emit_persistent_kernel(EmitArgs A) 
   // per 256 (each reservation waits on the atomic's return).
   constexpr int kLevel0 = 8;
   const long long span = (long long)blockDim.x * kLevel0;
-  for (long long base = (long long)blockIdx.x * span; base < A.nsurv; base += (long long)gridDim.x * span) {
-    // a chain exists only on arcs that the image's output takes (length 0 otherwise)
-    int mine = 0;
+#pragma unroll 1
+  for (int sd = 0; sd < 2; ++sd) {
+    const EmitArgs& A = sd ? P.s[1] : P.s[0];
+    const EmitCtx& E = A.E;
+    if (!A.cnt) continue;
+    for (long long base = (long long)blockIdx.x * span; base < A.nsurv; base += (long long)gridDim.x * span) {
+      // a chain exists only on arcs that the image's output takes (length 0 otherwise)
+      int mine = 0;
 #pragma unroll
-    for (int k = 0; k < kLevel0; ++k) {
-      const long long i = base + (long long)k * blockDim.x + threadIdx.x;
-      if (i >= A.nsurv) continue;
-      const int2 cl = *reinterpret_cast<const int2*>(E.fin + i);
-      mine += (cl.x > 0) + (cl.y > 0);
-    }
-    // most arcs have no chain (at threshold 0 nearly all): a block reserves
-    // queue slots only when one of its threads has a task
-    if (!__syncthreads_or(mine > 0)) continue;
-    int p, pb;
-    block_reserve2(A.cnt, mine, n_base, 0, p, pb);
-    if (mine == 0) continue;
-    for (int k = 0; k < kLevel0; ++k) {
-      const long long i = base + (long long)k * blockDim.x + threadIdx.x;
-      if (i >= A.nsurv) break;
-      const int4 fin = E.fin[i];
-      if (fin.x <= 0 && fin.y <= 0) continue;
-      const int4 a = E.arc[i];
-      const int pos = surv_start(E, (int)i, E.head[i].img);
+      for (int k = 0; k < kLevel0; ++k) {
+        const long long i = base + (long long)k * blockDim.x + threadIdx.x;
+        if (i >= A.nsurv) continue;
+        const int2 cl = *reinterpret_cast<const int2*>(E.fin + i);
+        mine += (cl.x > 0) + (cl.y > 0);
+      }
+      // most arcs have no chain (at threshold 0 nearly all): a block reserves
+      // queue slots only when one of its threads has a task
+      if (!__syncthreads_or(mine > 0)) continue;
+      int p, pb;
+      block_reserve2(A.cnt, mine, A.cnt + 3, 0, p, pb);
+      if (mine == 0) continue;
+      for (int k = 0; k < kLevel0; ++k) {
+        const long long i = base + (long long)k * blockDim.x + threadIdx.x;
+        if (i >= A.nsurv) break;
+        const int4 fin = E.fin[i];
+        if (fin.x <= 0 && fin.y <= 0) continue;
+        const int4 a = E.arc[i];
+        const int pos = surv_start(E, (int)i, E.head[i].img);
 #pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        if ((j ? fin.y : fin.x) <= 0) continue;
-        if (p < E.q_cap)
-          A.q0[p] = make_task(kTaskChain, 0, j ? a.y : a.x, j ? fin.w : fin.z, pos + a.z + (j ? fin.x + a.w : 0));
-        else
-          set_status(E.status, kStatusQueueOverflow);
-        ++p;
+        for (int j = 0; j < 2; ++j) {
+          if ((j ? fin.y : fin.x) <= 0) continue;
+          if (p < E.q_cap)
+            A.q0[p] = make_task(kTaskChain, 0, j ? a.y : a.x, j ? fin.w : fin.z, pos + a.z + (j ? fin.x + a.w : 0));
+          else
+            set_status(E.status, kStatusQueueOverflow);
+          ++p;
+        }
       }
     }
   }
   grid.sync();
-  bool solo = false;
+  bool solo = false, done[2] = {false, false};
   for (int lv = 0;; ++lv) {
-    int n = *(volatile int*)(A.cnt + lv % 3);
-    if (tid == 0 && A.timeline && lv < kTimeline - 2) {
-      A.timeline[lv] = global_ns();
-      A.timeline[kTimelineCounts + lv] = n;
+    int n[2];
+#pragma unroll
+    for (int sd = 0; sd < 2; ++sd) {
+      const EmitArgs& A = sd ? P.s[1] : P.s[0];
+      // in the solo levels the other side's counters are its own block's
+      n[sd] = A.cnt && !(solo && (int)blockIdx.x != sd) ? *(volatile int*)(A.cnt + lv % 3) : 0;
+      if (!A.cnt || (solo ? threadIdx.x != 0 || (int)blockIdx.x != sd : tid != 0) || done[sd]) continue;
+      if (A.timeline && lv < kTimeline - 2) {
+        A.timeline[lv] = global_ns();
+        A.timeline[kTimelineCounts + lv] = n[sd];
+      }
+      if (n[sd] == 0) {
+        if (A.levels) *A.levels = lv;
+        done[sd] = true;
+      }
     }
-    if (n == 0) {
-      if (tid == 0 && A.levels) *A.levels = lv;
-      break;
+    if (n[0] == 0 && n[1] == 0) break;
+    bool over = false;
+#pragma unroll
+    for (int sd = 0; sd < 2; ++sd) {
+      const EmitArgs& A = sd ? P.s[1] : P.s[0];
+      if (n[sd] == 0 || (lv < A.max_levels && n[sd] <= A.E.q_cap)) continue;
+      over = true;
+      if (solo ? threadIdx.x == 0 : tid == 0)
+        set_status(A.E.status, lv >= A.max_levels ? kStatusRoundCap : kStatusQueueOverflow);
     }
-    if (lv >= A.max_levels || n > E.q_cap) {
-      if (tid == 0) set_status(E.status, lv >= A.max_levels ? kStatusRoundCap : kStatusQueueOverflow);
-      break;
-    }
-    // a level of at most one task per thread of a block finishes the
-    // expansion in block 0 alone (each task is one thread's work either way)
-    if (!solo && n <= 256) {
+    if (over) break;  // every thread leaves: the counters are the same for all
+    // levels of at most one task per thread of a block finish in one block
+    // per side (each task is one thread's work either way)
+    if (!solo && n[0] <= 256 && n[1] <= 256) {
       solo = true;
-      if (blockIdx.x != 0) break;
+      if (blockIdx.x >= 2) break;
+      if (n[blockIdx.x] == 0) break;
     }
-    const long long t0 = solo ? threadIdx.x : tid, nt = solo ? blockDim.x : nth;
+    // this block's side, and its place among that side's blocks
+    int sd = (int)blockIdx.x, at = 0, blocks = 1;
+    if (!solo) {
+      const int g = (int)gridDim.x;
+      int g0 = (int)((long long)g * n[0] / ((long long)n[0] + n[1]));
+      if (n[0] && n[1]) g0 = min(g - 1, max(1, g0));
+      sd = (int)blockIdx.x >= g0;
+      at = sd ? (int)blockIdx.x - g0 : (int)blockIdx.x;
+      blocks = sd ? g - g0 : g0;
+    }
+    const EmitArgs& A = sd ? P.s[1] : P.s[0];
     const int4* in = (lv & 1) ? A.q1 : A.q0;
     int4* q_out = (lv & 1) ? A.q0 : A.q1;
-    int* n_out = A.cnt + (lv + 1) % 3;
-    if (tid == 0) A.cnt[(lv + 2) % 3] = 0;
-    for (long long base = 0; base < n; base += nt * U) emit_batch<U>(E, q_out, n_out, n_base, in, base + t0, nt, n);
+    if (solo ? threadIdx.x == 0 : tid == 0) {
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const EmitArgs& C = k ? P.s[1] : P.s[0];
+        if (C.cnt && (!solo || k == sd)) C.cnt[(lv + 2) % 3] = 0;
+      }
+    }
+    const int ns = sd ? n[1] : n[0];
+    const long long nt = (long long)blocks * 256;
+    const long long t0 = ((long long)(threadIdx.x >> 5) * blocks + at) * 32 + (threadIdx.x & 31);
+    for (long long base = 0; base < ns; base += nt * U)
+      emit_batch<U>(A.E, q_out, A.cnt + (lv + 1) % 3, A.cnt + 3, in, base + t0, nt, ns);
     if (solo)
       __syncthreads();
     else
@@ -1111,8 +1157,17 @@ constexpr int kSegRange = 128;
 constexpr int kSegSteps = 4;
 constexpr int kSegCursorShapes = 2;  // NC = 1 or 2 (tuned)
 
+struct SegArgs {
+  EmitCtx E[2];
+  const int* count[2];  // nullptr: nothing to write on this side
+};
+
+// Both sides in one launch (blockIdx.y).
 template <int NC>
-__global__ void __launch_bounds__(256) emit_segments_kernel(EmitCtx E, const int* __restrict__ count) {
+__global__ void __launch_bounds__(256) emit_segments_kernel(SegArgs A) {
+  const EmitCtx& E = blockIdx.y ? A.E[1] : A.E[0];
+  const int* count = blockIdx.y ? A.count[1] : A.count[0];
+  if (!count) return;
   const long long nb = E.nvirt + min((long long)*count, E.base_cap);
   const int lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
