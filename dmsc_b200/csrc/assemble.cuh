@@ -35,35 +35,25 @@ struct RouteF {
   }
 };
 
-// Surviving extrema, image-local cell ids, into the routed point lists.
-__global__ void points_kernel(int n, const uint8_t* __restrict__ alive, const int* __restrict__ to_out_excl,
-                              const int* __restrict__ alive_base, const int2* __restrict__ key,
-                              const int* __restrict__ ext_img, Imgs I, Route R) {
-  int x = blockIdx.x * blockDim.x + threadIdx.x;
-  if (x >= n || !alive[x]) return;
-  int b = ext_img[x];
-  int* dst = R.at(I.dual[b], b);
-  if (dst) dst[to_out_excl[x] - alive_base[b]] = key[x].y - 4 * I.idx_base[b];
-}
+// Surviving extrema of both sides (blockIdx.y), image-local cell ids, into the
+// routed point lists.
+struct PointSide {
+  int n;
+  const uint8_t* alive;
+  const int* rank;
+  const int* alive_base;
+  const int2* key;
+  const int* ext_img;
+  Route out;
+};
 
-// Survivor count and first survivor of every image, from the exclusive scan
-// `pos` of the survivors' flags; the count, the two cancellation counts and
-// the status word go straight to the mapped readback area.
-__global__ void survivor_base_kernel(int B, const int* __restrict__ sad_base, int nsad,
-                                     const uint8_t* __restrict__ survive, const int* __restrict__ pos,
-                                     const int* __restrict__ n_cancel, const unsigned* __restrict__ status,
-                                     int* __restrict__ surv_base, long long* __restrict__ rb) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b > B) return;
-  const int total = nsad > 0 ? pos[nsad - 1] + survive[nsad - 1] : 0;
-  const int f = b < B ? sad_base[b] : nsad;
-  surv_base[b] = f < nsad ? pos[f] : total;
-  if (b == 0) {
-    rb[0] = total;
-    rb[1] = n_cancel[0];
-    rb[2] = n_cancel[1];
-    rb[3] = *status;
-  }
+__global__ void points_kernel(PointSide F, PointSide V, Imgs I) {
+  const PointSide& S = blockIdx.y ? V : F;
+  const int x = blockIdx.x * blockDim.x + threadIdx.x;
+  if (x >= S.n || !S.alive[x]) return;
+  const int b = S.ext_img[x];
+  int* dst = S.out.at(I.dual[b], b);
+  if (dst) dst[S.rank[x] - S.alive_base[b]] = S.key[x].y - 4 * I.idx_base[b];
 }
 
 // Image, global cell and list index of a survivor, in output order.
@@ -85,33 +75,8 @@ __global__ void survivor_gather_kernel(int nsad, const uint8_t* __restrict__ fla
   idx_out[pos[s]] = s;
 }
 
-// Per-image first positions (B + 1 entries, the last one the total):
-// base[b] = excl[first[b]] where first[] are the image's first items.
-__global__ void image_base_kernel(int B, const int* __restrict__ first, int n_items, const int* __restrict__ excl,
-                                  int total, int* __restrict__ base) {
-  int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b > B) return;
-  int f = b < B ? first[b] : n_items;
-  base[b] = f < n_items ? excl[f] : total;
-}
-
-// First rank of each image's alive extrema on both sides (B + 1 entries, the
-// last one the side's total), from the scan over both sides' flags.
-__global__ void alive_base_kernel(int B, int M0, int M1, const int* __restrict__ first0, const int* __restrict__ first1,
-                                  const int* __restrict__ rank, const uint8_t* __restrict__ alive,
-                                  int* __restrict__ base0, int* __restrict__ base1) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b > B) return;
-  const int n = M0 + M1;
-  const int total = n > 0 ? rank[n - 1] + alive[n - 1] : 0;
-  const int f0 = b < B ? first0[b] : M0, f1 = M0 + (b < B ? first1[b] : M1);
-  base0[b] = f0 < n ? rank[f0] : total;
-  base1[b] = f1 < n ? rank[f1] : total;
-}
-
-// Two 32-bit counts scanned at once in one 64-bit sum: side 0 in the low half,
-// side 1 in the high half (a total of 2^31 or more fails the call, so no count
-// that is used ever carries).
+// Two 32-bit counts in one word: side 0 in the low half, side 1 in the high
+// half (a total of 2^31 or more fails the call).
 __device__ __forceinline__ unsigned long long pack2(unsigned f, unsigned v) { return f | (unsigned long long)v << 32; }
 __device__ __forceinline__ int half_of(unsigned long long p, int sd) { return (int)(unsigned)(sd ? p >> 32 : p); }
 

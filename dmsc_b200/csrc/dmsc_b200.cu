@@ -15,7 +15,6 @@
 #include <chrono>
 #include <cub/cub.cuh>
 #include <cudaTypedefs.h>
-#include <thrust/iterator/transform_iterator.h>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -31,6 +30,7 @@
 #include "persistent.cuh"
 #include "replay.cuh"
 #include "pairs.cuh"
+#include "scan.cuh"
 #include "walks.cuh"
 
 using namespace dmsc;
@@ -39,10 +39,10 @@ namespace {
 
 
 enum Slot {
-  S_MASK, S_FLOW, S_SEG0, S_SEG1, S_SEG2, S_OFF0, S_OFF1, S_OFF2, S_TOT, S_TAB, S_BASES,
+  S_MASK, S_FLOW, S_SEG0, S_SEG1, S_SEG2, S_OFF0, S_OFF1, S_OFF2, S_TAB, S_BASES, S_ZERO, S_SCAN,
   S_CSAD, S_IMIN, S_ISAD, S_IMAX, S_MINBITS, S_MAXBITS, S_KMIN, S_KMAX, S_SVAL, S_SKEY2, S_IOTA,
-  S_ASC, S_ARC, S_ALIVE, S_RANK, S_FLAG, S_FPOS, S_STATUS, S_NCANC, S_STATS, S_TIMELINE, S_ROUTE,
-  S_BKEY, S_BIDX, S_BKEY2, S_BIDX2, S_PERF, S_PERV, S_EXF, S_EXV, S_NEX, S_SKEY32B, S_SKEYS,
+  S_ASC, S_ARC, S_ALIVE, S_RANK, S_FLAG, S_FPOS, S_NCANC, S_ROUTE,
+  S_BKEY, S_BIDX, S_BKEY2, S_BIDX2, S_PERF, S_PERV, S_EXF, S_EXV, S_SKEY32B, S_SKEYS,
   S_SHEAD, S_LENS, S_ROWS, S_PP,
   S_SIDE0,  // per-side slots start here, kSideSlots each
 };
@@ -56,6 +56,16 @@ enum SideSlot {
 struct Buf {
   void* p = nullptr;
   size_t cap = 0;
+};
+
+// Small device state that starts a call as zero (one fill).
+struct ZeroArea {
+  unsigned status[4];
+  int stats[8];                  // rounds of the device loops, the pairing's handover round
+  int n_exits[4];                // cells whose label paths leave their tile
+  int total[4];                  // alive extrema of both sides, survivors
+  unsigned long long geom[2];    // exact geometry cells of each side
+  unsigned long long timeline[kTimelineSlots];
 };
 
 // Device-side per-image bases (B + 1 entries each) of the last extract.
@@ -122,7 +132,9 @@ struct dmsc_b200_context {
   SurvHead* head = nullptr;  // [nsurv] image, cell and list index of each survivor (output order)
   unsigned long long* lens = nullptr;  // [nsurv + 1] where its geometry starts (both sides packed)
   unsigned long long* rows = nullptr;  // [nsurv + 1] and its e rows
+  ZeroArea* zero = nullptr;
   unsigned* status = nullptr;
+  unsigned scan_epoch = 0;
   Side side[2];
   std::vector<dmsc_b200_sizes> sizes;
   std::vector<long long> geom[2];  // per-image geometry lengths of each side
@@ -183,13 +195,6 @@ struct dmsc_b200_context {
 
 
 namespace dmsc {
-
-__global__ void totals3_kernel(const int* o0, const int* s0, const int* o1, const int* s1, const int* o2,
-                               const int* s2, long long n, long long* out) {
-  out[0] = (long long)o0[n - 1] + s0[n - 1];
-  out[1] = (long long)o1[n - 1] + s1[n - 1];
-  out[2] = (long long)o2[n - 1] + s2[n - 1];
-}
 
 // 32-bit words from device memory into the mapped readback area.
 __global__ void copy_words_kernel(const uint32_t* __restrict__ src, uint32_t* __restrict__ dst, int n) {
@@ -268,24 +273,23 @@ void* cub_tmp(dmsc_b200_context* ctx, size_t bytes, cudaStream_t st) {
   return b.p;
 }
 
-template <class It, class Out>
-void excl_sum(dmsc_b200_context* ctx, It in, Out* out, int n, cudaStream_t st) {
+// One scan launch (scan.cuh) over n items on `st`.
+template <int V, class Op>
+void scan(dmsc_b200_context* ctx, Op op, long long n, cudaStream_t st) {
   if (n <= 0) return;
-  size_t bytes = 0;
-  CK(cub::DeviceScan::ExclusiveSum(nullptr, bytes, in, out, n, st));
-  void* tmp = cub_tmp(ctx, bytes, st);
-  CK(cub::DeviceScan::ExclusiveSum(tmp, bytes, in, out, n, st));
-  ++ctx->launches;
-}
-
-template <class In, class Out>
-void incl_sum(dmsc_b200_context* ctx, const In* in, Out* out, int n, cudaStream_t st) {
-  if (n <= 0) return;
-  size_t bytes = 0;
-  CK(cub::DeviceScan::InclusiveSum(nullptr, bytes, in, out, n, st));
-  void* tmp = cub_tmp(ctx, bytes, st);
-  CK(cub::DeviceScan::InclusiveSum(tmp, bytes, in, out, n, st));
-  ++ctx->launches;
+  const long long tiles = (n + kScanTile - 1) / kScanTile;
+  const size_t words = 1 + (size_t)V * tiles;
+  const size_t had = ctx->bufs.size() > (size_t)S_SCAN ? ctx->bufs[S_SCAN].cap : 0;
+  unsigned long long* w = get<unsigned long long>(ctx, S_SCAN, words);
+  if (ctx->bufs[S_SCAN].cap != had) {  // a new buffer: no word carries an epoch yet
+    CK(cudaMemsetAsync(w, 0, ctx->bufs[S_SCAN].cap, st));
+    ctx->scan_epoch = 0;
+  }
+  ctx->scan_epoch = (ctx->scan_epoch + 1) & 0x3FFFFFFFu;
+  if (ctx->scan_epoch == 0) ctx->scan_epoch = 1;
+  const ScanState S{(unsigned*)w, w + 1, ctx->scan_epoch, ctx->status};
+  LK((scan_kernel<V, Op><<<(unsigned)tiles, kScanNT, 0, st>>>(op, n, S)));
+  LAUNCH_CHECK("scan_kernel");
 }
 
 template <class K>
@@ -393,12 +397,6 @@ void rb_copy(dmsc_b200_context* ctx, cudaStream_t st, size_t off, const void* sr
   LAUNCH_CHECK("copy_words_kernel");
 }
 
-// Host read of `k` device scalars (into rb, as long long) after the stream drains.
-void readback(dmsc_b200_context* ctx, cudaStream_t st, const long long* dev, int k) {
-  rb_reserve(ctx, k * sizeof(long long));
-  rb_copy(ctx, st, 0, dev, k * sizeof(long long));
-  wait_stream(ctx, st);
-}
 const long long* rb_ll(dmsc_b200_context* ctx) { return (const long long*)ctx->rb_h; }
 
 // Error of a device status word (0: none).
@@ -469,13 +467,13 @@ PairArgs pairing_args(dmsc_b200_context* ctx, int si, Side& S) {
   A.faces = S.faces;
   A.status = ctx->status;
   A.max_rounds = capped(M + 2, ctx->cap_pair_rounds);
-  A.rounds = get<int>(ctx, S_STATS, 8) + 0 + si;
-  A.handover = get<int>(ctx, S_STATS, 8) + 6;
+  A.rounds = ctx->zero->stats + 0 + si;
+  A.handover = ctx->zero->stats + 6;
   A.node = sget<int>(ctx, si, X_CROOT, M + 1);  // free until the thresholded union-find
   A.solo_key = sget<unsigned long long>(ctx, si, X_SOLO, kPairSoloEdges + kPairSoloEdges / 2 + kPairSoloNodes);
   A.solo_ext = (int2*)(A.solo_key + kPairSoloEdges);
   A.solo_ends = (uint32_t*)(A.solo_ext + kPairSoloNodes);
-  A.timeline = get<unsigned long long>(ctx, S_TIMELINE, kTimelineSlots) + si * kTimeline;
+  A.timeline = ctx->zero->timeline + si * kTimeline;
   return A;
 }
 
@@ -491,13 +489,20 @@ void run_pairing(dmsc_b200_context* ctx, PairTileArgs T, int nltile, cudaStream_
     T.key[si] = P.s[si].key;
   }
   if (ctx->nsad <= 0) return;
-  constexpr int kSm = (int)sizeof(PairTileSmem), kSolo = (int)sizeof(PairSoloSmem);
+  constexpr int kN0 = kTilePairNT[0], kN1 = kTilePairNT[1];
+  constexpr int kSm0 = (int)sizeof(PairTileSmem<kN0>), kSm1 = (int)sizeof(PairTileSmem<kN1>);
+  constexpr int kSolo = (int)sizeof(PairSoloSmem);
   if (!ctx->pair_smem_set) {  // more than the 48 KB of static shared memory
-    CK(cudaFuncSetAttribute(pair_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSm));
+    CK(cudaFuncSetAttribute(pair_tile_kernel<kN0>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSm0));
+    CK(cudaFuncSetAttribute(pair_tile_kernel<kN1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSm1));
     CK(cudaFuncSetAttribute(pair_solo_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSolo));
     ctx->pair_smem_set = true;
   }
-  LK(pair_tile_kernel<<<2u * (unsigned)nltile, kTilePairNT, kSm, st>>>(ctx->I, T));
+  const unsigned blocks = 2u * (unsigned)nltile;
+  if (blocks <= 3u * (unsigned)ctx->num_sms)  // all resident at once with 512 threads
+    LK(pair_tile_kernel<kN1><<<blocks, kN1, kSm1, st>>>(ctx->I, T));
+  else
+    LK(pair_tile_kernel<kN0><<<blocks, kN0, kSm0, st>>>(ctx->I, T));
   LAUNCH_CHECK("pair_tile_kernel");
   // one block per 1024 saddles, up to all that are resident: a grid barrier
   // costs 3 us more on 740 blocks than on 148, and the tile pass leaves about
@@ -508,12 +513,10 @@ void run_pairing(dmsc_b200_context* ctx, PairTileArgs T, int nltile, cudaStream_
   LAUNCH_CHECK("pair_solo_kernel");
 }
 
-struct ByteToInt {
-  __host__ __device__ int operator()(uint8_t v) const { return v; }
-};
-
-// Persistence, cancellation, thresholded union-find and output ranks of both
-// sides; `survive` / `pos`: the surviving saddles and their exclusive scan.
+// Persistence, cancellation, thresholded union-find, output ranks and image
+// bases of both sides; `survive` / `pos`: the surviving saddles and their
+// exclusive scan. The survivor and cancellation counts and the status word go
+// to the readback area.
 void finish_pairing(dmsc_b200_context* ctx, uint8_t* survive, int* pos, cudaStream_t st) {
   const int nsad = ctx->nsad;
   PersistArgs P{};
@@ -562,10 +565,29 @@ void finish_pairing(dmsc_b200_context* ctx, uint8_t* survive, int* pos, cudaStre
   LK(persistence_kernel<<<grid_for(std::max(nsad, most), TB), TB, 0, st>>>(P));
   if (nsad > 0) LK(ut_union_kernel<<<dim3(grid_for(nsad, TB), 2), TB, 0, st>>>(U));
   LK(ut_flatten_kernel<<<dim3(grid_for((most + kUtBatch - 1) / kUtBatch, TB), 2), TB, 0, st>>>(U));
-  auto as_int = [](const uint8_t* p) { return thrust::make_transform_iterator(p, ByteToInt{}); };
-  excl_sum(ctx, as_int(alive), rank, Mf + Mv, st);
-  LK(root_out_kernel<<<dim3(grid_for(most, TB), 2), TB, 0, st>>>(U));
-  excl_sum(ctx, as_int(survive), pos, nsad, st);
+  FlagScan A;
+  A.in[0] = alive;
+  A.in[1] = survive;
+  A.n[0] = (long long)Mf + Mv;
+  A.n[1] = nsad;
+  A.out[0] = rank;
+  A.out[1] = pos;
+  A.total = ctx->zero->total;
+  scan<2>(ctx, A, std::max(A.n[0], A.n[1]), st);
+  rb_reserve(ctx, 4 * sizeof(long long));
+  RankBases R;
+  R.B = ctx->B;
+  R.nsad = nsad;
+  R.first[0] = ctx->bases.max;
+  R.first[1] = ctx->bases.min;
+  R.first_sad = ctx->bases.sad;
+  R.pos = pos;
+  R.total = A.total;
+  R.alive_base[0] = ctx->bases.alive[0];
+  R.alive_base[1] = ctx->bases.alive[1];
+  R.surv_base = ctx->bases.surv;
+  R.rb = (long long*)ctx->rb_d;
+  LK(root_out_kernel<<<dim3(grid_for(std::max(most, ctx->B + 1), TB), 2), TB, 0, st>>>(U, R));
   LAUNCH_CHECK("persistence and ranks");
 }
 
@@ -597,8 +619,8 @@ ReplayArgs replay_prepare(dmsc_b200_context* ctx, int si, Side& S, cudaStream_t 
   A.wa = sget<long long>(ctx, si, X_WA, 2 * (size_t)nsad);
   A.status = ctx->status;
   A.max_rounds = capped(nsad + 2, ctx->cap_replay_rounds);
-  A.rounds = get<int>(ctx, S_STATS, 8) + 2 + si;
-  A.timeline = get<unsigned long long>(ctx, S_TIMELINE, kTimelineSlots) + (4 + si) * kTimeline;
+  A.rounds = ctx->zero->stats + 2 + si;
+  A.timeline = ctx->zero->timeline + (4 + si) * kTimeline;
   return A;
 }
 
@@ -628,12 +650,10 @@ void replay_final(dmsc_b200_context* ctx, const int* sorted, unsigned long long*
     P.primal = S.arcs_primal;
     P.dual = S.arcs_dual;
   }
-  CK(cudaMemsetAsync(total, 0, 2 * sizeof(unsigned long long), st));
   LK(survivor_final_kernel<<<grid_for(2 * (nsurv + 1LL), TB), TB, 0, st>>>(
       nsurv, sorted, ctx->B, ctx->sad_img, ctx->crit_sad, ctx->I.dual, ctx->bases.surv, A[0], A[1], ctx->nsad + 1,
       ctx->head, ctx->lens, ctx->rows, total, ctx->status));
-  excl_sum(ctx, ctx->lens, ctx->lens, nsurv + 1, st);
-  excl_sum(ctx, ctx->rows, ctx->rows, nsurv + 1, st);
+  scan<4>(ctx, PackedScan{{ctx->lens, ctx->rows}}, nsurv + 1LL, st);
   LAUNCH_CHECK("final arcs");
 }
 
@@ -854,14 +874,12 @@ int extract_batch_impl(dmsc_b200_context* ctx, int B, const float* img, const in
   ctx->hH.assign(hH, hH + B);
   ctx->hW.assign(hW, hW + B);
   ctx->hdual.assign(hdual, hdual + B);
-  ctx->status = get<unsigned>(ctx, S_STATUS, 4);
+  ctx->zero = get<ZeroArea>(ctx, S_ZERO, 1);
+  ctx->status = ctx->zero->status;
   ctx->launches = 0;
   join_copies(ctx, st);  // host copies of an earlier call still reading its outputs
   mark(ctx, 0, st);
-  CK(cudaMemsetAsync(ctx->status, 0, sizeof(unsigned), st));
-  CK(cudaMemsetAsync(get<int>(ctx, S_STATS, 8), 0, 8 * sizeof(int), st));
-  CK(cudaMemsetAsync(get<unsigned long long>(ctx, S_TIMELINE, kTimelineSlots), 0,
-                     kTimelineSlots * sizeof(unsigned long long), st));
+  CK(cudaMemsetAsync(ctx->zero, 0, sizeof(ZeroArea), st));
   {  // upload the tables: 9 int arrays, then thr (float) and dual (u8)
     size_t ib = tab.size() * sizeof(int), fb = (size_t)B * sizeof(float);
     size_t total = ib + fb + B + 16;
@@ -903,11 +921,15 @@ int extract_batch_impl(dmsc_b200_context* ctx, int B, const float* img, const in
                                            ret_grad ? ctx->host_grad : nullptr);
   mark(ctx, 1, st);
   if (ret_grad && !grad_copied) copy_out_async(ctx, ctx->host_grad, grad, 16 * (size_t)nidx, st);
-  for (int k = 0; k < 3; ++k) excl_sum(ctx, seg[k], off[k], (int)nseg, st);
-  long long* tot = get<long long>(ctx, S_TOT, 8);
-  LK(totals3_kernel<<<1, 1, 0, st>>>(off[0], seg[0], off[1], seg[1], off[2], seg[2], nseg, tot));
-  LAUNCH_CHECK("totals3_kernel");
-  readback(ctx, st, tot, 3);
+  rb_reserve(ctx, 4 * sizeof(long long));
+  SegScan SS;
+  for (int k = 0; k < 3; ++k) {
+    SS.in[k] = seg[k];
+    SS.out[k] = off[k];
+  }
+  SS.rb = (long long*)ctx->rb_d;
+  scan<3>(ctx, SS, nseg, st);
+  wait_stream(ctx, st);
   const int nmin = (int)rb_ll(ctx)[0], nsad = (int)rb_ll(ctx)[1], nmax = (int)rb_ll(ctx)[2];
   ctx->nmin = nmin;
   ctx->nsad = nsad;
@@ -941,9 +963,6 @@ int extract_batch_impl(dmsc_b200_context* ctx, int B, const float* img, const in
     ps.g12[si] = sget<int2>(ctx, si, X_G12, nsad);
     ps.dying[si] = sget<int>(ctx, si, X_DYING, nsad);
   }
-  LK(compact_kernel<<<grid_for(nseg, 8 * kCompactSegs), 256, 0, st>>>(
-      I, img, nseg, flow, off[0], off[1], off[2], csad, imin, isad, imax, bmin, bmax, kmin, kmax, sval, ps));
-  LAUNCH_CHECK("compact_kernel");
   // per-image bases of the critical lists (B + 1 entries each)
   int* bases = get<int>(ctx, S_BASES, 8 * (size_t)(B + 1));
   Bases& BS = ctx->bases;
@@ -955,10 +974,10 @@ int extract_batch_impl(dmsc_b200_context* ctx, int B, const float* img, const in
   BS.alive[1] = bases + 5 * (B + 1);
   BS.erow[0] = bases + 6 * (B + 1);
   BS.erow[1] = bases + 7 * (B + 1);
-  LK(image_base_kernel<<<grid_for(B + 1LL, TB), TB, 0, st>>>(B, I.seg_base, (int)nseg, off[0], nmin, BS.min));
-  LK(image_base_kernel<<<grid_for(B + 1LL, TB), TB, 0, st>>>(B, I.seg_base, (int)nseg, off[1], nsad, BS.sad));
-  LK(image_base_kernel<<<grid_for(B + 1LL, TB), TB, 0, st>>>(B, I.seg_base, (int)nseg, off[2], nmax, BS.max));
-  LAUNCH_CHECK("image_base_kernel");
+  const ListBases LB{{BS.min, BS.sad, BS.max}, {nmin, nsad, nmax}};
+  LK(compact_kernel<<<grid_for(nseg, 8 * kCompactSegs), 256, 0, st>>>(
+      I, img, nseg, flow, off[0], off[1], off[2], csad, imin, isad, imax, bmin, bmax, kmin, kmax, sval, LB, ps));
+  LAUNCH_CHECK("compact_kernel");
   mark(ctx, 2, st);
 
   // ---- K4 saddle walks ----
@@ -1020,10 +1039,6 @@ int extract_batch_impl(dmsc_b200_context* ctx, int B, const float* img, const in
   // ---- surviving saddles in minima-sweep (vertex side) order ----
   // the status word rides along: a capped pairing or union-find loop ends the
   // call here, before the replay
-  rb_reserve(ctx, 4 * sizeof(long long));
-  LK(survivor_base_kernel<<<grid_for(B + 1LL, TB), TB, 0, st>>>(B, BS.sad, nsad, flag, fpos, get<int>(ctx, S_NCANC, 4),
-                                                               ctx->status, BS.surv, (long long*)ctx->rb_d));
-  LAUNCH_CHECK("survivor_base_kernel");
   wait_stream(ctx, st);
   raise_status(ctx, (unsigned)rb_ll(ctx)[3]);
   ctx->nsurv = (int)rb_ll(ctx)[0];
@@ -1078,10 +1093,6 @@ int extract_batch_impl(dmsc_b200_context* ctx, int B, const float* img, const in
   CK(cudaEventRecord(ctx->join_ev, ss));
 
   // ---- labels (region id = rank among the image's alive extrema) ----
-  // alive bases first (needed by the labels and the outputs)
-  LK(alive_base_kernel<<<grid_for(B + 1LL, TB), TB, 0, st>>>(B, nmax, nmin, BS.max, BS.min, F.to_out_excl, F.alive,
-                                                            BS.alive[0], BS.alive[1]));
-  LAUNCH_CHECK("alive bases");
   LabelOut OF{}, OV{};
   LabelSide LF{}, LV{};
   for (int si = 0; si < 2; ++si) {
@@ -1105,8 +1116,7 @@ int extract_batch_impl(dmsc_b200_context* ctx, int B, const float* img, const in
     L.abase = BS.alive[si];
     L.perim = get<int>(ctx, S.faces ? S_PERF : S_PERV, (size_t)nltile * kPerim);
   }
-  int* nex = get<int>(ctx, S_NEX, 2);
-  CK(cudaMemsetAsync(nex, 0, 2 * sizeof(int), st));
+  int* nex = ctx->zero->n_exits;
   mark(ctx, 16, st);  // the labels stage times the label kernels alone
   if (F.groups || V.groups) {
     int2* exf = F.groups ? get<int2>(ctx, S_EXF, nidx) : nullptr;
@@ -1125,12 +1135,11 @@ int extract_batch_impl(dmsc_b200_context* ctx, int B, const float* img, const in
                                                                                     exv, nex, ctx->status)));
     LAUNCH_CHECK("label_tile_kernel");
     int per = 0;
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, label_exit_kernel<true>, 256, 0));
-    const unsigned eg = (unsigned)std::max(1, per) * ctx->num_sms;
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, label_exit_kernel, 256, 0));
     // a path enters a tile through each of its border cells at most once
     const int hops = (int)std::min<long long>(nltile * kPerim + 2, 2147483647LL);
-    if (F.groups) LK(label_exit_kernel<true><<<eg, 256, 0, st>>>(I, exf, nex + 0, LF.perim, OF, hops, ctx->status));
-    if (V.groups) LK(label_exit_kernel<false><<<eg, 256, 0, st>>>(I, exv, nex + 1, LV.perim, OV, hops, ctx->status));
+    const unsigned eg = (unsigned)std::min<long long>((long long)std::max(1, per) * ctx->num_sms, 4 * nltile);
+    LK(label_exit_kernel<<<dim3(eg, 2), 256, 0, st>>>(I, exf, exv, nex, LF.perim, LV.perim, OF, OV, hops, ctx->status));
     LAUNCH_CHECK("label_exit_kernel");
   }
   mark(ctx, 10, st);
@@ -1144,7 +1153,7 @@ int extract_batch_impl(dmsc_b200_context* ctx, int B, const float* img, const in
     ctx->side[si].gbase = sget<long long>(ctx, si, X_GBASE, B + 1);
     ctx->side[si].total = 0;
   }
-  unsigned long long* total = get<unsigned long long>(ctx, S_TOT, 8) + 4;
+  unsigned long long* total = ctx->zero->geom;
   replay_final(ctx, sorted, total, st);
   mark(ctx, 9, st);
 
@@ -1248,8 +1257,8 @@ void emit_expand(dmsc_b200_context* ctx, cudaStream_t st) {
     E.base_q = sget<int4>(ctx, si, X_QB, cap);
     E.base_cap = cap;
     A.max_levels = capped(ctx->nsad + 4, ctx->cap_emit_levels);
-    A.levels = get<int>(ctx, S_STATS, 8) + 4 + si;
-    A.timeline = get<unsigned long long>(ctx, S_TIMELINE, kTimelineSlots) + (2 + si) * kTimeline;
+    A.levels = ctx->zero->stats + 4 + si;
+    A.timeline = ctx->zero->timeline + (2 + si) * kTimeline;
     ctx->emit[si] = A;
     most += cap;
   }
@@ -1330,12 +1339,18 @@ int fetch_batch_impl(dmsc_b200_context* ctx, const dmsc_b200_outputs* o, cudaStr
   const int* rt = (const int*)ctx->bufs[S_ROUTE].p;
   auto rt_of = [&](int k) { return rt + (size_t)k * B; };
   // extrema lists
-  for (int si = 0; si < 2; ++si) {
-    Side& S = ctx->side[si];
-    Route R{S.faces ? o->max_pts : o->min_pts, S.faces ? o->min_pts : o->max_pts, rt_of(si == 0 ? R_PTS0 : R_PTS1)};
-    if (S.M > 0)
-      LK(points_kernel<<<grid_for(S.M, TB), TB, 0, st>>>(S.M, S.alive, S.to_out_excl, ctx->bases.alive[si], S.key,
-                                                         S.ext_img, I, R));
+  {
+    PointSide PS[2];
+    int most = 0;
+    for (int si = 0; si < 2; ++si) {
+      Side& S = ctx->side[si];
+      PS[si] = PointSide{S.M, S.alive, S.to_out_excl, ctx->bases.alive[si], S.key, S.ext_img,
+                         Route{S.faces ? o->max_pts : o->min_pts, S.faces ? o->min_pts : o->max_pts,
+                               rt_of(si == 0 ? R_PTS0 : R_PTS1)}};
+      most = std::max(most, S.M);
+    }
+    if (most > 0) LK(points_kernel<<<dim3(grid_for(most, TB), 2), TB, 0, st>>>(PS[0], PS[1], I));
+    LAUNCH_CHECK("points_kernel");
   }
   // per-survivor outputs; a side's arcs go to the arrays that some image takes
   // (faces: ridges in the primal, valleys in the dual)
@@ -1707,19 +1722,19 @@ int dmsc_b200_stage_times(dmsc_b200_context* ctx, float* ms, int n) {
 long long dmsc_b200_launch_count(const dmsc_b200_context* ctx) { return ctx ? ctx->launches : -1; }
 
 int dmsc_b200_pairing_timeline(dmsc_b200_context* ctx, long long* out, int n) {
-  if (!ctx || !out || ctx->bufs.size() <= (size_t)S_TIMELINE || !ctx->bufs[S_TIMELINE].p) return -1;
+  if (!ctx || !out || !ctx->zero) return -1;
   int k = n < kTimelineSlots ? n : kTimelineSlots;
   if (cudaSetDevice(ctx->device) != cudaSuccess ||
-      cudaMemcpy(out, ctx->bufs[S_TIMELINE].p, k * sizeof(long long), cudaMemcpyDeviceToHost) != cudaSuccess)
+      cudaMemcpy(out, ctx->zero->timeline, k * sizeof(long long), cudaMemcpyDeviceToHost) != cudaSuccess)
     return -1;
   return k;
 }
 
 int dmsc_b200_loop_counts(dmsc_b200_context* ctx, int* out, int n) {
-  if (!ctx || !out || ctx->bufs.size() <= (size_t)S_STATS || !ctx->bufs[S_STATS].p) return -1;
+  if (!ctx || !out || !ctx->zero) return -1;
   int h[6] = {0};
   if (cudaSetDevice(ctx->device) != cudaSuccess ||
-      cudaMemcpy(h, ctx->bufs[S_STATS].p, sizeof h, cudaMemcpyDeviceToHost) != cudaSuccess)
+      cudaMemcpy(h, ctx->zero->stats, sizeof h, cudaMemcpyDeviceToHost) != cudaSuccess)
     return -1;
   for (int k = 0; k < 6 && k < n; ++k) out[k] = h[k];
   return 6;

@@ -740,14 +740,30 @@ __host__ __device__ __forceinline__ unsigned crit_bits(unsigned fl, bool vin) {
 // the pairing's starting state of the groups (PairStart).
 constexpr int kCompactSegs = 2;
 
+// First entry of each image in the lists of minima, saddles and maxima (B + 1
+// entries each), and the lists' lengths.
+struct ListBases {
+  int* base[3];
+  int total[3];
+};
+
 static __global__ void __launch_bounds__(256) compact_kernel(
     Imgs I, const float* __restrict__ img_all, long long nseg, const uint8_t* __restrict__ flow,
     const int* __restrict__ off_min, const int* __restrict__ off_sad, const int* __restrict__ off_max,
     int* __restrict__ crit_sad, int* __restrict__ min_img, int* __restrict__ sad_img, int* __restrict__ max_img,
     uint32_t* __restrict__ min_bits, uint32_t* __restrict__ max_bits, int2* __restrict__ min_key,
-    int2* __restrict__ max_key, float* __restrict__ sad_val, PairStart ps) {
+    int2* __restrict__ max_key, float* __restrict__ sad_val, ListBases lb, PairStart ps) {
   constexpr int K = kCompactSegs;
   const int lane = threadIdx.x & 31;
+  {  // an image has a segment, so there are at least B + 1 threads
+    const long long b = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (b <= I.B) {
+      const long long q = b < I.B ? I.seg_base[b] : nseg;
+#pragma unroll
+      for (int k = 0; k < 3; ++k)
+        lb.base[k][b] = q < nseg ? (k == 0 ? off_min : k == 1 ? off_sad : off_max)[q] : lb.total[k];
+    }
+  }
   const long long seg0 = ((long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * K;
   if (seg0 >= nseg) return;
   if (seg0 == 0 && lane == 0) {  // the pairing's void groups and round counters

@@ -171,22 +171,26 @@ __global__ void __launch_bounds__(256) saddle_walk_kernel(Imgs I, const uint8_t*
 // 1.13 -> 0.76 ms (this pass 0.37), 8192^2 noise 7.80 -> 4.75, 509 x 1531
 // 0.287 -> 0.166.
 constexpr int kTileNodes = 896, kTileEdges = 1664;
-constexpr int kTilePairNT = 256, kTilePairWarps = kTilePairNT / 32;
-constexpr int kTileRounds = 6;    // later rounds decide less than 1% of what is left
+// Threads per block: 256 when the blocks fill the device several times over,
+// 512 when one wave holds them all and a block's own latency counts (24% less
+// at 256^2, 8% more at 4096^2).
+constexpr int kTilePairNT[2] = {256, 512};
+constexpr int kTileRounds = 6;    // 4, 6, 8 rounds: stage of 5.68, 4.75, 4.93 ms at 8192^2 noise, 0.765, 0.753, 0.763 at 4096^2
 constexpr int kTilePairs = 512;   // slots of the table of group pairs
-constexpr int kTileList = (kTileEdges / 32 + kTilePairWarps - 1) / kTilePairWarps * 32;  // a warp's edges
+constexpr int tile_list(int warps) { return (kTileEdges / 32 + warps - 1) / warps * 32; }  // a warp's edges
 constexpr unsigned kTileVoid = 0xFFFEu;
 // `ends` of an edge that is no longer undecided: dead node | kTileDead, or a
 // cycle (or not the first between its groups); of one that leaves the tile
 constexpr uint32_t kTileDead = 0xFFFF0000u, kTileCycle = 0xFFFFFFFFu, kTileOut = 0xFFFEFFFEu;
 
+template <int NT>
 struct PairTileSmem {
   unsigned long long minedge[kTileNodes];  // (value key, edge or its complement) of a root's first local saddle
   float val[kTileNodes];
   uint32_t leave[kTileNodes];   // value key of the group's first saddle out of the tile
   uint32_t ends[kTileEdges];    // nodes of both ends (roots as of the last phase A)
   uint32_t hi[kTileEdges];      // value key
-  uint16_t list[kTilePairWarps][kTileList];  // each warp's undecided edges
+  uint16_t list[NT / 32][tile_list(NT / 32)];  // each warp's undecided edges
   uint16_t link[kTileNodes];
   uint8_t seg[kTileNodes];      // segment of each node
   uint8_t row[kTileEdges];      // row of each edge
@@ -225,10 +229,11 @@ __device__ __forceinline__ unsigned tile_root(volatile uint16_t* link, unsigned 
   return x;
 }
 
-__global__ void __launch_bounds__(kTilePairNT, 6) pair_tile_kernel(Imgs I, PairTileArgs A) {
+template <int NT>
+__global__ void __launch_bounds__(NT, 1536 / NT) pair_tile_kernel(Imgs I, PairTileArgs A) {
   extern __shared__ __align__(16) unsigned char pair_tile_smem[];
-  PairTileSmem& S = *reinterpret_cast<PairTileSmem*>(pair_tile_smem);
-  constexpr int NT = kTilePairNT, NW = kTilePairWarps, kNodesPer = (kTileNodes + NT - 1) / NT;
+  PairTileSmem<NT>& S = *reinterpret_cast<PairTileSmem<NT>*>(pair_tile_smem);
+  constexpr int NW = NT / 32, kNodesPer = (kTileNodes + NT - 1) / NT;
   const bool s1 = blockIdx.x & 1;  // consecutive blocks: the two sides of one tile
   const LabelTile g = label_tile_of(I, blockIdx.x >> 1);
   const bool dual = I.dual[g.b];
@@ -334,9 +339,10 @@ __global__ void __launch_bounds__(kTilePairNT, 6) pair_tile_kernel(Imgs I, PairT
     return;
   }
   {  // row of every edge, segment of every node
-    const int r = tid >> 2, q = tid >> 1;
-    for (int k = S.spre[r] + (tid & 3); k < S.spre[r + 1]; k += 4) S.row[k] = (uint8_t)r;
-    for (int i = S.npre[q] + (tid & 1); i < S.npre[q + 1]; i += 2) S.seg[i] = (uint8_t)q;
+    constexpr int kR = NT / kLT, kQ = NT / (2 * kLT);  // threads per row and segment
+    const int r = tid / kR, q = tid / kQ;
+    for (int k = S.spre[r] + tid % kR; k < S.spre[r + 1]; k += kR) S.row[k] = (uint8_t)r;
+    for (int i = S.npre[q] + tid % kQ; i < S.npre[q + 1]; i += kQ) S.seg[i] = (uint8_t)q;
   }
   __syncthreads();
   auto saddle_of = [&](int k) { return saddle_in_row(k, S.row[k]); };
@@ -748,11 +754,43 @@ __global__ void ut_flatten_kernel(UtArgs A) {
 
 // Rank of each extremum's thresholded root among the alive extrema: the
 // component's alive member (comp_root of its flattened union-find root; -1
-// for the void's component).
-__global__ void root_out_kernel(UtArgs A) {
+// for the void's component); and the images' first alive ranks and survivors
+// (B + 1 entries, the last ones the totals), with the counts and the status
+// word for the host straight to the mapped readback area.
+struct RankBases {
+  int B, nsad;
+  const int* first[2];   // [B + 1] first extremum of each image and side
+  const int* first_sad;  // [B + 1] first saddle
+  const int* pos;        // [nsad] survivors before each saddle
+  const int* total;      // alive extrema of both sides, survivors
+  int* alive_base[2];
+  int* surv_base;
+  long long* rb;
+};
+
+__global__ void __launch_bounds__(256) root_out_kernel(UtArgs A, RankBases R) {
   const bool s1 = blockIdx.y != 0;
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  if (x >= (s1 ? A.M[1] : A.M[0])) return;
+  const int M = s1 ? A.M[1] : A.M[0];
+  if (x <= R.B) {
+    // ranks run over both sides' lists, the vertex side's after the faces'
+    const int f = (s1 ? R.first[1] : R.first[0])[x];
+    const int* rank = s1 ? A.rank[1] : A.rank[0];
+    const bool end = f >= M;
+    (s1 ? R.alive_base[1] : R.alive_base[0])[x] =
+        !end ? rank[f] : s1 || A.M[1] == 0 ? R.total[0] : A.rank[1][0];
+    if (!s1) {
+      const int q = R.first_sad[x];
+      R.surv_base[x] = q < R.nsad ? R.pos[q] : R.total[1];
+      if (x == 0) {
+        R.rb[0] = R.total[1];
+        R.rb[1] = A.count[0];
+        R.rb[2] = A.count[1];
+        R.rb[3] = *A.status;
+      }
+    }
+  }
+  if (x >= M) return;
   const int u = (s1 ? A.comp_root[1] : A.comp_root[0])[(s1 ? A.p[1] : A.p[0])[x]];
   (s1 ? A.rout[1] : A.rout[0])[x] = u >= 0 ? (s1 ? A.rank[1] : A.rank[0])[u] : -1;
 }

@@ -390,12 +390,19 @@ __global__ void __launch_bounds__(NT, 2048 / NT) label_tile_kernel(Imgs I, const
   }
 }
 
-// Cells whose paths leave their tile: follow the border map to the label.
-template <bool FACES>
-__global__ void __launch_bounds__(256) label_exit_kernel(Imgs I, const int2* __restrict__ exits,
-                                                         const int* __restrict__ n_exits, const int* __restrict__ perim,
-                                                         LabelOut O, int cap, unsigned* status) {
-  const int n = *n_exits;
+// Cells whose paths leave their tile: follow the border map to the label
+// (both sides in one launch, blockIdx.y).
+__global__ void __launch_bounds__(256) label_exit_kernel(Imgs I, const int2* __restrict__ exits_f,
+                                                         const int2* __restrict__ exits_v,
+                                                         const int* __restrict__ n_exits,
+                                                         const int* __restrict__ perim_f,
+                                                         const int* __restrict__ perim_v, LabelOut OF, LabelOut OV,
+                                                         int cap, unsigned* status) {
+  const bool faces = blockIdx.y == 0;
+  const int2* __restrict__ exits = faces ? exits_f : exits_v;
+  const int* __restrict__ perim = faces ? perim_f : perim_v;
+  const LabelOut& O = faces ? OF : OV;
+  const int n = n_exits[blockIdx.y];
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
     const int2 e = exits[q];
     const int b = find_image(I.idx_base, I.B, e.x);
@@ -405,7 +412,7 @@ __global__ void __launch_bounds__(256) label_exit_kernel(Imgs I, const int2* __r
     const int lidx = e.x - I.idx_base[b];
     const int y = lidx / Nx, x = lidx - y * Nx;
     out += (d ? O.dual_off : O.primal_off)[b];
-    out[FACES ? lidx : y * W + x] = entry_label(e.y, perim, cap, status);
+    out[faces ? lidx : y * W + x] = entry_label(e.y, perim, cap, status);
   }
 }
 
