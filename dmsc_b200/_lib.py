@@ -21,6 +21,8 @@ EXPORTS = (
     "dmsc_b200_destroy",
     "dmsc_b200_extract",
     "dmsc_b200_fetch",
+    "dmsc_b200_fetch_start",
+    "dmsc_b200_fetch_finish",
     "dmsc_b200_set_host_outputs",
     "dmsc_b200_set_host_fetch_outputs",
     "dmsc_b200_set_host_input",
@@ -94,6 +96,10 @@ def load():
         lib.dmsc_b200_extract.restype = ctypes.c_int
         lib.dmsc_b200_fetch.argtypes = [ctypes.c_void_p, ctypes.POINTER(Outputs), ctypes.c_void_p]
         lib.dmsc_b200_fetch.restype = ctypes.c_int
+        lib.dmsc_b200_fetch_start.argtypes = [ctypes.c_void_p, ctypes.POINTER(Outputs), ctypes.c_void_p]
+        lib.dmsc_b200_fetch_start.restype = ctypes.c_int
+        lib.dmsc_b200_fetch_finish.argtypes = [ctypes.c_void_p, ctypes.c_void_p]
+        lib.dmsc_b200_fetch_finish.restype = ctypes.c_int
         lib.dmsc_b200_set_host_outputs.argtypes = [ctypes.c_void_p] * 4
         lib.dmsc_b200_set_host_outputs.restype = ctypes.c_int
         lib.dmsc_b200_set_host_input.argtypes = [ctypes.c_void_p, ctypes.c_void_p]

@@ -148,7 +148,8 @@ struct dmsc_b200_context {
   // writer in fetch reads its segment list (expanded: launched this call)
   EmitArgs emit[2] = {};
   bool expanded[2] = {false, false};
-  cudaEvent_t sync_ev = nullptr;   // polled by wait_stream
+  cudaEvent_t sync_ev = nullptr;   // polled by wait_event
+  bool fetch_pending = false;      // a fetch_start whose fetch_finish is due
   // host destinations of the fixed-size outputs for the next extract (copied
   // on copy_st as soon as each is produced; see dmsc_b200_set_host_outputs)
   int32_t* host_grad = nullptr;
@@ -326,14 +327,14 @@ void coop_launch(dmsc_b200_context* ctx, void (*kernel)(T), T args, cudaStream_t
   ++ctx->launches;
 }
 
-// Waits until the stream has drained by polling an event: the host thread
+// Waits for the last recorded event (wait_stream: until the stream has
+// drained) by polling it: the host thread
 // spins instead of sleeping in the driver, so the next launches follow the
 // readback without an operating-system wake-up delay (the few host round
 // trips of a call are on its critical path). Gives up after the context's
 // wait deadline with DMSC_B200_ERR_CUDA; the work may still be running then,
 // so the context must be destroyed, not reused.
-void wait_stream(dmsc_b200_context* ctx, cudaStream_t st) {
-  CK(cudaEventRecord(ctx->sync_ev, st));
+void wait_event(dmsc_b200_context* ctx) {
   const auto t0 = std::chrono::steady_clock::now();
   for (unsigned k = 0;; ++k) {
     const cudaError_t e = cudaEventQuery(ctx->sync_ev);
@@ -345,6 +346,11 @@ void wait_stream(dmsc_b200_context* ctx, cudaStream_t st) {
       throw Fail{kErrCuda};
     }
   }
+}
+
+void wait_stream(dmsc_b200_context* ctx, cudaStream_t st) {
+  CK(cudaEventRecord(ctx->sync_ev, st));
+  wait_event(ctx);
 }
 
 // Device -> host copy of a finished output on the context's copy stream,
@@ -418,15 +424,6 @@ void raise_status(dmsc_b200_context* ctx, unsigned h) {
     throw Fail{kErrInternal};
   }
 }
-
-void check_status(dmsc_b200_context* ctx, cudaStream_t st) {
-  rb_reserve(ctx, 64);
-  rb_copy(ctx, st, 0, ctx->status, sizeof(unsigned));
-  wait_stream(ctx, st);
-  raise_status(ctx, *(const unsigned*)ctx->rb_h);
-}
-
-
 
 constexpr int TB = 256;
 
@@ -791,6 +788,7 @@ int extract_batch_impl(dmsc_b200_context* ctx, int B, const float* img, const in
                        const float* hthr, const unsigned char* hdual, unsigned flags, int32_t* grad_out,
                        int32_t* peaks_out, int32_t* basins_out, dmsc_b200_sizes* sizes_out, cudaStream_t st) {
   ctx->valid = false;
+  ctx->fetch_pending = false;
   const float* host_img = ctx->host_img;  // the registration covers this call only
   ctx->host_img = nullptr;
   if (host_img && B != 1) {
@@ -1291,7 +1289,8 @@ void emit_write(dmsc_b200_context* ctx, int32_t* const (*out)[2], const int* con
   LAUNCH_CHECK("emit_segments_kernel");
 }
 
-int fetch_batch_impl(dmsc_b200_context* ctx, const dmsc_b200_outputs* o, cudaStream_t st) {
+// Enqueues every output of the last extract; fetch_finish_impl waits for them.
+int fetch_start_impl(dmsc_b200_context* ctx, const dmsc_b200_outputs* o, cudaStream_t st) {
   if (!ctx->valid || !o) {
     set_err(ctx, "fetch without a successful extract");
     return kErrInvalidArgument;
@@ -1406,7 +1405,22 @@ int fetch_batch_impl(dmsc_b200_context* ctx, const dmsc_b200_outputs* o, cudaStr
   if (ctx->host_fetch_set)
     for (int k = 9; k < 15; ++k) copy_out_async(ctx, host_f[k], dev_f[k], 4 * (size_t)tot_n[k], st);
   ctx->host_fetch_set = false;  // one fetch only
-  check_status(ctx, st);
+  rb_reserve(ctx, 64);
+  rb_copy(ctx, st, 0, ctx->status, sizeof(unsigned));
+  CK(cudaEventRecord(ctx->sync_ev, st));
+  ctx->fetch_pending = true;
+  return kOk;
+}
+
+int fetch_finish_impl(dmsc_b200_context* ctx, cudaStream_t st) {
+  if (!ctx->fetch_pending) {
+    set_err(ctx, "fetch_finish without a fetch_start");
+    return kErrInvalidArgument;
+  }
+  ctx->fetch_pending = false;
+  CK(cudaSetDevice(ctx->device));
+  wait_event(ctx);
+  raise_status(ctx, *(const unsigned*)ctx->rb_h);
   join_copies(ctx, st);  // the caller's stream passes here only once the host copies are done
   return kOk;
 }
@@ -1586,7 +1600,30 @@ int dmsc_b200_fetch(dmsc_b200_context* ctx, const dmsc_b200_outputs* out, void* 
   if (!ctx) return kErrInvalidArgument;
   ctx->err.clear();
   try {
-    return fetch_batch_impl(ctx, out, (cudaStream_t)stream);
+    const int rc = fetch_start_impl(ctx, out, (cudaStream_t)stream);
+    return rc == kOk ? fetch_finish_impl(ctx, (cudaStream_t)stream) : rc;
+  } catch (const Fail& f) {
+    abandon_copies(ctx);
+    return f.code;
+  }
+}
+
+int dmsc_b200_fetch_start(dmsc_b200_context* ctx, const dmsc_b200_outputs* out, void* stream) {
+  if (!ctx) return kErrInvalidArgument;
+  ctx->err.clear();
+  try {
+    return fetch_start_impl(ctx, out, (cudaStream_t)stream);
+  } catch (const Fail& f) {
+    abandon_copies(ctx);
+    return f.code;
+  }
+}
+
+int dmsc_b200_fetch_finish(dmsc_b200_context* ctx, void* stream) {
+  if (!ctx) return kErrInvalidArgument;
+  ctx->err.clear();
+  try {
+    return fetch_finish_impl(ctx, (cudaStream_t)stream);
   } catch (const Fail& f) {
     abandon_copies(ctx);
     return f.code;

@@ -254,20 +254,27 @@ def extract_single(img: torch.Tensor, persistence_threshold: float, flags: int, 
         hout = {k: _host_like(v) for k, v in out.items()}
         ho = _lib.Outputs(**{k: _ptr(v) for k, v in hout.items()})
         ctx.check(ctx.lib.dmsc_b200_set_host_fetch_outputs(ctx.h, ctypes.byref(ho)), "dmsc_b200_set_host_fetch_outputs")
-    ctx.check(ctx.lib.dmsc_b200_fetch(ctx.h, ctypes.byref(o), ctypes.c_void_p(s.cuda_stream)), "dmsc_b200_fetch")
-    empty = torch.empty(0, **i32)
-    empty2 = torch.empty((0, 0), **i32)
-    shape = torch.tensor([H, W], dtype=torch.int32)
-    if host_fixed:  # host tensors, complete once the stream has passed the fetch
-        grad, peaks, basins = hg, hp, hb
-        out = hout
-        empty = torch.empty(0, dtype=torch.int32)
-        empty2 = torch.empty((0, 0), dtype=torch.int32)
-    return (shape, out["max_pts"], out["min_pts"], out["sad_pts"], out["e_max"], out["e_min"], out["p_max"],
-            out["p_min"], out["ppairs_max"], out["ppairs_min"], grad if grad is not None else empty,
-            peaks if peaks is not None else empty2, out["ridges"], out["ridge_offsets"], out["ridge_arc_offsets"],
-            basins if basins is not None else empty2, out["valleys"], out["valley_offsets"],
-            out["valley_arc_offsets"])
+    ctx.check(ctx.lib.dmsc_b200_fetch_start(ctx.h, ctypes.byref(o), ctypes.c_void_p(s.cuda_stream)), "dmsc_b200_fetch")
+    on_device = (grad, peaks, basins, out)  # held until the copies from them are ordered before later work
+    try:  # the result is put together while the device writes the outputs
+        empty = torch.empty(0, **i32)
+        empty2 = torch.empty((0, 0), **i32)
+        shape = torch.tensor([H, W], dtype=torch.int32)
+        if host_fixed:  # host tensors, complete once the stream has passed the fetch
+            grad, peaks, basins = hg, hp, hb
+            out = hout
+            empty = torch.empty(0, dtype=torch.int32)
+            empty2 = torch.empty((0, 0), dtype=torch.int32)
+        res = (shape, out["max_pts"], out["min_pts"], out["sad_pts"], out["e_max"], out["e_min"], out["p_max"],
+               out["p_min"], out["ppairs_max"], out["ppairs_min"], grad if grad is not None else empty,
+               peaks if peaks is not None else empty2, out["ridges"], out["ridge_offsets"], out["ridge_arc_offsets"],
+               basins if basins is not None else empty2, out["valleys"], out["valley_offsets"],
+               out["valley_arc_offsets"])
+    finally:
+        rc = ctx.lib.dmsc_b200_fetch_finish(ctx.h, ctypes.c_void_p(s.cuda_stream))
+    del on_device
+    ctx.check(rc, "dmsc_b200_fetch")
+    return res
 
 
 # Indices (H+1)*(W+1) summed over the images of one device batch. The library
@@ -303,10 +310,11 @@ def _extract_raw(x3, thresholds, duals):
 
 
 def _batch_raw(images, thresholds, is_dual, flags: int, stream=None, host_fixed=False):
-    """Both C-ABI phases of one device batch. Returns the batch-wide output
-    tensors (``out``, field -> tensor, images back to back), the per-image
-    lengths of each (``lens``), the image shapes and orientations and the
-    stream."""
+    """Both C-ABI phases of one device batch, the second one enqueued only: the
+    caller ends it with ``finish()``. Returns the batch-wide output tensors
+    (``out``, field -> tensor, images back to back), the per-image lengths of
+    each (``lens``), the image shapes and orientations, the stream and
+    ``finish``."""
     B = len(images)
     dev = images[0].device
     ctx = _lib.context(dev.index if dev.index is not None else torch.cuda.current_device())
@@ -347,7 +355,15 @@ def _batch_raw(images, thresholds, is_dual, flags: int, stream=None, host_fixed=
         hout = {k: _host_like(v) for k, v in out.items()}
         ho = _lib.Outputs(**{k: _ptr(v) for k, v in hout.items()})
         ctx.check(ctx.lib.dmsc_b200_set_host_fetch_outputs(ctx.h, ctypes.byref(ho)), "dmsc_b200_set_host_fetch_outputs")
-    ctx.check(ctx.lib.dmsc_b200_fetch(ctx.h, ctypes.byref(o), ctypes.c_void_p(s.cuda_stream)), "dmsc_b200_fetch")
+    ctx.check(ctx.lib.dmsc_b200_fetch_start(ctx.h, ctypes.byref(o), ctypes.c_void_p(s.cuda_stream)), "dmsc_b200_fetch")
+    on_device = (grad, peaks, basins, out)  # held until the copies from them are ordered before later work
+
+    def finish():
+        nonlocal on_device
+        rc = ctx.lib.dmsc_b200_fetch_finish(ctx.h, ctypes.c_void_p(s.cuda_stream))
+        on_device = None
+        return rc
+
     if host_fixed:
         out = hout
     if host_fixed:
@@ -361,7 +377,7 @@ def _batch_raw(images, thresholds, is_dual, flags: int, stream=None, host_fixed=
     if basins is not None:
         out["basins"] = basins
         lens["basins"] = bs_n
-    return out, lens, Hs, Ws, duals, s
+    return out, lens, Hs, Ws, duals, s, ctx, finish
 
 
 def extract_batch(images, thresholds, is_dual, flags: int, to_host: bool = False, stream=None) -> list:
@@ -372,26 +388,32 @@ def extract_batch(images, thresholds, is_dual, flags: int, to_host: bool = False
     ``to_host``). ``flags``' DUAL bit is ignored in favour of ``is_dual``."""
     B = len(images)
     dev = images[0].device
-    out, lens, Hs, Ws, duals, s = _batch_raw(images, thresholds, is_dual, flags, stream, host_fixed=to_host)
-    grad, peaks, basins = out.get("grad_indices"), out.get("peaks"), out.get("basins")
-    if to_host:
-        with torch.cuda.stream(s):
-            out = dict(zip(out.keys(), _to_host(tuple(out.values()))))
-    parts = {k: torch.split(v, lens[k]) for k, v in out.items()}
-    odev = torch.device("cpu") if to_host else dev
-    empty = torch.empty(0, dtype=torch.int32, device=odev)
-    empty2 = torch.empty((0, 0), dtype=torch.int32, device=odev)
-    res = []
-    for b in range(B):
-        H, W, d = Hs[b], Ws[b], duals[b]
-        g = parts["grad_indices"][b] if grad is not None else empty
-        pk = parts["peaks"][b].view((H, W) if d else (H + 1, W + 1)) if peaks is not None else empty2
-        bs = parts["basins"][b].view((H + 1, W + 1) if d else (H, W)) if basins is not None else empty2
-        q = {f: parts[f][b] for f in _FIELDS}
-        res.append((torch.tensor([H, W], dtype=torch.int32), q["max_pts"], q["min_pts"], q["sad_pts"], q["e_max"],
-                    q["e_min"], q["p_max"], q["p_min"], q["ppairs_max"], q["ppairs_min"], g, pk, q["ridges"],
-                    q["ridge_offsets"], q["ridge_arc_offsets"], bs, q["valleys"], q["valley_offsets"],
-                    q["valley_arc_offsets"]))
+    out, lens, Hs, Ws, duals, s, ctx, finish = _batch_raw(images, thresholds, is_dual, flags, stream,
+                                                          host_fixed=to_host)
+    try:  # the views are made while the device writes the outputs
+        grad, peaks, basins = out.get("grad_indices"), out.get("peaks"), out.get("basins")
+        parts = {k: torch.split(v, lens[k]) for k, v in out.items()}
+        odev = torch.device("cpu") if to_host else dev
+        empty = torch.empty(0, dtype=torch.int32, device=odev)
+        empty2 = torch.empty((0, 0), dtype=torch.int32, device=odev)
+        shapes = torch.tensor([Hs, Ws], dtype=torch.int32).t().contiguous().unbind(0)
+        g = parts["grad_indices"] if grad is not None else [empty] * B
+        pk = parts["peaks"] if peaks is not None else None
+        bs = parts["basins"] if basins is not None else None
+        res = []
+        for b in range(B):
+            H, W, d = Hs[b], Ws[b], duals[b]
+            px, ix = (H, W), (H + 1, W + 1)
+            res.append((shapes[b], *(parts[f][b] for f in _FIELDS[:9]), g[b],
+                        pk[b].view(px if d else ix) if pk is not None else empty2,
+                        *(parts[f][b] for f in _FIELDS[9:12]),
+                        bs[b].view(ix if d else px) if bs is not None else empty2,
+                        *(parts[f][b] for f in _FIELDS[12:])))
+    finally:
+        rc = finish()
+    ctx.check(rc, "dmsc_b200_fetch")
+    if to_host:  # the host copies are complete once the stream has passed the fetch
+        s.synchronize()
     return res
 
 

@@ -112,6 +112,13 @@ int dmsc_b200_extract(dmsc_b200_context* ctx, const float* image, int H, int W, 
    of image b, and so on); all values are image-local. */
 int dmsc_b200_fetch(dmsc_b200_context* ctx, const dmsc_b200_outputs* out, void* stream);
 
+/* dmsc_b200_fetch() in two halves: fetch_start() enqueues the outputs and
+   returns, fetch_finish() (same context and stream, before any other call on
+   the context) waits for them and reports the device loops' errors, so the
+   host can prepare its result objects meanwhile. */
+int dmsc_b200_fetch_start(dmsc_b200_context* ctx, const dmsc_b200_outputs* out, void* stream);
+int dmsc_b200_fetch_finish(dmsc_b200_context* ctx, void* stream);
+
 /* Optional host destinations for the fixed-size outputs of the next
    extract() / extract_batch() on this context (no counterpart in the
    reference, whose CPU callers get host tensors only after the whole call).
