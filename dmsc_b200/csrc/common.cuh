@@ -120,8 +120,8 @@ struct Imgs {
 // The persistence pairing's starting state, written by the kernels that
 // produce its inputs instead of a pass of its own: the ordered compaction
 // sets every group's union-find link (itself) and smallest outgoing keys
-// (none) and its alive flag as it lists the extrema, plus the void's link
-// and the counters; the saddle walks record each saddle's ends as they find them and
+// (none), its alive flag and its place in the forest of the thresholded roots
+// (itself) as it lists the extrema, plus the void's links and the counters; the saddle walks record each saddle's ends as they find them and
 // reduce the saddles' keys into the minima (see pairing.cuh). Side 0
 // is the face side (maxima), side 1 the vertex side (minima).
 struct PairStart {
@@ -132,6 +132,7 @@ struct PairStart {
   int* cnt[2];                     // [6] rotating active-saddle and live-root counters
   int* n_cancel;                   // [2] cancellation counters
   uint8_t* alive[2];               // [M] extrema that no cancelled saddle kills
+  int* par[2];                     // [M + 1] forest of the thresholded roots
   int2* g12[2];                    // [nsad] groups of each saddle's two ends
   int* dying[2];                   // [nsad] decision of each saddle
   const float* sval;               // [nsad] saddle values

@@ -50,7 +50,7 @@ enum SideSlot {
   X_ROUT, X_DYING, X_GRP, X_LINK, X_MINE, X_ACT0, X_ACT1, X_CNT,
   X_UF, X_CROOT, X_CKEY, X_CVAL, X_NODE,
   X_SARC, X_SOUT, X_SFIN, X_Q0, X_Q1, X_QB, X_G12,
-  X_GBASE, X_WX, X_WA, X_CENDS, X_SOLO, kSideSlots
+  X_GBASE, X_WX, X_WA, X_PAR, X_SOLO, kSideSlots
 };
 
 struct Buf {
@@ -514,7 +514,8 @@ void run_pairing(dmsc_b200_context* ctx, PairTileArgs T, int nltile, cudaStream_
 // bases of both sides; `survive` / `pos`: the surviving saddles and their
 // exclusive scan. The survivor and cancellation counts and the status word go
 // to the readback area.
-void finish_pairing(dmsc_b200_context* ctx, uint8_t* survive, int* pos, cudaStream_t st) {
+void finish_pairing(dmsc_b200_context* ctx, const PairTileArgs& T, int nltile, uint8_t* survive, int* pos,
+                    cudaStream_t st) {
   const int nsad = ctx->nsad;
   PersistArgs P{};
   UtArgs U{};
@@ -528,7 +529,7 @@ void finish_pairing(dmsc_b200_context* ctx, uint8_t* survive, int* pos, cudaStre
   P.n_cancel = get<int>(ctx, S_NCANC, 4);
   P.pp = get<int4>(ctx, S_PP, nsad);
   P.arc = ctx->side[0].arc;
-  U.count = P.n_cancel;
+  U.n_cancel = P.n_cancel;
   U.status = ctx->status;
   const int Mf = ctx->side[0].M, Mv = ctx->side[1].M, most = std::max(Mf, Mv) + 1;
   // both sides' flags and ranks back to back, so one scan ranks them all (a
@@ -545,23 +546,22 @@ void finish_pairing(dmsc_b200_context* ctx, uint8_t* survive, int* pos, cudaStre
     P.dying[si] = S.dying;
     P.key[si] = S.key;
     P.alive[si] = S.alive;
-    P.ends[si] = sget<int2>(ctx, si, X_CENDS, nsad);
     // the replay's cancellation list (keys and saddles) comes out of the same
     // pass when this side's arcs are simplified
     P.ckey[si] = S.arcs ? sget<unsigned long long>(ctx, si, X_CKEY, nsad) : nullptr;
     P.cval[si] = S.arcs ? sget<int>(ctx, si, X_CVAL, nsad) : nullptr;
     P.node[si] = S.arcs ? sget<ReplayNode>(ctx, si, X_NODE, S.M + 1) : nullptr;
-    P.uf[si] = sget<int>(ctx, si, X_UF, S.M + 1);
-    U.ends[si] = P.ends[si];
-    U.p[si] = P.uf[si];
-    U.alive[si] = S.alive;
-    U.comp_root[si] = sget<int>(ctx, si, X_CROOT, S.M + 1);
+    P.par[si] = T.ps.par[si];
+    U.par[si] = P.par[si];
+    U.off[si] = T.off[si];
+    U.bits[si] = T.bits[si];
     U.rank[si] = S.to_out_excl;
     U.rout[si] = S.rout;
   }
-  LK(persistence_kernel<<<grid_for(std::max(nsad, most), TB), TB, 0, st>>>(P));
-  if (nsad > 0) LK(ut_union_kernel<<<dim3(grid_for(nsad, TB), 2), TB, 0, st>>>(U));
-  LK(ut_flatten_kernel<<<dim3(grid_for((most + kUtBatch - 1) / kUtBatch, TB), 2), TB, 0, st>>>(U));
+  if (nsad > 0) {
+    LK(persistence_kernel<<<grid_for(nsad, TB), TB, 0, st>>>(P));
+    LK(ut_tile_kernel<<<2u * (unsigned)nltile, 256, 0, st>>>(ctx->I, U));
+  }
   FlagScan A;
   A.in[0] = alive;
   A.in[1] = survive;
@@ -584,7 +584,7 @@ void finish_pairing(dmsc_b200_context* ctx, uint8_t* survive, int* pos, cudaStre
   R.alive_base[1] = ctx->bases.alive[1];
   R.surv_base = ctx->bases.surv;
   R.rb = (long long*)ctx->rb_d;
-  LK(root_out_kernel<<<dim3(grid_for(std::max(most, ctx->B + 1), TB), 2), TB, 0, st>>>(U, R));
+  LK(root_out_kernel<<<dim3(grid_for(std::max((most + kUtBatch - 1) / kUtBatch, ctx->B + 1), TB), 2), TB, 0, st>>>(U, R));
   LAUNCH_CHECK("persistence and ranks");
 }
 
@@ -957,6 +957,7 @@ int extract_batch_impl(dmsc_b200_context* ctx, int B, const float* img, const in
     ps.minedge[si] = sget<unsigned long long>(ctx, si, X_MINE, M + 1);
     ps.leave[si] = sget<unsigned>(ctx, si, X_CROOT, M + 1);  // free until the thresholded union-find
     ps.link[si] = sget<int>(ctx, si, X_LINK, M + 1);
+    ps.par[si] = sget<int>(ctx, si, X_PAR, M + 1);
     ps.cnt[si] = sget<int>(ctx, si, X_CNT, 8);
     ps.g12[si] = sget<int2>(ctx, si, X_G12, nsad);
     ps.dying[si] = sget<int>(ctx, si, X_DYING, nsad);
@@ -1017,21 +1018,19 @@ int extract_batch_impl(dmsc_b200_context* ctx, int B, const float* img, const in
   }
 
   mark(ctx, 4, st);
-  {
-    PairTileArgs T{};
-    T.ps = ps;
-    T.off[0] = off[2];
-    T.off[1] = off[0];
-    T.bits[0] = bmax;
-    T.bits[1] = bmin;
-    T.off_sad = off[1];
-    T.seg_sad = seg[1];
-    run_pairing(ctx, T, (int)nltile, st);
-  }
+  PairTileArgs T{};
+  T.ps = ps;
+  T.off[0] = off[2];
+  T.off[1] = off[0];
+  T.bits[0] = bmax;
+  T.bits[1] = bmin;
+  T.off_sad = off[1];
+  T.seg_sad = seg[1];
+  run_pairing(ctx, T, (int)nltile, st);
   mark(ctx, 5, st);
   uint8_t* flag = get<uint8_t>(ctx, S_FLAG, nsad);  // surviving saddles
   int* fpos = get<int>(ctx, S_FPOS, nsad);
-  finish_pairing(ctx, flag, fpos, st);
+  finish_pairing(ctx, T, (int)nltile, flag, fpos, st);
   mark(ctx, 6, st);
 
   // ---- surviving saddles in minima-sweep (vertex side) order ----

@@ -770,6 +770,7 @@ static __global__ void __launch_bounds__(256) compact_kernel(
 #pragma unroll
     for (int sd = 0; sd < 2; ++sd) {
       ps.link[sd][ps.M[sd]] = ps.M[sd];
+      ps.par[sd][ps.M[sd]] = ps.M[sd];
 #pragma unroll
       for (int k = 0; k < 6; ++k) ps.cnt[sd][k] = 0;
       ps.n_cancel[sd] = 0;
@@ -828,6 +829,7 @@ static __global__ void __launch_bounds__(256) compact_kernel(
       ps.leave[1][q] = ~0u;
       ps.link[1][q] = q;
       ps.alive[1][q] = 1;
+      ps.par[1][q] = q;
     }
     if (m & 8u) {
       const int q = o_max[k] + __popc(bmax & lt);
@@ -837,6 +839,7 @@ static __global__ void __launch_bounds__(256) compact_kernel(
       ps.leave[0][q] = ~0u;
       ps.link[0][q] = q;
       ps.alive[0][q] = 1;
+      ps.par[0][q] = q;
     }
 #pragma unroll
     for (int t = 1; t <= 2; ++t) {

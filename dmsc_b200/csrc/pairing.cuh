@@ -18,9 +18,6 @@
 // side is exactly known; the globally first remaining saddle is always
 // decided, so every round makes progress.
 //
-// The thresholded union-find (the reference's uf_min / uf_max) ends with one
-// component per connected set of cancelled saddles; its root is the unique
-// member not killed by a cancelled saddle, or the void.
 #pragma once
 
 #include <cuda/atomic>
@@ -48,6 +45,13 @@ __device__ __forceinline__ int sweep_key_saddle(unsigned long long k, bool desc)
   const int lo = (int)(uint32_t)k;
   return desc ? 0x7FFFFFFF - lo : lo;
 }
+
+// A saddle's decision on one side: the extremum that dies at it with the arc end
+// it dies on (bit 30: the second; extremum indices stay below 2^29), -1 for a
+// cycle or a saddle that is not decided yet.
+__device__ __forceinline__ int dying_word(int x, bool second) { return second ? x | 0x40000000 : x; }
+__device__ __forceinline__ int dying_of(int w) { return w < 0 ? -1 : w & 0x3FFFFFFF; }
+__device__ __forceinline__ bool dying_second(int w) { return (w >> 30) & 1; }
 
 // older(a, b) for extremum dense indices of one image; `void_id` is older
 // than all. Older = smaller (value, cell) under value_less on the vertex side
@@ -179,8 +183,8 @@ constexpr int kTileRounds = 6;    // 4, 6, 8 rounds: stage of 5.68, 4.75, 4.93 m
 constexpr int kTilePairs = 512;   // slots of the table of group pairs
 constexpr int tile_list(int warps) { return (kTileEdges / 32 + warps - 1) / warps * 32; }  // a warp's edges
 constexpr unsigned kTileVoid = 0xFFFEu;
-// `ends` of an edge that is no longer undecided: dead node | kTileDead, or a
-// cycle (or not the first between its groups); of one that leaves the tile
+// `ends` of an edge that is no longer undecided: kTileDead | the dying end (0x8000:
+// the second) | the dead node, or a cycle (or not the first between its groups); of one that leaves the tile
 constexpr uint32_t kTileDead = 0xFFFF0000u, kTileCycle = 0xFFFFFFFFu, kTileOut = 0xFFFEFFFEu;
 
 template <int NT>
@@ -402,15 +406,17 @@ __global__ void __launch_bounds__(NT, 1536 / NT) pair_tile_kernel(Imgs I, PairTi
   // A root's decision on its first outgoing edge k (value key h1): it dies
   // there when the group behind it is older and no saddle out of the tile
   // comes first. (The other end's root may read `ends` after it was marked:
-  // it finds the dead node, its own partner, there.)
+  // the dead node is then its own partner, and younger.)
   auto decide = [&](int i, uint32_t h1, int k) -> bool {
     const uint32_t e = S.ends[k];
-    const unsigned h = (e & 0xFFFFu) == (unsigned)i ? e >> 16 : e & 0xFFFFu;
+    if (e >= kTileDead) return false;
+    const bool second = (e & 0xFFFFu) != (unsigned)i;
+    const unsigned h = second ? e & 0xFFFFu : e >> 16;
     if (h != kTileVoid) {  // nodes are numbered in cell order
       const float vh = S.val[h], vi = S.val[i];
       if (!(older_less ? tie_lt(vh, (int)h, vi, i) : tie_lt(vi, i, vh, (int)h))) return false;
     }
-    S.ends[k] = kTileDead | (uint32_t)i;
+    S.ends[k] = kTileDead | (second ? 0x8000u : 0u) | (uint32_t)i;
     S.link[i] = (uint16_t)h;
     return true;
   };
@@ -496,9 +502,9 @@ __global__ void __launch_bounds__(NT, 1536 / NT) pair_tile_kernel(Imgs I, PairTi
     const uint32_t e = S.ends[k];
     if (e >= kTileDead) continue;
     const unsigned a = tile_root(S.link, e & 0xFFFFu), b = tile_root(S.link, e >> 16);
-    const uint32_t pr = a == b ? kTileCycle : min(a, b) | max(a, b) << 16;  // the void is the larger node
-    S.ends[k] = pr;
+    S.ends[k] = a == b ? kTileCycle : a | b << 16;
     if (!dedupe || a == b) continue;
+    const uint32_t pr = min(a, b) | max(a, b) << 16;
     unsigned h = (pr * 0x9E3779B1u) >> 23;  // 9 bits; there are no more pairs than slots
     for (int t = 0; t < kTilePairs; ++t) {
       const uint32_t old = atomicCAS(&tab[h], kTileCycle, pr);
@@ -524,7 +530,7 @@ __global__ void __launch_bounds__(NT, 1536 / NT) pair_tile_kernel(Imgs I, PairTi
     const int k = c * 32 + lane;
     if (k >= ne) continue;
     const uint32_t e = S.ends[k];
-    dying[saddle_of(k)] = e >= kTileDead && e != kTileCycle ? rank_of(e & 0xFFFFu) : -1;
+    dying[saddle_of(k)] = e >= kTileDead && e != kTileCycle ? dying_word(rank_of(e & 0x7FFFu), e & 0x8000u) : -1;
     n_act += e < kTileDead;
   }
 #pragma unroll
@@ -545,7 +551,9 @@ __global__ void __launch_bounds__(NT, 1536 / NT) pair_tile_kernel(Imgs I, PairTi
     const uint32_t e = S.ends[k];
     if (e >= kTileDead) continue;
     const int s = saddle_of(k);
-    if (e != kTileOut) g12[s] = make_int2(rank_of(e & 0xFFFFu), (e >> 16) == kTileVoid ? M : rank_of(e >> 16));
+    if (e != kTileOut)
+      g12[s] = make_int2((e & 0xFFFFu) == kTileVoid ? M : rank_of(e & 0xFFFFu),
+                         (e >> 16) == kTileVoid ? M : rank_of(e >> 16));
     act[pa++] = s;
   }
 #pragma unroll
@@ -562,8 +570,8 @@ __global__ void __launch_bounds__(NT, 1536 / NT) pair_tile_kernel(Imgs I, PairTi
 // 139-161), both sides of a saddle in one thread, with the saddle's image's
 // orientation and threshold: pp[s] = (paired extremum or -1, persistence bits;
 // -1 for a cycle) of the face and the vertex side, alive[d] = 0 for an extremum that a cancelled saddle
-// kills, survive[s] = 1 when neither side cancels the saddle; and the starting
-// links of the thresholded union-find.
+// kills, survive[s] = 1 when neither side cancels the saddle; and the forest of
+// the thresholded roots (ut_tile_kernel).
 struct PersistArgs {
   int nsad;
   int M[2];
@@ -579,28 +587,27 @@ struct PersistArgs {
   int4* pp;                    // [nsad] both sides
   uint8_t* alive[2];
   const int4* arc;             // [2 nsad]
-  int2* ends[2];               // cancelled saddles' arc ends, compacted
-  unsigned long long* ckey[2];  // and their replay keys and saddles (nullptr: arcs not simplified)
+  unsigned long long* ckey[2];  // cancellations' replay keys and saddles (nullptr: arcs not simplified)
   int* cval[2];
   ReplayNode* node[2];
-  int* uf[2];                  // [M + 1]
+  int* par[2];                 // [M + 1] parent of each extremum (itself when it survives)
 };
 
 __global__ void __launch_bounds__(256) persistence_kernel(PersistArgs A) {
   // saddles in list order: every per-saddle access is sequential
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   bool canc[2] = {false, false};
-  int d[2] = {-1, -1};
+  int d[2] = {-1, -1}, w[2] = {-1, -1};
   float p[2] = {-1.0f, -1.0f};
-#pragma unroll
-  for (int sd = 0; sd < 2; ++sd)
-    if (s <= A.M[sd]) A.uf[sd][s] = s;
   if (s < A.nsad) {
     const int b = A.sad_img[s];
     const bool du = A.dual[b];
     const float sv = A.sval[s], thr = A.thr[b];
 #pragma unroll
-    for (int sd = 0; sd < 2; ++sd) d[sd] = A.dying[sd][s];
+    for (int sd = 0; sd < 2; ++sd) {
+      w[sd] = A.dying[sd][s];
+      d[sd] = dying_of(w[sd]);
+    }
     float ev[2];
 #pragma unroll
     for (int sd = 0; sd < 2; ++sd) ev[sd] = d[sd] >= 0 ? __int_as_float(A.key[sd][d[sd]].x) : 0.f;
@@ -617,18 +624,19 @@ __global__ void __launch_bounds__(256) persistence_kernel(PersistArgs A) {
     A.pp[s] = make_int4(d[0], __float_as_int(p[0]), d[1], __float_as_int(p[1]));
     A.survive[s] = !(canc[0] || canc[1]);
   }
-  // cancelled edges' ends, compacted for the thresholded union-find, and (when
-  // the side's arcs are simplified) the same cancellations with their replay
-  // keys (CancelEvent::operator<, cpu/persistence_struct.hxx:16-21):
-  // (persistence, saddle cell); a saddle is cancelled at most once per side,
-  // so the pair is unique and the target cell never breaks a tie
+  // the cancelled edge hangs the extremum it kills under its other end; and,
+  // when the side's arcs are simplified, its replay key joins the list
+  // (CancelEvent::operator<, cpu/persistence_struct.hxx:16-21): (persistence,
+  // saddle cell); a saddle is cancelled at most once per side, so the pair is
+  // unique and the target cell never breaks a tie
   int slot[2];
-  block_reserve2(A.n_cancel, canc[0], A.n_cancel + 1, canc[1], slot[0], slot[1]);
+  block_reserve2(A.n_cancel, canc[0] && A.ckey[0], A.n_cancel + 1, canc[1] && A.ckey[1], slot[0], slot[1]);
 #pragma unroll
   for (int sd = 0; sd < 2; ++sd) {
     if (!canc[sd]) continue;
     const int4 a = A.arc[2 * (long long)s + sd];
-    A.ends[sd][slot[sd]] = make_int2(a.x, a.y);
+    const int t = dying_second(w[sd]) ? a.x : a.y;
+    A.par[sd][d[sd]] = t >= 0 ? t : A.M[sd];
     if (!A.ckey[sd]) continue;
     const unsigned long long key = ((unsigned long long)orderable_key(p[sd]) << 32) | (unsigned)A.crit_sad[s];
     A.ckey[sd][slot[sd]] = key;
@@ -640,123 +648,130 @@ __global__ void __launch_bounds__(256) persistence_kernel(PersistArgs A) {
   }
 }
 
-// Thresholded union-find (the reference's uf_min / uf_max, persistence.hxx:
-// 90-104, 147-161): lock-free union of the ends of every cancelled saddle
-// (link the larger root under the smaller), over the compact list of
-// cancelled edges written by persistence_kernel. Every link points to a
-// smaller index, so a root search takes at most n steps and every failed CAS
-// means another thread linked one of the two roots (at most n - 1 links
-// exist); both loops are capped at the node count anyway, and a cap sets
-// kStatusFindCap and returns the node reached (a valid index). One edge per
-// thread: advancing 4 edges' searches in lockstep measured slower here (the
-// forest is deep while the unions run, and a thread waits for its longest).
-// Both sides in one launch (blockIdx.y).
+// Thresholded roots (the reference's uf_min / uf_max, persistence.hxx:90-104,
+// 147-161): one component per connected set of cancelled saddles, whose root
+// is its one surviving extremum, or the void. No union is needed: every killed
+// extremum d hangs under the extremum t at the other end of the saddle that
+// kills it.
+//   * d and t are in one component: everything that merged into d's pairing
+//     group before died younger than d and earlier in the sweep, so with no
+//     larger persistence (float subtraction is monotone) and was cancelled too;
+//     so d's end of the saddle hangs together with d.
+//   * There is no cycle: links put both ends into one pairing group for good,
+//     and the last link of a cycle would join two ends that the earlier ones had
+//     joined already.
+// Chains are long (means of 20 to 70 links on the bump fields, up to 350) but
+// stay local: followed inside 64 x 64 tiles first (ut_tile_kernel, pointer
+// jumping in shared memory), 2 to 6 links are left for root_out_kernel. With
+// a lock-free union of the cancelled edges and its flattening instead the
+// persistence and rank stage took 0.57 ms at 4096^2, threshold 0.05, now 0.36;
+// 0.196 -> 0.128 at 2048^2, threshold 0.25.
 struct UtArgs {
   int M[2];                  // the void is node M
-  const int2* ends[2];
-  const int* count;          // [2] cancelled edges
-  int* p[2];                 // [M + 1] links
-  const uint8_t* alive[2];
-  int* comp_root[2];         // [M + 1] alive member of each root's component, -1 for the void's
+  const int* off[2];         // segment offsets and bit masks of each side's extrema
+  const uint32_t* bits[2];
+  int* par[2];               // [M + 1] parents, then roots
   const int* rank[2];        // [M] alive extrema before each extremum
   int* rout[2];              // [M] rank of each extremum's thresholded root, -1 for the void
+  const int* n_cancel;       // [2]
   unsigned* status;
 };
 
-__device__ __forceinline__ int uf_root(int* p, int x, int cap, unsigned* status) {
-  for (int k = 0;; ++k) {
-    int px = p[x];
-    if (px == x) return x;
-    if (k >= cap) {
-      set_status(status, kStatusFindCap);
-      return x;
+// One tile and side per block: every extremum's parent becomes the first
+// extremum on its chain that survives or lies in another tile (or the void).
+constexpr int kUtNodes = 2048;  // a tile with more is left as it is
+__global__ void __launch_bounds__(256) ut_tile_kernel(Imgs I, UtArgs A) {
+  __shared__ int target[kUtNodes];     // a chain's end: its rank
+  __shared__ uint16_t next[kUtNodes];  // node in the tile, or kUtEnd | itself
+  __shared__ int base[kLT], pre[kLT + 1];
+  constexpr unsigned kUtEnd = 0x8000u;
+  const bool s1 = blockIdx.x & 1;
+  const LabelTile g = label_tile_of(I, blockIdx.x >> 1);
+  int* par = s1 ? A.par[1] : A.par[0];
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int nsegx = (g.W + kTileX) / kTileX;
+  if (tid < kLT) {  // a row's extrema are consecutive ranks
+    const int y = g.y0 + tid, sx = g.x0 >> 5;
+    const bool in = y <= g.H;
+    const long long q = (long long)I.seg_base[g.b] + (long long)y * nsegx + sx;
+    const uint32_t* bits = s1 ? A.bits[1] : A.bits[0];
+    base[tid] = in ? __ldg((s1 ? A.off[1] : A.off[0]) + q) : 0x7FFFFFFF;
+    int n = in ? __popc(__ldg(bits + q)) + (sx + 1 < nsegx ? __popc(__ldg(bits + q + 1)) : 0) : 0;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, n, o);
+      if (lane >= o) n += v;
     }
-    int ppx = p[px];
-    if (ppx != px) p[x] = ppx;  // path halving; benign race
-    x = ppx;
+    pre[tid + 1] = n;  // inside its half
+    if (tid == 0) pre[0] = 0;
+  }
+  __syncthreads();
+  const int half = pre[32];
+  __syncthreads();
+  if (tid >= 32 && tid < kLT) pre[tid + 1] += half;
+  __syncthreads();
+  const int nn = pre[kLT];
+  if (nn > kUtNodes) return;
+  auto row_of = [&](int i) {
+    int r = 0;
+#pragma unroll
+    for (int w = kLT / 2; w > 0; w >>= 1)
+      if (pre[r + w] <= i) r += w;
+    return r;
+  };
+  constexpr int kPer = kUtNodes / 256;
+  int x[kPer], p[kPer];
+#pragma unroll
+  for (int j = 0; j < kPer; ++j) {
+    const int i = tid + 256 * j;
+    x[j] = -1;
+    if (i < nn) {
+      const int r = row_of(i);
+      x[j] = base[r] + i - pre[r];
+      p[j] = par[x[j]];
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < kPer; ++j) {
+    const int i = tid + 256 * j;
+    if (x[j] < 0) continue;
+    unsigned nx = kUtEnd | (unsigned)i;
+    if (p[j] != x[j]) {  // the parent's node, when it lies in the tile
+      int r = 0;
+#pragma unroll
+      for (int w = kLT / 2; w > 0; w >>= 1)
+        if (base[r + w] <= p[j]) r += w;
+      const int k = p[j] - base[r];
+      if (k >= 0 && k < pre[r + 1] - pre[r]) nx = (unsigned)(pre[r] + k);
+    }
+    target[i] = p[j];
+    next[i] = (uint16_t)nx;
+  }
+  __syncthreads();
+  // barrier-free pointer jumping: any value read lies further along the same
+  // chain, so a pointer only moves toward the chain's end
+  volatile uint16_t* vn = next;
+#pragma unroll
+  for (int j = 0; j < kPer; ++j) {
+    const int i = tid + 256 * j;
+    if (x[j] < 0) continue;
+    unsigned nx = vn[i];
+    const bool moved = !(nx & kUtEnd);
+    for (int k = 0; !(nx & kUtEnd) && k <= kUtNodes; ++k) {
+      nx = vn[nx];
+      vn[i] = (uint16_t)nx;
+    }
+    if (moved && (nx & kUtEnd)) par[x[j]] = target[nx & (kUtEnd - 1u)];
   }
 }
 
-__global__ void __launch_bounds__(256) ut_union_kernel(UtArgs A) {
-  const bool s1 = blockIdx.y != 0;
-  const int2* __restrict__ ends = s1 ? A.ends[1] : A.ends[0];
-  int* p = s1 ? A.p[1] : A.p[0];
-  const int void_id = s1 ? A.M[1] : A.M[0], cap = void_id + 2, n = A.count[s1];
-  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
-    const int2 e = ends[q];
-    int a = e.x < 0 ? void_id : e.x;
-    int b = e.y < 0 ? void_id : e.y;
-    for (int tries = 0;; ++tries) {
-      if (tries >= cap) {
-        set_status(A.status, kStatusFindCap);
-        break;
-      }
-      a = uf_root(p, a, cap, A.status);
-      b = uf_root(p, b, cap, A.status);
-      if (a == b) break;
-      if (a > b) {
-        int t = a;
-        a = b;
-        b = t;
-      }
-      if (atomicCAS(p + b, b, a) == b) break;
-    }
-  }
-}
-
+// Rank of each extremum's thresholded root among the alive extrema (-1 for the
+// void), kUtBatch extrema per thread with their chains followed in lockstep (a
+// written root is further along the same chain for every reader); and the
+// images' first alive ranks and survivors (B + 1 entries, the last ones the
+// totals), with the counts and the status word for the host straight to the
+// mapped readback area.
 constexpr int kUtBatch = 4;
-
-// Every node's root, kUtBatch nodes per thread with their pointer chains
-// followed in lockstep (a written root is an ancestor for every reader), and
-// each component's alive member.
-__global__ void ut_flatten_kernel(UtArgs A) {
-  const bool s1 = blockIdx.y != 0;
-  int* p = s1 ? A.p[1] : A.p[0];
-  const uint8_t* alive = s1 ? A.alive[1] : A.alive[0];
-  int* comp_root = s1 ? A.comp_root[1] : A.comp_root[0];
-  const int M = s1 ? A.M[1] : A.M[0], n = M + 1, cap = M + 2;
-  const long long nt = (long long)gridDim.x * blockDim.x;
-  const long long x0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  int r[kUtBatch];
-  unsigned live = 0;
-#pragma unroll
-  for (int u = 0; u < kUtBatch; ++u) {
-    const long long x = x0 + nt * u;
-    r[u] = (int)x;
-    if (x < n) live |= 1u << u;
-  }
-  const unsigned own = live;
-  for (int k = 0; live; ++k) {
-    if (k >= cap) {
-      set_status(A.status, kStatusFindCap);
-      break;
-    }
-    int pr[kUtBatch];
-#pragma unroll
-    for (int u = 0; u < kUtBatch; ++u) pr[u] = ((live >> u) & 1u) ? p[r[u]] : r[u];
-#pragma unroll
-    for (int u = 0; u < kUtBatch; ++u) {
-      if (pr[u] == r[u]) live &= ~(1u << u);
-      r[u] = pr[u];
-    }
-  }
-#pragma unroll
-  for (int u = 0; u < kUtBatch; ++u) {
-    if (!((own >> u) & 1u)) continue;
-    const int x = (int)(x0 + nt * u);
-    p[x] = r[u];
-    if (x == M)
-      comp_root[r[u]] = -1;
-    else if (alive[x])
-      comp_root[r[u]] = x;
-  }
-}
-
-// Rank of each extremum's thresholded root among the alive extrema: the
-// component's alive member (comp_root of its flattened union-find root; -1
-// for the void's component); and the images' first alive ranks and survivors
-// (B + 1 entries, the last ones the totals), with the counts and the status
-// word for the host straight to the mapped readback area.
 struct RankBases {
   int B, nsad;
   const int* first[2];   // [B + 1] first extremum of each image and side
@@ -784,15 +799,44 @@ __global__ void __launch_bounds__(256) root_out_kernel(UtArgs A, RankBases R) {
       R.surv_base[x] = q < R.nsad ? R.pos[q] : R.total[1];
       if (x == 0) {
         R.rb[0] = R.total[1];
-        R.rb[1] = A.count[0];
-        R.rb[2] = A.count[1];
+        R.rb[1] = A.n_cancel[0];
+        R.rb[2] = A.n_cancel[1];
         R.rb[3] = *A.status;
       }
     }
   }
-  if (x >= M) return;
-  const int u = (s1 ? A.comp_root[1] : A.comp_root[0])[(s1 ? A.p[1] : A.p[0])[x]];
-  (s1 ? A.rout[1] : A.rout[0])[x] = u >= 0 ? (s1 ? A.rank[1] : A.rank[0])[u] : -1;
+  int* par = s1 ? A.par[1] : A.par[0];
+  const int nt = gridDim.x * blockDim.x;
+  int r[kUtBatch];
+  unsigned live = 0, own = 0;
+#pragma unroll
+  for (int u = 0; u < kUtBatch; ++u) {
+    const long long i = x + (long long)nt * u;
+    r[u] = (int)i;
+    if (i < M) own |= 1u << u;
+  }
+  live = own;
+  for (int k = 0; live; ++k) {
+    if (k > M) {  // a chain visits a node at most once: never reached
+      set_status(A.status, kStatusFindCap);
+      break;
+    }
+    int q[kUtBatch];
+#pragma unroll
+    for (int u = 0; u < kUtBatch; ++u) q[u] = ((live >> u) & 1u) ? par[r[u]] : r[u];
+#pragma unroll
+    for (int u = 0; u < kUtBatch; ++u) {
+      if (q[u] == r[u]) live &= ~(1u << u);
+      r[u] = q[u];
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < kUtBatch; ++u) {
+    if (!((own >> u) & 1u)) continue;
+    const int i = x + nt * u;
+    par[i] = r[u];
+    (s1 ? A.rout[1] : A.rout[0])[i] = r[u] == M ? -1 : (s1 ? A.rank[1] : A.rank[0])[r[u]];
+  }
 }
 
 }  // namespace dmsc

@@ -318,6 +318,7 @@ __device__ __forceinline__ void pair_batch_b(const PairArgs2& P, int r, long lon
     older_less |= (unsigned)(s1 ? !d : d) << u;
   }
   int h[U];
+  unsigned sec = 0;  // the root's end is the saddle's second
 #pragma unroll
   for (int u = 0; u < U; ++u) {
     h[u] = 0;
@@ -325,6 +326,7 @@ __device__ __forceinline__ void pair_batch_b(const PairArgs2& P, int r, long lon
     const bool s1 = (s1m >> u) & 1u;
     const int2 gg = PSIDE(g12)[e[u]];  // roots as of phase A
     h[u] = gg.x == g[u] ? gg.y : gg.x;
+    sec |= (unsigned)(gg.x != g[u]) << u;
   }
   int2 kh[U];
 #pragma unroll
@@ -345,7 +347,7 @@ __device__ __forceinline__ void pair_batch_b(const PairArgs2& P, int r, long lon
       dies = ((older_less >> u) & 1u) ? tie_lt(vh, kh[u].y, vg, kg[u].y) : tie_lt(vg, kg[u].y, vh, kh[u].y);
     }
     if (dies) {
-      PSIDE(dying)[e[u]] = g[u];
+      PSIDE(dying)[e[u]] = dying_word(g[u], (sec >> u) & 1u);
       PSIDE(link)[g[u]] = h[u];
     } else {
       chunk_keep(L, s1, g[u]);
@@ -562,7 +564,7 @@ __global__ void __launch_bounds__(kSoloNT) pair_solo_kernel(PairArgs2 P) {
           const float vh = __int_as_float(kh.x), vg = __int_as_float(kg.x);
           if (!(older_less ? tie_lt(vh, kh.y, vg, kg.y) : tie_lt(vg, kg.y, vh, kh.y))) continue;
         }
-        A.dying[sweep_key_saddle(m, e >> 31)] = S.rank[g];
+        A.dying[sweep_key_saddle(m, e >> 31)] = dying_word(S.rank[g], j != 0);
         S.link[g] = (uint16_t)h;
       }
     }
@@ -675,7 +677,7 @@ __device__ __forceinline__ void replay_batch(const ReplayArgs2& P, int rd, long 
 #pragma unroll
   for (int u = 0; u < U; ++u) {
     const bool s1 = (s1m >> u) & 1u;
-    d[u] = ((act >> u) & 1u) ? RSIDE(dying)[sd[u]] : 0;
+    d[u] = ((act >> u) & 1u) ? dying_of(RSIDE(dying)[sd[u]]) : 0;
   }
   // bit c of `live` is a walk that has not ended (the root as of the step's
   // key is not reached), bit c of `wait` one that met an undecided node
@@ -828,7 +830,7 @@ __global__ void __launch_bounds__(256, MINB) replay_persistent_kernel(ReplayArgs
         const ReplayArgs& A = i < na ? P.s[0] : P.s[1];
         const long long k = i < na ? i : i - na;
         const int r = rd == 0 ? (int)k : ((rd & 1) ? A.act1 : A.act0)[k];
-        A.S.node[A.dying[A.cj[r]]].status = kRootForever;
+        A.S.node[dying_of(A.dying[A.cj[r]])].status = kRootForever;
       }
       break;
     }
