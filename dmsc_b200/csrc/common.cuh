@@ -113,9 +113,25 @@ struct Imgs {
   const int* tile_base;  // 32 x 64 gradient index tiles
   const int* seg_base;   // 32-index row segments
   const int* ltile_base;  // 64 x 64 label tiles
+  const unsigned* magic;  // row_of's multiplier and shift
+  const int* shift;
   const uint8_t* dual;
   const float* thr;
 };
+
+// Row of the image-local index l of image b: l / (W + 1) by a multiplication.
+// With c = ceil(log2(W + 1)), shift = 29 + c and magic = ceil(2^shift / (W + 1))
+// < 2^30, the product is exact for l < 2^29 (an image's indices: 4 l is an int),
+// since magic (W + 1) exceeds 2^shift by less than 2^c.
+__device__ __forceinline__ int row_of(const Imgs& I, int b, int l) {
+  return (int)(((unsigned long long)(unsigned)l * I.magic[b]) >> I.shift[b]);
+}
+inline void row_magic(int Nx, unsigned* magic, int* shift) {
+  int c = 0;
+  while ((1LL << c) < Nx) ++c;
+  *shift = 29 + c;
+  *magic = (unsigned)(((1ULL << *shift) + (unsigned)Nx - 1) / (unsigned)Nx);
+}
 
 // The persistence pairing's starting state, written by the kernels that
 // produce its inputs instead of a pass of its own: the ordered compaction

@@ -811,7 +811,7 @@ int extract_batch_impl(dmsc_b200_context* ctx, int B, const float* img, const in
     return kErrInvalidArgument;
   }
   // per-image tables (host): 32-bit cell ids per image (input_validation.hxx:24-26) and for the batch
-  std::vector<int> tab(9 * (size_t)(B + 1), 0);
+  std::vector<int> tab(11 * (size_t)(B + 1), 0);
   int* tH = tab.data();
   int* tW = tH + (B + 1);
   int* idx_base = tW + (B + 1);
@@ -821,6 +821,8 @@ int extract_batch_impl(dmsc_b200_context* ctx, int B, const float* img, const in
   int* peaks_off = seg_base + (B + 1);
   int* basins_off = peaks_off + (B + 1);
   int* ltile_base = basins_off + (B + 1);
+  int* magic = ltile_base + (B + 1);
+  int* shift = magic + (B + 1);
   const int gshape = ctx->grad_shape;
   const int gTY = kGradTY[gshape];
   long long nidx = 0, npx = 0, ntile = 0, nseg = 0, npk = 0, nbs = 0, nltile = 0;
@@ -844,6 +846,7 @@ int extract_batch_impl(dmsc_b200_context* ctx, int B, const float* img, const in
     peaks_off[b] = (int)npk;
     basins_off[b] = (int)nbs;
     ltile_base[b] = (int)nltile;
+    row_magic((int)W + 1, (unsigned*)magic + b, shift + b);
     nltile += ((W + kLT) / kLT) * ((H + kLT) / kLT);
     const long long ntx = (W + 1 + kTileX - 1) / kTileX, nty = (H + 1 + gTY - 1) / gTY;
     nidx += (H + 1) * (W + 1);
@@ -878,7 +881,7 @@ int extract_batch_impl(dmsc_b200_context* ctx, int B, const float* img, const in
   join_copies(ctx, st);  // host copies of an earlier call still reading its outputs
   mark(ctx, 0, st);
   CK(cudaMemsetAsync(ctx->zero, 0, sizeof(ZeroArea), st));
-  {  // upload the tables: 9 int arrays, then thr (float) and dual (u8)
+  {  // upload the tables: 11 int arrays, then thr (float) and dual (u8)
     size_t ib = tab.size() * sizeof(int), fb = (size_t)B * sizeof(float);
     size_t total = ib + fb + B + 16;
     char* h = (char*)staging(ctx, total);
@@ -896,6 +899,8 @@ int extract_batch_impl(dmsc_b200_context* ctx, int B, const float* img, const in
     ctx->I.tile_base = di + 4 * (B + 1);
     ctx->I.seg_base = di + 5 * (B + 1);
     ctx->I.ltile_base = di + 8 * (B + 1);
+    ctx->I.magic = (const unsigned*)(di + 9 * (B + 1));
+    ctx->I.shift = di + 10 * (B + 1);
     ctx->I.thr = (const float*)(d + ib);
     ctx->I.dual = (const uint8_t*)(d + ib + fb);
   }
@@ -984,7 +989,7 @@ int extract_batch_impl(dmsc_b200_context* ctx, int B, const float* img, const in
   int4* arc = get<int4>(ctx, S_ARC, 2 * (size_t)nsad);
   if (nsad > 0) {
     LK(saddle_walk_kernel<<<grid_for(nsad, TB), TB, 0, st>>>(I, flow, nsad, csad, isad, off[2], bmax, off[0], bmin,
-                                                             arc, ncells, ps, ctx->status));
+                                                             arc, (int)ncells, ps, ctx->status));
     LAUNCH_CHECK("saddle_walk_kernel");
   }
 

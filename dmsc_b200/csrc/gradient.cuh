@@ -638,16 +638,7 @@ __global__ void __launch_bounds__(NT) gradient_batch_kernel(Imgs I, const float*
 // cell_value (cpu/cell_compare.hxx:82-87): value of the highest (dual: lowest)
 // vertex, chosen by (value, pixel id) in the reference's scan order (each
 // candidate replaces the current choice when value_greater); the chosen
-// pixel's own value is returned, so -0.0 survives. `pick` adds one candidate.
-template <bool DUAL>
-__device__ __forceinline__ void pick(bool& have, float& bv, int& bi, bool valid, float v, int id) {
-  if (valid && (!have || value_greater<DUAL>(v, id, bv, bi))) {
-    have = true;
-    bv = v;
-    bi = id;
-  }
-}
-
+// pixel's own value is returned, so -0.0 survives.
 // Values of the four cells of index (y, x) for a whole warp of consecutive
 // columns: every lane loads its pixel and the one above it, takes its left
 // neighbours' from the lane to its left (lane 0 loads them), and evaluates
@@ -678,44 +669,44 @@ __device__ __forceinline__ CellPixels warp_cell_loads(const float* __restrict__ 
   return c;
 }
 
-template <bool DUAL>
+// The candidates of a cell come in ascending pixel id, so each one is compared
+// as the later pixel (gt_after). INTERIOR: every lane's four pixels exist.
+template <bool DUAL, bool INTERIOR>
 __device__ __forceinline__ CellValues cell_values_of(CellPixels px, int y, int x, int H, int W, int lane) {
-  const bool in_x = x < W, up = y >= 1, here = y < H;
   const float a = px.a, u = px.u;
   float aL = __shfl_up_sync(0xffffffffu, a, 1), uL = __shfl_up_sync(0xffffffffu, u, 1);
   if (lane == 0) {
     aL = px.aL;
     uL = px.uL;
   }
-  const int id = y * W + x, idu = id - W;
   CellValues c;
   c.v = a;
-  {
-    bool hv = false;
-    float bv = 0.f;
-    int bi = 0;
-    pick<DUAL>(hv, bv, bi, here && x >= 1, aL, id - 1);
-    pick<DUAL>(hv, bv, bi, here && in_x, a, id);
-    c.h = bv;
+  if (INTERIOR) {
+    const bool ga = gt_after<DUAL>(a, aL);
+    c.h = ga ? a : aL;
+    c.e = gt_after<DUAL>(a, u) ? a : u;
+    float f = gt_after<DUAL>(u, uL) ? u : uL;
+    f = gt_after<DUAL>(aL, f) ? aL : f;
+    c.f = gt_after<DUAL>(a, f) ? a : f;
+    return c;
   }
-  {
-    bool hv = false;
-    float bv = 0.f;
-    int bi = 0;
-    pick<DUAL>(hv, bv, bi, up && in_x, u, idu);
-    pick<DUAL>(hv, bv, bi, here && in_x, a, id);
-    c.e = bv;
-  }
-  {
-    bool hv = false;
-    float bv = 0.f;
-    int bi = 0;
-    pick<DUAL>(hv, bv, bi, up && x >= 1, uL, idu - 1);
-    pick<DUAL>(hv, bv, bi, up && in_x, u, idu);
-    pick<DUAL>(hv, bv, bi, here && x >= 1, aL, id - 1);
-    pick<DUAL>(hv, bv, bi, here && in_x, a, id);
-    c.f = bv;
-  }
+  const bool in_x = x < W, in_l = x >= 1, up = y >= 1, here = y < H;
+  auto pick = [](bool& have, float& best, bool valid, float v) {
+    if (valid && (!have || gt_after<DUAL>(v, best))) {
+      have = true;
+      best = v;
+    }
+  };
+  bool hh = false, he = false, hf = false;
+  c.h = c.e = c.f = 0.f;
+  pick(hh, c.h, here && in_l, aL);
+  pick(hh, c.h, here && in_x, a);
+  pick(he, c.e, up && in_x, u);
+  pick(he, c.e, here && in_x, a);
+  pick(hf, c.f, up && in_l, uL);
+  pick(hf, c.f, up && in_x, u);
+  pick(hf, c.f, here && in_l, aL);
+  pick(hf, c.f, here && in_x, a);
   return c;
 }
 
@@ -817,8 +808,13 @@ static __global__ void __launch_bounds__(256) compact_kernel(
       max_bits[seg] = bmax;
     }
     if ((bmin | bmax | bh | bv) == 0u) continue;  // the whole warp together
-    const CellValues cv = I.dual[bk] ? cell_values_of<true>(px[k], iy[k], ix[k], H, W, lane)
-                                     : cell_values_of<false>(px[k], iy[k], ix[k], H, W, lane);
+    const int xs = ix[k] - lane;  // warp-uniform
+    const bool inside = iy[k] >= 1 && iy[k] < H && xs >= 1 && xs + 31 < W;
+    const CellValues cv =
+        I.dual[bk] ? (inside ? cell_values_of<true, true>(px[k], iy[k], ix[k], H, W, lane)
+                             : cell_values_of<true, false>(px[k], iy[k], ix[k], H, W, lane))
+                   : (inside ? cell_values_of<false, true>(px[k], iy[k], ix[k], H, W, lane)
+                             : cell_values_of<false, false>(px[k], iy[k], ix[k], H, W, lane));
     // saddles before this lane's: both edge kinds of the lanes below it
     int p = o_sad[k] + __popc(bh & lt) + __popc(bv & lt);
     if (m & 1u) {

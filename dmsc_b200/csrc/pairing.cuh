@@ -79,9 +79,11 @@ constexpr int kCycleEnd = (int)0x80000000;
 // in one 32-byte sector, for the random reads); and the pairing's starting
 // state: a saddle whose two ends coincide is a cycle, the others
 // record their ends and reduce their sweep key into both ends' minima
-// (nothing waits for these reductions: 0.03 ms of the 0.33 ms at 4096^2), and
-// a saddle that is not local to its tile reduces the value part of its key
-// into its ends' `leave` too.
+// (nothing waits for these reductions), and a saddle that is not local to its
+// tile reduces the value part of its key into its ends' `leave` too. Bound by
+// instruction issue: the rows of the four ends by multiplication instead of
+// division and 32-bit step counts took it from 38 to 32 registers (all 64
+// warps of an SM resident) and from 0.373 to 0.266 ms at 4096^2.
 __global__ void __launch_bounds__(256) saddle_walk_kernel(Imgs I, const uint8_t* __restrict__ flow, int nsad,
                                                           const int* __restrict__ crit_sad,
                                                           const int* __restrict__ sad_img,
@@ -89,28 +91,28 @@ __global__ void __launch_bounds__(256) saddle_walk_kernel(Imgs I, const uint8_t*
                                                           const uint32_t* __restrict__ max_bits,
                                                           const int* __restrict__ off_min,
                                                           const uint32_t* __restrict__ min_bits,
-                                                          int4* __restrict__ arc, long long cap, PairStart ps, unsigned* status) {
+                                                          int4* __restrict__ arc, int cap, PairStart ps, unsigned* status) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= nsad) return;
   const int b = sad_img[s];
   const int H = I.H[b], W = I.W[b], Nx = W + 1;
   const int sc = crit_sad[s];
-  const int sl = (sc >> 2) - I.idx_base[b], sy = sl / Nx, sx = sl - sy * Nx;
+  const int sl = (sc >> 2) - I.idx_base[b], sy = row_of(I, b, sl), sx = sl - sy * Nx;
   int te[2][2], len[2][2], loc[2][2];  // loc: the end's cell in the saddle's tile, -1 when it lies in another
 #pragma unroll
   for (int j = 0; j < 2; ++j) {
-    long long steps;
+    int steps;
     const int end = flow_walk<4>(flow, face_start(sc, j, Nx) >> 2, Nx, cap, &steps, status);
     int y, x;
     const int target = seg_rank(I, b, end, Nx, off_max, max_bits, y, x);
     te[0][j] = target;
-    len[0][j] = target >= 0 ? (int)steps + 1 : 0;  // cells of the raw arc, start and end included
+    len[0][j] = target >= 0 ? steps + 1 : 0;  // cells of the raw arc, start and end included
     loc[0][j] = ((y ^ sy) | (x ^ sx)) >> 6 ? -1 : (y & 63) << 6 | (x & 63);
   }
 #pragma unroll
   for (int j = 0; j < 2; ++j) {
-    const int start = vertex_start(sc, j, H, W, Nx, I.idx_base[b]);
-    long long steps = 0;
+    const int start = vertex_start(sc, j, sy, sx, H, W, Nx);
+    int steps = 0;
     int target = -1, at = kLocalVoid;
     if (start >= 0) {
       const int end = flow_walk<0>(flow, start >> 2, Nx, cap, &steps, status);
@@ -119,7 +121,7 @@ __global__ void __launch_bounds__(256) saddle_walk_kernel(Imgs I, const uint8_t*
       at = ((y ^ sy) | (x ^ sx)) >> 6 ? -1 : (y & 63) << 6 | (x & 63);
     }
     te[1][j] = target;
-    len[1][j] = target >= 0 ? (int)steps + 1 : 0;  // an arc that leaves the image is empty
+    len[1][j] = target >= 0 ? steps + 1 : 0;  // an arc that leaves the image is empty
     loc[1][j] = at;
   }
   // a raw arc has fewer cells than the batch (cell ids are int32)

@@ -74,7 +74,7 @@ __device__ __forceinline__ int cell_pixel_g(const float* __restrict__ img, int t
 __device__ __forceinline__ int value_pixel(const float* __restrict__ img_all, const Imgs& I, int b, int cell) {
   const int H = I.H[b], W = I.W[b], Nx = W + 1;
   const int lidx = (cell >> 2) - I.idx_base[b];
-  const int y = lidx / Nx, x = lidx - y * Nx;
+  const int y = row_of(I, b, lidx), x = lidx - y * Nx;
   const float* img = img_all + I.px_base[b];
   return I.dual[b] ? cell_pixel_g<true>(img, cell & 3, y, x, H, W) : cell_pixel_g<false>(img, cell & 3, y, x, H, W);
 }

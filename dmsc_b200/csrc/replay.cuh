@@ -277,8 +277,9 @@ __device__ __forceinline__ int surv_start(const EmitCtx& E, int i, int b) {
 // cell from the saddle's cell with no further load.
 __device__ __forceinline__ int arc_start_of_cell(const EmitCtx& E, int sc, int j, int b) {
   const int W = E.I.W[b], Nx = W + 1;
-  const int cell = E.faces ? face_start(sc, j, Nx) : vertex_start(sc, j, E.I.H[b], W, Nx, E.I.idx_base[b]);
-  return cell >> 2;
+  if (E.faces) return face_start(sc, j, Nx) >> 2;
+  const int l = (sc >> 2) - E.I.idx_base[b], y = row_of(E.I, b, l);
+  return vertex_start(sc, j, y, l - y * Nx, E.I.H[b], W, Nx) >> 2;
 }
 __device__ __forceinline__ int4 make_saddle_seg(int scell, int j, int rev, long long len, long long pos) {
   return make_int4(rev | (j << 1), scell, (int)len, (int)pos);

@@ -21,29 +21,22 @@ __device__ __forceinline__ int face_start(int s_cell, int j, int Nx) {
   return (cell_type(s_cell) == 1) ? 3 + 4 * (idx + Nx) : 3 + 4 * (idx + 1);
 }
 
-// The j-th valid start cell on the vertex side, or -1. `s_cell` may be a
-// global cell id of a batch whose image starts at index `ibase`.
-__device__ __forceinline__ int vertex_start(int s_cell, int j, int H, int W, int Nx, int ibase = 0) {
-  int idx = s_cell >> 2, t = cell_type(s_cell);
-  int lidx = idx - ibase;
-  int ey = lidx / Nx, ex = lidx - ey * Nx;
-  int v[2], n = 0;
-  if (t == 1) {
-    if (ex - 1 >= 0) v[n++] = 4 * (idx - 1);
-    if (ex < W) v[n++] = 4 * idx;
-  } else {
-    if (ey - 1 >= 0) v[n++] = 4 * (idx - Nx);
-    if (ey < H) v[n++] = 4 * idx;
-  }
-  return j < n ? v[j] : -1;
+// The j-th valid start cell on the vertex side, or -1; the saddle lies at
+// (ey, ex) of its image (`s_cell` may be a global cell id).
+__device__ __forceinline__ int vertex_start(int s_cell, int j, int ey, int ex, int H, int W, int Nx) {
+  const int idx = s_cell >> 2;
+  const bool h = cell_type(s_cell) == 1;
+  const bool low = h ? ex >= 1 : ey >= 1, high = h ? ex < W : ey < H;
+  if (j == 0 && low) return 4 * (h ? idx - 1 : idx - Nx);
+  return (j == 0 || low) && high ? 4 * idx : -1;
 }
 
 // Walks from index `idx` along the flow codes (nibble shift 0 = vertices,
 // 4 = faces) to the index of the critical cell; counts the steps.
 template <int SHIFT>
-__device__ __forceinline__ int flow_walk(const uint8_t* __restrict__ flow, int idx, int Nx, long long cap,
-                                         long long* steps, unsigned* status) {
-  long long n = 0;
+__device__ __forceinline__ int flow_walk(const uint8_t* __restrict__ flow, int idx, int Nx, int cap, int* steps,
+                                         unsigned* status) {
+  int n = 0;
   unsigned c;
   while ((c = (__ldg(flow + idx) >> SHIFT) & 7u) != kFlowNone) {
     idx += flow_step(c, Nx);
@@ -63,7 +56,7 @@ __device__ __forceinline__ int flow_walk(const uint8_t* __restrict__ flow, int i
 __device__ __forceinline__ int seg_rank(const Imgs& I, int b, int g, int Nx, const int* __restrict__ off,
                                         const uint32_t* __restrict__ bits, int& y, int& x) {
   const int l = g - I.idx_base[b];
-  y = l / Nx;
+  y = row_of(I, b, l);
   x = l - y * Nx;
   const int seg = I.seg_base[b] + y * ((Nx + 31) >> 5) + (x >> 5);
   return __ldg(off + seg) + __popc(__ldg(bits + seg) & ((1u << (x & 31)) - 1u));
@@ -410,7 +403,7 @@ __global__ void __launch_bounds__(256) label_exit_kernel(Imgs I, const int2* __r
     int* out = d ? O.dual : O.primal;
     const int W = I.W[b], Nx = W + 1;
     const int lidx = e.x - I.idx_base[b];
-    const int y = lidx / Nx, x = lidx - y * Nx;
+    const int y = row_of(I, b, lidx), x = lidx - y * Nx;
     out += (d ? O.dual_off : O.primal_off)[b];
     out[faces ? lidx : y * W + x] = entry_label(e.y, perim, cap, status);
   }
