@@ -61,20 +61,6 @@ struct SurvHead {
   int img, cell, sad, pad;
 };
 
-// The survivors in list order with their sort keys ((image, s_val) order:
-// the image id above the orderable value, so one sort orders every image;
-// a 32-bit key of the value alone for one image).
-template <class K>
-__global__ void survivor_gather_kernel(int nsad, const uint8_t* __restrict__ flag, const int* __restrict__ pos,
-                                       const float* __restrict__ sval, const int* __restrict__ sad_img,
-                                       K* __restrict__ key_out, int* __restrict__ idx_out) {
-  int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= nsad || !flag[s]) return;
-  const uint32_t o = orderable_key(sval[s]);
-  key_out[pos[s]] = sizeof(K) > 4 ? (K)(((unsigned long long)sad_img[s] << 32) | o) : (K)o;
-  idx_out[pos[s]] = s;
-}
-
 // Two 32-bit counts in one word: side 0 in the low half, side 1 in the high
 // half (a total of 2^31 or more fails the call).
 __device__ __forceinline__ unsigned long long pack2(unsigned f, unsigned v) { return f | (unsigned long long)v << 32; }

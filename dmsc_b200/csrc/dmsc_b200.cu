@@ -43,7 +43,7 @@ enum Slot {
   S_CSAD, S_IMIN, S_ISAD, S_IMAX, S_MINBITS, S_MAXBITS, S_KMIN, S_KMAX, S_SVAL, S_SKEY2, S_IOTA,
   S_ASC, S_ARC, S_ALIVE, S_RANK, S_FLAG, S_FPOS, S_NCANC, S_ROUTE,
   S_BKEY, S_BIDX, S_BKEY2, S_BIDX2, S_PERF, S_PERV, S_EXF, S_EXV, S_SKEY32B, S_SKEYS,
-  S_SHEAD, S_LENS, S_ROWS, S_PP,
+  S_SREC, S_SHEAD, S_LENS, S_ROWS, S_PP,
   S_SIDE0,  // per-side slots start here, kSideSlots each
 };
 enum SideSlot {
@@ -624,7 +624,8 @@ ReplayArgs replay_prepare(dmsc_b200_context* ctx, int si, Side& S, cudaStream_t 
 // The survivors in output order with their final arcs (after the replay and
 // the sort, `sorted`), and the scans of their geometry cells and e rows; the
 // exact geometry totals stay on the device (read back with the sizes).
-void replay_final(dmsc_b200_context* ctx, const int* sorted, unsigned long long* total, cudaStream_t st) {
+void replay_final(dmsc_b200_context* ctx, const int* sorted, const SurvRec* rec, unsigned long long* total,
+                  cudaStream_t st) {
   const int nsurv = ctx->nsurv;
   ctx->head = get<SurvHead>(ctx, S_SHEAD, nsurv);
   ctx->lens = get<unsigned long long>(ctx, S_LENS, (size_t)nsurv + 1);
@@ -636,9 +637,6 @@ void replay_final(dmsc_b200_context* ctx, const int* sorted, unsigned long long*
     S.s_arc = S.arcs ? sget<int4>(ctx, si, X_SARC, nsurv) : nullptr;
     S.s_fin = S.arcs ? sget<int4>(ctx, si, X_SFIN, nsurv) : nullptr;
     FinalSide& P = A[si];
-    P.arc = ctx->side[0].arc;
-    P.pp = ctx->side[0].pp;
-    P.rout = S.rout;
     P.s_arc = S.s_arc;
     P.s_out = S.s_out;
     P.s_fin = S.s_fin;
@@ -648,8 +646,8 @@ void replay_final(dmsc_b200_context* ctx, const int* sorted, unsigned long long*
     P.dual = S.arcs_dual;
   }
   LK(survivor_final_kernel<<<grid_for(2 * (nsurv + 1LL), TB), TB, 0, st>>>(
-      nsurv, sorted, ctx->B, ctx->sad_img, ctx->crit_sad, ctx->I.dual, ctx->bases.surv, A[0], A[1], ctx->nsad + 1,
-      ctx->head, ctx->lens, ctx->rows, total, ctx->status));
+      nsurv, sorted, rec, ctx->side[0].arc, ctx->I, ctx->bases.surv, A[0], A[1], ctx->nsad + 1, ctx->head, ctx->lens,
+      ctx->rows, total, ctx->status));
   scan<4>(ctx, PackedScan{{ctx->lens, ctx->rows}}, nsurv + 1LL, st);
   LAUNCH_CHECK("final arcs");
 }
@@ -1075,19 +1073,22 @@ int extract_batch_impl(dmsc_b200_context* ctx, int B, const float* img, const in
   // so the device starts the replay while the host sets up the sort
   CK(cudaStreamWaitEvent(ss, ctx->fork_ev, 0));
   int* sorted = get<int>(ctx, S_ASC, nsurv);
+  SurvRec* rec = get<SurvRec>(ctx, S_SREC, nsurv);
   if (nsurv > 0) {
+    const SurvSource SRC{arc, (const int4*)F.pp, {F.rout, V.rout}, {F.alive, V.alive}};
     // the survivors (list order) sorted by (image, s_val) with the list index
     // as the stable tie-break, then each image's range in its vertex-side
     // sweep direction (reversed for a dual image)
     int* sidx = get<int>(ctx, S_IOTA, nsurv);
     if (B > 1) {
       unsigned long long* k = get<unsigned long long>(ctx, S_SKEY2, nsurv);
-      LK(survivor_gather_kernel<unsigned long long><<<grid_for(nsad, TB), TB, 0, ss>>>(nsad, flag, fpos, sval, isad, k,
-                                                                                       sidx));
+      LK(survivor_gather_kernel<unsigned long long><<<grid_for(nsad, TB), TB, 0, ss>>>(nsad, flag, fpos, sval, isad,
+                                                                                       csad, SRC, k, sidx, rec));
       sort_pairs(ctx, k, get<unsigned long long>(ctx, S_SKEYS, nsurv), sidx, sorted, nsurv, ss, 32 + bits_for(B));
     } else {
       uint32_t* k = get<uint32_t>(ctx, S_SKEY32B, nsurv);
-      LK(survivor_gather_kernel<uint32_t><<<grid_for(nsad, TB), TB, 0, ss>>>(nsad, flag, fpos, sval, isad, k, sidx));
+      LK(survivor_gather_kernel<uint32_t><<<grid_for(nsad, TB), TB, 0, ss>>>(nsad, flag, fpos, sval, isad, csad, SRC,
+                                                                             k, sidx, rec));
       sort_pairs(ctx, k, get<uint32_t>(ctx, S_SKEYS, nsurv), sidx, sorted, nsurv, ss, 32);
     }
     LAUNCH_CHECK("survivor order");
@@ -1156,7 +1157,7 @@ int extract_batch_impl(dmsc_b200_context* ctx, int B, const float* img, const in
     ctx->side[si].total = 0;
   }
   unsigned long long* total = ctx->zero->geom;
-  replay_final(ctx, sorted, total, st);
+  replay_final(ctx, sorted, rec, total, st);
   mark(ctx, 9, st);
 
   // ---- per-image sizes: one read of the bases ----

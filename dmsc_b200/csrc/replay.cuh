@@ -141,27 +141,82 @@ __device__ __forceinline__ bool walk_root(const ReplayState& S, const uint8_t* _
   return true;
 }
 
+// A survivor's record, one 64-byte line (32 bytes a side): its arc ends, the
+// ranks of the thresholded roots of its ends and of its pair (-1 for the
+// void), the persistence bits and the raw-arc lengths (15 bits each, with a
+// bit for an end that a cancellation kills; kLongArc: look the lengths up).
+struct alignas(64) SurvRec {
+  struct Side {
+    int t0, t1, r0, r1;
+    int rp, p;
+    unsigned lens;
+    int id;  // faces: the saddle's cell, vertices: its list index
+  } side[2];
+};
+constexpr unsigned kLongArc = 0x7FFFu;
+
+struct SurvSource {
+  const int4* arc;       // [2 nsad] both sides' records, interleaved
+  const int4* pp;        // [nsad] paired extremum and persistence bits of both sides
+  const int* rout[2];    // [M] rank of each extremum's root
+  const uint8_t* alive[2];
+};
+
+// The survivors in list order: their sort keys ((image, s_val) order: the
+// image id above the orderable value, so one sort orders every image; a
+// 32-bit key of the value alone for one image) and their records. Everything
+// is read in list order here, or near it, so that the sort's random
+// permutation later costs a survivor one line; gathering the same from the
+// saddles' arrays in output order cost it eleven sectors, most of them in DRAM
+// for large calls. With 24 M survivors (8192^2 noise, threshold 0) the labels,
+// which this pass and the sort run beside, and the final arcs took 5.3 ms
+// before and take 3.9 ms.
+template <class K>
+__global__ void __launch_bounds__(256) survivor_gather_kernel(int nsad, const uint8_t* __restrict__ flag,
+                                                              const int* __restrict__ pos,
+                                                              const float* __restrict__ sval,
+                                                              const int* __restrict__ sad_img,
+                                                              const int* __restrict__ crit_sad, SurvSource A,
+                                                              K* __restrict__ key_out, int* __restrict__ idx_out,
+                                                              SurvRec* __restrict__ rec) {
+  const int s = blockIdx.x * blockDim.x + threadIdx.x;
+  if (s >= nsad || !flag[s]) return;
+  const int q = pos[s];
+  const uint32_t o = orderable_key(sval[s]);
+  key_out[q] = sizeof(K) > 4 ? (K)(((unsigned long long)sad_img[s] << 32) | o) : (K)o;
+  idx_out[q] = q;
+  const int4 pr = A.pp[s];
+  SurvRec r;
+#pragma unroll
+  for (int sd = 0; sd < 2; ++sd) {
+    const int4 a = A.arc[2 * (long long)s + sd];
+    const int e = sd ? pr.z : pr.x;
+    const bool long_arc = a.z >= (int)kLongArc || a.w >= (int)kLongArc;
+    const unsigned l0 = long_arc ? kLongArc : (unsigned)a.z, l1 = long_arc ? kLongArc : (unsigned)a.w;
+    const bool d0 = a.x >= 0 && !A.alive[sd][a.x], d1 = a.y >= 0 && !A.alive[sd][a.y];
+    SurvRec::Side& v = r.side[sd];
+    v.t0 = a.x;
+    v.t1 = a.y;
+    v.r0 = a.x >= 0 ? A.rout[sd][a.x] : -1;
+    v.r1 = a.y >= 0 ? A.rout[sd][a.y] : -1;
+    v.rp = e >= 0 ? A.rout[sd][e] : -1;
+    v.p = sd ? pr.w : pr.y;
+    v.lens = l0 | (d0 ? 0x8000u : 0u) | l1 << 16 | (d1 ? 0x80000000u : 0u);
+    v.id = sd ? s : crit_sad[s];
+  }
+  rec[q] = r;
+}
+
 // The survivors in output order and their final arcs, two threads (sides) a
-// survivor. `sorted` lists them by ascending (image, s_val, cell id), the
-// vertex side's sweep order (arcs_topology.hxx:99-102); an image whose vertex
-// side sweeps descending (dual) takes its range reversed. A side's thread
-// gathers its arc ends and raw-arc lengths, its persistence and the ranks of
-// the thresholded roots of its ends and pair (-1 for the void), walks its
-// ends' chains to their final roots, and writes all of it in output order, so
-// that the later per-survivor kernels read in order; the survivor's geometry
-// cells and e rows go to the scans (entry nsurv is zero: the totals). Images
-// whose output does not take a side's arcs (`primal` / `dual` by orientation)
-// get empty arcs there.
-//
-// Bound by L2 sectors (180 G/s): the sort's random permutation makes every
-// read its own sector, so both sides' records of a saddle are interleaved.
-// Measured at 4096^2 noise, threshold 0 (5.9 M survivors), gathers, final
-// arcs, row counts, scans and positions: 0.76 ms in eleven passes, 0.58 ms in
-// this one and two scans.
+// survivor. `sorted` lists their records by ascending (image, s_val, cell id),
+// the vertex side's sweep order (arcs_topology.hxx:99-102); an image whose
+// vertex side sweeps descending (dual) takes its range reversed. A side's
+// thread reads its half of the record, walks its ends' chains to their final
+// roots, and writes everything in output order, so that the later per-survivor
+// kernels read in order; the survivor's geometry cells and e rows go to the
+// scans (entry nsurv is zero: the totals). Images whose output does not take a
+// side's arcs (`primal` / `dual` by orientation) get empty arcs there.
 struct FinalSide {
-  const int4* arc;        // [2 nsad] both sides' records, interleaved
-  const int2* pp;         // [2 nsad] paired extremum and persistence bits, interleaved
-  const int* rout;        // [M] rank of each extremum's root
   int4* s_arc;            // [nsurv] arc ends, raw-arc lengths
   int4* s_out;            // [nsurv] ranks of the ends' roots, persistence bits, rank of the pair's root
   int4* s_fin;            // [nsurv] chain lengths and roots; nullptr: no image takes the arcs
@@ -171,10 +226,10 @@ struct FinalSide {
 };
 
 __global__ void __launch_bounds__(256) survivor_final_kernel(
-    int nsurv, const int* __restrict__ sorted, int B, const int* __restrict__ sad_img,
-    const int* __restrict__ crit_sad, const uint8_t* __restrict__ dual, const int* __restrict__ surv_base, FinalSide F,
-    FinalSide V, int max_steps, SurvHead* __restrict__ head, unsigned long long* __restrict__ lens,
-    unsigned long long* __restrict__ rows, unsigned long long* __restrict__ total, unsigned* status) {
+    int nsurv, const int* __restrict__ sorted, const SurvRec* __restrict__ rec, const int4* __restrict__ arc, Imgs I,
+    const int* __restrict__ surv_base, FinalSide F, FinalSide V, int max_steps, SurvHead* __restrict__ head,
+    unsigned long long* __restrict__ lens, unsigned long long* __restrict__ rows,
+    unsigned long long* __restrict__ total, unsigned* status) {
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int p = (int)(t >> 1), sd = (int)(t & 1);
   __shared__ unsigned long long sum[2];
@@ -183,43 +238,50 @@ __global__ void __launch_bounds__(256) survivor_final_kernel(
   int q = p;
   unsigned n_rows = 0;
   unsigned long long len = 0;
+  int4 v0 = make_int4(0, 0, 0, 0), v1 = v0;  // this side's half of the record
   if (p < nsurv) {
-    const int s = sorted[p], b = B > 1 ? sad_img[s] : 0;
-    const bool d = dual[b];
+    const int4* half = reinterpret_cast<const int4*>(rec + sorted[p]) + 2 * sd;
+    v0 = half[0];
+    v1 = half[1];
+  }
+  const int other = __shfl_xor_sync(0xffffffffu, v1.w, 1);
+  const int cell = sd ? other : v1.w, s = sd ? v1.w : other;
+  if (p < nsurv) {
+    const int b = I.B > 1 ? find_image(I.idx_base, I.B, cell >> 2) : 0;
+    const bool d = I.dual[b];
     if (d) {
       const int base = surv_base[b], cnt = surv_base[b + 1] - base;
       q = base + cnt - 1 - (p - base);
     }
     const FinalSide& A = sd ? V : F;
-    const int4 a = A.arc[2 * (long long)s + sd];
-    const int2 pr = A.pp[2 * (long long)s + sd];
-    const int4 o = make_int4(a.x >= 0 ? A.rout[a.x] : -1, a.y >= 0 ? A.rout[a.y] : -1, pr.y,
-                             pr.x >= 0 ? A.rout[pr.x] : -1);
-    A.s_out[q] = o;
+    A.s_out[q] = make_int4(v0.z, v0.w, v1.y, v1.x);
     int x, y;
-    n_rows = erow_ends(o.x, o.y, &x, &y);
+    n_rows = erow_ends(v0.z, v0.w, &x, &y);
     if (A.s_fin) {
+      const unsigned l = (unsigned)v1.z;
+      int l0 = (int)(l & 0x7FFFu), l1 = (int)(l >> 16 & 0x7FFFu);
+      if (l0 == (int)kLongArc) {
+        const int4 a = arc[2 * (long long)s + sd];
+        l0 = a.z;
+        l1 = a.w;
+      }
       int4 fin = make_int4(0, 0, -1, -1);
       if (d ? A.dual : A.primal) {
         long long c[2] = {0, 0};
-        int root[2];
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          const int T = j ? a.y : a.x;
-          root[j] = T;
-          // an extremum that no cancellation kills (alive) is its own final
-          // root; only the others walk their parent chains
-          if (T >= 0 && !A.alive[T]) walk_root(A.S, A.alive, T, kNever, &root[j], &c[j], max_steps, status);
-        }
+        int root[2] = {v0.x, v0.y};
+        // an extremum that no cancellation kills is its own final root; only
+        // the others walk their parent chains
+        if (l & 0x8000u) walk_root(A.S, A.alive, v0.x, kNever, &root[0], &c[0], max_steps, status);
+        if (l >> 31) walk_root(A.S, A.alive, v0.y, kNever, &root[1], &c[1], max_steps, status);
         // a chain beyond 32 bits makes the side's geometry overflow (the
         // exact total says so): its stored length is not used then
         fin = make_int4((int)c[0], (int)c[1], root[0], root[1]);
-        len = (unsigned long long)((long long)a.z + a.w + c[0] + c[1]);
+        len = (unsigned long long)((long long)l0 + l1 + c[0] + c[1]);
       }
-      A.s_arc[q] = a;
+      A.s_arc[q] = make_int4(v0.x, v0.y, l0, l1);
       A.s_fin[q] = fin;
     }
-    if (sd == 0) *reinterpret_cast<int4*>(head + q) = make_int4(b, crit_sad[s], s, 0);
+    if (sd == 0) *reinterpret_cast<int4*>(head + q) = make_int4(b, cell, s, 0);
   }
   const unsigned other_rows = __shfl_xor_sync(0xffffffffu, n_rows, 1);
   const unsigned other_len = __shfl_xor_sync(0xffffffffu, (unsigned)len, 1);
