@@ -216,6 +216,33 @@ __device__ __forceinline__ void block_reserve2(int* c0, int n0, int* c1, int n1,
   __syncthreads();
 }
 
+// The same for one counter.
+__device__ __forceinline__ int block_reserve(int* c0, int n0) {
+  __shared__ int wsum1[32], bbase1;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  int x0 = n0;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y0 = __shfl_up_sync(0xffffffffu, x0, o);
+    if (lane >= o) x0 += y0;
+  }
+  if (lane == 31) wsum1[warp] = x0;
+  __syncthreads();
+  if (warp == 0) {
+    const int s0 = lane < nw ? wsum1[lane] : 0;
+    int i0 = s0;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y0 = __shfl_up_sync(0xffffffffu, i0, o);
+      if (lane >= o) i0 += y0;
+    }
+    if (lane < nw) wsum1[lane] = i0 - s0;
+    if (lane == 31) bbase1 = i0 ? atomicAdd(c0, i0) : 0;
+  }
+  __syncthreads();
+  return bbase1 + wsum1[warp] + x0 - n0;
+}
+
 // Block-aggregated append: one global atomic per block. Every thread of the
 // block must call it (with blockDim.x a multiple of 32, at most 1024).
 // Returns the slot of this thread's item, or -1 when `take` is false.

@@ -188,7 +188,6 @@ struct dmsc_b200_context {
   int replay_shape = 0;  // replay items per thread batch: 0 -> 1, 1 -> 2
   int emit_shape = 0;    // expansion chain tasks per thread batch: 0 -> 1, 1 -> 2
   int seg_cursors = 1;  // raw-arc cursors per lane of the segment writer
-  bool label_smem_set = false;  // dynamic shared memory limit raised for the label kernels
   bool pair_smem_set = false;   // and for the pairing's tile kernel
   int cap_pair_rounds = 0, cap_replay_rounds = 0, cap_emit_levels = 0;
 };
@@ -911,7 +910,7 @@ int extract_batch_impl(dmsc_b200_context* ctx, int B, const float* img, const in
   // the 16 B/index gradient is written only when returned; every later stage
   // works from the flow codes, which also carry the criticality bits
   int* grad = ret_grad ? grad_out : nullptr;
-  uint8_t* flow = get<uint8_t>(ctx, S_FLOW, nidx);
+  uint8_t* flow = get<uint8_t>(ctx, S_FLOW, nidx + 8);  // the label tiles read whole words
   ctx->flow = flow;
   ctx->img = img;
   int* seg[3] = {get<int>(ctx, S_SEG0, nseg), get<int>(ctx, S_SEG1, nseg), get<int>(ctx, S_SEG2, nseg)};
@@ -1096,12 +1095,12 @@ int extract_batch_impl(dmsc_b200_context* ctx, int B, const float* img, const in
   CK(cudaEventRecord(ctx->join_ev, ss));
 
   // ---- labels (region id = rank among the image's alive extrema) ----
-  LabelOut OF{}, OV{};
   LabelSide LF{}, LV{};
   for (int si = 0; si < 2; ++si) {
     Side& S = ctx->side[si];
     if (!S.groups) continue;
-    LabelOut& O = S.faces ? OF : OV;
+    LabelSide& L = S.faces ? LF : LV;
+    LabelOut& O = L.out;
     if (S.faces) {
       O.primal = f_peaks ? peaks_out : nullptr;
       O.dual = f_basins ? basins_out : nullptr;
@@ -1113,36 +1112,30 @@ int extract_batch_impl(dmsc_b200_context* ctx, int B, const float* img, const in
       O.primal_off = d_basins_off;
       O.dual_off = d_peaks_off;
     }
-    LabelSide& L = S.faces ? LF : LV;
     L.off = S.faces ? off[2] : off[0];
+    L.bits = S.faces ? bmax : bmin;
     L.rout = S.rout;
     L.abase = BS.alive[si];
     L.perim = get<int>(ctx, S.faces ? S_PERF : S_PERV, (size_t)nltile * kPerim);
+    L.exits = get<int2>(ctx, S.faces ? S_EXF : S_EXV, nidx);
+    L.n_exits = ctx->zero->n_exits + (S.faces ? 0 : 1);
   }
-  int* nex = ctx->zero->n_exits;
   mark(ctx, 16, st);  // the labels stage times the label kernels alone
   if (F.groups || V.groups) {
-    int2* exf = F.groups ? get<int2>(ctx, S_EXF, nidx) : nullptr;
-    int2* exv = V.groups ? get<int2>(ctx, S_EXV, nidx) : nullptr;
-    constexpr int kLSm = (int)sizeof(LabelSmem);
-    if (!ctx->label_smem_set) {  // more than the 48 KB of static shared memory
-      CK(cudaFuncSetAttribute(label_tile_kernel<kLabelNT[0]>, cudaFuncAttributeMaxDynamicSharedMemorySize, kLSm));
-      CK(cudaFuncSetAttribute(label_tile_kernel<kLabelNT[1]>, cudaFuncAttributeMaxDynamicSharedMemorySize, kLSm));
-      ctx->label_smem_set = true;
-    }
+    const int first = F.groups ? 0 : 1;
+    const unsigned sides = F.groups && V.groups ? 2 : 1;
+    const dim3 grid((unsigned)nltile, sides);
     if (ctx->label_shape == 1)
-      LK((label_tile_kernel<kLabelNT[1]><<<(unsigned)nltile, kLabelNT[1], kLSm, st>>>(I, flow, LF, LV, OF, OV, exf,
-                                                                                    exv, nex, ctx->status)));
+      LK((label_tile_kernel<kLabelNT[1]><<<grid, kLabelNT[1], 0, st>>>(I, flow, LF, LV, first, ctx->status)));
     else
-      LK((label_tile_kernel<kLabelNT[0]><<<(unsigned)nltile, kLabelNT[0], kLSm, st>>>(I, flow, LF, LV, OF, OV, exf,
-                                                                                    exv, nex, ctx->status)));
+      LK((label_tile_kernel<kLabelNT[0]><<<grid, kLabelNT[0], 0, st>>>(I, flow, LF, LV, first, ctx->status)));
     LAUNCH_CHECK("label_tile_kernel");
     int per = 0;
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, label_exit_kernel, 256, 0));
     // a path enters a tile through each of its border cells at most once
     const int hops = (int)std::min<long long>(nltile * kPerim + 2, 2147483647LL);
     const unsigned eg = (unsigned)std::min<long long>((long long)std::max(1, per) * ctx->num_sms, 4 * nltile);
-    LK(label_exit_kernel<<<dim3(eg, 2), 256, 0, st>>>(I, exf, exv, nex, LF.perim, LV.perim, OF, OV, hops, ctx->status));
+    LK(label_exit_kernel<<<dim3(eg, sides), 256, 0, st>>>(I, LF, LV, first, hops, ctx->status));
     LAUNCH_CHECK("label_exit_kernel");
   }
   mark(ctx, 10, st);

@@ -104,84 +104,46 @@ __device__ __forceinline__ LabelTile label_tile_of(const Imgs& I, int t) {
   return g;
 }
 
-// Flow bytes of the tile; cells beyond the image read as critical (never reached).
-__device__ __forceinline__ void load_flow_tile(const uint8_t* __restrict__ flow, const LabelTile& g,
-                                               uint8_t (*fl)[kLT], int tid, int nthreads) {
-  for (int i = tid; i < kLTN; i += nthreads) {
-    const int r = i / kLT, c = i % kLT;
-    const bool in = g.y0 + r <= g.H && g.x0 + c <= g.W;
-    fl[r][c] = in ? __ldg(flow + g.base + (long long)r * g.Nx + c) : (uint8_t)0;
-  }
-}
-
 __device__ __forceinline__ int perim_slot(int r, int c) {
   return r == 0 ? c : r == kLT - 1 ? kLT + c : c == 0 ? 2 * kLT + r : 3 * kLT + r;
 }
 
-// In-tile resolution. Every (side, cell) of the tile has a 16-bit successor
-// and a 32-bit state. A terminal cell (critical, or whose successor lies
-// outside the tile) has successor kTerm | itself and a final state from the
-// start: the entry (label << 1) | 1 of its extremum (label -1 encodes as all
-// ones), or (border-map index of the cell its path enters next, in the
-// neighbouring tile) << 1. Every other cell walks its successors for up to
-// kWalk steps (paths are short: means of 3.2 steps for faces and 1.5 for
-// vertices on the bench field) and takes the state of the terminal cell it
-// reaches; a cell still walking after kWalk steps becomes pending (kPend | the
-// cell reached), and pending cells then jump their pointers,
-// state = state of the pointed-to cell, without block barriers: any state
-// read belongs to a cell further along the same path (written by any thread,
-// at any time), so a pointer only moves toward the path's end and gets there
-// in at most the path's length of jumps. Border-map indices and labels stay
-// below 2^30, so the top two bits tell a pending state apart.
-constexpr uint32_t kPend = 0x40000000u, kCellMask = 0x0FFFu;
-constexpr unsigned kTerm = 0x8000u;
-constexpr int kWalk = 8;
-__device__ __forceinline__ bool st_pending(uint32_t v) { return (v >> 30) == 1u; }
+// In-tile resolution, one side per block. The tile lies in shared memory as
+// one signed byte per cell, the distance in the array to the cell its path
+// visits next (0: the path ends here), inside a ring of one cell of the
+// neighbouring tiles, whose distance is 0: a step of a walk is one byte read
+// and one addition, with no test of the code, of the tile's edge or of the
+// end. Every cell takes kLabelSteps of them, the thread's cells together, and
+// one that has not ended then jumps through the cells that the others reached.
+// The state of a final cell is (label << 1) | 1 of its extremum (label -1
+// encodes as all ones), or, on the ring, (border-map index of that cell in
+// its own tile) << 1.
+//
+// What bounds it is the instructions: with 16-bit successors and 32-bit states
+// for every cell of both sides and a tested loop for each walk it issued 465
+// warp instructions for 32 cells of both sides, now 274. Labels at 4096^2
+// (smooth, threshold 0.05) 302 -> 205 us, at 8192^2 noise 1461 -> 1107 us, at
+// 256^2 29 -> 17 us; the issue slots and the shared-memory pipe are both at
+// four fifths. 4 to 12 steps before the jumps are within 3 %, 1536 threads
+// per SM instead of 2048 are 9 % slower.
+constexpr int kLabelPitch = 72;  // 64 columns from 4 on (words of steps are aligned), the ring in columns 3 and 68
+constexpr int kLabelCells = (kLT + 2) * kLabelPitch;
+constexpr int kLabelSteps = 8;
+__device__ __forceinline__ int label_pos(int r, int c) { return (r + 1) * kLabelPitch + 4 + c; }
 
 // Threads per label tile (the tuner picks one): each thread owns column
 // tid % 64 of rows tid / 64 + (NT / 64) k, k < 4096 / NT.
 constexpr int kLabelShapes = 2;
 constexpr int kLabelNT[kLabelShapes] = {1024, 512};
 
-// Successor set-up of one (row, 32-cell segment) item of a tile for both
-// sides, one lane per cell: a critical cell (terminal) takes the state
-// (label << 1) | 1 of its extremum, lab[rank], where rank is the segment's
-// first rank in the batch-wide critical list (the compaction's exclusive
-// scan) plus the critical cells before it in the segment (a ballot); a cell
-// whose successor lies in another tile (terminal) takes the border-map entry
-// of that cell; any other cell gets its successor's tile-local id. Cells
-// outside the image are terminal and never reached. `labf` / `labv`: the
-// labels loaded for this lane's critical cells (issued for a group of a
-// warp's items before any is used).
-__device__ __forceinline__ void tile_cell_setup(const uint8_t (*fl)[kLT], const LabelTile& g, int tile, int ntx,
-                                                int r, int c, bool do_f, bool do_v, bool critf, bool critv,
-                                                int labf, int labv, uint16_t (*succ)[kLTN], uint32_t (*st)[kLTN]) {
-  const int i = r * kLT + c;
-  const unsigned code = fl[r][c];
-  const int y = g.y0 + r, x = g.x0 + c;
-#pragma unroll
-  for (int sd = 0; sd < 2; ++sd) {
-    const bool in = sd == 0 ? (do_f && y <= g.H && x <= g.W) : (do_v && y < g.H && x < g.W);
-    const unsigned k = sd == 0 ? (code >> 4) & 7u : code & 7u;
-    uint16_t sc = (uint16_t)(kTerm | i);
-    uint32_t state = 1u;
-    if (in) {
-      if (sd == 0 ? critf : critv) {
-        state = ((uint32_t)(sd == 0 ? labf : labv) << 1) | 1u;
-      } else {
-        const int dc = (k == kFlowRight) - (k == kFlowLeft), dr = (k == kFlowDown) - (k == kFlowUp);
-        const int nr = r + dr, nc = c + dc;
-        if ((unsigned)nr < (unsigned)kLT && (unsigned)nc < (unsigned)kLT) {
-          sc = (uint16_t)(nr * kLT + nc);
-        } else {  // enters the neighbouring tile at its border cell (nr, nc) mod 64
-          const int nt = tile + dc + dr * ntx;
-          state = (uint32_t)(((long long)nt * kPerim + perim_slot(nr & (kLT - 1), nc & (kLT - 1))) << 1);
-        }
-      }
-    }
-    succ[sd][i] = sc;
-    if (sc & kTerm) st[sd][i] = state;
-  }
+// Steps of four cells from their four flow codes (one per byte, 0 .. 4): the
+// codes, packed to nibbles, select the bytes of a table.
+__device__ __forceinline__ unsigned label_steps(unsigned codes) {
+  unsigned s = codes & 0x07070707u;
+  s = (s | s >> 4) & 0x00FF00FFu;
+  s |= s >> 8;
+  constexpr unsigned lo = (0xFFu << 8) | (1u << 16) | ((unsigned)(256 - kLabelPitch) << 24);  // none, left, right, up
+  return __byte_perm(lo, (unsigned)kLabelPitch, s);                                           // down
 }
 
 // Follows border-map entries to a label.
@@ -196,9 +158,13 @@ __device__ __forceinline__ int entry_label(int e, const int* __restrict__ perim,
 
 struct LabelSide {
   const int* off;    // segment offsets of this side's critical list (exclusive scan)
+  const uint32_t* bits;  // critical cells of each segment
   const int* rout;   // per critical extremum (batch-wide rank): out rank of its thresholded root, -1 for the void
   const int* abase;  // [B + 1] first out rank of each image's alive extrema
-  int* perim;        // border map (nullptr: side not labelled)
+  int* perim;        // border map
+  int2* exits;       // cells whose paths leave their tile: (global index, entry)
+  int* n_exits;
+  LabelOut out;
 };
 
 // Label of an extremum from its root's batch-wide out rank: the root's rank
@@ -208,194 +174,173 @@ __device__ __forceinline__ int region_label(int rout, int abase) { return rout <
 
 __device__ __forceinline__ int label_ntx(const LabelTile& g) { return (g.W + kLT) / kLT; }
 
-// Labels of every cell of a tile: face labels over the (H+1) x (W+1) indices,
-// vertex labels over the H x W pixels (cpu/cell_groups.hxx:151-228). A cell
-// whose path ends inside the tile gets its label here; the tile's border
-// cells also get their border-map entries; a cell whose path leaves the tile
-// is appended to its side's exit list (global index, entry) and finished by
-// label_exit_kernel once every tile's border map is written.
-// Shared memory of a label tile (55 KB: dynamic shared memory).
 struct LabelSmem {
-  uint32_t st[2][kLTN];
-  uint16_t succ[2][kLTN];
-  uint8_t fl[kLT][kLT];
+  uint32_t st[kLabelCells];      // states of the final cells
+  uint16_t ptr[kLabelCells];     // cell reached by each cell's walk
+  __align__(4) int8_t step[kLabelCells];
 };
 
-template <int NT>
-__global__ void __launch_bounds__(NT, 2048 / NT) label_tile_kernel(Imgs I, const uint8_t* __restrict__ flow,
-                                                                   LabelSide F, LabelSide V, LabelOut OF, LabelOut OV,
-                                                                   int2* __restrict__ exits_f, int2* __restrict__ exits_v,
-                                                                   int* __restrict__ n_exits, unsigned* status) {
-  extern __shared__ __align__(16) unsigned char label_smem[];
-  LabelSmem& SM = *reinterpret_cast<LabelSmem*>(label_smem);
-  uint8_t (*fl)[kLT] = SM.fl;
-  uint16_t (*succ)[kLTN] = SM.succ;
-  uint32_t (*st)[kLTN] = SM.st;
-  constexpr int kTileCells = kLTN / NT, kStep = NT / kLT;
-  constexpr int NW = NT / 32, kItems = 2 * kLT / NW;  // (row, segment) items per warp
+// Labels of a tile's cells on one side: face labels over the (H+1) x (W+1)
+// indices or vertex labels over the H x W pixels
+// (cpu/cell_groups.hxx:151-228). A cell whose path ends inside the tile gets
+// its label here; the tile's border cells also get their border-map entries; a
+// cell whose path leaves the tile is appended to its side's exit list and
+// finished by label_exit_kernel once every tile's border map is written.
+template <int NT, bool FACES>
+__device__ __forceinline__ void label_tile(LabelSmem& S, const Imgs& I, const uint8_t* __restrict__ flow,
+                                           const LabelSide& L, unsigned* status) {
+  constexpr int kCells = kLTN / NT, kStep = NT / kLT, kItems = 2 * kLT / (NT / 32);
   const LabelTile g = label_tile_of(I, blockIdx.x);
-  const bool d = I.dual[g.b];
-  int* of = d ? OF.dual : OF.primal;
-  int* ov = d ? OV.dual : OV.primal;
-  if (of) of += (d ? OF.dual_off : OF.primal_off)[g.b];
-  if (ov) ov += (d ? OV.dual_off : OV.primal_off)[g.b];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int ntx = label_ntx(g);
-  const bool do_f = F.perim != nullptr, do_v = V.perim != nullptr;
-  // the first ranks of this warp's items: lane k loads item k's (issued
-  // before the flow tile is waited for)
-  int offf = 0, offv = 0;
-  const int abf = do_f ? __ldg(F.abase + g.b) : 0, abv = do_v ? __ldg(V.abase + g.b) : 0;
+  // the (row, 32-cell segment) items of this warp: lane k loads the first rank
+  // and the extrema of item k, used once the steps are on their way
+  int off = 0;
+  unsigned bits = 0;
   if (lane < kItems) {
-    const int rs = warp + NW * lane, r = rs >> 1, sg = rs & 1;
-    const int y = g.y0 + r;
-    if (y <= g.H && g.x0 + sg * 32 <= g.W) {
-      const int nsegx = (g.W + 32) / 32;  // 32-index row segments of the compaction: ceil((W + 1) / 32)
-      const long long sid = (long long)I.seg_base[g.b] + (long long)y * nsegx + (g.x0 >> 5) + sg;
-      if (do_f && F.off) offf = __ldg(F.off + sid);
-      if (do_v && V.off) offv = __ldg(V.off + sid);
+    const int rs = warp * kItems + lane, y = g.y0 + (rs >> 1), sx = (g.x0 >> 5) + (rs & 1);
+    const int nsegx = (g.W + 32) / 32;  // 32-index row segments of the compaction: ceil((W + 1) / 32)
+    if (y <= g.H && sx < nsegx) {
+      const long long q = (long long)I.seg_base[g.b] + (long long)y * nsegx + sx;
+      off = __ldg(L.off + q);
+      bits = __ldg(L.bits + q);
     }
   }
-  load_flow_tile(flow, g, fl, threadIdx.x, blockDim.x);
-  __syncthreads();
-  {  // successors and terminal states, one warp per (row, segment) item, in
-     // groups of 4 items whose label loads are issued together
-    const unsigned lt = (1u << lane) - 1u;
-    constexpr int kGroup = kItems < 4 ? kItems : 4;
+  const int abase = __ldg(L.abase + g.b);
+  // steps, a word of four cells at a time (rows start at any byte: two aligned
+  // words and a shift). A word is read when its first cell lies in the image;
+  // what lies beyond is never reached from inside.
 #pragma unroll
-    for (int k0 = 0; k0 < kItems; k0 += kGroup) {
-      int labf[kGroup], labv[kGroup];
-      unsigned cf = 0, cv = 0;  // bit k: this lane's cell of item k0 + k is critical
+  for (int k = 0; k < kLTN / 4 / NT + (kLTN / 4 % NT != 0); ++k) {
+    const int i = tid + k * NT, r = i >> 4, c = (i & 15) * 4;
+    unsigned w = 0;
+    if (g.y0 + r <= g.H && g.x0 + c <= g.W) {
+      const long long o = g.base + (long long)r * g.Nx + c;
+      const unsigned* p = reinterpret_cast<const unsigned*>(flow) + (o >> 2);
+      w = __funnelshift_r(__ldg(p), __ldg(p + 1), 8 * (unsigned)(o & 3));
+    }
+    *reinterpret_cast<unsigned*>(S.step + label_pos(r, c)) = label_steps(FACES ? w >> 4 : w);
+  }
+  for (int i = tid; i < 4 * kLT; i += NT) {  // the ring
+    const int k = i & (kLT - 1), e = i / kLT;
+    const int r = e == 0 ? -1 : e == 1 ? kLT : k, c = e == 2 ? -1 : e == 3 ? kLT : k;
+    const int nt = blockIdx.x + (e == 0 ? -ntx : e == 1 ? ntx : e == 2 ? -1 : 1);
+    S.step[label_pos(r, c)] = 0;
+    S.st[label_pos(r, c)] = (unsigned)(nt * kPerim + perim_slot(r & (kLT - 1), c & (kLT - 1))) << 1;
+  }
+  {  // labels of the extrema
+    int lab[kItems];
 #pragma unroll
-      for (int k = 0; k < kGroup; ++k) {  // ranks and label loads of the critical cells
-        const int rs = warp + NW * (k0 + k), r = rs >> 1, c = (rs & 1) * 32 + lane;
-        const int y = g.y0 + r, x = g.x0 + c;
-        const unsigned code = fl[r][c];
-        const bool fcrit = do_f && y <= g.H && x <= g.W && ((code >> 4) & 7u) == kFlowNone;
-        const bool vcrit = do_v && y < g.H && x < g.W && (code & 7u) == kFlowNone;
-        const unsigned fb = __ballot_sync(0xffffffffu, fcrit), vb = __ballot_sync(0xffffffffu, vcrit);
-        const int of0 = __shfl_sync(0xffffffffu, offf, k0 + k), ov0 = __shfl_sync(0xffffffffu, offv, k0 + k);
-        labf[k] = fcrit ? region_label(__ldg(F.rout + of0 + __popc(fb & lt)), abf) : 0;
-        labv[k] = vcrit ? region_label(__ldg(V.rout + ov0 + __popc(vb & lt)), abv) : 0;
-        cf |= (unsigned)fcrit << k;
-        cv |= (unsigned)vcrit << k;
-      }
+    for (int k = 0; k < kItems; ++k) {
+      const unsigned m = __shfl_sync(0xffffffffu, bits, k);
+      const int o = __shfl_sync(0xffffffffu, off, k);
+      lab[k] = (m >> lane) & 1u ? __ldg(L.rout + o + __popc(m & ((1u << lane) - 1u))) : 0;
+    }
 #pragma unroll
-      for (int k = 0; k < kGroup; ++k) {
-        const int rs = warp + NW * (k0 + k);
-        tile_cell_setup(fl, g, blockIdx.x, ntx, rs >> 1, (rs & 1) * 32 + lane, do_f, do_v, (cf >> k) & 1u,
-                        (cv >> k) & 1u, labf[k], labv[k], succ, st);
-      }
+    for (int k = 0; k < kItems; ++k) {
+      const int rs = warp * kItems + k;
+      if ((__shfl_sync(0xffffffffu, bits, k) >> lane) & 1u)
+        S.st[label_pos(rs >> 1, (rs & 1) * 32 + lane)] = ((unsigned)region_label(lab[k], abase) << 1) | 1u;
     }
   }
   __syncthreads();
-  const int c = threadIdx.x % kLT, rb = threadIdx.x / kLT;
-  // short walks to the terminal cell; bit 2k + side of `pend`: still walking
+  const int c = tid % kLT, rb = tid / kLT, x = g.x0 + c;
+  int pos[kCells];
+#pragma unroll
+  for (int k = 0; k < kCells; ++k) pos[k] = label_pos(rb + kStep * k, c);
   unsigned pend = 0;
+  {
+    int last[kCells];
 #pragma unroll
-  for (int q = 0; q < 2 * kTileCells; ++q) {
-    const int sd = q & 1, i = (rb + kStep * (q >> 1)) * kLT + c;
-    unsigned cur = succ[sd][i];
-    if (cur & kTerm) continue;
-    unsigned nx = succ[sd][cur];
-#pragma unroll 1
-    for (int w = 1; w < kWalk && !(nx & kTerm); ++w) {
-      cur = nx;
-      nx = succ[sd][cur];
-    }
-    if (nx & kTerm) {
-      st[sd][i] = st[sd][cur];  // cur is terminal: its state is final
-    } else {
-      st[sd][i] = kPend | cur;
-      pend |= 1u << q;
+    for (int w = 0; w < kLabelSteps; ++w)
+#pragma unroll
+      for (int k = 0; k < kCells; ++k) {
+        last[k] = S.step[pos[k]];
+        pos[k] += last[k];
+      }
+    const int rows = FACES ? g.H + 1 - g.y0 : g.H - g.y0;
+    const bool in = FACES ? x <= g.W : x < g.W;
+#pragma unroll
+    for (int k = 0; k < kCells; ++k) {
+      S.ptr[label_pos(rb + kStep * k, c)] = (uint16_t)pos[k];
+      if (last[k] != 0 && in && rb + kStep * k < rows) pend |= 1u << k;
     }
   }
   __syncthreads();
-  {  // barrier-free pointer jumping of this thread's pending cells (only this
-     // thread writes its cells' states; other threads read them at any time)
-    volatile uint32_t* vs = &st[0][0];
-    for (int it = 0; pend; ++it) {
-      if (it >= kLTN) {  // a path is at most kLTN cells long inside a tile
-        set_status(status, kStatusWalkCap);
-        break;
-      }
+  // barrier-free pointer jumping of this thread's unfinished cells: a cell's
+  // pointer only moves on along its path, whichever thread reads it, so a
+  // path's end is reached in at most its length of jumps
+  for (int it = 0; pend; ++it) {
+    if (it >= kLTN) {
+      set_status(status, kStatusWalkCap);
+      break;
+    }
 #pragma unroll
-      for (int q = 0; q < 2 * kTileCells; ++q) {
-        if (!((pend >> q) & 1u)) continue;
-        const int side = (q & 1) * kLTN, i = side + (rb + kStep * (q >> 1)) * kLT + c;
-        const uint32_t w = vs[side + (vs[i] & kCellMask)];
-        vs[i] = w;
-        if (!st_pending(w)) pend &= ~(1u << q);
+    for (int k = 0; k < kCells; ++k) {
+      if (!((pend >> k) & 1u)) continue;
+      if (S.step[pos[k]] == 0) {
+        pend &= ~(1u << k);
+      } else {
+        pos[k] = *reinterpret_cast<volatile uint16_t*>(S.ptr + pos[k]);
+        *reinterpret_cast<volatile uint16_t*>(S.ptr + label_pos(rb + kStep * k, c)) = (uint16_t)pos[k];
       }
     }
   }
-  // this thread's own states are final now (read back from shared memory):
-  // labels of paths that end in the tile, border-map entries of the border
-  // cells, and a bit per cell whose path leaves the tile on a side whose
-  // labels this image outputs (bit 2k: faces, 2k + 1: vertices); those are
-  // reserved in the exit lists at once and written afterwards
+  // labels of the paths that end in the tile, entries of the border cells, and
+  // a bit per cell whose path leaves the tile if this image outputs the side's
+  // labels; those are reserved in the exit list at once and written afterwards
+  const bool d = I.dual[g.b];
+  int* out = d ? L.out.dual : L.out.primal;
+  const int pitch = FACES ? g.Nx : g.W;
+  if (out) out += (d ? L.out.dual_off : L.out.primal_off)[g.b] + (g.y0 + rb) * pitch + x;  // image-local: below 2^31
   const bool border_c = c == 0 || c == kLT - 1;
-  const int x = g.x0 + c;
-  const bool fx = do_f && x <= g.W, vx = do_v && x < g.W;
   unsigned xm = 0;
-  {
-    int* ofr = of ? of + (g.y0 + rb) * g.Nx + x : nullptr;  // image-local outputs stay below 2^31
-    int* ovr = ov ? ov + (g.y0 + rb) * g.W + x : nullptr;
+  if (FACES ? x <= g.W : x < g.W) {
 #pragma unroll
-    for (int k = 0; k < kTileCells; ++k) {
-      const int r = rb + kStep * k, y = g.y0 + r, i = r * kLT + c;
-      const bool border = border_c || r == 0 || r == kLT - 1;
-      if (fx && y <= g.H) {
-        // odd: (label << 1) | 1 of a path ending in the tile; even: exit entry
-        const uint32_t ef = st[0][i];
-        if (border) F.perim[blockIdx.x * kPerim + perim_slot(r, c)] = (int)ef;
-        if (ofr) {
-          if (ef & 1u)
-            ofr[k * kStep * g.Nx] = (int)ef >> 1;
-          else
-            xm |= 1u << (2 * k);
-        }
-      }
-      if (vx && y < g.H) {
-        const uint32_t ev = st[1][i];
-        if (border) V.perim[blockIdx.x * kPerim + perim_slot(r, c)] = (int)ev;
-        if (ovr) {
-          if (ev & 1u)
-            ovr[k * kStep * g.W] = (int)ev >> 1;
-          else
-            xm |= 2u << (2 * k);
-        }
+    for (int k = 0; k < kCells; ++k) {
+      const int r = rb + kStep * k, y = g.y0 + r;
+      if (FACES ? y > g.H : y >= g.H) break;
+      const unsigned e = S.st[pos[k]];
+      if (border_c || r == 0 || r == kLT - 1) L.perim[blockIdx.x * kPerim + perim_slot(r, c)] = (int)e;
+      if (out) {
+        if (e & 1u)
+          out[k * kStep * pitch] = (int)e >> 1;
+        else
+          xm |= 1u << k;
       }
     }
   }
-  int pf, pv;
-  block_reserve2(n_exits + 0, __popc(xm & 0x55555555u), n_exits + 1, __popc(xm & 0xAAAAAAAAu), pf, pv);
+  int at = block_reserve(L.n_exits, __popc(xm));
   while (xm) {  // the few cells whose paths leave the tile
-    const int q = __ffs(xm) - 1, k = q >> 1, sd = q & 1;
+    const int k = __ffs(xm) - 1;
     xm &= xm - 1u;
     const int r = rb + kStep * k;
-    const int gidx = (int)(g.base + (long long)r * g.Nx + c);  // global indices stay below 2^29
-    const int e = (int)st[sd][r * kLT + c];
-    if (sd == 0)
-      exits_f[pf++] = make_int2(gidx, e);
-    else
-      exits_v[pv++] = make_int2(gidx, e);
+    // global indices stay below 2^29
+    L.exits[at++] = make_int2((int)(g.base + (long long)r * g.Nx + c), (int)S.st[S.ptr[label_pos(r, c)]]);
   }
+}
+
+// Side `first` (0 faces, 1 vertices), or both (grid y = 2, first = 0).
+template <int NT>
+__global__ void __launch_bounds__(NT, 2048 / NT) label_tile_kernel(Imgs I, const uint8_t* __restrict__ flow,
+                                                                   LabelSide F, LabelSide V, int first,
+                                                                   unsigned* status) {
+  __shared__ LabelSmem S;
+  if (blockIdx.y + first == 0)
+    label_tile<NT, true>(S, I, flow, F, status);
+  else
+    label_tile<NT, false>(S, I, flow, V, status);
 }
 
 // Cells whose paths leave their tile: follow the border map to the label
 // (both sides in one launch, blockIdx.y).
-__global__ void __launch_bounds__(256) label_exit_kernel(Imgs I, const int2* __restrict__ exits_f,
-                                                         const int2* __restrict__ exits_v,
-                                                         const int* __restrict__ n_exits,
-                                                         const int* __restrict__ perim_f,
-                                                         const int* __restrict__ perim_v, LabelOut OF, LabelOut OV,
-                                                         int cap, unsigned* status) {
-  const bool faces = blockIdx.y == 0;
-  const int2* __restrict__ exits = faces ? exits_f : exits_v;
-  const int* __restrict__ perim = faces ? perim_f : perim_v;
-  const LabelOut& O = faces ? OF : OV;
-  const int n = n_exits[blockIdx.y];
+__global__ void __launch_bounds__(256) label_exit_kernel(Imgs I, LabelSide F, LabelSide V, int first, int cap,
+                                                         unsigned* status) {
+  const bool faces = blockIdx.y + first == 0;
+  const int2* __restrict__ exits = faces ? F.exits : V.exits;
+  const int* __restrict__ perim = faces ? F.perim : V.perim;
+  const LabelOut& O = faces ? F.out : V.out;
+  const int n = faces ? *F.n_exits : *V.n_exits;
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
     const int2 e = exits[q];
     const int b = find_image(I.idx_base, I.B, e.x);
