@@ -1280,10 +1280,8 @@ void emit_write(dmsc_b200_context* ctx, int32_t* const (*out)[2], const int* con
     A.count[si] = ctx->emit[si].cnt + 3;
   }
   if (!any) return;
-  int per = 0;
   auto kernel = ctx->seg_cursors == 1 ? emit_segments_kernel<1> : emit_segments_kernel<2>;
-  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, 256, 0));
-  LK(kernel<<<dim3(per * ctx->num_sms * 4, 2), 256, 0, st>>>(A));
+  LK(kernel<<<dim3(kSegBlocks * ctx->num_sms, 2), 256, 0, st>>>(A));
   LAUNCH_CHECK("emit_segments_kernel");
 }
 

@@ -337,9 +337,10 @@ __device__ __forceinline__ int surv_start(const EmitCtx& E, int i, int b) {
 // A raw-arc segment task of the chain expansion: {reversed | arc << 1,
 // saddle cell, cells, output position}: the writer finds the arc's start
 // cell from the saddle's cell with no further load.
+template <bool FACES>
 __device__ __forceinline__ int arc_start_of_cell(const EmitCtx& E, int sc, int j, int b) {
   const int W = E.I.W[b], Nx = W + 1;
-  if (E.faces) return face_start(sc, j, Nx) >> 2;
+  if (FACES) return face_start(sc, j, Nx) >> 2;
   const int l = (sc >> 2) - E.I.idx_base[b], y = row_of(E.I, b, l);
   return vertex_start(sc, j, y, l - y * Nx, E.I.H[b], W, Nx) >> 2;
 }
@@ -362,6 +363,7 @@ struct SegCursor {
 // forward at its arc's output position; the others are the chain
 // expansion's tasks. rem = 0 when it writes nothing (no arc, or its image's
 // output does not take this side's arcs).
+template <bool FACES>
 __device__ __forceinline__ void seg_start(const EmitCtx& E, long long q, SegCursor& c) {
   c.rem = 0;
   int b, idx, len, pos;
@@ -373,7 +375,7 @@ __device__ __forceinline__ void seg_start(const EmitCtx& E, long long q, SegCurs
     if ((j ? a.y : a.x) < 0 || len <= 0) return;
     const int2 ic = *reinterpret_cast<const int2*>(E.head + i);
     b = ic.x;
-    idx = arc_start_of_cell(E, ic.y, j, b);
+    idx = arc_start_of_cell<FACES>(E, ic.y, j, b);
     pos = surv_start(E, i, b) + (j ? a.z + E.fin[i].x : 0);
     rev = false;
   } else {
@@ -381,7 +383,7 @@ __device__ __forceinline__ void seg_start(const EmitCtx& E, long long q, SegCurs
     const int j = (t.x >> 1) & 1;
     len = t.z;
     b = find_image(E.I.idx_base, E.I.B, t.y >> 2);
-    idx = arc_start_of_cell(E, t.y, j, b);
+    idx = arc_start_of_cell<FACES>(E, t.y, j, b);
     pos = t.w;
     rev = t.x & 1;
   }
