@@ -83,7 +83,8 @@ constexpr int kCycleEnd = (int)0x80000000;
 // tile reduces the value part of its key into its ends' `leave` too. Bound by
 // instruction issue: the rows of the four ends by multiplication instead of
 // division and 32-bit step counts took it from 38 to 32 registers (all 64
-// warps of an SM resident) and from 0.373 to 0.266 ms at 4096^2.
+// warps of an SM resident) and from 0.373 to 0.266 ms at 4096^2, a step's
+// distance from two selects (flow_step) to 0.206 (8192^2 noise: 0.694).
 __global__ void __launch_bounds__(256) saddle_walk_kernel(Imgs I, const uint8_t* __restrict__ flow, int nsad,
                                                           const int* __restrict__ crit_sad,
                                                           const int* __restrict__ sad_img,
