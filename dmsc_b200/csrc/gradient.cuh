@@ -636,79 +636,19 @@ __global__ void __launch_bounds__(NT) gradient_batch_kernel(Imgs I, const float*
 }
 
 // cell_value (cpu/cell_compare.hxx:82-87): value of the highest (dual: lowest)
-// vertex, chosen by (value, pixel id) in the reference's scan order (each
-// candidate replaces the current choice when value_greater); the chosen
-// pixel's own value is returned, so -0.0 survives.
-// Values of the four cells of index (y, x) for a whole warp of consecutive
-// columns: every lane loads its pixel and the one above it, takes its left
-// neighbours' from the lane to its left (lane 0 loads them), and evaluates
-// the candidates of cpu/cell_compare.hxx:82-87 in the reference's order
-// (vertex (y-1, x-1), (y-1, x), (y, x-1), (y, x) among those in the image).
-// Every lane of the warp must call it.
-struct CellValues {
-  float v, h, e, f;  // vertex, H edge (t = 1), V edge (t = 2), face (t = 3)
-};
-
-// The four pixel values an index's cells need: its own (y, x), the one above
-// and their left neighbours (0 outside the image).
-struct CellPixels {
-  float a, u, aL, uL;
-};
-
-// The loads of the cell values: every lane loads its pixel and the one above
-// it; lane 0 also loads its left neighbours (the other lanes take theirs from
-// the lane to their left in cell_values_of).
-__device__ __forceinline__ CellPixels warp_cell_loads(const float* __restrict__ img, int y, int x, int H, int W,
-                                                      int lane) {
-  const bool in_x = x < W, in_xl = x >= 1 && x - 1 < W, up = y >= 1, here = y < H;
-  CellPixels c;
-  c.a = (here && in_x) ? __ldg(img + (size_t)y * W + x) : 0.f;
-  c.u = (up && in_x) ? __ldg(img + (size_t)(y - 1) * W + x) : 0.f;
-  c.aL = (lane == 0 && here && in_xl) ? __ldg(img + (size_t)y * W + x - 1) : 0.f;
-  c.uL = (lane == 0 && up && in_xl) ? __ldg(img + (size_t)(y - 1) * W + x - 1) : 0.f;
-  return c;
-}
-
-// The candidates of a cell come in ascending pixel id, so each one is compared
-// as the later pixel (gt_after). INTERIOR: every lane's four pixels exist.
-template <bool DUAL, bool INTERIOR>
-__device__ __forceinline__ CellValues cell_values_of(CellPixels px, int y, int x, int H, int W, int lane) {
-  const float a = px.a, u = px.u;
-  float aL = __shfl_up_sync(0xffffffffu, a, 1), uL = __shfl_up_sync(0xffffffffu, u, 1);
-  if (lane == 0) {
-    aL = px.aL;
-    uL = px.uL;
+// vertex, chosen by (value, pixel id) in the reference's scan order, that is
+// among (y-1, x-1), (y-1, x), (y, x-1), (y, x) those in the image, in ascending
+// pixel id, so each candidate is compared as the later pixel (gt_after); the
+// chosen pixel's own value is returned, so -0.0 survives.
+struct CellValue {
+  bool dual, have = false;
+  float best = 0.f;
+  __device__ __forceinline__ CellValue(bool d) : dual(d) {}
+  __device__ __forceinline__ void add(bool valid, float v) {
+    if (valid && (!have || (dual ? gt_after<true>(v, best) : gt_after<false>(v, best)))) best = v;
+    have = have || valid;
   }
-  CellValues c;
-  c.v = a;
-  if (INTERIOR) {
-    const bool ga = gt_after<DUAL>(a, aL);
-    c.h = ga ? a : aL;
-    c.e = gt_after<DUAL>(a, u) ? a : u;
-    float f = gt_after<DUAL>(u, uL) ? u : uL;
-    f = gt_after<DUAL>(aL, f) ? aL : f;
-    c.f = gt_after<DUAL>(a, f) ? a : f;
-    return c;
-  }
-  const bool in_x = x < W, in_l = x >= 1, up = y >= 1, here = y < H;
-  auto pick = [](bool& have, float& best, bool valid, float v) {
-    if (valid && (!have || gt_after<DUAL>(v, best))) {
-      have = true;
-      best = v;
-    }
-  };
-  bool hh = false, he = false, hf = false;
-  c.h = c.e = c.f = 0.f;
-  pick(hh, c.h, here && in_l, aL);
-  pick(hh, c.h, here && in_x, a);
-  pick(he, c.e, up && in_x, u);
-  pick(he, c.e, here && in_x, a);
-  pick(hf, c.f, up && in_l, uL);
-  pick(hf, c.f, up && in_x, u);
-  pick(hf, c.f, here && in_l, aL);
-  pick(hf, c.f, here && in_x, a);
-  return c;
-}
+};
 
 // Criticality bits of an index (bit t: slot t is an unpaired valid cell) from
 // its flow byte; `vin`: the index's vertex is a pixel.
@@ -716,20 +656,27 @@ __host__ __device__ __forceinline__ unsigned crit_bits(unsigned fl, bool vin) {
   return (unsigned)((fl & 7u) == 0u && vin) | ((fl >> 2) & 2u) | ((fl >> 5) & 4u) | (unsigned)(((fl >> 4) & 7u) == 0u) << 3;
 }
 
-// K2: ordered compaction. One warp per (row, 32-column) segment of an image,
-// kCompactSegs consecutive segments per warp with every load of all of them
-// (flow bytes, pixel values, list offsets) issued before any is used, so a
-// warp waits on one round of loads instead of three per segment; segment
-// offsets are exclusive scans of the per-segment counts over the whole batch
-// (images in order, rows in order), so each image's lists are a contiguous
-// slice in ascending cell-id order. Writes the saddle list as global cell
-// ids with each saddle's image and value; each extremum's image and its
-// (value bits, global cell id) record (the extremum lists, read by the
+// K2: ordered compaction. A warp takes K consecutive (row, 32-column)
+// segments; segment offsets are exclusive scans of the per-segment counts over
+// the whole batch (images in order, rows in order), so each image's lists are
+// a contiguous slice in ascending cell-id order, and so are the entries of the
+// warp's segments: the warp first collects its critical cells of each kind in
+// order in shared memory (ballots of the criticality bits), then handles them
+// 32 at a time, one per lane, with coalesced writes. Writes the saddle list as
+// global cell ids with each saddle's image and value; each extremum's image
+// and its (value bits, global cell id) record (the extremum lists, read by the
 // elder comparisons of the pairing, the persistence pass and the outputs);
 // the per-segment bit masks of the minima and maxima (an extremum's list
 // rank is its segment's offset plus the extrema before it in the mask); and
 // the pairing's starting state of the groups (PairStart).
-constexpr int kCompactSegs = 2;
+//
+// Bound by instruction issue: one cell in six is critical, and a pass over
+// each segment's cells by kind kept three lanes of a warp busy for all of an
+// entry's writes and evaluated the values of all cells.
+// Compaction stage before -> now: 239 -> 119 us (4096^2), 870 -> 417 (8192^2
+// noise), 50 -> 34 (1080 x 1920), within 1 us at 256^2 and below. K = 1, 2 and
+// 4: 270, 188 and 135 us at 4096^2, and no faster on small images.
+constexpr int kCompactSegs = 8;
 
 // First entry of each image in the lists of minima, saddles and maxima (B + 1
 // entries each), and the lists' lengths.
@@ -738,15 +685,23 @@ struct ListBases {
   int total[3];
 };
 
+struct __align__(16) CompactSeg {
+  int g0, pix0, b, W;  // first index, its pixel (px_base + y W + x), image, width
+  int lim, flags;      // indices to the right of the first one; bit 0: y >= 1, 1: y < H, 2: x >= 1, 3: dual
+  int pad[2];
+};
+
 static __global__ void __launch_bounds__(256) compact_kernel(
-    Imgs I, const float* __restrict__ img_all, long long nseg, const uint8_t* __restrict__ flow,
+    Imgs I, const float* __restrict__ img, long long nseg, const uint8_t* __restrict__ flow,
     const int* __restrict__ off_min, const int* __restrict__ off_sad, const int* __restrict__ off_max,
     int* __restrict__ crit_sad, int* __restrict__ min_img, int* __restrict__ sad_img, int* __restrict__ max_img,
     uint32_t* __restrict__ min_bits, uint32_t* __restrict__ max_bits, int2* __restrict__ min_key,
     int2* __restrict__ max_key, float* __restrict__ sad_val, ListBases lb, PairStart ps) {
-  constexpr int K = kCompactSegs;
-  const int lane = threadIdx.x & 31;
-  {  // an image has a segment, so there are at least B + 1 threads
+  constexpr int K = kCompactSegs, kVEdge = 32 * K;
+  __shared__ CompactSeg segs[8][K];
+  __shared__ uint16_t lists[8][4 * 32 * K];  // segment << 5 | column (| kVEdge) of the minima, maxima, saddles
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  {  // an image has two segments at least, so there are at least B + 1 threads
     const long long b = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (b <= I.B) {
       const long long q = b < I.B ? I.seg_base[b] : nseg;
@@ -755,7 +710,7 @@ static __global__ void __launch_bounds__(256) compact_kernel(
         lb.base[k][b] = q < nseg ? (k == 0 ? off_min : k == 1 ? off_sad : off_max)[q] : lb.total[k];
     }
   }
-  const long long seg0 = ((long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * K;
+  const long long seg0 = ((long long)blockIdx.x * (blockDim.x >> 5) + warp) * K;
   if (seg0 >= nseg) return;
   if (seg0 == 0 && lane == 0) {  // the pairing's void groups and round counters
 #pragma unroll
@@ -767,85 +722,101 @@ static __global__ void __launch_bounds__(256) compact_kernel(
       ps.n_cancel[sd] = 0;
     }
   }
-  const unsigned lt = (1u << lane) - 1u;
-  int b[K], iy[K], ix[K], o_min[K], o_sad[K], o_max[K];
-  unsigned fl[K];
-  CellPixels px[K];
-  // every load of the warp's segments first
-#pragma unroll
-  for (int k = 0; k < K; ++k) {
-    const long long seg = seg0 + k;
-    b[k] = 0;
-    iy[k] = ix[k] = 0;
-    fl[k] = 0;
-    o_min[k] = o_sad[k] = o_max[k] = 0;
-    px[k] = CellPixels{0.f, 0.f, 0.f, 0.f};
-    if (seg >= nseg) continue;  // warp-uniform
-    b[k] = find_image(I.seg_base, I.B, seg);
-    const int H = I.H[b[k]], W = I.W[b[k]], Nx = W + 1;
-    const int nsegx = (W + 1 + kTileX - 1) / kTileX;
-    const int lseg = (int)(seg - I.seg_base[b[k]]);  // an image has fewer than 2^31 / 4 indices
-    iy[k] = lseg / nsegx;
-    ix[k] = (lseg - iy[k] * nsegx) * kTileX + lane;
-    if (ix[k] <= W) fl[k] = flow[(long long)I.idx_base[b[k]] + (long long)iy[k] * Nx + ix[k]];
-    px[k] = warp_cell_loads(img_all + I.px_base[b[k]], iy[k], ix[k], H, W, lane);
-    o_min[k] = off_min[seg];
-    o_sad[k] = off_sad[seg];
-    o_max[k] = off_max[seg];
+  const int o_min = off_min[seg0], o_sad = off_sad[seg0], o_max = off_max[seg0];
+  int g0 = 0, lim = -1, vlim = 0;  // lane k: segment k
+  if (lane < K && seg0 + lane < nseg) {
+    const long long seg = seg0 + lane;
+    const int b = find_image(I.seg_base, I.B, seg);
+    const int H = I.H[b], W = I.W[b];
+    const int nsegx = (W + kTileX) / kTileX;
+    const int lseg = (int)(seg - I.seg_base[b]);  // an image has fewer than 2^31 / 4 indices
+    const int y = lseg / nsegx, x = (lseg - y * nsegx) * kTileX;
+    g0 = I.idx_base[b] + y * (W + 1) + x;
+    lim = W - x;
+    vlim = y < H ? lim : 0;
+    segs[warp][lane] = CompactSeg{g0,  I.px_base[b] + y * W + x, b, W,
+                                  lim, (int)(y >= 1) | (int)(y < H) << 1 | (int)(x >= 1) << 2 | (int)I.dual[b] << 3};
   }
+  unsigned fl[K];
 #pragma unroll
   for (int k = 0; k < K; ++k) {
-    const long long seg = seg0 + k;
-    if (seg >= nseg) break;  // warp-uniform
-    const int bk = b[k], H = I.H[bk], W = I.W[bk], Nx = W + 1;
-    const long long gidx = (long long)I.idx_base[bk] + (long long)iy[k] * Nx + ix[k];
-    const unsigned m = ix[k] <= W ? crit_bits(fl[k], iy[k] < H && ix[k] < W) : 0u;
-    const unsigned bmin = __ballot_sync(0xffffffffu, m & 1u);
-    const unsigned bmax = __ballot_sync(0xffffffffu, m & 8u);
-    const unsigned bh = __ballot_sync(0xffffffffu, m & 2u), bv = __ballot_sync(0xffffffffu, m & 4u);
-    if (lane == 0) {
-      min_bits[seg] = bmin;
-      max_bits[seg] = bmax;
-    }
-    if ((bmin | bmax | bh | bv) == 0u) continue;  // the whole warp together
-    const int xs = ix[k] - lane;  // warp-uniform
-    const bool inside = iy[k] >= 1 && iy[k] < H && xs >= 1 && xs + 31 < W;
-    const CellValues cv =
-        I.dual[bk] ? (inside ? cell_values_of<true, true>(px[k], iy[k], ix[k], H, W, lane)
-                             : cell_values_of<true, false>(px[k], iy[k], ix[k], H, W, lane))
-                   : (inside ? cell_values_of<false, true>(px[k], iy[k], ix[k], H, W, lane)
-                             : cell_values_of<false, false>(px[k], iy[k], ix[k], H, W, lane));
-    // saddles before this lane's: both edge kinds of the lanes below it
-    int p = o_sad[k] + __popc(bh & lt) + __popc(bv & lt);
-    if (m & 1u) {
-      const int q = o_min[k] + __popc(bmin & lt);
-      min_img[q] = bk;
-      min_key[q] = make_int2(__float_as_int(cv.v), (int)(4 * gidx));
-      ps.minedge[1][q] = ~0ull;  // a single-extremum group without outgoing saddles yet
-      ps.leave[1][q] = ~0u;
-      ps.link[1][q] = q;
-      ps.alive[1][q] = 1;
-      ps.par[1][q] = q;
-    }
-    if (m & 8u) {
-      const int q = o_max[k] + __popc(bmax & lt);
-      max_img[q] = bk;
-      max_key[q] = make_int2(__float_as_int(cv.f), (int)(4 * gidx + 3));
-      ps.minedge[0][q] = ~0ull;
-      ps.leave[0][q] = ~0u;
-      ps.link[0][q] = q;
-      ps.alive[0][q] = 1;
-      ps.par[0][q] = q;
-    }
+    const int g = __shfl_sync(0xffffffffu, g0, k);
+    fl[k] = lane <= __shfl_sync(0xffffffffu, lim, k) ? flow[g + lane] : 0x11u;  // 0x11: nothing critical
+  }
+  uint16_t *lmin = lists[warp], *lmax = lmin + 32 * K, *lsad = lmax + 32 * K;
+  const unsigned lt = (1u << lane) - 1u;
+  int nmin = 0, nmax = 0, nsad = 0;
+  unsigned mymin = 0, mymax = 0;
 #pragma unroll
-    for (int t = 1; t <= 2; ++t) {
-      if (!(m & (1u << t))) continue;
-      const float v = t == 1 ? cv.h : cv.e;
-      crit_sad[p] = (int)(4 * gidx + t);
-      sad_img[p] = bk;
-      sad_val[p] = v;
-      p++;
+  for (int k = 0; k < K; ++k) {
+    const unsigned m = crit_bits(fl[k], lane < __shfl_sync(0xffffffffu, vlim, k));
+    const unsigned bmin = __ballot_sync(0xffffffffu, m & 1u), bmax = __ballot_sync(0xffffffffu, m & 8u);
+    const unsigned bh = __ballot_sync(0xffffffffu, m & 2u), bv = __ballot_sync(0xffffffffu, m & 4u);
+    const int at = k << 5 | lane;
+    if (lane == k) {
+      mymin = bmin;
+      mymax = bmax;
     }
+    if (m & 1u) lmin[nmin + __popc(bmin & lt)] = (uint16_t)at;
+    if (m & 8u) lmax[nmax + __popc(bmax & lt)] = (uint16_t)at;
+    // saddles before this lane's: both edge kinds of the lanes below it
+    const int p = nsad + __popc(bh & lt) + __popc(bv & lt);
+    if (m & 2u) lsad[p] = (uint16_t)at;
+    if (m & 4u) lsad[p + ((m >> 1) & 1u)] = (uint16_t)(at | kVEdge);
+    nmin += __popc(bmin);
+    nmax += __popc(bmax);
+    nsad += __popc(bh) + __popc(bv);
+  }
+  if (lane < K && seg0 + lane < nseg) {
+    min_bits[seg0 + lane] = mymin;
+    max_bits[seg0 + lane] = mymax;
+  }
+  __syncwarp();
+  auto pixel = [&](bool valid, int at) { return valid ? __ldg(img + at) : 0.f; };
+  for (int i = lane; i < nmin; i += 32) {
+    const int at = lmin[i], c = at & 31, q = o_min + i;
+    const CompactSeg S = segs[warp][at >> 5];
+    min_img[q] = S.b;
+    min_key[q] = make_int2(__float_as_int(__ldg(img + S.pix0 + c)), 4 * (S.g0 + c));
+    ps.minedge[1][q] = ~0ull;  // a single-extremum group without outgoing saddles yet
+    ps.leave[1][q] = ~0u;
+    ps.link[1][q] = q;
+    ps.alive[1][q] = 1;
+    ps.par[1][q] = q;
+  }
+  for (int i = lane; i < nmax; i += 32) {
+    const int at = lmax[i], c = at & 31, q = o_max + i;
+    const CompactSeg S = segs[warp][at >> 5];
+    const int p = S.pix0 + c;
+    const bool up = S.flags & 1, here = S.flags & 2, in_x = c < S.lim, in_l = c > 0 || (S.flags & 4);
+    const float uL = pixel(up && in_l, p - S.W - 1), u = pixel(up && in_x, p - S.W);
+    const float aL = pixel(here && in_l, p - 1), a = pixel(here && in_x, p);
+    CellValue v(S.flags & 8);
+    v.add(up && in_l, uL);
+    v.add(up && in_x, u);
+    v.add(here && in_l, aL);
+    v.add(here && in_x, a);
+    max_img[q] = S.b;
+    max_key[q] = make_int2(__float_as_int(v.best), 4 * (S.g0 + c) + 3);
+    ps.minedge[0][q] = ~0ull;
+    ps.leave[0][q] = ~0u;
+    ps.link[0][q] = q;
+    ps.alive[0][q] = 1;
+    ps.par[0][q] = q;
+  }
+  for (int i = lane; i < nsad; i += 32) {
+    const int at = lsad[i], c = at & 31, q = o_sad + i;
+    const CompactSeg S = segs[warp][(at & (kVEdge - 1)) >> 5];
+    const int p = S.pix0 + c;
+    const bool ve = at & kVEdge, up = S.flags & 1, here = S.flags & 2, in_x = c < S.lim, in_l = c > 0 || (S.flags & 4);
+    const bool v0 = ve ? up && in_x : here && in_l, v1 = here && in_x;
+    const float f0 = pixel(v0, ve ? p - S.W : p - 1), f1 = pixel(v1, p);
+    CellValue v(S.flags & 8);
+    v.add(v0, f0);
+    v.add(v1, f1);
+    crit_sad[q] = 4 * (S.g0 + c) + (ve ? 2 : 1);
+    sad_img[q] = S.b;
+    sad_val[q] = v.best;
   }
 }
 
