@@ -1054,17 +1054,21 @@ int extract_batch_impl(dmsc_b200_context* ctx, int B, const float* img, const in
   {
     ReplayArgs2 RA{};
     bool any = false;
+    long long items = 0;
     for (int si = 0; si < 2; ++si) {
       Side& S = ctx->side[si];
       RA.s[si].status = ctx->status;
       if (S.arcs && nsad > 0) {
         RA.s[si] = replay_prepare(ctx, si, S, st);
         any = any || RA.s[si].n_cancel != nullptr;
+        items += S.C;
       }
     }
+    // one thread per cancellation at most: a grid barrier waits for every
+    // block (48 -> 39 us at 256^2, where 592 blocks shared 20 thousand)
     if (any)
       coop_launch(ctx, ctx->replay_shape ? replay_persistent_kernel<2, 3> : replay_persistent_kernel<1, 4>, RA, st,
-                  "replay_persistent_kernel", ctx->replay_per_sm);
+                  "replay_persistent_kernel", ctx->replay_per_sm, (int)std::min<long long>(1 + items / 256, 1 << 20));
     mark(ctx, 8, st);
   }
 
@@ -1259,9 +1263,11 @@ void emit_expand(dmsc_b200_context* ctx, cudaStream_t st) {
     most += cap;
   }
   // few tasks for small geometry: a grid barrier costs less on fewer blocks
+  // (geometry with a block per 512, 2048 and 8192 cells: 100, 91 and 101 us at
+  // 256^2, 164, 154 and 150 us at 2048^2, threshold 0.25)
   if (most > 0)
-    coop_launch(ctx, ctx->emit_shape ? emit_persistent_kernel<2, 3> : emit_persistent_kernel<1, 5>, P, st,
-                "emit_persistent_kernel", ctx->emit_per_sm, (int)std::min<long long>(2 + most / 512, 1 << 20));
+    coop_launch(ctx, ctx->emit_shape ? emit_persistent_kernel<2, 3> : emit_persistent_kernel<1, 4>, P, st,
+                "emit_persistent_kernel", ctx->emit_per_sm, (int)std::min<long long>(2 + most / 2048, 1 << 20));
 }
 
 // Geometry, second half (fetch): the writer of every raw-arc segment into the
@@ -1825,7 +1831,7 @@ int dmsc_b200_tuning_limits(dmsc_b200_context* ctx, int* out, int n) {
           &v[3], ctx->replay_shape ? replay_persistent_kernel<2, 3> : replay_persistent_kernel<1, 4>, 256, 0) !=
           cudaSuccess ||
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-          &v[4], ctx->emit_shape ? emit_persistent_kernel<2, 3> : emit_persistent_kernel<1, 5>, 256, 0) !=
+          &v[4], ctx->emit_shape ? emit_persistent_kernel<2, 3> : emit_persistent_kernel<1, 4>, 256, 0) !=
           cudaSuccess)
     return -1;
   for (int k = 0; k < 9 && k < n; ++k) out[k] = v[k];
