@@ -30,7 +30,7 @@ enum : unsigned {
   kStatusChainCap = 4u,     // a replay chain walk exceeded its bound
   kStatusQueueOverflow = 8u,
   kStatusBadIndex = 16u,
-  kStatusFindCap = 32u,     // a union-find root search or union retry loop exceeded its bound
+  kStatusFindCap = 32u,     // a search for a root exceeded its bound
   kStatusCopyWait = 64u,    // a bulk copy into shared memory did not complete within its time bound
 };
 

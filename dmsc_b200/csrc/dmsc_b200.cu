@@ -39,7 +39,7 @@ namespace {
 
 
 enum Slot {
-  S_MASK, S_FLOW, S_SEG0, S_SEG1, S_SEG2, S_OFF0, S_OFF1, S_OFF2, S_TAB, S_BASES, S_ZERO, S_SCAN,
+  S_FLOW, S_SEG0, S_SEG1, S_SEG2, S_OFF0, S_OFF1, S_OFF2, S_TAB, S_BASES, S_ZERO, S_SCAN,
   S_CSAD, S_IMIN, S_ISAD, S_IMAX, S_MINBITS, S_MAXBITS, S_KMIN, S_KMAX, S_SVAL, S_SKEY2, S_IOTA,
   S_ASC, S_ARC, S_ALIVE, S_RANK, S_FLAG, S_FPOS, S_NCANC, S_ROUTE,
   S_BKEY, S_BIDX, S_BKEY2, S_BIDX2, S_PERF, S_PERV, S_EXF, S_EXV, S_SKEY32B, S_SKEYS,
@@ -48,7 +48,7 @@ enum Slot {
 };
 enum SideSlot {
   X_ROUT, X_DYING, X_GRP, X_LINK, X_MINE, X_ACT0, X_ACT1, X_CNT,
-  X_UF, X_CROOT, X_CKEY, X_CVAL, X_NODE,
+  X_ROOTS1, X_LEAVE, X_CKEY, X_CVAL, X_NODE,
   X_SARC, X_SOUT, X_SFIN, X_Q0, X_Q1, X_QB, X_G12,
   X_GBASE, X_WX, X_WA, X_PAR, X_SOLO, kSideSlots
 };
@@ -443,7 +443,6 @@ PairArgs pairing_args(dmsc_b200_context* ctx, int si, Side& S) {
   const int nsad = ctx->nsad, M = S.M;
   S.dying = sget<int>(ctx, si, X_DYING, nsad);  // list order
   PairArgs A;
-  A.nsad = nsad;
   A.M = M;
   A.sval = get<float>(ctx, S_SVAL, nsad);
   A.sad_img = ctx->sad_img;
@@ -454,7 +453,7 @@ PairArgs pairing_args(dmsc_b200_context* ctx, int si, Side& S) {
   A.act0 = sget<int>(ctx, si, X_ACT0, nsad);
   A.act1 = sget<int>(ctx, si, X_ACT1, nsad);
   A.roots0 = sget<int>(ctx, si, X_GRP, M + 1);
-  A.roots1 = sget<int>(ctx, si, X_UF, M + 1);
+  A.roots1 = sget<int>(ctx, si, X_ROOTS1, M + 1);
   A.cnt = sget<int>(ctx, si, X_CNT, 8);
   A.key = S.key;
   A.idx_base = ctx->I.idx_base;
@@ -465,7 +464,7 @@ PairArgs pairing_args(dmsc_b200_context* ctx, int si, Side& S) {
   A.max_rounds = capped(M + 2, ctx->cap_pair_rounds);
   A.rounds = ctx->zero->stats + 0 + si;
   A.handover = ctx->zero->stats + 6;
-  A.node = sget<int>(ctx, si, X_CROOT, M + 1);  // free until the thresholded union-find
+  A.node = sget<int>(ctx, si, X_LEAVE, M + 1);  // the tile pass was the last to read the `leave` keys
   A.solo_key = sget<unsigned long long>(ctx, si, X_SOLO, kPairSoloEdges + kPairSoloEdges / 2 + kPairSoloNodes);
   A.solo_ext = (int2*)(A.solo_key + kPairSoloEdges);
   A.solo_ends = (uint32_t*)(A.solo_ext + kPairSoloNodes);
@@ -509,7 +508,7 @@ void run_pairing(dmsc_b200_context* ctx, PairTileArgs T, int nltile, cudaStream_
   LAUNCH_CHECK("pair_solo_kernel");
 }
 
-// Persistence, cancellation, thresholded union-find, output ranks and image
+// Persistence, cancellation, thresholded roots, output ranks and image
 // bases of both sides; `survive` / `pos`: the surviving saddles and their
 // exclusive scan. The survivor and cancellation counts and the status word go
 // to the readback area.
@@ -957,7 +956,7 @@ int extract_batch_impl(dmsc_b200_context* ctx, int B, const float* img, const in
     const int M = si ? nmin : nmax;
     ps.M[si] = M;
     ps.minedge[si] = sget<unsigned long long>(ctx, si, X_MINE, M + 1);
-    ps.leave[si] = sget<unsigned>(ctx, si, X_CROOT, M + 1);  // free until the thresholded union-find
+    ps.leave[si] = sget<unsigned>(ctx, si, X_LEAVE, M + 1);
     ps.link[si] = sget<int>(ctx, si, X_LINK, M + 1);
     ps.par[si] = sget<int>(ctx, si, X_PAR, M + 1);
     ps.cnt[si] = sget<int>(ctx, si, X_CNT, 8);
@@ -1036,7 +1035,7 @@ int extract_batch_impl(dmsc_b200_context* ctx, int B, const float* img, const in
   mark(ctx, 6, st);
 
   // ---- surviving saddles in minima-sweep (vertex side) order ----
-  // the status word rides along: a capped pairing or union-find loop ends the
+  // the status word rides along: a capped pairing or root loop ends the
   // call here, before the replay
   wait_stream(ctx, st);
   raise_status(ctx, (unsigned)rb_ll(ctx)[3]);

@@ -51,8 +51,6 @@ __device__ __forceinline__ int find_halving(int* link, int x, int cap, unsigned*
   }
 }
 
-
-
 // Chunked processing with two output lists: each block takes contiguous
 // chunks of items (up to kChunkPer per thread, fewer when there are few
 // items, so small rounds still spread over the whole grid; no barrier between
@@ -107,7 +105,7 @@ __device__ __forceinline__ void chunk_flush(ChunkLists& L, int* cnt0, int* out0,
 // pairing rounds (see pairing.cuh for the algorithm)
 // ---------------------------------------------------------------------------
 struct PairArgs {
-  int nsad, M;  // void group = M
+  int M;  // void group = M
   // saddles are indexed in list order (ascending cell id); a saddle's sweep
   // key (sweep_key) orders the saddles of its image in this side's sweep
   // and is the atomicMin key, so no sorted copy of the saddles is needed

@@ -16,7 +16,7 @@ changes an output bit:
 * ``replay_shape``: replay cancellations each thread advances together (1 or
   2, with 4 or 3 resident blocks per SM);
 * ``emit_shape``: geometry-expansion chain tasks each thread advances
-  together (1 or 2, with 5 or 3 resident blocks per SM);
+  together (1 or 2, with 4 or 3 resident blocks per SM);
 * ``pair_blocks_per_sm``, ``replay_blocks_per_sm``, ``emit_blocks_per_sm``:
   resident blocks per SM of the three persistent round loops (0 = all that
   fit); fewer blocks make each grid barrier cheaper, more hide more latency;

@@ -258,7 +258,7 @@ int dmsc_b200_pairing_timeline(dmsc_b200_context* ctx, long long* out, int n);
 /* Failure handling (no counterpart in the reference). Every device loop of
    the pipeline has a bound that no input reaches: pairing rounds (extrema of
    a side + 2), replay rounds (saddles + 2), geometry expansion levels
-   (saddles + 4), union-find searches and retries (extrema + 2), V-path walks
+   (saddles + 4), group and root searches (extrema + 2), V-path walks
    (cells) and chain walks (saddles + 1). A loop that reaches its bound stops,
    leaves the device state consistent (undecided saddles become cycles,
    pending cancellations are dropped), sets a bit of a device status word,
@@ -287,11 +287,11 @@ int dmsc_b200_set_loop_caps(dmsc_b200_context* ctx, int pair_rounds, int replay_
    seg_cursors  : raw-arc walks each lane of the segment writer drives at
                   once, 1..2; default 1.
    pair_shape   : pairing items each thread advances together, {2, 4}
-                  (with {5, 4} resident blocks per SM), 0..1; default 0.
+                  (with 4 resident blocks per SM), 0..1; default 0.
    replay_shape : replay cancellations each thread advances together, {1, 2}
                   (with {4, 3} resident blocks per SM), 0..1; default 0.
    emit_shape   : geometry-expansion chain tasks each thread advances
-                  together, {1, 2} (with {5, 3} resident blocks per SM),
+                  together, {1, 2} (with {4, 3} resident blocks per SM),
                   0..1; default 0. */
 typedef struct {
   int grad_shape;
