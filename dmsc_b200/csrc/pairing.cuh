@@ -182,7 +182,7 @@ constexpr int kTileNodes = 896, kTileEdges = 1664;
 // 512 when one wave holds them all and a block's own latency counts (24% less
 // at 256^2, 8% more at 4096^2).
 constexpr int kTilePairNT[2] = {256, 512};
-constexpr int kTileRounds = 6;    // 4, 6, 8 rounds: stage of 5.68, 4.75, 4.93 ms at 8192^2 noise, 0.765, 0.753, 0.763 at 4096^2
+constexpr int kTileRounds = 5;    // 4, 5, 6, 8 rounds: stage of 5.68, 4.69, 4.67, 4.93 ms at 8192^2 noise, 0.765, 0.728, 0.738, 0.763 at 4096^2
 constexpr int kTilePairs = 512;   // slots of the table of group pairs
 constexpr int tile_list(int warps) { return (kTileEdges / 32 + warps - 1) / warps * 32; }  // a warp's edges
 constexpr unsigned kTileVoid = 0xFFFEu;
@@ -373,7 +373,7 @@ __global__ void __launch_bounds__(NT, 1536 / NT) pair_tile_kernel(Imgs I, PairTi
   }
   uint16_t* const list = S.list[warp];
   int n = 0;  // edges in the warp's list
-  constexpr int kBatch = 4;  // chunks whose loads are issued together
+  constexpr int kBatch = 2;  // chunks whose loads are issued together (a warp has three or so; 4 spill)
   for (int c0 = warp; c0 * 32 < ne; c0 += NW * kBatch) {
     int2 en[kBatch];
     float sv[kBatch];
