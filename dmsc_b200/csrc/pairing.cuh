@@ -171,12 +171,12 @@ __global__ void __launch_bounds__(256) saddle_walk_kernel(Imgs I, const uint8_t*
 // noise, 820 and 1460 of 4096 cells) hands everything on.
 //
 // Bound: instruction issue (short dependent shared-memory chains and block
-// barriers, 48 warps per SM). On the bump fields 12% of the saddles and 8% of
-// the groups are left to the global rounds, on i.i.d. noise 15% and 10% (with
-// tiles of 128: 5 to 8%, but one block per SM). Measured, the whole pairing
-// stage without and with this pass and the last block's rounds: 4096^2 bumps
-// 1.13 -> 0.76 ms (this pass 0.37), 8192^2 noise 7.80 -> 4.75, 509 x 1531
-// 0.287 -> 0.166.
+// barriers, 48 warps per SM). On the bump fields about 12% of the saddles and 8%
+// of the groups are left to the global rounds, on i.i.d. noise 15% and 10%
+// (with tiles of 128: 5 to 8%, but one block per SM). Measured, the whole
+// pairing stage without and with this pass and the last block's rounds: 4096^2
+// bumps 1.13 -> 0.725 ms (this pass 0.43), 8192^2 noise 7.80 -> 4.69, 509 x
+// 1531 0.287 -> 0.147.
 constexpr int kTileNodes = 896, kTileEdges = 1664;
 // Threads per block: 256 when the blocks fill the device several times over,
 // 512 when one wave holds them all and a block's own latency counts (24% less
