@@ -149,6 +149,10 @@ struct dmsc_b200_context {
   EmitArgs emit[2] = {};
   bool expanded[2] = {false, false};
   cudaEvent_t sync_ev = nullptr;   // polled by wait_event
+  // the work that calls left on the device when they returned; it reads the
+  // context's buffers, so the next call's stream waits for it (begin_work)
+  cudaEvent_t work_ev = nullptr;
+  bool drain = false;  // and the host too: its uploads read the host staging
   bool fetch_pending = false;      // a fetch_start whose fetch_finish is due
   // host destinations of the fixed-size outputs for the next extract (copied
   // on copy_st as soon as each is produced; see dmsc_b200_set_host_outputs)
@@ -326,17 +330,16 @@ void coop_launch(dmsc_b200_context* ctx, void (*kernel)(T), T args, cudaStream_t
   ++ctx->launches;
 }
 
-// Waits for the last recorded event (wait_stream: until the stream has
-// drained) by polling it: the host thread
-// spins instead of sleeping in the driver, so the next launches follow the
-// readback without an operating-system wake-up delay (the few host round
-// trips of a call are on its critical path). Gives up after the context's
+// Waits for an event (wait_stream: until the stream has drained) by polling
+// it: the host thread spins instead of sleeping in the driver, so the next
+// launches follow the readback without an operating-system wake-up delay (the
+// few host round trips of a call are on its critical path). Gives up after the context's
 // wait deadline with DMSC_B200_ERR_CUDA; the work may still be running then,
 // so the context must be destroyed, not reused.
-void wait_event(dmsc_b200_context* ctx) {
+void wait_event(dmsc_b200_context* ctx, cudaEvent_t ev) {
   const auto t0 = std::chrono::steady_clock::now();
   for (unsigned k = 0;; ++k) {
-    const cudaError_t e = cudaEventQuery(ctx->sync_ev);
+    const cudaError_t e = cudaEventQuery(ev);
     if (e == cudaSuccess) return;
     if (e != cudaErrorNotReady) CK(e);
     if ((k & 15u) == 15u &&
@@ -349,7 +352,33 @@ void wait_event(dmsc_b200_context* ctx) {
 
 void wait_stream(dmsc_b200_context* ctx, cudaStream_t st) {
   CK(cudaEventRecord(ctx->sync_ev, st));
-  wait_event(ctx);
+  wait_event(ctx, ctx->sync_ev);
+}
+
+bool capturing(cudaStream_t st) {
+  cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &c) == cudaSuccess) return c != cudaStreamCaptureStatusNone;
+  cudaGetLastError();  // the legacy stream while another one is captured: its own launches say so
+  return true;
+}
+
+// A context serves one thread, but that thread may change streams between
+// calls, and calls return with work still running that uses the context's
+// buffers: the expansion at the end of extract, and all of fetch_start,
+// fetch_pairs, fetch_pair_pixels and scatter_pair_grads. So every call makes
+// its stream wait for what the calls before it left (begin_work) and marks
+// what it leaves itself (leave_work). A captured call does neither: events do
+// not cross a capture, and its graph runs when the caller launches it.
+void begin_work(dmsc_b200_context* ctx, cudaStream_t st) {
+  if (capturing(st)) return;
+  if (ctx->drain) {
+    wait_event(ctx, ctx->work_ev);
+    ctx->drain = false;
+  }
+  CK(cudaStreamWaitEvent(st, ctx->work_ev, 0));
+}
+void leave_work(dmsc_b200_context* ctx, cudaStream_t st) {
+  if (!capturing(st)) CK(cudaEventRecord(ctx->work_ev, st));
 }
 
 // Device -> host copy of a finished output on the context's copy stream,
@@ -370,9 +399,15 @@ void join_copies(dmsc_b200_context* ctx, cudaStream_t st) {
   ctx->copies_pending = false;
 }
 
-// After a failure: wait for the copies already issued, so no host buffer is
-// written after the call returns, and forget the registered destinations.
-void abandon_copies(dmsc_b200_context* ctx) {
+// After a failure: mark what the call left running on `st` and the side
+// stream, wait for the copies already issued, so no host buffer is written
+// after the call returns, and forget the registered destinations.
+void abandon_work(dmsc_b200_context* ctx, cudaStream_t st) {
+  if (!capturing(st)) {
+    cudaEventRecord(ctx->join_ev, ctx->side_st);
+    cudaStreamWaitEvent(st, ctx->join_ev, 0);
+    ctx->drain = cudaEventRecord(ctx->work_ev, st) == cudaSuccess;
+  }
   if (ctx->copy_st) cudaStreamSynchronize(ctx->copy_st);
   if (ctx->in_st) cudaStreamSynchronize(ctx->in_st);  // uploads from a host image source
   ctx->copies_pending = false;
@@ -784,7 +819,6 @@ int extract_batch_impl(dmsc_b200_context* ctx, int B, const float* img, const in
                        const float* hthr, const unsigned char* hdual, unsigned flags, int32_t* grad_out,
                        int32_t* peaks_out, int32_t* basins_out, dmsc_b200_sizes* sizes_out, cudaStream_t st) {
   ctx->valid = false;
-  ctx->fetch_pending = false;
   const float* host_img = ctx->host_img;  // the registration covers this call only
   ctx->host_img = nullptr;
   if (host_img && B != 1) {
@@ -865,6 +899,9 @@ int extract_batch_impl(dmsc_b200_context* ctx, int B, const float* img, const in
   basins_off[B] = (int)nbs;
   ltile_base[B] = (int)nltile;
   CK(cudaSetDevice(ctx->device));
+  if (ctx->fetch_pending) ctx->drain = true;  // its fetch_finish never came
+  ctx->fetch_pending = false;
+  begin_work(ctx, st);
   ctx->B = B;
   ctx->flags = flags;
   ctx->nidx = nidx;
@@ -1217,6 +1254,7 @@ int extract_batch_impl(dmsc_b200_context* ctx, int B, const float* img, const in
   mark(ctx, 17, st);
   emit_expand(ctx, st);
   mark(ctx, 18, st);
+  leave_work(ctx, st);
   ctx->valid = true;
   return kOk;
 }
@@ -1297,6 +1335,8 @@ int fetch_start_impl(dmsc_b200_context* ctx, const dmsc_b200_outputs* o, cudaStr
     return kErrInvalidArgument;
   }
   CK(cudaSetDevice(ctx->device));
+  if (ctx->fetch_pending) ctx->drain = true;
+  begin_work(ctx, st);
   mark(ctx, 12, st);
   const int B = ctx->B, nsurv = ctx->nsurv;
   const Imgs I = ctx->I;
@@ -1409,6 +1449,7 @@ int fetch_start_impl(dmsc_b200_context* ctx, const dmsc_b200_outputs* o, cudaStr
   rb_reserve(ctx, 64);
   rb_copy(ctx, st, 0, ctx->status, sizeof(unsigned));
   CK(cudaEventRecord(ctx->sync_ev, st));
+  leave_work(ctx, st);
   ctx->fetch_pending = true;
   return kOk;
 }
@@ -1420,7 +1461,7 @@ int fetch_finish_impl(dmsc_b200_context* ctx, cudaStream_t st) {
   }
   ctx->fetch_pending = false;
   CK(cudaSetDevice(ctx->device));
-  wait_event(ctx);
+  wait_event(ctx, ctx->sync_ev);
   raise_status(ctx, *(const unsigned*)ctx->rb_h);
   join_copies(ctx, st);  // the caller's stream passes here only once the host copies are done
   return kOk;
@@ -1436,6 +1477,7 @@ int fetch_pair_pixels_impl(dmsc_b200_context* ctx, int32_t* plus_max, int32_t* m
   CK(cudaSetDevice(ctx->device));
   const int nsurv = ctx->nsurv;
   if (nsurv == 0) return kOk;
+  begin_work(ctx, st);
   for (int si = 0; si < 2; ++si) {
     Side& S = ctx->side[si];
     // faces: the max side in the primal, the min side in the dual
@@ -1445,6 +1487,7 @@ int fetch_pair_pixels_impl(dmsc_b200_context* ctx, int32_t* plus_max, int32_t* m
                                                               ctx->head, S.pp, S.key, PLUS, MINUS));
   }
   LAUNCH_CHECK("pair_pixels_kernel");
+  leave_work(ctx, st);
   return kOk;
 }
 
@@ -1461,6 +1504,7 @@ int fetch_pairs_impl(dmsc_b200_context* ctx, PairEntries E, cudaStream_t st) {
   }
   CK(cudaSetDevice(ctx->device));
   if (nsurv == 0) return kOk;
+  begin_work(ctx, st);
   PairSide P[2];
   for (int si = 0; si < 2; ++si) {
     const Side& S = ctx->side[si];
@@ -1469,6 +1513,7 @@ int fetch_pairs_impl(dmsc_b200_context* ctx, PairEntries E, cudaStream_t st) {
   LK(pair_entries_out_kernel<<<grid_for(2LL * nsurv, TB), TB, 0, st>>>(nsurv, ctx->I, ctx->bases.surv, ctx->img,
                                                                        ctx->head, P[0], P[1], E));
   LAUNCH_CHECK("pair_entries_out_kernel");
+  leave_work(ctx, st);
   return kOk;
 }
 
@@ -1486,6 +1531,7 @@ int scatter_pair_grads_impl(dmsc_b200_context* ctx, const int32_t* plus, const i
   CK(cudaSetDevice(ctx->device));
   if (npx > 0) CK(cudaMemsetAsync(grad_img, 0, npx * sizeof(float), st));
   if (n == 0 || npx == 0) return kOk;
+  begin_work(ctx, st);
   const int m = (int)(2 * n);
   int* key = get<int>(ctx, S_BKEY, m);
   int* idx = get<int>(ctx, S_BIDX, m);
@@ -1496,6 +1542,7 @@ int scatter_pair_grads_impl(dmsc_b200_context* ctx, const int32_t* plus, const i
   sort_pairs(ctx, key, key2, idx, idx2, m, st, bits_for((int)npx + 1));
   LK(pair_segments_kernel<<<grid_for(m, TB), TB, 0, st>>>(m, key2, idx2, grad, (int)npx, grad_img));
   LAUNCH_CHECK("pair_segments_kernel");
+  leave_work(ctx, st);
   return kOk;
 }
 
@@ -1516,6 +1563,7 @@ int dmsc_b200_create(dmsc_b200_context** out, int device) {
   }
   c->pinned_cap = 64 * sizeof(long long);
   if (cudaEventCreateWithFlags(&c->sync_ev, cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&c->work_ev, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&c->copy_ev, cudaEventDisableTiming) != cudaSuccess ||
       cudaStreamCreateWithFlags(&c->copy_st, cudaStreamNonBlocking) != cudaSuccess ||
       cudaStreamCreateWithFlags(&c->side_st, cudaStreamNonBlocking) != cudaSuccess ||
@@ -1565,6 +1613,7 @@ void dmsc_b200_destroy(dmsc_b200_context* c) {
   if (c->pinned) cudaFreeHost(c->pinned);
   if (c->rb_h) cudaFreeHost(c->rb_h);
   if (c->sync_ev) cudaEventDestroy(c->sync_ev);
+  if (c->work_ev) cudaEventDestroy(c->work_ev);
   if (c->copy_st) {
     cudaStreamSynchronize(c->copy_st);
     cudaStreamDestroy(c->copy_st);
@@ -1592,7 +1641,7 @@ int dmsc_b200_extract(dmsc_b200_context* ctx, const float* image, int H, int W, 
                               (cudaStream_t)stream);
   } catch (const Fail& f) {
     ctx->valid = false;
-    abandon_copies(ctx);
+    abandon_work(ctx, (cudaStream_t)stream);
     return f.code;
   }
 }
@@ -1604,7 +1653,7 @@ int dmsc_b200_fetch(dmsc_b200_context* ctx, const dmsc_b200_outputs* out, void* 
     const int rc = fetch_start_impl(ctx, out, (cudaStream_t)stream);
     return rc == kOk ? fetch_finish_impl(ctx, (cudaStream_t)stream) : rc;
   } catch (const Fail& f) {
-    abandon_copies(ctx);
+    abandon_work(ctx, (cudaStream_t)stream);
     return f.code;
   }
 }
@@ -1615,7 +1664,7 @@ int dmsc_b200_fetch_start(dmsc_b200_context* ctx, const dmsc_b200_outputs* out, 
   try {
     return fetch_start_impl(ctx, out, (cudaStream_t)stream);
   } catch (const Fail& f) {
-    abandon_copies(ctx);
+    abandon_work(ctx, (cudaStream_t)stream);
     return f.code;
   }
 }
@@ -1626,7 +1675,7 @@ int dmsc_b200_fetch_finish(dmsc_b200_context* ctx, void* stream) {
   try {
     return fetch_finish_impl(ctx, (cudaStream_t)stream);
   } catch (const Fail& f) {
-    abandon_copies(ctx);
+    abandon_work(ctx, (cudaStream_t)stream);
     return f.code;
   }
 }
@@ -1668,7 +1717,7 @@ int dmsc_b200_extract_batch(dmsc_b200_context* ctx, const float* images, int B, 
                               sizes, (cudaStream_t)stream);
   } catch (const Fail& f) {
     ctx->valid = false;
-    abandon_copies(ctx);
+    abandon_work(ctx, (cudaStream_t)stream);
     return f.code;
   }
 }
@@ -1680,6 +1729,7 @@ int dmsc_b200_fetch_pair_pixels(dmsc_b200_context* ctx, int32_t* plus_max, int32
   try {
     return fetch_pair_pixels_impl(ctx, plus_max, minus_max, plus_min, minus_min, (cudaStream_t)stream);
   } catch (const Fail& f) {
+    abandon_work(ctx, (cudaStream_t)stream);
     return f.code;
   }
 }
@@ -1694,6 +1744,7 @@ int dmsc_b200_fetch_pairs(dmsc_b200_context* ctx, float* persistence, int64_t* i
                         plus_pixel,  minus_pixel,       plus_flat,          minus_flat};
     return fetch_pairs_impl(ctx, E, (cudaStream_t)stream);
   } catch (const Fail& f) {
+    abandon_work(ctx, (cudaStream_t)stream);
     return f.code;
   }
 }
@@ -1705,6 +1756,7 @@ int dmsc_b200_scatter_pair_grads(dmsc_b200_context* ctx, const int32_t* plus, co
   try {
     return scatter_pair_grads_impl(ctx, plus, minus, grad, n, grad_img, npx, (cudaStream_t)stream);
   } catch (const Fail& f) {
+    abandon_work(ctx, (cudaStream_t)stream);
     return f.code;
   }
 }

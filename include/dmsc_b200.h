@@ -17,7 +17,10 @@
  *   2. dmsc_b200_fetch() writes the variable-size outputs into caller buffers
  *      sized from phase 1.
  * A context keeps the device workspace between the two phases and across
- * calls; a context is not thread-safe, use one per host thread.
+ * calls; a context is not thread-safe, use one per host thread. Its calls may
+ * come on different streams: each waits on the device for what the ones before
+ * it left running on the context's buffers (calls under stream capture do
+ * not). The caller's own buffers are the caller's to order.
  */
 #ifndef DMSC_B200_H
 #define DMSC_B200_H
