@@ -66,6 +66,7 @@ def _run(x3, thresholds, duals):
     ctx.check(ctx.lib.dmsc_b200_fetch_pairs(
         ctx.h, *(_ptr(t) for t in (p, image, side, ppairs, plus, minus, plus_g, minus_g)),
         ctypes.c_void_p(s.cuda_stream)), "dmsc_b200_fetch_pairs")
+    x3.record_stream(s)  # the pixels are still being looked up in it; its memory may be another stream's
     return p, image, side, ppairs, plus, minus, plus_g, minus_g
 
 
