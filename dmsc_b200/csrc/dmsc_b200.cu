@@ -1320,7 +1320,7 @@ void emit_write(dmsc_b200_context* ctx, int32_t* const (*out)[2], const int* con
     A.E[si].out_primal = out[si][0];
     A.E[si].out_dual = out[si][1];
     A.E[si].dst_off = dst_off[si];
-    A.count[si] = ctx->emit[si].cnt + 3;
+    A.count[si] = ctx->emit[si].cnt + kEmitSegs;
   }
   if (!any) return;
   auto kernel = ctx->seg_cursors == 1 ? emit_segments_kernel<1> : emit_segments_kernel<2>;

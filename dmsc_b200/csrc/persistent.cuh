@@ -863,7 +863,7 @@ struct EmitArgs {
   int nsurv;
   int4* q0;
   int4* q1;
-  int* cnt;  // [0..2] rotating level counts, [3] raw-arc segment count
+  int* cnt;  // [8] level counts at emit_slot, raw-arc segment count at kEmitSegs
   int max_levels;
   int* levels;                   // receives the number of levels (statistics)
   unsigned long long* timeline;  // [kTimeline] level start times (ns), optional
@@ -872,6 +872,14 @@ struct EmitArgs {
 struct EmitArgs2 {
   EmitArgs s[2];
 };
+
+// Where level `lv` counts its tasks: three rotating slots for the levels of the
+// whole grid and three others for the last levels, which one block per side
+// goes through alone (solo) while the blocks that leave may still be reading
+// the last count of the grid's. That one is not written again: a block that
+// found it changed could stay and wait for the others for good.
+constexpr int kEmitSegs = 3;
+__host__ __device__ constexpr int emit_slot(int lv, bool solo) { return lv % 3 + (solo ? kEmitSegs + 1 : 0); }
 
 // One batch of a thread's chain tasks at one expansion level, in[i0 + nt u]
 // (u < U) below n: the U chains are counted in lockstep (one node-record load
@@ -1025,9 +1033,9 @@ template <int U, int MINB>
 __global__ void __launch_bounds__(256, MINB) emit_persistent_kernel(EmitArgs2 P) {
   cg::grid_group grid = cg::this_grid();
   const long long tid = grid.thread_rank();
-  if (tid < 8) {
-    const EmitArgs& A = tid < 4 ? P.s[0] : P.s[1];
-    if (A.cnt) A.cnt[tid & 3] = 0;
+  if (tid < 16) {
+    const EmitArgs& A = tid < 8 ? P.s[0] : P.s[1];
+    if (A.cnt) A.cnt[tid & 7] = 0;
   }
   grid.sync();
   // level 0: the chain of each surviving arc (its own raw arc is a segment
@@ -1057,7 +1065,7 @@ __global__ void __launch_bounds__(256, MINB) emit_persistent_kernel(EmitArgs2 P)
       // queue slots only when one of its threads has a task
       if (!__syncthreads_or(mine > 0)) continue;
       int p, pb;
-      block_reserve2(A.cnt, mine, A.cnt + 3, 0, p, pb);
+      block_reserve2(A.cnt + emit_slot(0, false), mine, A.cnt + kEmitSegs, 0, p, pb);
       if (mine == 0) continue;
       for (int k = 0; k < kLevel0; ++k) {
         const long long i = base + (long long)k * blockDim.x + threadIdx.x;
@@ -1086,7 +1094,7 @@ __global__ void __launch_bounds__(256, MINB) emit_persistent_kernel(EmitArgs2 P)
     for (int sd = 0; sd < 2; ++sd) {
       const EmitArgs& A = sd ? P.s[1] : P.s[0];
       // in the solo levels the other side's counters are its own block's
-      n[sd] = A.cnt && !(solo && (int)blockIdx.x != sd) ? *(volatile int*)(A.cnt + lv % 3) : 0;
+      n[sd] = A.cnt && !(solo && (int)blockIdx.x != sd) ? *(volatile int*)(A.cnt + emit_slot(lv, solo)) : 0;
       if (!A.cnt || (solo ? threadIdx.x != 0 || (int)blockIdx.x != sd : tid != 0) || done[sd]) continue;
       if (A.timeline && lv < kTimeline - 2) {
         A.timeline[lv] = global_ns();
@@ -1132,14 +1140,14 @@ __global__ void __launch_bounds__(256, MINB) emit_persistent_kernel(EmitArgs2 P)
 #pragma unroll
       for (int k = 0; k < 2; ++k) {
         const EmitArgs& C = k ? P.s[1] : P.s[0];
-        if (C.cnt && (!solo || k == sd)) C.cnt[(lv + 2) % 3] = 0;
+        if (C.cnt && (!solo || k == sd)) C.cnt[emit_slot(lv + 2, solo)] = 0;
       }
     }
     const int ns = sd ? n[1] : n[0];
     const long long nt = (long long)blocks * 256;
     const long long t0 = ((long long)(threadIdx.x >> 5) * blocks + at) * 32 + (threadIdx.x & 31);
     for (long long base = 0; base < ns; base += nt * U)
-      emit_batch<U>(A.E, q_out, A.cnt + (lv + 1) % 3, A.cnt + 3, in, base + t0, nt, ns);
+      emit_batch<U>(A.E, q_out, A.cnt + emit_slot(lv + 1, solo), A.cnt + kEmitSegs, in, base + t0, nt, ns);
     if (solo)
       __syncthreads();
     else
