@@ -38,6 +38,7 @@ EXPORTS = (
     "dmsc_b200_loop_counts",
     "dmsc_b200_pairing_timeline",
     "dmsc_b200_set_loop_caps",
+    "dmsc_b200_set_scan_looks",
     "dmsc_b200_set_tuning",
     "dmsc_b200_get_tuning",
     "dmsc_b200_tuning_limits",
@@ -135,6 +136,8 @@ def load():
         lib.dmsc_b200_pairing_timeline.restype = ctypes.c_int
         lib.dmsc_b200_set_loop_caps.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.c_int]
         lib.dmsc_b200_set_loop_caps.restype = ctypes.c_int
+        lib.dmsc_b200_set_scan_looks.argtypes = [ctypes.c_void_p, ctypes.c_int]
+        lib.dmsc_b200_set_scan_looks.restype = ctypes.c_int
         lib.dmsc_b200_set_tuning.argtypes = [ctypes.c_void_p, ctypes.POINTER(Tuning)]
         lib.dmsc_b200_set_tuning.restype = ctypes.c_int
         lib.dmsc_b200_get_tuning.argtypes = [ctypes.c_void_p, ctypes.POINTER(Tuning)]
@@ -193,6 +196,10 @@ class Context:
         """Lowers the device loop bounds of the following calls (0 = normal)."""
         self.check(self.lib.dmsc_b200_set_loop_caps(self.h, pair_rounds, replay_rounds, emit_levels),
                    "dmsc_b200_set_loop_caps")
+
+    def set_scan_looks(self, looks: int = 0):
+        """The scans' bound on looks at a predecessor (0 = normal, negative = none)."""
+        self.check(self.lib.dmsc_b200_set_scan_looks(self.h, looks), "dmsc_b200_set_scan_looks")
 
     def set_tuning(self, **kw):
         t = self.get_tuning()

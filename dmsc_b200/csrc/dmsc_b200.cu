@@ -194,6 +194,7 @@ struct dmsc_b200_context {
   int seg_cursors = 1;  // raw-arc cursors per lane of the segment writer
   bool pair_smem_set = false;   // and for the pairing's tile kernel
   int cap_pair_rounds = 0, cap_replay_rounds = 0, cap_emit_levels = 0;
+  int cap_scan_looks = 0;  // negative: none at all
 };
 
 
@@ -291,7 +292,8 @@ void scan(dmsc_b200_context* ctx, Op op, long long n, cudaStream_t st) {
   }
   ctx->scan_epoch = (ctx->scan_epoch + 1) & 0x3FFFFFFFu;
   if (ctx->scan_epoch == 0) ctx->scan_epoch = 1;
-  const ScanState S{(unsigned*)w, w + 1, ctx->scan_epoch, ctx->status};
+  const int looks = ctx->cap_scan_looks ? std::max(ctx->cap_scan_looks, 0) : kScanLooks;
+  const ScanState S{(unsigned*)w, w + 1, ctx->scan_epoch, looks, ctx->status};
   LK((scan_kernel<V, Op><<<(unsigned)tiles, kScanNT, 0, st>>>(op, n, S)));
   LAUNCH_CHECK("scan_kernel");
 }
@@ -964,8 +966,11 @@ int extract_batch_impl(dmsc_b200_context* ctx, int B, const float* img, const in
     SS.out[k] = off[k];
   }
   SS.rb = (long long*)ctx->rb_d;
+  reinterpret_cast<long long*>(ctx->rb_h)[3] = 0;
   scan<3>(ctx, SS, nseg, st);
   wait_stream(ctx, st);
+  // a tile of the scan gave up: neither the counts nor the offsets hold
+  if (rb_ll(ctx)[3]) raise_status(ctx, kStatusRoundCap);
   const int nmin = (int)rb_ll(ctx)[0], nsad = (int)rb_ll(ctx)[1], nmax = (int)rb_ll(ctx)[2];
   ctx->nmin = nmin;
   ctx->nsad = nsad;
@@ -1835,6 +1840,12 @@ int dmsc_b200_set_loop_caps(dmsc_b200_context* ctx, int pair_rounds, int replay_
   ctx->cap_pair_rounds = pair_rounds;
   ctx->cap_replay_rounds = replay_rounds;
   ctx->cap_emit_levels = emit_levels;
+  return kOk;
+}
+
+int dmsc_b200_set_scan_looks(dmsc_b200_context* ctx, int looks) {
+  if (!ctx) return kErrInvalidArgument;
+  ctx->cap_scan_looks = looks;
   return kOk;
 }
 

@@ -16,6 +16,11 @@
 // scan's own work is 4 to 50 us), so what counts most is the number of launches:
 // the library scan took two per array and a kernel to fetch the totals, ten
 // to twelve where one is left.
+//
+// A tile looks for its predecessors' sums a bounded number of times. One that
+// gives up sets the status word and calls op.gave_up(): its sums are wrong, so
+// nothing may be addressed by them before the host or a later kernel has seen
+// either.
 #pragma once
 
 #include "common.cuh"
@@ -28,13 +33,15 @@ struct ScanState {
   unsigned* ticket;
   unsigned long long* word;  // [V][tiles] (epoch << 2 | state) << 32 | count
   unsigned epoch;
+  int looks;  // bound on a lane's looks at words that are not published yet
   unsigned* status;
 };
+// Predecessors are running, so no tile comes near it (about half a second).
+constexpr int kScanLooks = 1 << 20;
 
 template <int V, class Op>
 __global__ void __launch_bounds__(kScanNT) scan_kernel(Op op, long long n, ScanState st) {
   constexpr int NW = kScanNT / 32;
-  constexpr int kMaxPolls = 1 << 20;  // predecessors are running: never reached
   static_assert(V <= NW, "a warp per count");
   __shared__ unsigned tile, wsum[V][NW], pre[V], tot[V];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, tiles = (int)gridDim.x;
@@ -100,14 +107,13 @@ __global__ void __launch_bounds__(kScanNT) scan_kernel(Op op, long long n, ScanS
     unsigned before = 0;
     if (t > 0) {
       if (lane == 0) word[t] = agg | sum;
-      int polls = 0;
+      int looks = 0;
       for (int p0 = t - 1; p0 >= 0; p0 -= 32) {
         const int p = p0 - lane;  // lane 0: the nearest predecessor
         unsigned long long q = whole;
         if (p >= 0) {
-          do {
-            q = word[p];
-          } while ((unsigned)(q >> 34) != st.epoch && ++polls < kMaxPolls);
+          q = 0;
+          while (looks < st.looks && (unsigned)((q = word[p]) >> 34) != st.epoch) ++looks;
         }
         const unsigned done = __ballot_sync(0xffffffffu, ((unsigned)(q >> 32) & 3u) == 2u);
         // the counts up to the nearest whole prefix
@@ -115,7 +121,10 @@ __global__ void __launch_bounds__(kScanNT) scan_kernel(Op op, long long n, ScanS
         before += __reduce_add_sync(0xffffffffu, lane <= last ? (unsigned)q : 0u);
         if (done) break;
       }
-      if (polls >= kMaxPolls) set_status(st.status, kStatusRoundCap);
+      if (looks >= st.looks) {
+        set_status(st.status, kStatusRoundCap);
+        op.gave_up();
+      }
     }
     if (lane == 0) {
       word[t] = whole | (before + sum);
@@ -146,7 +155,8 @@ __global__ void __launch_bounds__(kScanNT) scan_kernel(Op op, long long n, ScanS
 }
 
 // Row-segment counts of minima, saddles and maxima; the totals go to the
-// mapped readback area.
+// mapped readback area, and a fourth word there is set when a tile gave up:
+// the host sizes the lists and launches their writer from what it reads there.
 struct SegScan {
   const int* in[3];
   int* out[3];
@@ -178,6 +188,7 @@ struct SegScan {
 #pragma unroll
     for (int k = 0; k < 3; ++k) rb[k] = v[k];
   }
+  __device__ void gave_up() const { rb[3] = 1; }
 };
 
 // Alive flags of both sides' extrema and survivor flags of the saddles.
@@ -228,6 +239,7 @@ struct FlagScan {
     total[0] = (int)v[0];
     total[1] = (int)v[1];
   }
+  __device__ void gave_up() const {}  // the host reads the status word with the counts
 };
 
 // Pairs of packed counts (side 0 low, side 1 high), in place.
@@ -267,6 +279,7 @@ struct PackedScan {
                       (int)v[2 * h + 1][2 * k + 1]);
   }
   __device__ void finish(const unsigned*) const {}
+  __device__ void gave_up() const {}  // the host reads the status word with the sizes
 };
 
 }  // namespace dmsc

@@ -262,7 +262,8 @@ int dmsc_b200_pairing_timeline(dmsc_b200_context* ctx, long long* out, int n);
    the pipeline has a bound that no input reaches: pairing rounds (extrema of
    a side + 2), replay rounds (saddles + 2), geometry expansion levels
    (saddles + 4), group and root searches (extrema + 2), V-path walks
-   (cells) and chain walks (saddles + 1). A loop that reaches its bound stops,
+   (cells), chain walks (saddles + 1) and the scans' looks at a predecessor's
+   sum. A loop that reaches its bound stops,
    leaves the device state consistent (undecided saddles become cycles,
    pending cancellations are dropped), sets a bit of a device status word,
    and the call returns DMSC_B200_ERR_ITERATION_CAP at its next readback;
@@ -271,6 +272,11 @@ int dmsc_b200_pairing_timeline(dmsc_b200_context* ctx, long long* out, int n);
    values (0 = the normal bound) so that tests can make them run out; the
    context stays usable after such an error. */
 int dmsc_b200_set_loop_caps(dmsc_b200_context* ctx, int pair_rounds, int replay_rounds, int emit_levels);
+
+/* The same for the scans of the following calls: the times a tile of a scan
+   looks for its predecessors' sums before it gives up (0: the normal bound,
+   negative: it does not look at all). */
+int dmsc_b200_set_scan_looks(dmsc_b200_context* ctx, int looks);
 
 /* Launch shapes (no counterpart in the reference, whose CPU path fixes its
    blocking at compile time, cpu/gradient.hxx:15 DEFAULT_GRADIENT_BLOCK_SIZE
