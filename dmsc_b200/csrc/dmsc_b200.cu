@@ -959,18 +959,18 @@ int extract_batch_impl(dmsc_b200_context* ctx, int B, const float* img, const in
                                            ret_grad ? ctx->host_grad : nullptr);
   mark(ctx, 1, st);
   if (ret_grad && !grad_copied) copy_out_async(ctx, ctx->host_grad, grad, 16 * (size_t)nidx, st);
-  rb_reserve(ctx, 4 * sizeof(long long));
+  rb_reserve(ctx, 5 * sizeof(long long));
   SegScan SS;
   for (int k = 0; k < 3; ++k) {
     SS.in[k] = seg[k];
     SS.out[k] = off[k];
   }
   SS.rb = (long long*)ctx->rb_d;
-  reinterpret_cast<long long*>(ctx->rb_h)[3] = 0;
+  SS.status = ctx->status;
+  reinterpret_cast<long long*>(ctx->rb_h)[4] = 0;
   scan<3>(ctx, SS, nseg, st);
   wait_stream(ctx, st);
-  // a tile of the scan gave up: neither the counts nor the offsets hold
-  if (rb_ll(ctx)[3]) raise_status(ctx, kStatusRoundCap);
+  raise_status(ctx, (unsigned)(rb_ll(ctx)[3] | rb_ll(ctx)[4]));  // before the counts are used
   const int nmin = (int)rb_ll(ctx)[0], nsad = (int)rb_ll(ctx)[1], nmax = (int)rb_ll(ctx)[2];
   ctx->nmin = nmin;
   ctx->nsad = nsad;

@@ -155,12 +155,16 @@ __global__ void __launch_bounds__(kScanNT) scan_kernel(Op op, long long n, ScanS
 }
 
 // Row-segment counts of minima, saddles and maxima; the totals go to the
-// mapped readback area, and a fourth word there is set when a tile gave up:
-// the host sizes the lists and launches their writer from what it reads there.
+// mapped readback area, since the host sizes the lists and launches their
+// writer from them. So that it can see first whether they hold, two more words
+// there take the status word (a gradient tile that gave up has written no
+// counts) and whether a tile of this scan gave up (it may end after the last
+// one).
 struct SegScan {
   const int* in[3];
   int* out[3];
-  long long* rb;
+  long long* rb;  // [5]
+  const unsigned* status;
   __device__ void load(long long i, unsigned* v) const {
 #pragma unroll
     for (int k = 0; k < 3; ++k) v[k] = (unsigned)in[k][i];
@@ -187,8 +191,9 @@ struct SegScan {
   __device__ void finish(const unsigned* v) const {
 #pragma unroll
     for (int k = 0; k < 3; ++k) rb[k] = v[k];
+    rb[3] = *status;
   }
-  __device__ void gave_up() const { rb[3] = 1; }
+  __device__ void gave_up() const { rb[4] = kStatusRoundCap; }
 };
 
 // Alive flags of both sides' extrema and survivor flags of the saddles.
