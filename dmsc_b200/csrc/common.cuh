@@ -127,7 +127,7 @@ struct Imgs {
 // With c = ceil(log2(W + 1)), shift = 29 + c and magic = ceil(2^shift / (W + 1))
 // < 2^30, the product is exact for l < 2^29 (an image's indices: 4 l is an int),
 // since magic (W + 1) exceeds 2^shift by less than 2^c.
-__device__ __forceinline__ int row_of(const Imgs& I, int b, int l) {
+__host__ __device__ __forceinline__ int row_of(const Imgs& I, int b, int l) {
   return (int)(((unsigned long long)(unsigned)l * I.magic[b]) >> I.shift[b]);
 }
 inline void row_magic(int Nx, unsigned* magic, int* shift) {
