@@ -659,7 +659,11 @@ __global__ void __launch_bounds__(256) persistence_kernel(PersistArgs A) {
 //   * d and t are in one component: everything that merged into d's pairing
 //     group before died younger than d and earlier in the sweep, so with no
 //     larger persistence (float subtraction is monotone) and was cancelled too;
-//     so d's end of the saddle hangs together with d.
+//     so d's end of the saddle hangs together with d. The one exception is
+//     threshold infinity on a field with infinite values: equal infinities
+//     leave NaN, which is never cancelled, where a later, infinite persistence
+//     is. The reference's roots depend on the order of its unions there (they
+//     may be killed extrema); these are survivors or the void, as everywhere.
 //   * There is no cycle: links put both ends into one pairing group for good,
 //     and the last link of a cycle would join two ends that the earlier ones had
 //     joined already.
