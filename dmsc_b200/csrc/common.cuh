@@ -29,14 +29,11 @@ enum : unsigned {
   kStatusRoundCap = 2u,     // a round loop exceeded its bound
   kStatusChainCap = 4u,     // a replay chain walk exceeded its bound
   kStatusQueueOverflow = 8u,
-  kStatusBadIndex = 16u,
   kStatusFindCap = 32u,     // a search for a root exceeded its bound
   kStatusCopyWait = 64u,    // a bulk copy into shared memory did not complete within its time bound
 };
 
-__host__ __device__ __forceinline__ int cell_id(int t, int y, int x, int Nx) { return t + 4 * (y * Nx + x); }
 __host__ __device__ __forceinline__ int cell_type(int id) { return id & 3; }
-__host__ __device__ __forceinline__ int cell_index(int id) { return id >> 2; }
 
 // std::tie(v1, id1) < std::tie(v2, id2) with IEEE '<' (cpu/cell_compare.hxx:10-12):
 // -0 == +0 and NaN compare as ties, broken by id.
@@ -78,15 +75,6 @@ enum : unsigned { kFlowNone = 0, kFlowLeft = 1, kFlowRight = 2, kFlowUp = 3, kFl
 __device__ __forceinline__ int flow_step(unsigned code, int Nx) {
   const int v = code >= kFlowUp ? Nx : 1;  // odd codes step back
   return (code & 1u) ? -v : v;
-}
-
-// Face code of the face at index `idx` paired with edge cell `e`: the other
-// coface of the edge (cpu/arcs_topology.hxx:19-39).
-__device__ __forceinline__ unsigned face_flow(int e, int idx) {
-  if (e < 0) return kFlowNone;
-  int eidx = e >> 2;
-  if ((e & 3) == 1) return eidx == idx ? kFlowDown : kFlowUp;  // H(fy,fx) -> F(fy+1,fx); H(fy-1,fx) -> F(fy-1,fx)
-  return eidx == idx ? kFlowRight : kFlowLeft;                 // V(fy,fx) -> F(fy,fx+1); V(fy,fx-1) -> F(fy,fx-1)
 }
 
 // a - b with the NaN results of the x86 SSE subtraction the reference CPU
@@ -141,9 +129,10 @@ inline void row_magic(int Nx, unsigned* magic, int* shift) {
 // produce its inputs instead of a pass of its own: the ordered compaction
 // sets every group's union-find link (itself) and smallest outgoing keys
 // (none), its alive flag and its place in the forest of the thresholded roots
-// (itself) as it lists the extrema, plus the void's links and the counters; the saddle walks record each saddle's ends as they find them and
-// reduce the saddles' keys into the minima (see pairing.cuh). Side 0
-// is the face side (maxima), side 1 the vertex side (minima).
+// (itself) as it lists the extrema, plus the void's links and the counters;
+// the saddle walks record each saddle's ends as they find them and reduce the
+// saddles' keys into the minima (see pairing.cuh). Side 0 is the face side
+// (maxima), side 1 the vertex side (minima).
 struct PairStart {
   int M[2];                        // extrema of each side; the void is group M
   unsigned long long* minedge[2];  // [M] smallest sweep key of each group's outgoing saddles
@@ -245,32 +234,6 @@ __device__ __forceinline__ int block_reserve(int* c0, int n0) {
   }
   __syncthreads();
   return bbase1 + wsum1[warp] + x0 - n0;
-}
-
-// Block-aggregated append: one global atomic per block. Every thread of the
-// block must call it (with blockDim.x a multiple of 32, at most 1024).
-// Returns the slot of this thread's item, or -1 when `take` is false.
-__device__ __forceinline__ int block_append(int* counter, bool take) {
-  __shared__ int wbase[32], bbase;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const unsigned b = __ballot_sync(0xffffffffu, take);
-  if (lane == 0) wbase[warp] = __popc(b);
-  __syncthreads();
-  if (warp == 0) {
-    const int s = lane < nw ? wbase[lane] : 0;
-    int incl = s;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int y = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += y;
-    }
-    if (lane < nw) wbase[lane] = incl - s;
-    if (lane == 31) bbase = incl ? atomicAdd(counter, incl) : 0;  // block total
-  }
-  __syncthreads();
-  const int r = take ? bbase + wbase[warp] + __popc(b & ((1u << lane) - 1u)) : -1;
-  __syncthreads();
-  return r;
 }
 
 inline unsigned grid_for(long long n, int block) {

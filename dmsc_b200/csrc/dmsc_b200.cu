@@ -163,8 +163,8 @@ struct dmsc_b200_context {
   bool host_fetch_set = false;
   bool copies_pending = false;
   cudaStream_t copy_st = nullptr;
-  // the second side's persistence, cancellation and rank kernels run on
-  // side_st, forked from and joined back to the call's stream
+  // the survivors' records and their sort run on side_st, forked from and
+  // joined back to the call's stream
   cudaStream_t side_st = nullptr;
   cudaEvent_t fork_ev = nullptr, join_ev = nullptr;
   cudaEvent_t copy_ev = nullptr;
@@ -192,7 +192,7 @@ struct dmsc_b200_context {
   int replay_shape = 0;  // replay items per thread batch: 0 -> 1, 1 -> 2
   int emit_shape = 0;    // expansion chain tasks per thread batch: 0 -> 1, 1 -> 2
   int seg_cursors = 1;  // raw-arc cursors per lane of the segment writer
-  bool pair_smem_set = false;   // and for the pairing's tile kernel
+  bool pair_smem_set = false;  // the pairing kernels' shared memory limits are raised
   int cap_pair_rounds = 0, cap_replay_rounds = 0, cap_emit_levels = 0;
   int cap_scan_looks = 0;  // negative: none at all
 };
@@ -1077,8 +1077,9 @@ int extract_batch_impl(dmsc_b200_context* ctx, int B, const float* img, const in
   mark(ctx, 6, st);
 
   // ---- surviving saddles in minima-sweep (vertex side) order ----
-  // the status word rides along: a capped pairing or root loop ends the
-  // call here, before the replay
+  // the status word rides along: a capped pairing loop ends the call here,
+  // before the replay (a capped root search sets its bit after the word is
+  // taken and ends the call with the sizes; its ranks are in range all the same)
   wait_stream(ctx, st);
   raise_status(ctx, (unsigned)rb_ll(ctx)[3]);
   ctx->nsurv = (int)rb_ll(ctx)[0];

@@ -53,18 +53,6 @@ __device__ __forceinline__ int dying_word(int x, bool second) { return second ? 
 __device__ __forceinline__ int dying_of(int w) { return w < 0 ? -1 : w & 0x3FFFFFFF; }
 __device__ __forceinline__ bool dying_second(int w) { return (w >> 30) & 1; }
 
-// older(a, b) for extremum dense indices of one image; `void_id` is older
-// than all. Older = smaller (value, cell) under value_less on the vertex side
-// in the primal and the face side in the dual, larger otherwise.
-// `key[x]` = (value bits, cell) of extremum x, one 8-byte record per extremum.
-__device__ __forceinline__ bool older(int a, int b, int void_id, const int2* __restrict__ key, bool older_less) {
-  if (a == void_id) return b != void_id;
-  if (b == void_id) return false;
-  const int2 ka = key[a], kb = key[b];
-  const float va = __int_as_float(ka.x), vb = __int_as_float(kb.x);
-  return older_less ? tie_lt(va, ka.y, vb, kb.y) : tie_lt(vb, kb.y, va, ka.y);
-}
-
 // Ends of a saddle as the walks record them for the tile pass below. A local
 // saddle has its two ends inside its own 64 x 64 index tile or in the void:
 // each end is ~(r * 64 + c) of the extremum's cell in the tile (negative), or
@@ -408,8 +396,8 @@ __global__ void __launch_bounds__(NT, 1536 / NT) pair_tile_kernel(Imgs I, PairTi
   __syncthreads();
   // A root's decision on its first outgoing edge k (value key h1): it dies
   // there when the group behind it is older and no saddle out of the tile
-  // comes first. (The other end's root may read `ends` after it was marked:
-  // the dead node is then its own partner, and younger.)
+  // comes first. (The other end's root, if this edge is its first too, is the
+  // older one: it stays alive, with or without seeing the mark.)
   auto decide = [&](int i, uint32_t h1, int k) -> bool {
     const uint32_t e = S.ends[k];
     if (e >= kTileDead) return false;

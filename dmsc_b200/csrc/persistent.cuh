@@ -72,15 +72,11 @@ __device__ __forceinline__ long long chunk_size(long long n, int blocks) {
   return 256LL * max(1LL, min((long long)kChunkPer, (n + lanes - 1) / lanes));
 }
 
-// Round loops whose active set has shrunk below a threshold leave the grid,
-// whose barriers cost several microseconds each. The replay and the geometry
-// expansion finish in block 0 alone (the other blocks leave: all decide
-// alike, from the same counters read after the grid barrier that ended the
-// previous round), with block barriers between the phases; a replay item
-// walks whole parent chains, so the replay does so only at one item per
-// thread. The pairing hands over to a kernel that holds what is left of a
-// side in one block's shared memory (pair_solo_kernel).
-constexpr long long kReplaySoloItems = 256;
+// Loops whose active set has shrunk below a threshold leave the grid, whose
+// barriers cost several microseconds each: the geometry expansion goes on in
+// one block per side (the other blocks leave: all decide alike, from counts
+// that are not written any more), the pairing hands over to a kernel that
+// holds what is left of a side in one block's shared memory (pair_solo_kernel).
 constexpr int kPairSoloEdges = 8192, kPairSoloNodes = 4096;  // per side
 constexpr unsigned kSoloVoid = 0x7FFFu;                      // the void's node
 
@@ -337,7 +333,7 @@ __device__ __forceinline__ void pair_batch_b(const PairArgs2& P, int r, long lon
   for (int u = 0; u < U; ++u) {
     if (!((act >> u) & 1u)) continue;
     const bool s1 = (s1m >> u) & 1u;
-    // older(h, g): the void is older than any extremum; else (value, cell)
+    // h older than g: the void is older than any extremum; else (value, cell)
     // under the side's order
     bool dies = h[u] == PSIDE(M);
     if (!dies) {
